@@ -22,7 +22,7 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
               "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall"]
 # the complex64 FP32 fused passes sit in translation units of their own (gsb_group_*.cu): the largest objects, compiled
 # in parallel with the rest
-LIB_SOURCES = ["gsb_engine.cu", "gsb_group_ws.cu", "gsb_group_wst.cu", "gsb_group_f32.cu", "gsb_group3.cu",
+LIB_SOURCES = ["gsb_engine.cu", "gsb_group_ws.cu", "gsb_group_ws3.cu", "gsb_group_wst.cu", "gsb_group_f32.cu", "gsb_group3.cu",
                "gsb_dp.cu", "gsb_grad.cu", "gsb_batch.cu", "gsb_probe.cu", "gsb_plan.cpp", "gsb_order.cpp", "gsb_fuse.cpp"]
 LIB_DEPS = LIB_SOURCES + ["gsb_kernels.cuh", "gsb_group.cuh", "gsb_step.h", "gsb_plan.h", "gsb_common.h", "gsb_fuse.h",
                           "gsb_pick.h"]
@@ -54,12 +54,15 @@ def build(force=False, verbose_ptxas=False):
         objdir = os.path.join(ROOT, "_build", "gsb")
         os.makedirs(objdir, exist_ok=True)
         cmds, objs = [], []
+        headers = [d for d in deps if not d.endswith((".cu", ".cpp"))]
         for f in LIB_SOURCES:
             obj = os.path.join(objdir, f + ".o")
             objs.append(obj)
+            if not force and not verbose_ptxas and not _stale(obj, headers + [os.path.join(CSRC, f)]):
+                continue
             cmds.append([_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose_ptxas else []) +
                         ["-c", "-I" + INCLUDE, "-I" + CSRC, "-o", obj, os.path.join(CSRC, f)])
-        with concurrent.futures.ThreadPoolExecutor(max_workers=min(len(cmds), os.cpu_count() or 1)) as ex:
+        with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(len(cmds), os.cpu_count() or 1))) as ex:
             list(ex.map(_run, cmds))
         _run([_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", LIB] + objs)
     cli_src = os.path.join(CSRC, "gsb_cli.cpp")

@@ -18,6 +18,7 @@
 #include <random>
 #include <string>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "gsb.h"
@@ -47,6 +48,7 @@ int fail(int code, const std::string &msg) {
 
 struct Launch {
     int grid = 1, block = 1, U = 1, tl = 0, cl = 0;
+    int cap = 1;                // blocks the device holds at once
     unsigned int nchunks = 1;
     void *fn = nullptr;
 };
@@ -117,6 +119,14 @@ static void *pick_group(int d, int tr) {
 // A fused pass's kernel parameters (GroupArgs, the arena pointer, Ctx) stay within the 4 KB of a classic launch.
 static_assert(sizeof(GroupArgs) + sizeof(void *) + sizeof(Ctx) <= 4096, "fused-pass parameters exceed 4 KB");
 
+// Items per launch (slots, gsb_kernels.cuh): at most MAX_SLOTS, with arenas of at most SLOT_BYTES together.  The bound
+// is well above the 126 MB L2: the narrow steps at both ends of an item cost time, not bandwidth, and more items
+// share it.  50 strings of width 19, complex128 'chain', at 64 / 128 / 256 / 512 MB: 1.91 / 1.36 / 0.91 / 0.78 ms (one at a
+// time: 14 ms); 9 strings of width 24, complex64: 3.06 / 2.30 / 1.82 / 1.57 ms.  Blocks of a launch: SLOT_WAVES rounds of
+// what the device holds; 1 and 2 measured alike, 4 was 10 % slower at width 19.
+constexpr int MAX_SLOTS = 1024, SLOT_WAVES = 2;
+constexpr size_t SLOT_BYTES = (size_t)512 << 20;
+
 struct Op {
     int k0 = 0, d = 1, tr = 0, lcap = 0;   // lcap: the tile-size cap the pass was built with (fused passes)
     int minb = 2;                          // CTAs per SM the fused kernel is built for (2, or 3: pick_group3)
@@ -126,7 +136,7 @@ struct Op {
     bool norm_first = false;  // sampling: a norm pass of step k0 runs first (its bit has no other source)
     GroupArgs ga;
     void *fn = nullptr;
-    int grid = 1;
+    int grid = 1, cap = 1;    // blocks of one item; blocks the device holds at once
     size_t smem = 0;
     unsigned int ntiles = 0;
     double entries = 0;       // entries read + written by the pass (the norm pass not included)
@@ -184,7 +194,13 @@ struct Engine {
     StepArgs *d_args = nullptr;          // device copy of args (read by the small-step runs, k_small_run)
     bool args_dirty = true;              // args changed since d_args was last written
     std::vector<Launch> lw, ln;
-    std::map<int, cudaGraphExec_t> graphs;   // key: graph kind
+    std::map<int, cudaGraphExec_t> graphs;   // key: graph kind << 16 | slots
+    size_t arena = 0;                    // entries of an arena
+    int max_slots = 1;                   // items per launch at most (a power of two, MAX_SLOTS and SLOT_BYTES)
+    int slots = 1;                       // items carried by the launches being queued
+    int used_slots = 1;                  // slots of the launches queued since the device's error flags were read
+    void *slot_mem = nullptr;            // the arenas of launches that carry several items
+    size_t slot_bytes = 0;
     std::map<void *, int> occ;
     // complex128 re-evaluation of unlikely strings (gsb_set_guard): the engine that re-evaluates this one's strings
     // whose log2 Pr + ns < guard_lx, and the engine this one re-evaluates for
@@ -206,6 +222,7 @@ struct Engine {
         DevGuard g(dev);
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
         cudaFree(mem);
+        cudaFree(slot_mem);
         cudaFree(d_args);
         cudaFree(st);
         cudaFree(partials);
@@ -246,8 +263,8 @@ struct Engine {
             L.cl = (wide64 ? 9 : 8) + (uw == 4 ? 2 : 1);
             L.nchunks = (unsigned int)(N >> L.cl);
             L.fn = pick_wide(prec, a.ntq, a.m, write, arith == 32);
-            const int cap_blocks = occupancy(L.fn, L.block) * sms;
-            L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)cap_blocks);
+            L.cap = occupancy(L.fn, L.block) * sms;
+            L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)L.cap);
             return L;
         }
         // blocks of at least one full warp (the reductions shuffle over 32 lanes); below 32 cosets the threads
@@ -258,8 +275,8 @@ struct Engine {
         L.cl = L.tl + (L.U == 4 ? 2 : 0);
         L.nchunks = (unsigned int)(N >> L.cl);
         L.fn = step_fn(a.ntq, a.m, L.U, write);
-        const int cap_blocks = occupancy(L.fn, L.block) * sms;
-        L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)cap_blocks);
+        L.cap = occupancy(L.fn, L.block) * sms;
+        L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)L.cap);
         return L;
     }
 
@@ -277,16 +294,29 @@ struct Engine {
         c.tpb_log2 = L.tl;
         c.chunk_log2 = L.cl;
         c.nchunks = L.nchunks;
+        c.arena = arena;
         return c;
     }
+
+    // x extent of a launch that carries `slots` items: one item alone takes `grid` blocks, the device holds `cap`.
+    // With several items the blocks are shared out (SLOT_WAVES rounds of `cap` in all), a power of two per item so that
+    // the items' tiles, a power of two as well, split evenly.
+    unsigned slot_grid(int grid, int cap) const {
+        if (slots == 1) return (unsigned)grid;
+        unsigned g = 1;
+        while (2 * g * (unsigned)slots <= (unsigned)(SLOT_WAVES * cap)) g *= 2;
+        return std::min((unsigned)grid, g);
+    }
+    void *arena_mem() const { return slots == 1 ? mem : slot_mem; }
 
     cudaError_t launch_step(int k, bool write, int driver, int k1, bool use_forced, bool use_unif) {
         const Launch &L = write ? lw[(size_t)k] : ln[(size_t)k];
         StepArgs a = args[(size_t)k];
         Ctx c = ctx(driver, k1, L, use_forced, use_unif);
-        void *memp = mem;
+        void *memp = arena_mem();
         void *kargs[] = {&a, &memp, &c};
-        return cudaLaunchKernel(L.fn, dim3((unsigned)L.grid), dim3((unsigned)L.block), kargs, 0, stream);
+        return cudaLaunchKernel(L.fn, dim3(slot_grid(L.grid, L.cap), (unsigned)slots), dim3((unsigned)L.block), kargs, 0,
+                                stream);
     }
 
     // Whether step k runs in a small-step run (k_small_run) when it is a single-step pass.
@@ -298,10 +328,10 @@ struct Engine {
         Ctx c = ctx(driver, plan.ns, L, use_forced, use_unif);
         const StepArgs *sa = d_args;
         int a0 = k0, a1 = k1, nm = norm ? 1 : 0;
-        void *memp = mem;
+        void *memp = arena_mem();
         void *kargs[] = {&sa, &a0, &a1, &nm, &memp, &c};
         void *fn = prec == 128 ? (void *)k_small_run<double2> : (void *)k_small_run<float2>;
-        return cudaLaunchKernel(fn, dim3(1), dim3(SMALL_THREADS), kargs, 0, stream);
+        return cudaLaunchKernel(fn, dim3(1, (unsigned)slots), dim3(SMALL_THREADS), kargs, 0, stream);
     }
 
     // Length of the run of consecutive single small-step passes that starts at ops[i] (0 or 1: no run).
@@ -324,8 +354,14 @@ struct Engine {
     }
 
     cudaError_t launch_begin() {
-        if (prec == 128) k_begin<double2><<<1, 1, 0, stream>>>((double2 *)mem, st);
-        else k_begin<float2><<<1, 1, 0, stream>>>((float2 *)mem, st);
+        const int b = std::min(slots, 64);
+        if (prec == 128) k_begin<double2><<<slots / b, b, 0, stream>>>((double2 *)arena_mem(), st, arena);
+        else k_begin<float2><<<slots / b, b, 0, stream>>>((float2 *)arena_mem(), st, arena);
+        return cudaGetLastError();
+    }
+    cudaError_t launch_finish(int driver) {
+        const int b = std::min(slots, 64);
+        k_finish<<<slots / b, b, 0, stream>>>(st, d_logp, d_aux, driver, plan.ns);
         return cudaGetLastError();
     }
 
@@ -340,9 +376,10 @@ struct Engine {
         Ctx c = ctx(driver, plan.ns, L, use_forced, use_unif);
         GroupArgs ga = op.ga;
         ga.withhold_loads = withhold_loads;
-        void *memp = mem;
+        void *memp = arena_mem();
         void *kargs[] = {&ga, &memp, &c};
-        return cudaLaunchKernel(op.fn, dim3((unsigned)op.grid), dim3((unsigned)op.threads), kargs, op.smem, stream);
+        return cudaLaunchKernel(op.fn, dim3(slot_grid(op.grid, op.cap), (unsigned)slots), dim3((unsigned)op.threads), kargs,
+                                op.smem, stream);
     }
 
     cudaError_t enqueue_item(int driver, bool use_forced, bool use_unif) {
@@ -360,8 +397,7 @@ struct Engine {
                 e = launch_op(chain_ops[i++], driver);
                 if (e != cudaSuccess) return e;
             }
-            k_finish<<<1, 1, 0, stream>>>(st, d_logp, d_aux, driver, plan.ns);
-            return cudaGetLastError();
+            return launch_finish(driver);
         }
         if (driver == DRV_CHAIN && !sample_ops.empty()) {
             for (size_t i = 0; i < sample_ops.size();) {
@@ -381,8 +417,7 @@ struct Engine {
                              : launch_step(op.k0, true, driver, plan.ns, use_forced, use_unif);
                 if (e != cudaSuccess) return e;
             }
-            k_finish<<<1, 1, 0, stream>>>(st, d_logp, d_aux, driver, plan.ns);
-            return cudaGetLastError();
+            return launch_finish(driver);
         }
         int k0 = 0;
         if (driver == DRV_HYBRID && hyb_K > 0) {
@@ -397,7 +432,8 @@ struct Engine {
                 e = launch_op(hyb_ops[i++], DRV_CHAIN1);
                 if (e != cudaSuccess) return e;
             }
-            k_hybrid_switch<<<1, 1, 0, stream>>>(st, d_forced, d_bits, plan.ns, hyb_K);
+            const int b = std::min(slots, 64);
+            k_hybrid_switch<<<slots / b, b, 0, stream>>>(st, d_forced, d_bits, plan.ns, hyb_K);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
             k0 = hyb_K;
         }
@@ -417,13 +453,30 @@ struct Engine {
             e = launch_step(k, true, driver, plan.ns, use_forced, use_unif);
             if (e != cudaSuccess) return e;
         }
-        k_finish<<<1, 1, 0, stream>>>(st, d_logp, d_aux, driver, plan.ns);
-        return cudaGetLastError();
+        return launch_finish(driver);
     }
 
-    int graph(int kind, cudaGraphExec_t *out) {
-        auto it = graphs.find(kind);
+    // The graph of one launch of `nslots` items of mode `kind`.
+    int graph(int kind, int nslots, cudaGraphExec_t *out) {
+        const int key = kind << 16 | nslots;
+        auto it = graphs.find(key);
         if (it != graphs.end()) { *out = it->second; return 0; }
+        if (nslots > 1 && (size_t)nslots * arena * esize > slot_bytes) {   // the slots' arenas, allocated on first use
+            GSB_CK(cudaStreamSynchronize(stream));
+            for (auto kv = graphs.begin(); kv != graphs.end();)            // those that point at the old ones
+                if ((kv->first & 0xffff) > 1) { cudaGraphExecDestroy(kv->second); kv = graphs.erase(kv); }
+                else ++kv;
+            cudaFree(slot_mem);
+            slot_mem = nullptr;
+            slot_bytes = 0;
+            const size_t bytes = (size_t)nslots * arena * esize;
+            if (cudaMalloc(&slot_mem, bytes) != cudaSuccess) {
+                cudaGetLastError();
+                slot_mem = nullptr;
+                return fail(GSB_E_ALLOC, "allocation of the slots' arenas failed");
+            }
+            slot_bytes = bytes;
+        }
         int driver = kind == 0 ? DRV_CHAIN1 : kind == 3 ? DRV_HYBRID : DRV_CHAIN;
         bool use_forced = kind != 2, use_unif = kind >= 2;
         if (args_dirty) {   // the small-step runs read the step descriptors from the device
@@ -433,7 +486,9 @@ struct Engine {
         }
         cudaGraph_t g = nullptr;
         GSB_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+        slots = nslots;
         cudaError_t e = enqueue_item(driver, use_forced, use_unif);
+        slots = 1;
         cudaError_t e2 = cudaStreamEndCapture(stream, &g);
         if (e != cudaSuccess) { if (g) cudaGraphDestroy(g); GSB_CK(e); }
         GSB_CK(e2);
@@ -441,19 +496,25 @@ struct Engine {
         e = cudaGraphInstantiate(&ex, g, 0);
         cudaGraphDestroy(g);
         GSB_CK(e);
-        graphs[kind] = ex;
+        graphs[key] = ex;
         *out = ex;
         return 0;
     }
 
     // Run `n` items of graph `kind` with inputs already in d_forced / d_unif rows 0..n-1.
     int run_graph_items(int kind, int64_t n) {
+        if (n < 1) return 0;
         cudaGraphExec_t ex;
-        int rc = graph(kind, &ex);
+        int s = 1;
+        while (s < max_slots && s < n) s *= 2;
+        int rc = graph(kind, s, &ex);
+        if (rc == GSB_E_ALLOC) rc = graph(kind, s = 1, &ex);   // no room for more than the engine's own arena
         if (rc) return rc;
-        k_set_item<<<1, 1, 0, stream>>>(st, 0);
+        used_slots = std::max(used_slots, s);
+        const int b = std::min(s, 64);
+        k_set_item<<<s / b, b, 0, stream>>>(st, 0, (int)n);
         GSB_CK(cudaGetLastError());
-        for (int64_t i = 0; i < n; i++) GSB_CK(cudaGraphLaunch(ex, stream));
+        for (int64_t i = 0; i < n; i += s) GSB_CK(cudaGraphLaunch(ex, stream));
         return 0;
     }
 };
@@ -576,8 +637,9 @@ static int make_args(Engine &E) {
         E.ln[(size_t)k] = E.shape(E.args[(size_t)k], false);
         maxgrid = std::max(maxgrid, (size_t)std::max(E.lw[(size_t)k].grid, E.ln[(size_t)k].grid));
     }
-    maxgrid = std::max(maxgrid, (size_t)E.sms * 8);
-    GSB_CK(cudaMalloc(&E.partials, maxgrid * 8 * sizeof(double)));   // up to 6 sums per block (fused groups)
+    // a launch of several slots: one block each, or blocks of 256 threads (8 per SM) in at most SLOT_WAVES rounds
+    maxgrid = std::max(maxgrid, std::max((size_t)E.sms * 8 * SLOT_WAVES, (size_t)MAX_SLOTS));
+    GSB_CK(cudaMalloc(&E.partials, maxgrid * PARTIAL_SUMS * sizeof(double)));
     GSB_CK(cudaMalloc(&E.d_args, (size_t)std::max(1, p.ns) * sizeof(StepArgs)));
     E.args_dirty = true;
     return 0;
@@ -766,7 +828,8 @@ static bool fill_group(Engine &E, const GroupPlan &gp, Op &op, int lcap = GROUP_
         return false;
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, op.fn, op.threads, op.smem) != cudaSuccess || nb < 1) nb = 1;
-    op.grid = (int)std::min<uint64_t>(op.ntiles, (uint64_t)nb * E.sms);
+    op.cap = nb * E.sms;
+    op.grid = (int)std::min<uint64_t>(op.ntiles, (uint64_t)op.cap);
     op.entries = gp.entries_moved;
     return true;
 }
@@ -954,7 +1017,9 @@ static int open_plan(const char *text, size_t len, int precision, int device, gs
     cudaError_t e = cudaStreamCreateWithFlags(&E->own_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_fail(e, "stream");
     E->stream = E->own_stream;
-    const size_t arena = ((size_t)1 << E->plan.R) * E->esize;
+    E->arena = (size_t)1 << E->plan.R;
+    const size_t arena = E->arena * E->esize;
+    while (E->max_slots < MAX_SLOTS && 2 * (size_t)E->max_slots * arena <= SLOT_BYTES) E->max_slots *= 2;
     e = cudaMalloc(&E->mem, arena);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -966,8 +1031,9 @@ static int open_plan(const char *text, size_t len, int precision, int device, gs
     e = cudaMemsetAsync(E->mem, 0, arena, E->stream);
     if (e != cudaSuccess) return cuda_fail(e, "arena clear");
     const size_t ns = (size_t)std::max(1, E->plan.ns), cap = (size_t)E->cap;
-    if ((e = cudaMalloc(&E->st, sizeof(DevState))) != cudaSuccess) return cuda_fail(e, "state");
-    if ((e = cudaMemsetAsync(E->st, 0, sizeof(DevState), E->stream)) != cudaSuccess) return cuda_fail(e, "state");
+    const size_t st_bytes = sizeof(DevState) * (size_t)E->max_slots;
+    if ((e = cudaMalloc(&E->st, st_bytes)) != cudaSuccess) return cuda_fail(e, "state");
+    if ((e = cudaMemsetAsync(E->st, 0, st_bytes, E->stream)) != cudaSuccess) return cuda_fail(e, "state");
     if ((e = cudaMalloc(&E->d_forced, cap * ns)) != cudaSuccess) return cuda_fail(e, "buffers");
     if ((e = cudaMalloc(&E->d_bits, cap * ns)) != cudaSuccess) return cuda_fail(e, "buffers");
     if ((e = cudaMalloc(&E->d_unif, cap * ns * 8)) != cudaSuccess) return cuda_fail(e, "buffers");
@@ -1081,11 +1147,13 @@ static int check_bits(const int8_t *b, int64_t n, int ns, bool allow_free) {
 // A fused pass whose tile loads did not complete within its bounded wait sets DevState::err and stops the item;
 // report it (and clear it) after the work has been synchronised.
 static int check_device(Engine *E) {
-    int v = 0;
-    GSB_CK(cudaMemcpy(&v, &E->st->err, sizeof v, cudaMemcpyDeviceToHost));
-    if (!v) return 0;
-    v = 0;
-    GSB_CK(cudaMemcpy(&E->st->err, &v, sizeof v, cudaMemcpyHostToDevice));
+    std::vector<int> v((size_t)std::exchange(E->used_slots, 1));   // those of the calls since the last check
+    const size_t pitch = sizeof(DevState);
+    if (v.size() == 1) GSB_CK(cudaMemcpy(v.data(), &E->st->err, sizeof(int), cudaMemcpyDeviceToHost));   // quicker
+    else GSB_CK(cudaMemcpy2D(v.data(), sizeof(int), &E->st->err, pitch, sizeof(int), v.size(), cudaMemcpyDeviceToHost));
+    if (std::all_of(v.begin(), v.end(), [](int x) { return x == 0; })) return 0;
+    std::fill(v.begin(), v.end(), 0);
+    GSB_CK(cudaMemcpy2D(&E->st->err, pitch, v.data(), sizeof(int), sizeof(int), v.size(), cudaMemcpyHostToDevice));
     return fail(GSB_E_CUDA, "a fused pass gave up waiting for its tile loads; results of this call are invalid");
 }
 
@@ -1332,7 +1400,7 @@ int gsb_prefix(gsb_engine *e, const int8_t *forced, int K, void *dump, double *l
     std::vector<int8_t> row((size_t)std::max(ns, 1), 0);
     for (int k = 0; k < Kr; k++) row[(size_t)k] = forced[k];
     if (ns) GSB_CK(cudaMemcpyAsync(E->d_forced, row.data(), (size_t)ns, cudaMemcpyHostToDevice, E->stream));
-    k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0);
+    k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0, 1);
     GSB_CK(E->launch_begin());
     for (int k = 0; k < Kr; k++) GSB_CK(E->launch_step(k, true, DRV_HYBRID, Kr, true, false));
     if (dump) {   // dump == NULL: only the prefix probability (a marginal) is wanted
@@ -1429,7 +1497,7 @@ int gsb_resume(gsb_engine *e, const int8_t *forced, int K, uint64_t seed, int64_
         GSB_CK(cudaMemcpyAsync(E->d_forced, row.data(), (size_t)ns, cudaMemcpyHostToDevice, E->stream));
         GSB_CK(cudaMemcpyAsync(E->d_unif, u.data(), (size_t)ns * 8, cudaMemcpyHostToDevice, E->stream));
     }
-    k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0);
+    k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0, 1);
     const uint64_t Nc = 1ULL << nk;
     Launch L1;
     L1.block = (int)std::max<uint64_t>(32, std::min<uint64_t>(256, Nc));
@@ -1509,11 +1577,9 @@ int gsb_set_hybrid_prefix(gsb_engine *e, int K) {
     DevGuard g(E->dev);
     GSB_CK(cudaStreamSynchronize(E->stream));
     E->hyb_K = K;
-    auto it = E->graphs.find(3);
-    if (it != E->graphs.end()) {
-        cudaGraphExecDestroy(it->second);
-        E->graphs.erase(it);
-    }
+    for (auto it = E->graphs.begin(); it != E->graphs.end();)
+        if (it->first >> 16 == 3) { cudaGraphExecDestroy(it->second); it = E->graphs.erase(it); }
+        else ++it;
     build_hyb_ops(*E);
     return 0;
 }
@@ -1607,7 +1673,7 @@ struct Timer {
     double operator()(F launch) {
         double tot = 0;
         for (int r = -1; r < reps; r++) {   // r = -1: untimed warm-up
-            k_set_item<<<1, 1, 0, E.stream>>>(E.st, 0);
+            k_set_item<<<1, 1, 0, E.stream>>>(E.st, 0, 1);
             if (E.launch_begin() != cudaSuccess) return -1;
             if (cudaEventRecord(e0, E.stream) != cudaSuccess) return -1;
             if (launch() != cudaSuccess) return -1;
@@ -1770,15 +1836,15 @@ int gsb_autotune(gsb_engine *e, int mode, int reps, float *ms_before, float *ms_
     // device time of one item of graph `kind` (replayed: one warm-up, then the mean of `reps`)
     auto item_ms = [&](int kind, float *out) -> int {
         cudaGraphExec_t ex;
-        if (int rc = E->graph(kind, &ex)) return rc;
+        if (int rc = E->graph(kind, 1, &ex)) return rc;
         cudaEvent_t a, b;
         GSB_CK(cudaEventCreate(&a));
         GSB_CK(cudaEventCreate(&b));
-        k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0);
+        k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0, 1);
         GSB_CK(cudaGraphLaunch(ex, E->stream));
         float tot = 0;
         for (int r = 0; r < reps; r++) {
-            k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0);
+            k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0, 1);
             GSB_CK(cudaEventRecord(a, E->stream));
             GSB_CK(cudaGraphLaunch(ex, E->stream));
             GSB_CK(cudaEventRecord(b, E->stream));
@@ -1941,7 +2007,7 @@ int gsb_profile_steps(gsb_engine *e, const int8_t *bits, int mode, float *ms_wri
     std::vector<cudaEvent_t> ev((size_t)(2 * ns + 1));
     for (auto &x : ev) GSB_CK(cudaEventCreate(&x));
     if (ns) GSB_CK(cudaMemcpyAsync(E->d_forced, bits, (size_t)ns, cudaMemcpyHostToDevice, E->stream));
-    k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0);
+    k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0, 1);
     GSB_CK(E->launch_begin());
     GSB_CK(cudaEventRecord(ev[0], E->stream));
     if (driver == DRV_CHAIN1 && !E->chain_ops.empty()) {   // one timing per pass, reported at its first step
@@ -1950,7 +2016,7 @@ int gsb_profile_steps(gsb_engine *e, const int8_t *bits, int mode, float *ms_wri
             GSB_CK(E->launch_op(E->chain_ops[i], driver));
             GSB_CK(cudaEventRecord(ev[i + 1], E->stream));
         }
-        k_finish<<<1, 1, 0, E->stream>>>(E->st, E->d_logp, E->d_aux, driver, ns);
+        GSB_CK(E->launch_finish(driver));
         GSB_CK(cudaStreamSynchronize(E->stream));
         for (size_t i = 0; i < E->chain_ops.size(); i++) {
             float a = 0;
@@ -1977,7 +2043,7 @@ int gsb_profile_steps(gsb_engine *e, const int8_t *bits, int mode, float *ms_wri
             else GSB_CK(E->launch_step(op.k0, true, driver, ns, true, false));
             GSB_CK(cudaEventRecord(ev2[2 * i + 2], E->stream));
         }
-        k_finish<<<1, 1, 0, E->stream>>>(E->st, E->d_logp, E->d_aux, driver, ns);
+        GSB_CK(E->launch_finish(driver));
         GSB_CK(cudaStreamSynchronize(E->stream));
         for (size_t i = 0; i < E->sample_ops.size(); i++) {
             float a = 0, b = 0;
@@ -2000,7 +2066,7 @@ int gsb_profile_steps(gsb_engine *e, const int8_t *bits, int mode, float *ms_wri
         GSB_CK(E->launch_step(k, true, driver, ns, true, false));
         GSB_CK(cudaEventRecord(ev[(size_t)(2 * k + 2)], E->stream));
     }
-    k_finish<<<1, 1, 0, E->stream>>>(E->st, E->d_logp, E->d_aux, driver, ns);
+    GSB_CK(E->launch_finish(driver));
     GSB_CK(cudaStreamSynchronize(E->stream));
     for (int k = 0; k < ns; k++) {
         float a = 0, b = 0;

@@ -97,7 +97,7 @@ __device__ __forceinline__ bool grid_reduceN(double (&a)[ND], const Ctx &cx, dou
         for (int i = 0; i < ND; i++) {
             double s = 0;
             for (int w = 0; w < nw; w++) s += red[i][w];
-            cx.partials[ND * blockIdx.x + i] = s;
+            cx.partials[PARTIAL_SUMS * blockIdx.x + i] = s;
         }
         __threadfence();
         const unsigned int done = atomicAdd(&cx.st->counter, 1u);
@@ -116,7 +116,7 @@ __device__ __forceinline__ bool grid_reduceN(double (&a)[ND], const Ctx &cx, dou
     for (int i = 0; i < ND; i++) s[i] = 0;
     for (unsigned int b = threadIdx.x; threadIdx.x < GROUP_NCT && b < gridDim.x; b += GROUP_NCT)
 #pragma unroll
-        for (int i = 0; i < ND; i++) s[i] += __ldcg(cx.partials + ND * b + i);
+        for (int i = 0; i < ND; i++) s[i] += __ldcg(cx.partials + PARTIAL_SUMS * b + i);
 #pragma unroll
     for (int i = 0; i < ND; i++) s[i] = warp_sum(s[i]);
     __syncthreads();
@@ -1624,7 +1624,9 @@ __host__ __device__ inline GroupSmem group_smem(const int (&ssz)[4], int L, bool
 // landed / every step warp done reading), so the step warps do not wait for one another within or between tiles.
 template <typename E, typename T, int D, int TR, int MINB = 2, bool WS = false>
 __global__ void __launch_bounds__(WS ? GROUP_NCT + 32 : GROUP_NCT, MINB)
-    k_group(const GroupArgs ga, E *__restrict__ mem, const Ctx cx) {
+    k_group(const GroupArgs ga, E *__restrict__ mem, const Ctx c0) {
+    const Ctx cx = slot_ctx(c0);
+    mem += (size_t)blockIdx.y * cx.arena;
     DevState *st = cx.st;
     if (*(volatile int *)&st->dead) return;
     extern __shared__ __align__(16) unsigned char smem[];

@@ -49,11 +49,12 @@ struct DevState {
     unsigned int counter;   // blocks finished in the current launch
     int err;                // a bounded pipeline wait gave up (reported to the host, cleared when read)
     int trx;                // n0, n1 were expanded from a trailing step's shared sums (fused sampling passes)
+    int nitems;             // items of the current call: a slot whose item is past them idles (dead) until the next call
 };
 
 struct Ctx {
     DevState *st;
-    double *partials;        // [gridDim][2]
+    double *partials;        // [slots][gridDim.x][PARTIAL_SUMS]
     const int8_t *forced;    // [cap][ns] or null
     const double *unif;      // [cap][ns] or null
     int8_t *bits_out;        // [cap][ns]
@@ -64,7 +65,22 @@ struct Ctx {
     int tpb_log2;            // log2 blockDim
     int chunk_log2;          // log2 cosets per chunk (= tpb_log2 + log2 U)
     unsigned int nchunks;
+    size_t arena;            // entries of one slot's arena
 };
+
+// Slots: a launch of an item's step sequence carries gridDim.y strings or samples side by side, one slot each, with an
+// arena, a DevState and a row of block partials of its own; the x extent of the grid is one slot's blocks.  A narrow
+// table cannot fill the chip, and its steps are a chain of launches of 7-17 us each: at width 19 one complex64 string took
+// 192 us for 28 launches, however few of the 148 SMs they used.
+constexpr int PARTIAL_SUMS = 8;   // doubles of a block's row in Ctx::partials (at most 7 sums)
+
+// A kernel's context with the state and partials of this block's slot (its arena starts at blockIdx.y * arena).
+__device__ __forceinline__ Ctx slot_ctx(const Ctx &c) {
+    Ctx r = c;
+    r.st += blockIdx.y;
+    r.partials += (size_t)blockIdx.y * gridDim.x * PARTIAL_SUMS;
+    return r;
+}
 
 __device__ __forceinline__ void load_entry(const float2 *p, double &re, double &im) {
     const float2 v = *p;
@@ -104,8 +120,8 @@ __device__ __forceinline__ bool grid_reduce2(double a0, double a1, const Ctx &cx
     if (threadIdx.x == 0) {
         double s0 = 0, s1 = 0;
         for (int w = 0; w < nw; w++) { s0 += red[0][w]; s1 += red[1][w]; }
-        cx.partials[2 * blockIdx.x] = s0;
-        cx.partials[2 * blockIdx.x + 1] = s1;
+        cx.partials[PARTIAL_SUMS * blockIdx.x] = s0;
+        cx.partials[PARTIAL_SUMS * blockIdx.x + 1] = s1;
         __threadfence();
         const unsigned int done = atomicAdd(&cx.st->counter, 1u);
         last = (done == gridDim.x - 1);
@@ -116,8 +132,8 @@ __device__ __forceinline__ bool grid_reduce2(double a0, double a1, const Ctx &cx
     // the last block sums the partials in block order: thread t takes blocks t, t + blockDim, ... then a fixed tree
     double s0 = 0, s1 = 0;
     for (unsigned int b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-        s0 += __ldcg(cx.partials + 2 * b);
-        s1 += __ldcg(cx.partials + 2 * b + 1);
+        s0 += __ldcg(cx.partials + PARTIAL_SUMS * b);
+        s1 += __ldcg(cx.partials + PARTIAL_SUMS * b + 1);
     }
     s0 = warp_sum(s0);
     s1 = warp_sum(s1);
@@ -202,7 +218,9 @@ __device__ __forceinline__ void write_epilogue(const Ctx &cx, int k, int bv, dou
 }
 
 template <typename E, int NTQ, int MOUT, int U, bool WRITE>
-__global__ void __launch_bounds__(256) k_step(const StepArgs s, E *__restrict__ mem, const Ctx cx) {
+__global__ void __launch_bounds__(256) k_step(const StepArgs s, E *__restrict__ mem, const Ctx c0) {
+    const Ctx cx = slot_ctx(c0);
+    mem += (size_t)blockIdx.y * cx.arena;
     DevState *st = cx.st;
     if (*(volatile int *)&st->dead) return;
     const size_t row = (size_t)st->item * (size_t)cx.ns;
@@ -328,7 +346,9 @@ constexpr int SMALL_U = (1 << SMALL_NK) / SMALL_THREADS;
 
 template <typename E>
 __global__ void __launch_bounds__(SMALL_THREADS) k_small_run(const StepArgs *__restrict__ sa, int k0, int k1, int norm,
-                                                             E *__restrict__ mem, const Ctx cx) {
+                                                             E *__restrict__ mem, const Ctx c0) {
+    const Ctx cx = slot_ctx(c0);
+    mem += (size_t)blockIdx.y * cx.arena;
     __shared__ StepArgs s;
     __shared__ double red[2][SMALL_THREADS / 32];
     __shared__ int sh_skip, sh_bv;
@@ -511,7 +531,9 @@ __device__ __forceinline__ double fmaT(double a, double b, double c) { return fm
 //   float : sums and rotation in FP32 (a few roundings per entry; faster on the FP32 pipe).
 // Chunk = 256 threads x U pairs = 2^(9 + log2 U) cosets; pair u of thread t covers cosets 2t + 512u + {0, 1}.
 template <typename T, int NTQ, int MOUT, int U, bool WRITE>
-__global__ void __launch_bounds__(256) k_pair64(const StepArgs s, float2 *__restrict__ mem, const Ctx cx) {
+__global__ void __launch_bounds__(256) k_pair64(const StepArgs s, float2 *__restrict__ mem, const Ctx c0) {
+    const Ctx cx = slot_ctx(c0);
+    mem += (size_t)blockIdx.y * cx.arena;
     const Prologue P = step_prologue(s, cx, WRITE);
     if (P.skip) return;
     __shared__ uint64_t tks[40];
@@ -641,7 +663,9 @@ __global__ void __launch_bounds__(256) k_pair64(const StepArgs s, float2 *__rest
 // complex128 arena, one coset per thread and per 16-byte entry; FP64 arithmetic.
 // Chunk = 256 threads x U cosets = 2^(8 + log2 U) cosets; coset u of thread t is t + 256u.
 template <int NTQ, int MOUT, int U, bool WRITE>
-__global__ void __launch_bounds__(256) k_wide128(const StepArgs s, double2 *__restrict__ mem, const Ctx cx) {
+__global__ void __launch_bounds__(256) k_wide128(const StepArgs s, double2 *__restrict__ mem, const Ctx c0) {
+    const Ctx cx = slot_ctx(c0);
+    mem += (size_t)blockIdx.y * cx.arena;
     const Prologue P = step_prologue(s, cx, WRITE);
     if (P.skip) return;
     __shared__ uint64_t tks[40];
@@ -730,9 +754,13 @@ __global__ void __launch_bounds__(256) k_wide128(const StepArgs s, double2 *__re
     else norm_epilogue(cx, s.k, t0, t1);
 }
 
-// Start of a string / sample: the unit table and a fresh state.
+// Start of a string / sample per slot (one thread each): the unit table and a fresh state; a slot with no item left is
+// dead, so the item's passes skip it.
 template <typename E>
-__global__ void k_begin(E *mem, DevState *st) {
+__global__ void k_begin(E *mem, DevState *st, size_t arena) {
+    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+    mem += (size_t)slot * arena;
+    st += slot;
     store_entry(mem, 1.0, 0.0);
     st->prev = 1.0;
     st->lsc = 0;
@@ -741,29 +769,38 @@ __global__ void k_begin(E *mem, DevState *st) {
     st->sc = 1.0;
     st->ek = 0;
     st->bv = 0;
-    st->dead = 0;
+    st->dead = st->item >= st->nitems;
     st->counter = 0;
     st->aux = 0;
     st->trx = 0;
 }
 
-// End of a string / sample: final log2 Pr, next item.
+// End of a string / sample per slot (one thread each): final log2 Pr, next item (the slots take every slots-th).
 static __global__ void k_finish(DevState *st, double *logp_out, double *aux_out, int driver, int ns) {
+    st += blockIdx.x * blockDim.x + threadIdx.x;
     const int it = st->item;
+    st->item = it + gridDim.x * blockDim.x;
+    if (it >= st->nitems) return;
     double lp;
     if (driver == DRV_CHAIN1) lp = st->dead ? -INFINITY : log2(st->prev) + 2.0 * st->lsc - ns;
     else lp = st->logp;
     logp_out[it] = lp;
     if (aux_out) aux_out[it] = driver == DRV_HYBRID ? st->logscale : st->aux;
-    st->item = it + 1;
 }
 
-static __global__ void k_set_item(DevState *st, int item) { st->item = item; }
+// Slot i takes item first + i next, of items first .. nitems - 1.
+static __global__ void k_set_item(DevState *st, int first, int nitems) {
+    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+    st[slot].item = first + slot;
+    st[slot].nitems = nitems;
+}
 
 // Hybrid item whose first K steps are forced and ran as 'chain' passes (DRV_CHAIN1): from here on the run_steps
 // conventions (gsamp2.cpp:77-98).  The stored table is the true one times 2^-lsc, which is run_steps' logscale;
 // log2 Pr of the prefix is log2 |table|^2 + 2 lsc - K.  The forced bits of the prefix go to the output row.
 static __global__ void k_hybrid_switch(DevState *st, const int8_t *forced, int8_t *bits_out, int ns, int K) {
+    st += blockIdx.x * blockDim.x + threadIdx.x;
+    if (st->item >= st->nitems) return;
     const size_t row = (size_t)st->item * (size_t)ns;
     for (int k = 0; k < K; k++) bits_out[row + k] = forced[row + k];
     if (st->dead) {   // a zero-probability prefix: the chain epilogue zeroed every conditional from there on
