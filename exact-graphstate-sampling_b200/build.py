@@ -24,7 +24,7 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
 # in parallel with the rest
 LIB_SOURCES = ["gsb_engine.cu", "gsb_group_ws.cu", "gsb_group_ws3.cu", "gsb_group_wst.cu", "gsb_group_f32.cu", "gsb_group3.cu",
                "gsb_dp.cu", "gsb_grad.cu", "gsb_batch.cu", "gsb_probe.cu", "gsb_plan.cpp", "gsb_order.cpp", "gsb_fuse.cpp"]
-LIB_DEPS = LIB_SOURCES + ["gsb_kernels.cuh", "gsb_group.cuh", "gsb_step.h", "gsb_plan.h", "gsb_common.h", "gsb_fuse.h",
+LIB_DEPS = LIB_SOURCES + ["gsb_kernels.cuh", "gsb_run.cuh", "gsb_group.cuh", "gsb_step.h", "gsb_plan.h", "gsb_common.h", "gsb_fuse.h",
                           "gsb_pick.h"]
 
 
@@ -55,10 +55,11 @@ def build(force=False, verbose_ptxas=False):
         os.makedirs(objdir, exist_ok=True)
         cmds, objs = [], []
         headers = [d for d in deps if not d.endswith((".cu", ".cpp"))]
+        only_engine = os.path.join(CSRC, "gsb_run.cuh")
         for f in LIB_SOURCES:
             obj = os.path.join(objdir, f + ".o")
             objs.append(obj)
-            if not force and not verbose_ptxas and not _stale(obj, headers + [os.path.join(CSRC, f)]):
+            if not force and not verbose_ptxas and not _stale(obj, [os.path.join(CSRC, f)] + [h for h in headers if h != only_engine or f == "gsb_engine.cu"]):
                 continue
             cmds.append([_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose_ptxas else []) +
                         ["-c", "-I" + INCLUDE, "-I" + CSRC, "-o", obj, os.path.join(CSRC, f)])

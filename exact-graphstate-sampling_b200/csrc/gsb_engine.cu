@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <random>
 #include <string>
 #include <tuple>
@@ -28,6 +29,7 @@
 #include "gsb_kernels.cuh"
 #include "gsb_pick.h"
 #include "gsb_plan.h"
+#include "gsb_run.cuh"
 
 namespace gsb {
 
@@ -66,23 +68,14 @@ struct DevGuard {
     }
 };
 
-template <typename E, int NTQ, int M, int U>
-static void *pick_w(bool write) {
-    return write ? (void *)k_step<E, NTQ, M, U, true> : (void *)k_step<E, NTQ, M, U, false>;
+template <int NTQ, int M>
+static void *pick_any64(bool write) {
+    return write ? (void *)k_step<float2, NTQ, M, 4, true> : (void *)k_step<float2, NTQ, M, 4, false>;
 }
-template <typename E, int NTQ, int M>
-static void *pick_u(int U, bool write) {
-    return U == 4 ? pick_w<E, NTQ, M, 4>(write) : pick_w<E, NTQ, M, 1>(write);
-}
-template <typename E, int NTQ>
-static void *pick_m(int m, int U, bool write) {
-    return m == 2 ? pick_u<E, NTQ, 2>(U, write) : pick_u<E, NTQ, 1>(U, write);
-}
-template <typename E>
-static void *pick_step_kernel(int ntq, int m, int U, bool write) {
-    if (ntq == 4) return pick_m<E, 4>(m, U, write);
-    if (ntq == 2) return pick_m<E, 2>(m, U, write);
-    return pick_m<E, 1>(m, U, write);
+static void *pick_step_kernel(int ntq, int m, bool write) {
+    if (ntq == 4) return m == 2 ? pick_any64<4, 2>(write) : pick_any64<4, 1>(write);
+    if (ntq == 2) return m == 2 ? pick_any64<2, 2>(write) : pick_any64<2, 1>(write);
+    return m == 2 ? pick_any64<1, 2>(write) : pick_any64<1, 1>(write);
 }
 
 // wide-step kernels: U = 4 coset groups per thread for 1-2 offsets, 2 for 4 offsets (register budget)
@@ -167,6 +160,49 @@ static uint32_t group_smem_bytes(int D, int TR, const int (&ssz)[4], int L, bool
     return D == 3 ? group_smem<E, T, 3, 0>(ssz, L).total : group_smem<E, T, 2, 0>(ssz, L).total;
 }
 
+// Device memory of the slots' arenas.  cudaMalloc and cudaFree cost about 25 us per MB here, more than a whole call
+// on a fresh engine (50 samples of width 19: 1.4 ms, 13 ms with 512 MB to allocate), so the arenas come from a CUDA
+// memory pool per device (stream ordered, safe with several threads) that keeps at most SLOT_BYTES of freed memory for
+// the next engine and returns it when the last engine that used it closes.
+class SlotPool {
+    struct Dev {
+        cudaMemPool_t pool = nullptr;
+        int users = 0;
+    };
+    std::mutex mu;
+    std::map<int, Dev> devs;
+
+public:
+    static SlotPool &get() {
+        static SlotPool *p = new SlotPool();   // never destroyed: engines may close while the process exits
+        return *p;
+    }
+    cudaError_t open(int dev, cudaMemPool_t *pool) {
+        std::lock_guard<std::mutex> lock(mu);
+        Dev &d = devs[dev];
+        if (!d.pool) {
+            cudaMemPoolProps props;
+            memset(&props, 0, sizeof props);
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            cudaError_t e = cudaMemPoolCreate(&d.pool, &props);
+            if (e != cudaSuccess) { d.pool = nullptr; return e; }
+            uint64_t keep = SLOT_BYTES;
+            e = cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            if (e != cudaSuccess) return e;
+        }
+        d.users++;
+        *pool = d.pool;
+        return cudaSuccess;
+    }
+    void close(int dev) {
+        std::lock_guard<std::mutex> lock(mu);
+        Dev &d = devs[dev];
+        if (--d.users == 0) cudaMemPoolTrimTo(d.pool, 0);
+    }
+};
+
 struct Engine {
     HPlan plan;
     int prec = 64, dev = 0, sms = 0;
@@ -191,8 +227,17 @@ struct Engine {
     void *d_dump = nullptr;
     size_t dump_bytes = 0;
     std::vector<StepArgs> args;
-    StepArgs *d_args = nullptr;          // device copy of args (read by the small-step runs, k_small_run)
-    bool args_dirty = true;              // args changed since d_args was last written
+    // runs of small steps (gsb_run.cuh): maximal parts of consecutive steps, and each step's part (-1: none)
+    struct RunPart {
+        int k0, k1, dim;
+        size_t off;                      // first entry in rsteps (one per step, then the table left)
+    };
+    std::vector<RunPart> parts;
+    std::vector<int> part_of;
+    std::vector<RunStep> rsteps;
+    RunStep *d_rs = nullptr;             // device copies, read by the runs
+    StepArgs *d_args = nullptr;          // args, then a one-entry table
+    bool args_dirty = true;              // args changed since the device copies were last written
     std::vector<Launch> lw, ln;
     std::map<int, cudaGraphExec_t> graphs;   // key: graph kind << 16 | slots
     size_t arena = 0;                    // entries of an arena
@@ -201,6 +246,7 @@ struct Engine {
     int used_slots = 1;                  // slots of the launches queued since the device's error flags were read
     void *slot_mem = nullptr;            // the arenas of launches that carry several items
     size_t slot_bytes = 0;
+    cudaMemPool_t slot_pool = nullptr;
     std::map<void *, int> occ;
     // complex128 re-evaluation of unlikely strings (gsb_set_guard): the engine that re-evaluates this one's strings
     // whose log2 Pr + ns < guard_lx, and the engine this one re-evaluates for
@@ -221,9 +267,11 @@ struct Engine {
         if (guarded) guarded->guard = nullptr;
         DevGuard g(dev);
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
-        cudaFree(mem);
-        cudaFree(slot_mem);
+        cudaFree(mem);   // waits for the device, so nothing queued uses the slots' arenas any more
+        free_slots();
+        if (slot_pool) SlotPool::get().close(dev);
         cudaFree(d_args);
+        cudaFree(d_rs);
         cudaFree(st);
         cudaFree(partials);
         cudaFree(d_forced);
@@ -236,6 +284,22 @@ struct Engine {
         if (own_stream) cudaStreamDestroy(own_stream);
     }
 
+    void free_slots() {
+        if (!slot_mem) return;
+        cudaFreeAsync(slot_mem, own_stream);
+        cudaStreamSynchronize(own_stream);
+        slot_mem = nullptr;
+        slot_bytes = 0;
+    }
+    cudaError_t alloc_slots(size_t bytes) {
+        cudaError_t e = slot_pool ? cudaSuccess : SlotPool::get().open(dev, &slot_pool);
+        if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&slot_mem, bytes, slot_pool, own_stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(own_stream);
+        if (e != cudaSuccess) { cudaGetLastError(); slot_mem = nullptr; return e; }
+        slot_bytes = bytes;
+        return e;
+    }
+
     int occupancy(void *fn, int block) {
         auto it = occ.find(fn);
         if (it != occ.end()) return it->second;
@@ -243,10 +307,6 @@ struct Engine {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, block, 0) != cudaSuccess || nb < 1) nb = 1;
         occ[fn] = nb;
         return nb;
-    }
-
-    void *step_fn(int ntq, int m, int U, bool write) const {
-        return prec == 128 ? pick_step_kernel<double2>(ntq, m, U, write) : pick_step_kernel<float2>(ntq, m, U, write);
     }
 
     Launch shape(const StepArgs &a, bool write) {
@@ -267,14 +327,13 @@ struct Engine {
             L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)L.cap);
             return L;
         }
-        // blocks of at least one full warp (the reductions shuffle over 32 lanes); below 32 cosets the threads
-        // tid >= 2^nk idle
-        if (N >= 1024) { L.block = 256; L.U = 4; L.tl = 8; }
-        else if (N >= 256) { L.block = 256; L.U = 1; L.tl = 8; }
-        else { L.block = (int)std::max<uint64_t>(32, N); L.U = 1; L.tl = a.nk; }
-        L.cl = L.tl + (L.U == 4 ? 2 : 0);
+        if (prec == 128 || N < 1024) return L;   // always in a run
+        L.block = 256;
+        L.U = 4;
+        L.tl = 8;
+        L.cl = 10;
         L.nchunks = (unsigned int)(N >> L.cl);
-        L.fn = step_fn(a.ntq, a.m, L.U, write);
+        L.fn = pick_step_kernel(a.ntq, a.m, write);
         L.cap = occupancy(L.fn, L.block) * sms;
         L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)L.cap);
         return L;
@@ -319,38 +378,101 @@ struct Engine {
                                 stream);
     }
 
-    // Whether step k runs in a small-step run (k_small_run) when it is a single-step pass.
-    bool small_step(int k) const { return args[(size_t)k].nk <= SMALL_NK; }
-
-    // Steps k0 .. k1-1 as one k_small_run launch; norm: each step's norm pass runs before its write pass.
-    cudaError_t launch_small_run(int k0, int k1, int driver, bool norm, bool use_forced, bool use_unif) {
-        Launch L;
-        Ctx c = ctx(driver, plan.ns, L, use_forced, use_unif);
-        const StepArgs *sa = d_args;
-        int a0 = k0, a1 = k1, nm = norm ? 1 : 0;
+    // Steps k0 .. k1 - 1, all of one run part, as one k_run launch; norm: the branch norms of steps whose bit is drawn.
+    cudaError_t launch_run(int k0, int k1, int driver, int k_end, bool norm, bool use_forced, bool use_unif, bool begin,
+                           bool finish, bool direct = false) {
+        const RunPart &p = parts[(size_t)part_of[(size_t)k0]];
+        RunArgs ra;
+        ra.rs = d_rs + p.off + (k0 - p.k0);
+        ra.sa = d_args;
+        ra.k0 = k0;
+        ra.k1 = k1;
+        ra.dim = p.dim;
+        ra.norm = norm ? 1 : 0;
+        ra.begin = begin ? 1 : 0;
+        ra.finish = finish ? 1 : 0;
+        ra.direct = direct ? 1 : 0;
+        ra.logp = d_logp;
+        ra.aux = d_aux;
+        int nk = 0;
+        for (int k = k0; k < k1; k++) nk = std::max(nk, args[(size_t)k].nk);
+        // four cosets of the widest step per thread, at least a warp and at most 512 threads
+        const unsigned T = 1u << std::min(9, std::max(5, nk - 2));
+        Ctx c = ctx(driver, k_end, Launch(), use_forced, use_unif);
         void *memp = arena_mem();
-        void *kargs[] = {&sa, &a0, &a1, &nm, &memp, &c};
-        void *fn = prec == 128 ? (void *)k_small_run<double2> : (void *)k_small_run<float2>;
-        return cudaLaunchKernel(fn, dim3(1, (unsigned)slots), dim3(SMALL_THREADS), kargs, 0, stream);
+        void *kargs[] = {&ra, &memp, &c};
+        return cudaLaunchKernel(run_fn(), dim3(1, (unsigned)slots), dim3(T), kargs, run_smem(p.dim, k1 - k0, esize), stream);
+    }
+    void *run_fn() const { return prec == 128 ? (void *)k_run<double2> : (void *)k_run<float2>; }
+    // Whether one run is the whole plan: items then are one CTA each, all of a call in one launch.
+    bool whole() const { return parts.size() == 1 && plan.ns > 0 && parts[0].k0 == 0 && parts[0].k1 == plan.ns; }
+
+    // A single step alone, as a run or as its write pass (the caller queues the norm pass of a step in no part).
+    cudaError_t launch_single(int k, int driver, bool use_forced, bool use_unif) {
+        if (part_of[(size_t)k] < 0) return launch_step(k, true, driver, plan.ns, use_forced, use_unif);
+        return launch_run(k, k + 1, driver, plan.ns, driver != DRV_CHAIN1, use_forced, use_unif, false, false);
+    }
+    bool in_run(int k) const { return part_of[(size_t)k] >= 0; }
+
+    // A queued item sequence: whether its start is queued, whether its end is, and the launches so far.
+    struct Seq {
+        bool begun = false, finished = false;
+        int64_t launches = 0;
+        bool dry = false;      // count the launches only
+    };
+    cudaError_t seq_begin(Seq &q) {
+        if (q.begun) return cudaSuccess;
+        q.begun = true;
+        q.launches++;
+        return q.dry ? cudaSuccess : launch_begin();
     }
 
-    // Length of the run of consecutive single small-step passes that starts at ops[i] (0 or 1: no run).
-    size_t small_run_len(const std::vector<Op> &ops, size_t i) const {
-        size_t j = i;
-        while (j < ops.size() && !ops[j].group && small_step(ops[j].k0)) j++;
-        return j - i >= 2 ? j - i : 0;
-    }
-
-    // Launches of one item over a pass list (small-step runs count once), begin and finish included.
-    int64_t item_launches(const std::vector<Op> &ops, bool norm) const {
-        int64_t n = 2;
-        for (size_t i = 0; i < ops.size();) {
-            const size_t r = small_run_len(ops, i);
-            if (r) { n++; i += r; continue; }
-            n += 1 + ((norm && !ops[i].group) || ops[i].norm_first ? 1 : 0);
-            i++;
+    // Steps a .. b - 1 as runs where they are small enough, else one launch each (two with a norm pass); with `finish`
+    // the item ends with step b - 1, and a run that ends there records its results.
+    cudaError_t enqueue_steps(Seq &q, int a, int b, int driver, int k_end, bool norm, bool use_forced, bool use_unif,
+                              bool finish) {
+        cudaError_t e = cudaSuccess;
+        for (int k = a; k < b && e == cudaSuccess;) {
+            if (part_of[(size_t)k] >= 0) {
+                const int k1 = std::min(b, parts[(size_t)part_of[(size_t)k]].k1);
+                const bool last = finish && k1 == b;
+                q.launches++;
+                if (!q.dry)
+                    e = launch_run(k, k1, driver, k_end, norm, use_forced, use_unif, !q.begun, last);
+                q.begun = true;
+                q.finished = last;
+                k = k1;
+                continue;
+            }
+            e = seq_begin(q);
+            q.launches += norm ? 2 : 1;
+            if (e == cudaSuccess && norm && !q.dry) e = launch_step(k, false, driver, k_end, use_forced, use_unif);
+            if (e == cudaSuccess && !q.dry) e = launch_step(k, true, driver, k_end, use_forced, use_unif);
+            k++;
         }
-        return n;
+        return e;
+    }
+
+    // A pass list: fused passes, and the single steps between them.
+    cudaError_t enqueue_ops(Seq &q, const std::vector<Op> &ops, int driver, bool norm, bool use_forced, bool use_unif,
+                            bool finish) {
+        cudaError_t e = cudaSuccess;
+        for (size_t i = 0; i < ops.size() && e == cudaSuccess;) {
+            if (!ops[i].group) {
+                const int a = ops[i].k0;
+                while (i < ops.size() && !ops[i].group) i++;
+                e = enqueue_steps(q, a, ops[i - 1].k0 + 1, driver, plan.ns, norm, use_forced, use_unif,
+                                  finish && i == ops.size());
+                continue;
+            }
+            const Op &op = ops[i++];
+            e = seq_begin(q);
+            q.launches += op.norm_first ? 2 : 1;
+            if (q.dry) continue;
+            if (e == cudaSuccess && op.norm_first) e = launch_step(op.k0, false, driver, plan.ns, use_forced, use_unif);
+            if (e == cudaSuccess) e = launch_op(op, driver, use_forced, use_unif);
+        }
+        return e;
     }
 
     cudaError_t launch_begin() {
@@ -368,7 +490,7 @@ struct Engine {
     // One item: begin, steps k0..k1-1, finish.  driver decides the passes:
     //   CHAIN: norm + write per step; CHAIN1: write; HYBRID: norm (skipped on device when forced) + write.
     cudaError_t launch_op(const Op &op, int driver, bool use_forced = true, bool use_unif = false) {
-        if (!op.group) return launch_step(op.k0, true, driver, plan.ns, use_forced, use_unif);
+        if (!op.group) return launch_single(op.k0, driver, use_forced, use_unif);
         Launch L;
         L.tl = 8;
         L.cl = op.ga.L;
@@ -382,79 +504,63 @@ struct Engine {
                                 op.smem, stream);
     }
 
-    cudaError_t enqueue_item(int driver, bool use_forced, bool use_unif) {
-        cudaError_t e = launch_begin();
-        if (e != cudaSuccess) return e;
+    cudaError_t enqueue_item(int driver, bool use_forced, bool use_unif, Seq &q) {
+        const int ns = plan.ns;
+        const bool norm = driver != DRV_CHAIN1;
+        cudaError_t e = cudaSuccess;
         if (driver == DRV_CHAIN1 && !chain_ops.empty()) {
-            for (size_t i = 0; i < chain_ops.size();) {
-                if (const size_t r = small_run_len(chain_ops, i)) {
-                    e = launch_small_run(chain_ops[i].k0, chain_ops[i + r - 1].k0 + 1, driver, false, use_forced,
-                                         use_unif);
-                    if (e != cudaSuccess) return e;
-                    i += r;
-                    continue;
+            e = enqueue_ops(q, chain_ops, driver, false, use_forced, use_unif, true);
+        } else if (driver == DRV_CHAIN && !sample_ops.empty()) {
+            e = enqueue_ops(q, sample_ops, driver, true, use_forced, use_unif, true);
+        } else {
+            int k0 = 0;
+            if (driver == DRV_HYBRID && hyb_K > 0) {
+                // forced prefix: 'chain' passes (fused where possible), then the run_steps state for the sampled steps
+                e = enqueue_ops(q, hyb_ops, DRV_CHAIN1, false, true, false, false);
+                q.launches++;
+                const int b = std::min(slots, 64);
+                if (e == cudaSuccess && !q.dry) {
+                    k_hybrid_switch<<<slots / b, b, 0, stream>>>(st, d_forced, d_bits, ns, hyb_K);
+                    e = cudaGetLastError();
                 }
-                e = launch_op(chain_ops[i++], driver);
-                if (e != cudaSuccess) return e;
+                k0 = hyb_K;
             }
-            return launch_finish(driver);
+            if (e == cudaSuccess) e = enqueue_steps(q, k0, ns, driver, ns, norm, use_forced, use_unif, true);
         }
-        if (driver == DRV_CHAIN && !sample_ops.empty()) {
-            for (size_t i = 0; i < sample_ops.size();) {
-                if (const size_t r = small_run_len(sample_ops, i)) {
-                    e = launch_small_run(sample_ops[i].k0, sample_ops[i + r - 1].k0 + 1, driver, true, use_forced,
-                                         use_unif);
-                    if (e != cudaSuccess) return e;
-                    i += r;
-                    continue;
-                }
-                const Op &op = sample_ops[i++];
-                if (!op.group || op.norm_first) {
-                    e = launch_step(op.k0, false, driver, plan.ns, use_forced, use_unif);
-                    if (e != cudaSuccess) return e;
-                }
-                e = op.group ? launch_op(op, driver, use_forced, use_unif)
-                             : launch_step(op.k0, true, driver, plan.ns, use_forced, use_unif);
-                if (e != cudaSuccess) return e;
-            }
-            return launch_finish(driver);
-        }
-        int k0 = 0;
-        if (driver == DRV_HYBRID && hyb_K > 0) {
-            // forced prefix: 'chain' passes (fused where possible), then the run_steps state for the sampled steps
-            for (size_t i = 0; i < hyb_ops.size();) {
-                if (const size_t r = small_run_len(hyb_ops, i)) {
-                    e = launch_small_run(hyb_ops[i].k0, hyb_ops[i + r - 1].k0 + 1, DRV_CHAIN1, false, true, false);
-                    if (e != cudaSuccess) return e;
-                    i += r;
-                    continue;
-                }
-                e = launch_op(hyb_ops[i++], DRV_CHAIN1);
-                if (e != cudaSuccess) return e;
-            }
-            const int b = std::min(slots, 64);
-            k_hybrid_switch<<<slots / b, b, 0, stream>>>(st, d_forced, d_bits, plan.ns, hyb_K);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            k0 = hyb_K;
-        }
-        for (int k = k0; k < plan.ns; k++) {
-            int k1 = k;
-            while (k1 < plan.ns && small_step(k1)) k1++;
-            if (k1 - k >= 2) {
-                e = launch_small_run(k, k1, driver, driver != DRV_CHAIN1, use_forced, use_unif);
-                if (e != cudaSuccess) return e;
-                k = k1 - 1;
-                continue;
-            }
-            if (driver != DRV_CHAIN1) {
-                e = launch_step(k, false, driver, plan.ns, use_forced, use_unif);
-                if (e != cudaSuccess) return e;
-            }
-            e = launch_step(k, true, driver, plan.ns, use_forced, use_unif);
-            if (e != cudaSuccess) return e;
-        }
-        return launch_finish(driver);
+        if (e == cudaSuccess) e = seq_begin(q);   // an empty plan
+        if (e != cudaSuccess || q.finished) return e;
+        q.launches++;
+        return q.dry ? cudaSuccess : launch_finish(driver);
     }
+
+    // Launches of one item (mode 0: 'chain', else 'prob' / 'sample').
+    int64_t item_launches(int mode) {
+        if (whole()) return 1;
+        Seq q;
+        q.dry = true;
+        enqueue_item(mode == 0 ? DRV_CHAIN1 : DRV_CHAIN, true, false, q);
+        return q.launches;
+    }
+
+    // The step descriptors that runs read, to the device.
+    int upload() {
+        if (!args_dirty) return 0;
+        for (const RunPart &p : parts)
+            for (int k = p.k0; k < p.k1; k++)
+                for (int b = 0; b < 2; b++)
+                    for (int x = 0; x < 2; x++) {
+                        RunStep &r = rsteps[p.off + (size_t)(k - p.k0)];
+                        r.M[b][x][0] = args[(size_t)k].Mr[b][x];
+                        r.M[b][x][1] = args[(size_t)k].Mi[b][x];
+                    }
+        GSB_CK(cudaMemcpyAsync(d_args, args.data(), args.size() * sizeof(StepArgs), cudaMemcpyHostToDevice, stream));
+        GSB_CK(cudaMemcpyAsync(d_rs, rsteps.data(), rsteps.size() * sizeof(RunStep), cudaMemcpyHostToDevice, stream));
+        GSB_CK(cudaStreamSynchronize(stream));
+        args_dirty = false;
+        return 0;
+    }
+
+    static int driver_of(int kind) { return kind == 0 ? DRV_CHAIN1 : kind == 3 ? DRV_HYBRID : DRV_CHAIN; }
 
     // The graph of one launch of `nslots` items of mode `kind`.
     int graph(int kind, int nslots, cudaGraphExec_t *out) {
@@ -466,28 +572,18 @@ struct Engine {
             for (auto kv = graphs.begin(); kv != graphs.end();)            // those that point at the old ones
                 if ((kv->first & 0xffff) > 1) { cudaGraphExecDestroy(kv->second); kv = graphs.erase(kv); }
                 else ++kv;
-            cudaFree(slot_mem);
-            slot_mem = nullptr;
-            slot_bytes = 0;
-            const size_t bytes = (size_t)nslots * arena * esize;
-            if (cudaMalloc(&slot_mem, bytes) != cudaSuccess) {
-                cudaGetLastError();
-                slot_mem = nullptr;
+            free_slots();
+            if (alloc_slots((size_t)nslots * arena * esize) != cudaSuccess)
                 return fail(GSB_E_ALLOC, "allocation of the slots' arenas failed");
-            }
-            slot_bytes = bytes;
         }
-        int driver = kind == 0 ? DRV_CHAIN1 : kind == 3 ? DRV_HYBRID : DRV_CHAIN;
-        bool use_forced = kind != 2, use_unif = kind >= 2;
-        if (args_dirty) {   // the small-step runs read the step descriptors from the device
-            GSB_CK(cudaMemcpyAsync(d_args, args.data(), args.size() * sizeof(StepArgs), cudaMemcpyHostToDevice, stream));
-            GSB_CK(cudaStreamSynchronize(stream));
-            args_dirty = false;
-        }
+        const int driver = driver_of(kind);
+        const bool use_forced = kind != 2, use_unif = kind >= 2;
+        if (int rc = upload()) return rc;
         cudaGraph_t g = nullptr;
         GSB_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         slots = nslots;
-        cudaError_t e = enqueue_item(driver, use_forced, use_unif);
+        Seq q;
+        cudaError_t e = enqueue_item(driver, use_forced, use_unif, q);
         slots = 1;
         cudaError_t e2 = cudaStreamEndCapture(stream, &g);
         if (e != cudaSuccess) { if (g) cudaGraphDestroy(g); GSB_CK(e); }
@@ -504,6 +600,16 @@ struct Engine {
     // Run `n` items of graph `kind` with inputs already in d_forced / d_unif rows 0..n-1.
     int run_graph_items(int kind, int64_t n) {
         if (n < 1) return 0;
+        if (whole()) {   // every item in one launch (a hybrid prefix runs with the run_steps conventions as well)
+            if (int rc = upload()) return rc;
+            const int driver = driver_of(kind);
+            slots = (int)n;
+            const cudaError_t e = launch_run(0, plan.ns, driver, plan.ns, driver != DRV_CHAIN1, kind != 2, kind >= 2, true,
+                                             true, true);
+            slots = 1;
+            GSB_CK(e);
+            return 0;
+        }
         cudaGraphExec_t ex;
         int s = 1;
         while (s < max_slots && s < n) s *= 2;
@@ -604,6 +710,81 @@ static void apply_coeffs(Engine &E) {
     E.args_dirty = true;   // every change of the descriptors (matrices, arithmetic) ends here
 }
 
+// Span of address columns with coordinates in the inserted columns.
+struct Coords {
+    std::vector<std::pair<uint64_t, uint32_t>> rows;   // (reduced column, inserted columns it is the sum of)
+    bool reduce(uint64_t &v, uint32_t &c) const {      // true: v was in the span, c its coordinates
+        for (const auto &r : rows)
+            if (v >> (63 - __builtin_clzll(r.first)) & 1) { v ^= r.first; c ^= r.second; }
+        return v == 0;
+    }
+    void add(uint64_t v) {
+        uint32_t c = 0;
+        if (reduce(v, c)) return;
+        rows.push_back({v, c ^ 1u << rows.size()});    // reduced by all earlier rows; later ones keep their leading bits
+    }
+    uint32_t of(uint64_t v) const {
+        uint32_t c = 0;
+        reduce(v, c);
+        return c;
+    }
+};
+
+// Parts of consecutive steps whose columns span at most 2^RUN_DIM addresses, each as long as it can be, with their steps
+// in compact coordinates.  Every step of at most 2^10 cosets fits one (its columns span nk + 2 dimensions at most).
+constexpr int RUN_MAX_STEPS = 1024;   // saved scalars of a run in shared memory: 25 B per step
+static void build_runs(Engine &E) {
+    const int ns = E.plan.ns;
+    E.parts.clear();
+    E.rsteps.clear();
+    E.part_of.assign((size_t)ns, -1);
+    auto columns = [&](const StepArgs &a, Coords &s) {
+        for (int j = 0; j < a.nk; j++) s.add(a.tk[j]);
+        for (int t = 0; t < a.ntq; t++) s.add(a.tq[t]);
+        if (a.m == 2) s.add(a.g);
+    };
+    for (int k0 = 0; k0 < ns;) {
+        Coords span;
+        int k1 = k0;
+        for (; k1 < ns && k1 - k0 < RUN_MAX_STEPS; k1++) {
+            Coords with = span;
+            columns(E.args[(size_t)k1], with);
+            if ((int)with.rows.size() > RUN_DIM) break;
+            span = with;
+        }
+        if (k1 == k0) { k0++; continue; }
+        std::vector<int> by((size_t)(k1 - k0));
+        for (int i = 0; i < k1 - k0; i++) by[(size_t)i] = k0 + i;
+        std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return E.args[(size_t)x].nk > E.args[(size_t)y].nk; });
+        Coords co;
+        for (int k : by) columns(E.args[(size_t)k], co);
+        E.parts.push_back({k0, k1, (int)co.rows.size(), E.rsteps.size()});
+        for (int k = k0; k <= k1; k++) {   // k1: the columns of the table the part leaves
+            RunStep r;
+            memset(&r, 0, sizeof r);
+            r.ntq = 1;
+            if (k < ns) {
+                const StepArgs &a = E.args[(size_t)k];
+                r.nk = a.nk;
+                r.ntq = a.ntq;
+                r.m = a.m;
+                r.g = co.of(a.g);
+                r.rhoc = (uint32_t)a.rhoc;
+                for (int j = 0; j < std::min(a.nk, RUN_DIM); j++) r.tk[j] = co.of(a.tk[j]);
+                for (int t = 0; t < a.ntq; t++) {
+                    r.tq[t] = co.of(a.tq[t]);
+                    r.tau0 |= a.tau0[t] << t;
+                    r.tau1 |= a.tau1[t] << t;
+                    r.par |= a.par[t] << t;
+                }
+            }
+            E.rsteps.push_back(r);
+            if (k < k1) E.part_of[(size_t)k] = (int)E.parts.size() - 1;
+        }
+        k0 = k1;
+    }
+}
+
 static int make_args(Engine &E) {
     const HPlan &p = E.plan;
     E.args.resize((size_t)p.ns);
@@ -637,11 +818,21 @@ static int make_args(Engine &E) {
         E.ln[(size_t)k] = E.shape(E.args[(size_t)k], false);
         maxgrid = std::max(maxgrid, (size_t)std::max(E.lw[(size_t)k].grid, E.ln[(size_t)k].grid));
     }
+    build_runs(E);
+    if (E.whole()) E.max_slots = 1;   // its items need no slots
     // a launch of several slots: one block each, or blocks of 256 threads (8 per SM) in at most SLOT_WAVES rounds
-    maxgrid = std::max(maxgrid, std::max((size_t)E.sms * 8 * SLOT_WAVES, (size_t)MAX_SLOTS));
+    maxgrid = std::max(maxgrid, E.max_slots > 1 ? std::max((size_t)E.sms * 8 * SLOT_WAVES, (size_t)E.max_slots)
+                                                : (size_t)E.sms * 8);
     GSB_CK(cudaMalloc(&E.partials, maxgrid * PARTIAL_SUMS * sizeof(double)));
-    GSB_CK(cudaMalloc(&E.d_args, (size_t)std::max(1, p.ns) * sizeof(StepArgs)));
+    GSB_CK(cudaMalloc(&E.d_args, ((size_t)p.ns + 1) * sizeof(StepArgs)));
+    GSB_CK(cudaMalloc(&E.d_rs, std::max<size_t>(E.rsteps.size(), 1) * sizeof(RunStep)));
+    StepArgs end;
+    memset(&end, 0, sizeof end);
+    end.ntq = 1;
+    GSB_CK(cudaMemcpy(E.d_args + p.ns, &end, sizeof end, cudaMemcpyHostToDevice));
     E.args_dirty = true;
+    GSB_CK(cudaFuncSetAttribute(E.run_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)run_smem(RUN_DIM, RUN_MAX_STEPS, sizeof(double2))));
     return 0;
 }
 
@@ -1031,9 +1222,6 @@ static int open_plan(const char *text, size_t len, int precision, int device, gs
     e = cudaMemsetAsync(E->mem, 0, arena, E->stream);
     if (e != cudaSuccess) return cuda_fail(e, "arena clear");
     const size_t ns = (size_t)std::max(1, E->plan.ns), cap = (size_t)E->cap;
-    const size_t st_bytes = sizeof(DevState) * (size_t)E->max_slots;
-    if ((e = cudaMalloc(&E->st, st_bytes)) != cudaSuccess) return cuda_fail(e, "state");
-    if ((e = cudaMemsetAsync(E->st, 0, st_bytes, E->stream)) != cudaSuccess) return cuda_fail(e, "state");
     if ((e = cudaMalloc(&E->d_forced, cap * ns)) != cudaSuccess) return cuda_fail(e, "buffers");
     if ((e = cudaMalloc(&E->d_bits, cap * ns)) != cudaSuccess) return cuda_fail(e, "buffers");
     if ((e = cudaMalloc(&E->d_unif, cap * ns * 8)) != cudaSuccess) return cuda_fail(e, "buffers");
@@ -1043,6 +1231,9 @@ static int open_plan(const char *text, size_t len, int precision, int device, gs
     if ((e = cudaMemsetAsync(E->d_forced, 0, cap * ns, E->stream)) != cudaSuccess) return cuda_fail(e, "buffers");
     rc = make_args(*E);
     if (rc) { std::string m = g_err; delete E; return fail(rc, m); }
+    const size_t st_bytes = sizeof(DevState) * (size_t)E->max_slots;
+    if ((e = cudaMalloc(&E->st, st_bytes)) != cudaSuccess) return cuda_fail(e, "state");
+    if ((e = cudaMemsetAsync(E->st, 0, st_bytes, E->stream)) != cudaSuccess) return cuda_fail(e, "state");
     build_chain_ops(*E);
     if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return cuda_fail(e, "set-up");
     *out = reinterpret_cast<gsb_engine *>(E);
@@ -1147,6 +1338,7 @@ static int check_bits(const int8_t *b, int64_t n, int ns, bool allow_free) {
 // A fused pass whose tile loads did not complete within its bounded wait sets DevState::err and stops the item;
 // report it (and clear it) after the work has been synchronised.
 static int check_device(Engine *E) {
+    if (E->whole()) return 0;   // runs only: nothing on the device waits
     std::vector<int> v((size_t)std::exchange(E->used_slots, 1));   // those of the calls since the last check
     const size_t pitch = sizeof(DevState);
     if (v.size() == 1) GSB_CK(cudaMemcpy(v.data(), &E->st->err, sizeof(int), cudaMemcpyDeviceToHost));   // quicker
@@ -1401,8 +1593,10 @@ int gsb_prefix(gsb_engine *e, const int8_t *forced, int K, void *dump, double *l
     for (int k = 0; k < Kr; k++) row[(size_t)k] = forced[k];
     if (ns) GSB_CK(cudaMemcpyAsync(E->d_forced, row.data(), (size_t)ns, cudaMemcpyHostToDevice, E->stream));
     k_set_item<<<1, 1, 0, E->stream>>>(E->st, 0, 1);
-    GSB_CK(E->launch_begin());
-    for (int k = 0; k < Kr; k++) GSB_CK(E->launch_step(k, true, DRV_HYBRID, Kr, true, false));
+    if (int rc = E->upload()) return rc;
+    Engine::Seq q;
+    GSB_CK(E->enqueue_steps(q, 0, Kr, DRV_HYBRID, Kr, false, true, false, false));
+    GSB_CK(E->seq_begin(q));   // K = 0
     if (dump) {   // dump == NULL: only the prefix probability (a marginal) is wanted
         int nk, ntq;
         gsb_dump_shape(e, K, &nk, &ntq);
@@ -1506,10 +1700,10 @@ int gsb_resume(gsb_engine *e, const int8_t *forced, int K, uint64_t seed, int64_
     if (E->prec == 128) k_resume_sum<double2><<<grid, L1.block, 0, E->stream>>>(a, (double2 *)E->mem, ra, c);
     else k_resume_sum<float2><<<grid, L1.block, 0, E->stream>>>(a, (float2 *)E->mem, ra, c);
     GSB_CK(cudaGetLastError());
-    for (int k = K; k < ns; k++) {
-        GSB_CK(E->launch_step(k, false, DRV_HYBRID, ns, true, true));
-        GSB_CK(E->launch_step(k, true, DRV_HYBRID, ns, true, true));
-    }
+    if ((rc = E->upload())) return rc;
+    Engine::Seq q;
+    q.begun = true;
+    GSB_CK(E->enqueue_steps(q, K, ns, DRV_HYBRID, ns, true, true, true, false));
     DevState hs;
     GSB_CK(cudaMemcpyAsync(&hs, E->st, sizeof hs, cudaMemcpyDeviceToHost, E->stream));
     std::vector<int8_t> hb((size_t)std::max(ns, 1), 0);
@@ -1706,8 +1900,10 @@ static int autotune(Engine &E, int mode, int reps) {
     std::vector<double> t_write((size_t)ns), t_norm((size_t)ns);
     const int drv = mode == 0 ? DRV_CHAIN1 : DRV_CHAIN;
     for (int k = 0; k < ns; k++) {
-        t_write[(size_t)k] = timer([&] { return E.launch_step(k, true, drv, ns, true, false); });
-        t_norm[(size_t)k] = mode == 0 ? 0 : timer([&] { return E.launch_step(k, false, drv, ns, true, false); });
+        t_write[(size_t)k] = timer([&] { return E.launch_single(k, drv, true, false); });
+        // a run evaluates the branch norms itself; a fused pass of a step in a run may still want a norm pass first
+        t_norm[(size_t)k] = mode == 0 || (E.in_run(k) && rof(k) < GROUP_MIN_R)
+                                ? 0 : timer([&] { return E.launch_step(k, false, drv, ns, true, false); });
         if (t_write[(size_t)k] < 0 || t_norm[(size_t)k] < 0) return fail(GSB_E_CUDA, "autotuner: a timing launch failed");
     }
     // fused candidates starting at k, with their times (distinct tile sizes only)
@@ -1787,7 +1983,7 @@ static int autotune(Engine &E, int mode, int reps) {
         for (int t = 0; t < 2; t++) {
             OpShape single;
             single.k0 = k;
-            double best = t_norm[(size_t)k] + t_write[(size_t)k] + cost[(size_t)k + 1][0];
+            double best = (E.in_run(k) ? 0 : t_norm[(size_t)k]) + t_write[(size_t)k] + cost[(size_t)k + 1][0];
             OpShape bp = single;
             for (auto &x : cands[(size_t)k]) {
                 const OpShape &sh = x.first;
@@ -2004,6 +2200,7 @@ int gsb_profile_steps(gsb_engine *e, const int8_t *bits, int mode, float *ms_wri
     int rc = check_bits(bits, 1, ns, false);
     if (rc) return rc;
     const int driver = mode == 0 ? DRV_CHAIN1 : DRV_CHAIN;
+    if ((rc = E->upload())) return rc;
     std::vector<cudaEvent_t> ev((size_t)(2 * ns + 1));
     for (auto &x : ev) GSB_CK(cudaEventCreate(&x));
     if (ns) GSB_CK(cudaMemcpyAsync(E->d_forced, bits, (size_t)ns, cudaMemcpyHostToDevice, E->stream));
@@ -2037,10 +2234,9 @@ int gsb_profile_steps(gsb_engine *e, const int8_t *bits, int mode, float *ms_wri
         GSB_CK(cudaEventRecord(ev2[0], E->stream));
         for (size_t i = 0; i < E->sample_ops.size(); i++) {
             const Op &op = E->sample_ops[i];
-            if (!op.group || op.norm_first) GSB_CK(E->launch_step(op.k0, false, driver, ns, true, false));
+            if (op.group ? op.norm_first : !E->in_run(op.k0)) GSB_CK(E->launch_step(op.k0, false, driver, ns, true, false));
             GSB_CK(cudaEventRecord(ev2[2 * i + 1], E->stream));
-            if (op.group) GSB_CK(E->launch_op(op, driver, true, false));
-            else GSB_CK(E->launch_step(op.k0, true, driver, ns, true, false));
+            GSB_CK(E->launch_op(op, driver, true, false));
             GSB_CK(cudaEventRecord(ev2[2 * i + 2], E->stream));
         }
         GSB_CK(E->launch_finish(driver));
@@ -2061,9 +2257,9 @@ int gsb_profile_steps(gsb_engine *e, const int8_t *bits, int mode, float *ms_wri
         return 0;
     }
     for (int k = 0; k < ns; k++) {
-        if (driver == DRV_CHAIN) GSB_CK(E->launch_step(k, false, driver, ns, true, false));
+        if (driver == DRV_CHAIN && !E->in_run(k)) GSB_CK(E->launch_step(k, false, driver, ns, true, false));
         GSB_CK(cudaEventRecord(ev[(size_t)(2 * k + 1)], E->stream));
-        GSB_CK(E->launch_step(k, true, driver, ns, true, false));
+        GSB_CK(E->launch_single(k, driver, true, false));
         GSB_CK(cudaEventRecord(ev[(size_t)(2 * k + 2)], E->stream));
     }
     GSB_CK(E->launch_finish(driver));
@@ -2081,21 +2277,7 @@ int gsb_profile_steps(gsb_engine *e, const int8_t *bits, int mode, float *ms_wri
 
 int gsb_launches_per_item(const gsb_engine *e, int mode, int64_t *launches) {
     if (!e || !launches) return fail(GSB_E_USAGE, "null argument");
-    const Engine *E = eng(e);
-    const int64_t ns = E->plan.ns;
-    if (mode == 0 && !E->chain_ops.empty()) *launches = E->item_launches(E->chain_ops, false);
-    else if (mode == 1 && !E->sample_ops.empty()) *launches = E->item_launches(E->sample_ops, true);
-    else {   // one norm and one write pass per step ('chain' mode: write only), small-step runs counted once
-        int64_t n = 2;
-        for (int k = 0; k < ns;) {
-            int k1 = k;
-            while (k1 < ns && E->small_step(k1)) k1++;
-            if (k1 - k >= 2) { n++; k = k1; continue; }
-            n += mode == 0 ? 1 : 2;
-            k++;
-        }
-        *launches = n;
-    }
+    *launches = const_cast<Engine *>(eng(e))->item_launches(mode);   // a dry run of the sequence: nothing is queued
     return 0;
 }
 
