@@ -5,17 +5,26 @@
 // with the step map of the executor (gsamp2.cpp:32-38, 59-66): for every coset c of step k, base = XOR of Tkeep
 // over the bits of c, the inputs v_t = T_k[base ^ tq_t] and
 //   out[tau] = sum_{t: tau0_t = tau} m0 v_t + sum_{t: tau1_t = tau} m1 s_t v_t,   s_t = (-1)^(parity(c & rhoc) ^ par_t),
-// m_x = M_k[b_k][x], stored at base (tau 0) and base ^ g (tau 1).  The reverse sweep carries lambda_k = dZ/dT_k
-// backwards through the transposed step map (the same cosets and slots, read and written the other way round):
+// m_x = M_k[b_k][x].  The reverse sweep carries lambda_k = dZ/dT_k backwards through the transposed step map:
 //   lambda_k[base ^ tq_t] = m0 lambda_{k+1}[tau0_t] + m1 s_t lambda_{k+1}[tau1_t],
 //   dZ/dm0 = sum_t lambda_{k+1}[tau0_t] v_t,       dZ/dm1 = sum_t s_t lambda_{k+1}[tau1_t] v_t,
-// with lambda_ns = 1 at the final entry.  Each coset reads and writes only its own slots, so the reverse pass is
-// in place and race-free like the forward one.  The reverse pass needs T_k: the forward sweep keeps a compact copy
-// of the live table ([coset][offset], 2^{r_k} entries) every `every` steps, and each segment between two
-// checkpoints is recomputed forward once, keeping its tables, before the reverse pass walks it.  Up to 32 strings
-// are swept together (grid dimension y: each string owns its arenas, checkpoints, segment tables and reduction
-// slots), and the whole sequence of such a launch (forward, then per segment: restore, recompute, reverse) is one
-// CUDA graph; the first string's index lives in device memory and advances at its end.
+// with lambda_ns = 1 at the final entry.
+//
+// Both sweeps run in passes of two steps (one where two do not fuse), out of place: the table before a pass is kept for
+// the reverse sweep, which computes the table between the pass's two steps again as it goes.  A pass of two steps then
+// reads and writes a table once forward, and reads T, reads lambda and writes lambda once in reverse: five table
+// transfers for two steps.  One step per pass with a checkpoint every four steps moved sixteen (forward, restore, the
+// segment's tables again, the reverse reads and writes), and both forms are bound by HBM.
+//
+// Tables are compact: the entry at address base(c) ^ tq_t of the table before step k has index c | t << nk, which is
+// XOR-linear in the address, so a pass walks its classes (gsb_fuse.h) with one running index per table.  A thread takes a
+// whole class; its values of every stage sit in shared-memory slots of its own ([value][thread]: no bank conflicts and
+// no barriers), filled by 16-byte asynchronous copies, all of a class at once.
+//
+// Up to 32 strings are swept together (grid dimension y: each string owns its tables and reduction slots), and the
+// whole sequence of such a launch is one CUDA graph; the first string's index lives in device memory and advances at its
+// end.  Where the tables of all passes do not fit, only every q-th is kept and the ones between are computed again,
+// segment by segment.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -26,6 +35,7 @@
 
 #include "gsb.h"
 #include "gsb_common.h"
+#include "gsb_fuse.h"
 #include "gsb_plan.h"
 #include "gsb_step.h"
 
@@ -36,214 +46,351 @@ struct GradCtx {
     const double *M;         // [ns][2][2] (re, im): the caller's matrices
     const int8_t *bits;      // [cap][ns]
     const int *item;         // first string of the launch
-    int ns, maxgrid;
-    size_t arena;            // entries per string: T and Lam arenas
+    int ns;
 };
 
-__device__ __forceinline__ uint64_t coset_base(const StepArgs &s, uint64_t c) {
-    uint64_t b = 0;
-    while (c) {
-        const int j = __ffsll((long long)c) - 1;
-        b ^= s.tk[j];
-        c &= c - 1;
-    }
-    return b;
-}
+// One step inside a pass: member j of a class reads values in[j][t] of its stage and writes values out[j][tau] of the
+// next one; its class sign is parity(class & lam) ^ mpar[j].
+struct GradStep {
+    int k, nmem, ntq, m;
+    int tau0, tau1, par;     // bit t: offset t's x = 0 / x = 1 output, x = 1 sign
+    uint64_t lam;
+    unsigned char in[16][4], out[16][2], mpar[16];
+};
 
-// The cosets a thread visits (grid x times block: a power of two, 2^ls threads): c = t | (g << ls) for the Gray
-// codes g of the high bits, so the base is the thread's fixed low part XOR one running value (one XOR per coset).
-template <typename F>
-__device__ __forceinline__ void grid_cosets(const StepArgs &s, F f) {
-    const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
-    const int ls = __ffsll((long long)nthreads) - 1;
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (s.nk < ls && t >= (1ULL << s.nk)) return;
-    const uint64_t lo = coset_base(s, t);
-    const uint64_t nh = s.nk > ls ? 1ULL << (s.nk - ls) : 1;
-    uint64_t hi = 0;
-    for (uint64_t n = 0; n < nh; n++) {
-        if (n) hi ^= s.tk[ls + __ffsll((long long)n) - 1];
-        f(t | ((n ^ (n >> 1)) << ls), lo ^ hi);
-    }
-}
+// A pass: 2^nb classes; class p has index XOR of cin[j] (cout[j]) over the bits of p in the table read (written), and
+// its value i of the first (last) stage sits at that index ^ zin[i] (zout[i]).
+struct GradPass {
+    int d, nb, ssz[3];
+    uint32_t cin[34], cout[34], zin[32], zout[32];
+    GradStep st[2];
+};
+static_assert(sizeof(GradPass) <= 3500, "a pass goes by value as a kernel parameter");
 
-// The same walk, two consecutive Gray-code cosets per call: f(c0, base0, c1, base1, two), the second only when two.
-template <typename F>
-__device__ __forceinline__ void grid_cosets2(const StepArgs &s, F f) {
-    const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
-    const int ls = __ffsll((long long)nthreads) - 1;
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (s.nk < ls && t >= (1ULL << s.nk)) return;
-    const uint64_t lo = coset_base(s, t);
-    const uint64_t nh = s.nk > ls ? 1ULL << (s.nk - ls) : 1;
-    uint64_t hi = 0;
-    for (uint64_t n = 0; n < nh; n += 2) {
-        if (n) hi ^= s.tk[ls + __ffsll((long long)n) - 1];
-        const bool two = n + 1 < nh;
-        const uint64_t hi1 = two ? hi ^ s.tk[ls] : hi;   // Gray step n -> n + 1 flips high bit 0
-        f(t | ((n ^ (n >> 1)) << ls), lo ^ hi, t | (((n + 1) ^ ((n + 1) >> 1)) << ls), lo ^ hi1, two);
-        hi = hi1;
-    }
-}
-
-__device__ __forceinline__ void step_row(const StepArgs &s, const GradCtx &g, double2 &m0, double2 &m1) {
-    const int b = g.bits[(size_t)(*g.item + (int)blockIdx.y) * (size_t)g.ns + (size_t)s.k];
-    const double *Mk = g.M + (size_t)s.k * 8 + 4 * b;
-    m0 = make_double2(Mk[0], Mk[1]);
-    m1 = make_double2(Mk[2], Mk[3]);
-}
+constexpr int GRAD_THREADS = 128;
+constexpr int GRAD_MAX_VALUES = 64;   // stage values of a class: 64 x 16 B x 128 threads = 128 KB of slots
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 cscale(double s, double2 a) { return make_double2(s * a.x, s * a.y); }
+__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {
+    return make_double2(fma(a.x, b.x, fma(-a.y, b.y, c.x)), fma(a.x, b.y, fma(a.y, b.x, c.y)));
+}
+__device__ __forceinline__ double2 csign(double2 a, int neg) {
+    const int f = neg << 31;
+    return make_double2(__hiloint2double(__double2hiint(a.x) ^ f, __double2loint(a.x)),
+                        __hiloint2double(__double2hiint(a.y) ^ f, __double2loint(a.y)));
+}
 
-__global__ void k_gr_begin(double2 *T, const GradCtx g) { T[blockIdx.y * g.arena] = make_double2(1.0, 0.0); }
+__device__ __forceinline__ void copy16(double2 *dst, const double2 *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Forward step on the T arena: gathers the input table to `gather` ([c][t], if given) and, if `write`, stores the
-// step's outputs in place.  Two cosets per iteration, both cosets' loads first (distinct cosets never share a slot),
-// so a thread has twice the loads in flight (7 % off the sweep); NTQ (the step's offsets) is a template parameter, so
-// the loaded values stay in registers.
-template <int NTQ>
-__global__ void __launch_bounds__(256) k_gr_fwd(const StepArgs s, double2 *__restrict__ T, double2 *__restrict__ gather,
-                                                size_t gather_stride, int write, const GradCtx g) {
+// The classes a thread visits (grid x times block: a power of two, 2^ls threads): p = t | (g << ls) for the Gray codes g
+// of the high bits, so both indices are running values (one XOR each per class).
+struct ClassWalk {
+    uint64_t p, n, count;
+    uint32_t in, out;
+    int ls;
+    __device__ ClassWalk(const GradPass &g) {
+        ls = __ffs((int)(gridDim.x * blockDim.x)) - 1;
+        p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+        n = 0;
+        in = out = 0;
+        count = g.nb > ls ? 1ULL << (g.nb - ls) : p < (1ULL << g.nb) ? 1 : 0;
+        for (int j = 0; j < min(g.nb, ls); j++)
+            if ((p >> j) & 1) { in ^= g.cin[j]; out ^= g.cout[j]; }
+    }
+    __device__ bool more() const { return n < count; }
+    __device__ void next(const GradPass &g) {
+        if (++n >= count) return;
+        const int j = ls + __ffsll((long long)n) - 1;
+        p ^= 1ULL << j;
+        in ^= g.cin[j];
+        out ^= g.cout[j];
+    }
+};
+
+struct MRow {
     double2 m0, m1;
-    step_row(s, g, m0, m1);
-    T += blockIdx.y * g.arena;
-    if (gather) gather += blockIdx.y * gather_stride;
-    auto one = [&](uint64_t c, uint64_t base, const double2 (&v)[NTQ]) {
-        const int pc = __popcll(c & s.rhoc) & 1;
-        double2 o0 = make_double2(0, 0), o1 = make_double2(0, 0);   // scalars: no runtime-indexed arrays
-#pragma unroll
-        for (int t = 0; t < NTQ; t++) {
-            if (gather) gather[c * (uint64_t)NTQ + (uint64_t)t] = v[t];
-            const double2 a = cmul(m0, v[t]), b = cscale((pc ^ s.par[t]) ? -1.0 : 1.0, cmul(m1, v[t]));
-            if (s.tau0[t]) o1 = cadd(o1, a); else o0 = cadd(o0, a);
-            if (s.tau1[t]) o1 = cadd(o1, b); else o0 = cadd(o0, b);
-        }
-        if (!write) return;
-        T[base] = o0;
-        if (s.m == 2) T[base ^ s.g] = o1;
-    };
-    grid_cosets2(s, [&](uint64_t c0, uint64_t b0, uint64_t c1, uint64_t b1, bool two) {
-        double2 v0[NTQ], v1[NTQ];
-#pragma unroll
-        for (int t = 0; t < NTQ; t++) {
-            v0[t] = T[b0 ^ s.tq[t]];
-            v1[t] = two ? T[b1 ^ s.tq[t]] : make_double2(0, 0);
-        }
-        one(c0, b0, v0);
-        if (two) one(c1, b1, v1);
-    });
+};
+__device__ __forceinline__ MRow step_row(const GradStep &s, const GradCtx &g) {
+    const int b = g.bits[(size_t)(*g.item + (int)blockIdx.y) * (size_t)g.ns + (size_t)s.k];
+    const double *Mk = g.M + (size_t)s.k * 8 + 4 * b;
+    return MRow{make_double2(Mk[0], Mk[1]), make_double2(Mk[2], Mk[3])};
 }
 
-// Restore a checkpoint: the compact table [c][t] back to its arena slots.
-__global__ void __launch_bounds__(256) k_gr_scatter(const StepArgs s, const double2 *__restrict__ src, size_t src_stride,
-                                                    double2 *__restrict__ T, const GradCtx g) {
-    src += blockIdx.y * src_stride;
-    T += blockIdx.y * g.arena;
-    grid_cosets(s, [&](uint64_t c, uint64_t base) {
-        for (int t = 0; t < s.ntq; t++) T[base ^ s.tq[t]] = src[c * (uint64_t)s.ntq + (uint64_t)t];
-    });
+// This thread's slot i.
+__device__ __forceinline__ double2 &slot(double2 *sh, int i) { return sh[i * GRAD_THREADS + (int)threadIdx.x]; }
+
+// Coset sums of a member: X[tau] of the x = 0 terms, Z[tau] of the x = 1 terms with their term signs.
+template <int NTQ>
+__device__ __forceinline__ void member_sums(const GradStep &s, const double2 (&v)[NTQ], double2 (&X)[2], double2 (&Z)[2]) {
+    X[0] = X[1] = Z[0] = Z[1] = make_double2(0, 0);
+#pragma unroll
+    for (int t = 0; t < NTQ; t++) {
+        if ((s.tau0 >> t) & 1) X[1] = cadd(X[1], v[t]);
+        else X[0] = cadd(X[0], v[t]);
+        const double2 w = csign(v[t], (s.par >> t) & 1);
+        if ((s.tau1 >> t) & 1) Z[1] = cadd(Z[1], w);
+        else Z[0] = cadd(Z[0], w);
+    }
 }
 
-// End of the forward sweep: Z = T[0]; lambda_ns = 1.
-__global__ void k_gr_final(const double2 *T, double2 *Lam, double2 *z_out, const GradCtx g) {
-    z_out[*g.item + (int)blockIdx.y] = T[blockIdx.y * g.arena];
-    Lam[blockIdx.y * g.arena] = make_double2(1.0, 0.0);
+// A step forward on one class: values in slots a.. to f(index, value).
+template <int NTQ, typename F>
+__device__ __forceinline__ void class_fwd(const GradStep &s, const MRow &m, double2 *sh, int a, int cpar, F f) {
+    for (int j = 0; j < s.nmem; j++) {
+        double2 v[NTQ], X[2], Z[2];
+#pragma unroll
+        for (int t = 0; t < NTQ; t++) v[t] = slot(sh, a + s.in[j][t]);
+        member_sums<NTQ>(s, v, X, Z);
+        const double2 m1 = csign(m.m1, (cpar ^ s.mpar[j]) & 1);
+        f(s.out[j][0], cfma(m.m0, X[0], cmul(m1, Z[0])));
+        if (s.m == 2) f(s.out[j][1], cfma(m.m0, X[1], cmul(m1, Z[1])));
+    }
+}
+
+// A step in reverse on one class: inputs in slots a.., lambda of its outputs in slots l..; lambda of its inputs to
+// f(index, value), the sums for dZ/dM to acc.
+template <int NTQ, typename F>
+__device__ __forceinline__ void class_bwd(const GradStep &s, const MRow &m, double2 *sh, int a, int l, int cpar,
+                                          double2 (&acc)[2], F f) {
+    for (int j = 0; j < s.nmem; j++) {
+        double2 v[NTQ], X[2], Z[2];
+#pragma unroll
+        for (int t = 0; t < NTQ; t++) v[t] = slot(sh, a + s.in[j][t]);
+        const double2 l0 = slot(sh, l + s.out[j][0]);
+        const double2 l1 = s.m == 2 ? slot(sh, l + s.out[j][1]) : make_double2(0, 0);
+        member_sums<NTQ>(s, v, X, Z);
+        const int cs = (cpar ^ s.mpar[j]) & 1;
+        acc[0] = cfma(l0, X[0], cfma(l1, X[1], acc[0]));
+        acc[1] = cadd(acc[1], csign(cfma(l0, Z[0], cmul(l1, Z[1])), cs));
+        const double2 m1 = csign(m.m1, cs);
+        const double2 a0 = cmul(m.m0, l0), a1 = cmul(m.m0, l1), b0 = cmul(m1, l0), b1 = cmul(m1, l1);
+#pragma unroll
+        for (int t = 0; t < NTQ; t++) {
+            const double2 x = (s.tau0 >> t) & 1 ? a1 : a0, y = (s.tau1 >> t) & 1 ? b1 : b0;
+            f(s.in[j][t], cadd(x, csign(y, (s.par >> t) & 1)));
+        }
+    }
+}
+
+template <typename F>
+__device__ __forceinline__ void class_fwd_any(const GradStep &s, const MRow &m, double2 *sh, int a, int cpar, F f) {
+    if (s.ntq == 4) class_fwd<4>(s, m, sh, a, cpar, f);
+    else if (s.ntq == 2) class_fwd<2>(s, m, sh, a, cpar, f);
+    else class_fwd<1>(s, m, sh, a, cpar, f);
+}
+template <typename F>
+__device__ __forceinline__ void class_bwd_any(const GradStep &s, const MRow &m, double2 *sh, int a, int l, int cpar,
+                                              double2 (&acc)[2], F f) {
+    if (s.ntq == 4) class_bwd<4>(s, m, sh, a, l, cpar, acc, f);
+    else if (s.ntq == 2) class_bwd<2>(s, m, sh, a, l, cpar, acc, f);
+    else class_bwd<1>(s, m, sh, a, l, cpar, acc, f);
+}
+
+__global__ void k_gr_begin(double2 *T, size_t stride) { T[blockIdx.y * stride] = make_double2(1.0, 0.0); }
+
+// Forward pass: the table `in` to the table `out` (strides: entries between two strings' tables).
+template <int D>
+__global__ void __launch_bounds__(GRAD_THREADS) k_gr_fwd(const GradPass g, const double2 *__restrict__ in, size_t in_stride,
+                                                         double2 *__restrict__ out, size_t out_stride, const GradCtx c) {
+    extern __shared__ __align__(16) double2 sh[];
+    const MRow ma = step_row(g.st[0], c), mb = step_row(g.st[D - 1], c);
+    in += blockIdx.y * in_stride;
+    out += blockIdx.y * out_stride;
+    ClassWalk w(g);
+    if (w.more())
+        for (int i = 0; i < g.ssz[0]; i++) copy16(&slot(sh, i), in + (w.in ^ g.zin[i]));
+    while (w.more()) {
+        copies_landed();
+        const uint64_t p = w.p;
+        const uint32_t o = w.out;
+        if (D == 1) {
+            class_fwd_any(g.st[0], ma, sh, 0, __popcll(p & g.st[0].lam), [&](int i, double2 v) { out[o ^ g.zout[i]] = v; });
+        } else {
+            const int s1 = g.ssz[0];
+            class_fwd_any(g.st[0], ma, sh, 0, __popcll(p & g.st[0].lam), [&](int i, double2 v) { slot(sh, s1 + i) = v; });
+        }
+        w.next(g);   // the first stage is done: the next class's values arrive while the second step runs
+        if (w.more())
+            for (int i = 0; i < g.ssz[0]; i++) copy16(&slot(sh, i), in + (w.in ^ g.zin[i]));
+        if (D == 2)
+            class_fwd_any(g.st[1], mb, sh, g.ssz[0], __popcll(p & g.st[D - 1].lam),
+                          [&](int i, double2 v) { out[o ^ g.zout[i]] = v; });
+    }
+}
+
+// End of the forward sweep: Z = T_ns[0]; lambda_ns = 1.
+__global__ void k_gr_final(const double2 *T, size_t t_stride, double2 *Lam, size_t l_stride, double2 *z_out,
+                           const GradCtx g) {
+    z_out[*g.item + (int)blockIdx.y] = T[blockIdx.y * t_stride];
+    Lam[blockIdx.y * l_stride] = make_double2(1.0, 0.0);
 }
 
 __global__ void k_gr_next(int *item, int bs) { *item += bs; }
 __global__ void k_gr_set_item(int *item, int v) { *item = v; }
 
-// Reverse step: lambda_{k+1} (output slots of the Lam arena) -> lambda_k (input slots, in place), and
-// dZ/dM_k[b_k][x] from the step's input table Tk ([c][t]).  Deterministic reduction: per-block partials, the last
-// block sums them in block order and writes grad[item][k] = (dZ/dm0, dZ/dm1).
-template <int NTQ>
-__global__ void __launch_bounds__(256) k_gr_bwd(const StepArgs s, const double2 *__restrict__ Tk, size_t tk_stride,
-                                                double2 *__restrict__ Lam, const GradCtx g, double *partials,
-                                                unsigned int *counter, double *grad) {
-    double2 m0, m1;
-    step_row(s, g, m0, m1);
-    Tk += blockIdx.y * tk_stride;
-    Lam += blockIdx.y * g.arena;
-    partials += (size_t)blockIdx.y * 4 * (size_t)g.maxgrid;
+// Measured on the width-20 workload (128 strings, loss and gradient): 23.1 -> 9.6 ms a call with both sweeps in two-step
+// passes.  The widest reverse pass moves 1.3 GB in 0.34 ms and is bound by issue (65 % of the slots, 900 instructions per
+// class of four values); five blocks per SM (96 registers, no spills) took 4 % off against four, six and eight spill.
+//
+// Reverse pass: lambda after the pass (`lo`) and the table before it (T) to lambda before it (`li`), and
+// dZ/dM_k[b_k][x] of its steps.  Deterministic reduction: per-block partials, the last block sums them in block order
+// and writes grad[item][k] = (dZ/dm0, dZ/dm1).
+template <int D>
+__global__ void __launch_bounds__(GRAD_THREADS, 5) k_gr_bwd(const GradPass g, const double2 *__restrict__ T, size_t t_stride,
+                                                         const double2 *__restrict__ lo, double2 *__restrict__ li,
+                                                         size_t l_stride, const GradCtx c, double *partials,
+                                                         unsigned int *counter, double *grad) {
+    extern __shared__ __align__(16) double2 sh[];
+    const MRow ma = step_row(g.st[0], c), mb = step_row(g.st[D - 1], c);
+    T += blockIdx.y * t_stride;
+    lo += blockIdx.y * l_stride;
+    li += blockIdx.y * l_stride;
     counter += blockIdx.y;
-    double a[4] = {0, 0, 0, 0};   // dZ/dm0 (re, im), dZ/dm1 (re, im)
-    // two cosets per iteration: both cosets' lambda and input values are read before either writes (a coset writes
-    // only its own slots)
-    auto one = [&](uint64_t c, uint64_t base, double2 lam0, double2 lam1, const double2 (&v)[NTQ]) {
-        const int pc = __popcll(c & s.rhoc) & 1;
+    const int s1 = g.ssz[0], s2 = D == 2 ? s1 + g.ssz[1] : s1, nl = g.ssz[D];   // slots of stage 1, and of lambda after
+    const double2 z = make_double2(0, 0);
+    double2 acc[D][2];
 #pragma unroll
-        for (int t = 0; t < NTQ; t++) {
-            const double sg = (pc ^ s.par[t]) ? -1.0 : 1.0;
-            const double2 la = s.tau0[t] ? lam1 : lam0, lb = cscale(sg, s.tau1[t] ? lam1 : lam0);
-            const double2 p0 = cmul(la, v[t]), p1 = cmul(lb, v[t]);
-            a[0] += p0.x;
-            a[1] += p0.y;
-            a[2] += p1.x;
-            a[3] += p1.y;
-            Lam[base ^ s.tq[t]] = cadd(cmul(m0, la), cmul(m1, lb));
+    for (int s = 0; s < D; s++) acc[s][0] = acc[s][1] = z;
+    for (ClassWalk w(g); w.more(); w.next(g)) {
+        for (int i = 0; i < g.ssz[0]; i++) copy16(&slot(sh, i), T + (w.in ^ g.zin[i]));
+        for (int i = 0; i < nl; i++) copy16(&slot(sh, s2 + i), lo + (w.out ^ g.zout[i]));
+        copies_landed();
+        const int pa = __popcll(w.p & g.st[0].lam);
+        const uint32_t in = w.in;
+        auto store = [&](int i, double2 v) { li[in ^ g.zin[i]] = v; };
+        if (D == 1) {
+            class_bwd_any(g.st[0], ma, sh, 0, s2, pa, acc[0], store);
+        } else {
+            // a stage-1 slot holds the step's input until the member that reads it, then its lambda
+            auto keep = [&](int i, double2 v) { slot(sh, s1 + i) = v; };
+            class_fwd_any(g.st[0], ma, sh, 0, pa, keep);
+            class_bwd_any(g.st[D - 1], mb, sh, s1, s2, __popcll(w.p & g.st[D - 1].lam), acc[D - 1], keep);
+            class_bwd_any(g.st[0], ma, sh, 0, s1, pa, acc[0], store);
         }
-    };
-    grid_cosets2(s, [&](uint64_t c0, uint64_t b0, uint64_t c1, uint64_t b1, bool two) {
-        const double2 z = make_double2(0, 0);
-        const double2 l00 = Lam[b0], l01 = s.m == 2 ? Lam[b0 ^ s.g] : z;
-        const double2 l10 = two ? Lam[b1] : z, l11 = two && s.m == 2 ? Lam[b1 ^ s.g] : z;
-        double2 v0[NTQ], v1[NTQ];
-#pragma unroll
-        for (int t = 0; t < NTQ; t++) {
-            v0[t] = Tk[c0 * (uint64_t)NTQ + (uint64_t)t];
-            v1[t] = two ? Tk[c1 * (uint64_t)NTQ + (uint64_t)t] : z;
-        }
-        one(c0, b0, l00, l01, v0);
-        if (two) one(c1, b1, l10, l11, v1);
-    });
-    __shared__ double red[4][8];
+    }
+    __shared__ double red[4 * D][GRAD_THREADS / 32];
     __shared__ int last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    for (int i = 0; i < 4; i++) a[i] = warp_sum(a[i]);
-    if (lane == 0)
-        for (int i = 0; i < 4; i++) red[i][warp] = a[i];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    partials += (size_t)blockIdx.y * gridDim.x * (4 * D);
+#pragma unroll
+    for (int s = 0; s < D; s++)
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+            const double r = warp_sum(acc[s][x].x), i = warp_sum(acc[s][x].y);
+            if (lane == 0) { red[4 * s + 2 * x][warp] = r; red[4 * s + 2 * x + 1][warp] = i; }
+        }
+    __syncthreads();
+    if (threadIdx.x < 4 * D) {
+        double t = 0;
+        for (int v = 0; v < GRAD_THREADS / 32; v++) t += red[threadIdx.x][v];
+        partials[4 * D * blockIdx.x + threadIdx.x] = t;
+        __threadfence();
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 4; i++) {
-            double t = 0;
-            for (int w = 0; w < nw; w++) t += red[i][w];
-            partials[4 * blockIdx.x + i] = t;
-        }
         __threadfence();
         last = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last || threadIdx.x != 0) return;
+    if (!last || threadIdx.x >= 4 * D) return;
     __threadfence();
-    double t[4] = {0, 0, 0, 0};
-    for (unsigned int b = 0; b < gridDim.x; b++)
-        for (int i = 0; i < 4; i++) t[i] += __ldcg(partials + 4 * b + i);
-    double *out = grad + ((size_t)(*g.item + (int)blockIdx.y) * (size_t)g.ns + (size_t)s.k) * 4;
-    for (int i = 0; i < 4; i++) out[i] = t[i];
-    *counter = 0;
+    double t = 0;
+    for (unsigned int b = 0; b < gridDim.x; b++) t += __ldcg(partials + 4 * D * b + threadIdx.x);
+    const GradStep &s = g.st[threadIdx.x >> 2 & (D - 1)];
+    grad[((size_t)(*c.item + (int)blockIdx.y) * (size_t)c.ns + (size_t)s.k) * 4 + (threadIdx.x & 3)] = t;
+    if (threadIdx.x == 0) *counter = 0;
 }
 
-// Blocks per launch: at most GSB_GRAD_GRID_MUL x maxgrid (8 per SM) over the launch's bs strings together.  Every
-// block ends in a block reduction and an atomic (the reverse step) or is short-lived (forward), so a thread should
-// walk several cosets: with the x extent sized per string alone, a launch of 32 strings made 32768 blocks of one or two
-// cosets per thread, and the sweep ran 28 % slower than with 4 (timed 1, 2, 4, 8: 0.400, 0.370, 0.364, 0.383 s for
-// 2048 strings at width 20, against 0.507 s uncapped).
-#ifndef GSB_GRAD_GRID_MUL
-#define GSB_GRAD_GRID_MUL 4
-#endif
+// Index of an address in the compact table before step k (HStep columns): XOR-linear, c | t << nk with the offsets in
+// ascending order (their index is linear too: the three nonzero ones XOR to 0).
+class TableIndex {
+    struct Row {
+        uint64_t v;
+        uint32_t i;
+    };
+    std::vector<Row> rows;   // each reduced by the ones before it
+
+public:
+    explicit TableIndex(const HStep *s) {
+        if (!s) return;      // the table after the last step: one entry
+        for (int j = 0; j < s->nk; j++) add(s->tk[(size_t)j], 1u << j);
+        if (s->tqs.size() > 1) add(s->tqs[1], 1u << s->nk);
+        if (s->tqs.size() > 2) add(s->tqs[2], 2u << s->nk);
+    }
+    void add(uint64_t v, uint32_t i) {
+        reduce(v, i);
+        if (v) rows.push_back({v, i});
+    }
+    void reduce(uint64_t &v, uint32_t &i) const {
+        for (const Row &r : rows)
+            if (v >> (63 - __builtin_clzll(r.v)) & 1) { v ^= r.v; i ^= r.i; }
+    }
+    uint32_t operator()(uint64_t v) const {
+        uint32_t i = 0;
+        reduce(v, i);
+        return i;
+    }
+};
+
+// The pass of steps gp.k0 .. gp.k0 + gp.d - 1; false when it is too large for the kernels.
+static bool make_pass(const HPlan &p, const GroupPlan &gp, GradPass &g) {
+    memset(&g, 0, sizeof g);
+    int values = 0;
+    for (int s = 0; s <= gp.d; s++) values += g.ssz[s] = gp.stage_size[s];
+    if (values > GRAD_MAX_VALUES || gp.nb > 32) return false;
+    g.d = gp.d;
+    g.nb = gp.nb;
+    const int k1 = gp.k0 + gp.d;
+    const TableIndex before(&p.st[(size_t)gp.k0]), after(k1 < p.ns ? &p.st[(size_t)k1] : nullptr);
+    std::vector<uint64_t> cols;
+    for (int j = 0; j < gp.L; j++) cols.push_back(1ULL << j);
+    cols.insert(cols.end(), gp.bhi.begin(), gp.bhi.end());
+    for (int j = 0; j < gp.nb; j++) {
+        g.cin[j] = before(cols[(size_t)j]);
+        g.cout[j] = after(cols[(size_t)j]);
+    }
+    for (int i = 0; i < gp.stage_size[0]; i++) g.zin[i] = before(gp.z_in[(size_t)i]);
+    for (int i = 0; i < gp.stage_size[gp.d]; i++) g.zout[i] = after(gp.z_out[(size_t)i]);
+    for (int s = 0; s < gp.d; s++) {
+        const HStep &hs = p.st[(size_t)(gp.k0 + s)];
+        const GroupPlan::Step &q = gp.step[s];
+        GradStep &a = g.st[s];
+        a.k = gp.k0 + s;
+        a.nmem = q.nmem;
+        a.ntq = q.ntq;
+        a.m = q.m;
+        for (int t = 0; t < q.ntq; t++) {
+            a.tau0 |= hs.tau0[t] << t;
+            a.tau1 |= hs.tau1[t] << t;
+            a.par |= hs.par[t] << t;
+        }
+        for (int j = 0; j < gp.nb; j++)
+            a.lam |= (uint64_t)(__builtin_popcountll(cols[(size_t)j] & q.lambda) & 1) << j;
+        for (int j = 0; j < q.nmem; j++) {
+            for (int t = 0; t < q.ntq; t++) a.in[j][t] = (unsigned char)q.in_idx[j][t];
+            for (int tau = 0; tau < q.m; tau++) a.out[j][tau] = (unsigned char)q.out_idx[j][tau];
+            a.mpar[j] = (unsigned char)q.mpar[j];
+        }
+    }
+    return true;
+}
 
 struct GradEngine {
     HPlan plan;
-    int dev = 0, sms = 0, every = 4, cap = 1024, bs = 1;   // cap: strings per host batch, a multiple of bs
-    std::vector<StepArgs> args;
-    std::vector<size_t> ckpt_off;      // offset (entries) of step k's checkpoint in a string's checkpoint slot
-    size_t arena = 0, ckpt_n = 0;      // entries per string: arena, checkpoints
-    double2 *T = nullptr, *Lam = nullptr, *d_ckpt = nullptr, *d_seg = nullptr;
-    size_t seg_stride = 0;             // entries per segment table
+    int dev = 0, sms = 0, cap = 1024, bs = 1;   // cap: strings per host batch, a multiple of bs
+    std::vector<GradPass> passes;
+    std::vector<size_t> entries;       // of the table before pass i; the last one (after all passes) is 1
+    int q = 1;                         // every q-th pass keeps its table
+    std::vector<size_t> kept_off;      // offset (entries) of pass i's kept table in a string's slot (i % q == 0)
+    size_t kept_n = 0, seg_stride = 0; // entries per string: kept tables; one table of a segment, or a lambda table
+    double2 *d_kept = nullptr, *d_seg = nullptr, *d_pair[2] = {nullptr, nullptr};
     double *d_M = nullptr, *partials = nullptr, *d_grad = nullptr;
     double2 *d_z = nullptr;
     int8_t *d_bits = nullptr;
@@ -251,17 +398,16 @@ struct GradEngine {
     unsigned int *d_counter = nullptr;
     cudaStream_t stream = nullptr;
     cudaGraphExec_t graph = nullptr;
-    int maxgrid = 1;
 
     ~GradEngine() {
         int prev = 0;
         cudaGetDevice(&prev);
         cudaSetDevice(dev);
         if (graph) cudaGraphExecDestroy(graph);
-        cudaFree(T);
-        cudaFree(Lam);
-        cudaFree(d_ckpt);
+        cudaFree(d_kept);
         cudaFree(d_seg);
+        cudaFree(d_pair[0]);
+        cudaFree(d_pair[1]);
         cudaFree(d_M);
         cudaFree(partials);
         cudaFree(d_grad);
@@ -273,57 +419,94 @@ struct GradEngine {
         cudaSetDevice(prev);
     }
 
-    // a power of two of blocks per string (grid_cosets splits a coset index into thread and Gray-walk bits), with
-    // the launch's bs strings together at most GSB_GRAD_GRID_MUL * maxgrid blocks
-    dim3 grid_of(const StepArgs &s) const {
-        const uint64_t N = 1ULL << s.nk;
-        const uint64_t cap = std::max<uint64_t>(1, (uint64_t)GSB_GRAD_GRID_MUL * (uint64_t)maxgrid / (uint64_t)bs);
-        uint64_t want = std::max<uint64_t>(1, std::min<uint64_t>((N + 255) / 256, std::min<uint64_t>(cap, maxgrid))), gx = 1;
+    // Kept tables for an interval of n passes; returns the device bytes a string needs.
+    size_t lay_out(int n) {
+        q = n;
+        kept_off.assign(passes.size(), 0);
+        kept_n = 0;
+        for (size_t i = 0; i < passes.size(); i += (size_t)n) {
+            kept_off[i] = kept_n;
+            kept_n += entries[i];
+        }
+        return 16 * (kept_n + (size_t)(n - 1) * seg_stride + 2 * seg_stride) + (size_t)max_blocks() * 8 * sizeof(double);
+    }
+    // Blocks of a launch over all its strings: four rounds of four per SM; every block ends in a block reduction and an
+    // atomic, so a thread walks several classes.
+    int max_blocks() const { return sms * 16; }
+    dim3 grid_of(const GradPass &g) const {
+        const uint64_t want = std::min<uint64_t>(((1ULL << g.nb) + GRAD_THREADS - 1) / GRAD_THREADS,
+                                                 std::max(1, max_blocks() / bs));
+        uint64_t gx = 1;   // a power of two: ClassWalk splits a class index into thread and Gray-walk bits
         while (gx * 2 <= want) gx *= 2;
         return dim3((unsigned)gx, (unsigned)bs);
     }
-    GradCtx ctx() const { return GradCtx{d_M, d_bits, d_item, plan.ns, maxgrid, arena}; }
-    size_t seg_per_string() const { return (size_t)std::max(0, every - 1) * seg_stride; }
-    double2 *seg(int pos) const { return d_seg + (size_t)(pos - 1) * seg_stride; }   // pos = 1 .. every-1 (slot 0)
+    GradCtx ctx() const { return GradCtx{d_M, d_bits, d_item, plan.ns}; }
 
-    // forward / reverse step launches, instantiated for the step's number of coset offsets
-    void fwd(const StepArgs &s, double2 *gather, size_t gstride, int write, const GradCtx &g) {
-        if (s.ntq == 1) k_gr_fwd<1><<<grid_of(s), 256, 0, stream>>>(s, T, gather, gstride, write, g);
-        else if (s.ntq == 2) k_gr_fwd<2><<<grid_of(s), 256, 0, stream>>>(s, T, gather, gstride, write, g);
-        else k_gr_fwd<4><<<grid_of(s), 256, 0, stream>>>(s, T, gather, gstride, write, g);
+    // Where the table before pass i lives while `seg0` is the first pass of the segment being worked on.
+    double2 *table(size_t i, size_t *stride) const {
+        if (i % (size_t)q == 0) {
+            *stride = kept_n;
+            return d_kept + kept_off[i];
+        }
+        *stride = (size_t)(q - 1) * seg_stride;
+        return d_seg + (i % (size_t)q - 1) * seg_stride;
     }
-    void bwd(const StepArgs &s, const double2 *tk, size_t tstride, const GradCtx &g) {
-        if (s.ntq == 1) k_gr_bwd<1><<<grid_of(s), 256, 0, stream>>>(s, tk, tstride, Lam, g, partials, d_counter, d_grad);
-        else if (s.ntq == 2) k_gr_bwd<2><<<grid_of(s), 256, 0, stream>>>(s, tk, tstride, Lam, g, partials, d_counter, d_grad);
-        else k_gr_bwd<4><<<grid_of(s), 256, 0, stream>>>(s, tk, tstride, Lam, g, partials, d_counter, d_grad);
+    cudaError_t fwd(size_t i, const double2 *in, size_t is, double2 *out, size_t os) {
+        const GradPass &g = passes[i];
+        const size_t sm = (size_t)(g.ssz[0] + (g.d == 2 ? g.ssz[1] : 0)) * 16 * GRAD_THREADS;
+        if (g.d == 2) k_gr_fwd<2><<<grid_of(g), GRAD_THREADS, sm, stream>>>(g, in, is, out, os, ctx());
+        else k_gr_fwd<1><<<grid_of(g), GRAD_THREADS, sm, stream>>>(g, in, is, out, os, ctx());
+        return cudaGetLastError();
+    }
+    cudaError_t bwd(size_t i, const double2 *T, size_t ts, const double2 *lo, double2 *li) {
+        const GradPass &g = passes[i];
+        const size_t sm = (size_t)(g.ssz[0] + g.ssz[1] + (g.d == 2 ? g.ssz[2] : 0)) * 16 * GRAD_THREADS;
+        if (g.d == 2)
+            k_gr_bwd<2><<<grid_of(g), GRAD_THREADS, sm, stream>>>(g, T, ts, lo, li, seg_stride, ctx(), partials, d_counter,
+                                                                  d_grad);
+        else
+            k_gr_bwd<1><<<grid_of(g), GRAD_THREADS, sm, stream>>>(g, T, ts, lo, li, seg_stride, ctx(), partials, d_counter,
+                                                                  d_grad);
+        return cudaGetLastError();
     }
 
     // The sequence of one launch of bs strings (captured once as a graph).
     cudaError_t enqueue() {
-        const int ns = plan.ns;
-        const GradCtx g = ctx();
         const dim3 one(1, (unsigned)bs);
-        k_gr_begin<<<one, 1, 0, stream>>>(T, g);
-        for (int k = 0; k < ns; k++) {
-            const StepArgs &s = args[(size_t)k];
-            fwd(s, k % every == 0 ? d_ckpt + ckpt_off[(size_t)k] : nullptr, ckpt_n, 1, g);
+        const size_t np = passes.size();
+        k_gr_begin<<<one, 1, 0, stream>>>(d_kept, kept_n);
+        cudaError_t e = cudaGetLastError();
+        // forward: tables that are not kept pass through the pair that holds lambda later
+        const double2 *in = d_kept;
+        size_t is = kept_n;
+        for (size_t i = 0; i < np && e == cudaSuccess; i++) {
+            double2 *out = d_pair[i & 1];
+            size_t os = seg_stride;
+            if (i + 1 < np && (i + 1) % (size_t)q == 0) out = table(i + 1, &os);
+            e = fwd(i, in, is, out, os);
+            in = out;
+            is = os;
         }
-        k_gr_final<<<one, 1, 0, stream>>>(T, Lam, d_z, g);
-        for (int c = ((ns - 1) / every) * every; c >= 0; c -= every) {
-            const int e = std::min(c + every, ns);
-            const StepArgs &sc = args[(size_t)c];
-            k_gr_scatter<<<grid_of(sc), 256, 0, stream>>>(sc, d_ckpt + ckpt_off[(size_t)c], ckpt_n, T, g);
-            for (int j = c; j < e; j++) {   // recompute: gather T_j (j > c), write T_{j+1} (j < e - 1)
-                if (j == c && e - 1 == c) break;
-                const StepArgs &s = args[(size_t)j];
-                fwd(s, j == c ? nullptr : seg(j - c), seg_per_string(), j < e - 1 ? 1 : 0, g);
+        if (e != cudaSuccess) return e;
+        int cur = in == d_pair[0] ? 1 : 0;   // lambda starts in the buffer that does not hold T_ns
+        k_gr_final<<<one, 1, 0, stream>>>(in, is, d_pair[cur], seg_stride, d_z, ctx());
+        e = cudaGetLastError();
+        for (size_t c = (np - 1) / (size_t)q * (size_t)q; e == cudaSuccess; c -= (size_t)q) {
+            const size_t end = std::min(c + (size_t)q, np);
+            for (size_t i = c; i + 1 < end && e == cudaSuccess; i++) {   // the segment's tables again
+                size_t a, b;
+                const double2 *src = table(i, &a);
+                double2 *dst = table(i + 1, &b);
+                e = fwd(i, src, a, dst, b);
             }
-            for (int j = e - 1; j >= c; j--) {
-                const StepArgs &s = args[(size_t)j];
-                const double2 *tk = j == c ? d_ckpt + ckpt_off[(size_t)c] : seg(j - c);
-                bwd(s, tk, j == c ? ckpt_n : seg_per_string(), g);
+            for (size_t i = end; i-- > c && e == cudaSuccess; cur ^= 1) {
+                size_t a;
+                const double2 *T = table(i, &a);
+                e = bwd(i, T, a, d_pair[cur], d_pair[cur ^ 1]);
             }
+            if (c == 0) break;
         }
+        if (e != cudaSuccess) return e;
         k_gr_next<<<1, 1, 0, stream>>>(d_item, bs);
         return cudaGetLastError();
     }
@@ -372,7 +555,6 @@ int gsb_grad_open_text(const char *text, size_t len, int device, int every, gsb_
         return fail(GSB_E_USAGE, "the last step must leave a single entry (nk = 0, m = 1)");
     }
     E.dev = device;
-    E.every = every;
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(device);
@@ -381,68 +563,52 @@ int gsb_grad_open_text(const char *text, size_t len, int device, int every, gsb_
         ~Restore() { cudaSetDevice(p); }
     } restore{prev};
     cudaDeviceGetAttribute(&E.sms, cudaDevAttrMultiProcessorCount, device);
-    E.maxgrid = std::max(1, E.sms * 8);
-    E.args.resize((size_t)p.ns);
-    E.ckpt_off.assign((size_t)p.ns, 0);
-    size_t ck = 0, maxr = 0;
-    for (int k = 0; k < p.ns; k++) {
-        const HStep &s = p.st[(size_t)k];
-        StepArgs a;
-        memset(&a, 0, sizeof a);
-        for (int j = 0; j < s.nk; j++) a.tk[j] = s.tk[(size_t)j];
-        a.ntq = (int)s.tqs.size();
-        for (int i = 0; i < a.ntq; i++) {
-            a.tq[i] = s.tqs[(size_t)i];
-            a.tau0[i] = s.tau0[i];
-            a.tau1[i] = s.tau1[i];
-            a.par[i] = s.par[i];
+    for (int k = 0; k < p.ns;) {
+        GradPass g;
+        GroupPlan gp;
+        int d = 2;
+        while (d > 0 && !(plan_group(p, k, d, 0, 30, gp) && make_pass(p, gp, g))) d--;
+        if (d == 0) {
+            delete h;
+            return fail(GSB_E_PLAN_LAYOUT, "step " + std::to_string(k) + " does not fit a pass of the adjoint sweep");
         }
-        a.g = s.m == 2 ? s.g : 0;
-        a.rhoc = s.rhoc;
-        a.nk = s.nk;
-        a.k = k;
-        a.m = s.m;
-        E.args[(size_t)k] = a;
-        const size_t entries = ((size_t)1 << s.nk) * (size_t)a.ntq;
-        maxr = std::max(maxr, entries);
-        if (k % every == 0) {
-            E.ckpt_off[(size_t)k] = ck;
-            ck += entries;
-        }
+        E.passes.push_back(g);
+        E.entries.push_back(((size_t)1 << p.st[(size_t)k].nk) * p.st[(size_t)k].tqs.size());
+        E.seg_stride = std::max(E.seg_stride, E.entries.back());
+        k += d;
     }
-    E.seg_stride = maxr;
-    E.ckpt_n = ck;
-    const size_t arena = (size_t)1 << p.R;
-    E.arena = arena;
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    // strings per launch: a power of two up to 32, each with its own arenas, checkpoints and segment tables, within
-    // half of the free device memory
-    const size_t per_string = 16 * (2 * arena + ck + (size_t)std::max(0, every - 1) * maxr) +
-                              (size_t)E.maxgrid * 4 * sizeof(double);
+    // The default interval of four steps keeps the table before every pass (half of all tables: less memory than
+    // checkpoints and the segments between them took), longer ones every (every / 4)-th; where that does not fit, fewer.
+    size_t per_string = E.lay_out(std::max(1, every / 4));
+    for (int n = E.q + 1; per_string > free_b / 10 * 9 && n <= (int)E.passes.size(); n++) per_string = E.lay_out(n);
     if (per_string > free_b / 10 * 9) {
         delete h;
-        return fail(GSB_E_ALLOC, "arena, checkpoints and segment tables need " + std::to_string(per_string) +
+        return fail(GSB_E_ALLOC, "kept tables, segment tables and lambda need " + std::to_string(per_string) +
                                      " bytes; the device has " + std::to_string(free_b) + " free");
     }
+    // strings per launch: a power of two up to 32, each with its own tables, within half of the free device memory
     E.bs = 1;
     while (E.bs < 32 && (size_t)(2 * E.bs) * per_string <= free_b / 2) E.bs *= 2;
     const size_t bs = (size_t)E.bs;
     cudaError_t e = cudaStreamCreateWithFlags(&E.stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&E.T, bs * arena * 16);
-    if (e == cudaSuccess) e = cudaMalloc(&E.Lam, bs * arena * 16);
-    if (e == cudaSuccess) e = cudaMalloc(&E.d_ckpt, bs * std::max<size_t>(ck, 1) * 16);
-    if (e == cudaSuccess) e = cudaMalloc(&E.d_seg, bs * std::max<size_t>(E.seg_per_string(), 1) * 16);
+    if (e == cudaSuccess) e = cudaMalloc(&E.d_kept, bs * E.kept_n * 16);
+    if (e == cudaSuccess && E.q > 1) e = cudaMalloc(&E.d_seg, bs * (size_t)(E.q - 1) * E.seg_stride * 16);
+    for (auto &b : E.d_pair)
+        if (e == cudaSuccess) e = cudaMalloc(&b, bs * E.seg_stride * 16);
     if (e == cudaSuccess) e = cudaMalloc(&E.d_M, (size_t)p.ns * 8 * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&E.partials, bs * (size_t)E.maxgrid * 4 * sizeof(double));
+    if (e == cudaSuccess) e = cudaMalloc(&E.partials, std::max<size_t>((size_t)E.max_blocks(), bs) * 8 * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&E.d_grad, (size_t)E.cap * (size_t)p.ns * 4 * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&E.d_z, (size_t)E.cap * sizeof(double2));
     if (e == cudaSuccess) e = cudaMalloc(&E.d_bits, (size_t)E.cap * (size_t)p.ns);
     if (e == cudaSuccess) e = cudaMalloc(&E.d_item, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&E.d_counter, bs * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMemsetAsync(E.d_counter, 0, bs * sizeof(unsigned int), E.stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(E.T, 0, bs * arena * 16, E.stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(E.Lam, 0, bs * arena * 16, E.stream);
+    const int most = GRAD_MAX_VALUES * 16 * GRAD_THREADS;   // shared memory of the largest pass
+    for (const void *f : {(const void *)k_gr_fwd<1>, (const void *)k_gr_fwd<2>, (const void *)k_gr_bwd<1>,
+                          (const void *)k_gr_bwd<2>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e == cudaSuccess) e = cudaStreamSynchronize(E.stream);
     if (e != cudaSuccess) {
         delete h;

@@ -206,8 +206,10 @@ int gsb_dp_extend_static(int r, int rn, uint64_t rho, uint64_t pivmask, int nker
 
 /* ---- adjoint sweep: gradients of log Pr(b) with respect to the step matrices (complex128) ----
  * No counterpart in the reference (it has no differentiation).  The plan text is the in-place plan (its own M
- * values are ignored: every run takes the matrices).  `every` is the checkpoint interval in steps; the segment
- * between two checkpoints is recomputed once during the reverse sweep. */
+ * values are ignored: every run takes the matrices).  `every` is the checkpoint interval in steps: up to 7
+ * (the default is 4) the table before every pass of two steps is kept, from 8 on the one before every (every / 4)-th pass,
+ * and the tables between two kept ones are computed again during the reverse sweep; fewer are kept where memory is
+ * short. */
 typedef struct gsb_grad gsb_grad;
 int gsb_grad_open_text(const char *plan_text, size_t len, int device, int every, gsb_grad **out);
 int gsb_grad_close(gsb_grad *g);
