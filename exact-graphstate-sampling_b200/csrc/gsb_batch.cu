@@ -5,15 +5,21 @@
 // resumes from it through steps [K_i, ns_i): one log2 Pr per (prefix, suffix) string.  Strings that share a prefix
 // share its DP work (the reference's prefix / resume, gsamp2.cpp:162-208, done in memory).
 //
-// A work item is (instance, prefix).  Items sit in two queues, each sorted by decreasing cost: wide instances are
-// run by a whole CTA ("block team"), narrow ones (R <= small_R) by one warp ("warp team").  The kernel is
-// persistent: every CTA first takes block-team items from the first queue, then each of its warps takes warp-team
-// items from the second, with one atomic per item.  A team owns an arena of 2^R entries and a snapshot buffer in its
-// slot, so a whole item runs without any grid-wide synchronisation: a step is a strided loop of the team over the
-// step's cosets (each coset reads and writes only its own slots, gsamp2.cpp:32-38 and 59-66), then a team reduction
-// of the written norm; the one-pass chain logic (power-of-two rescaling, gsamp2.cpp:59-70) runs redundantly in every
-// thread of the team.  Block size, the narrow-width threshold and CTAs per SM are chosen by an autotuner that times
-// the actual batch; each shape's launch is captured once as a CUDA graph (queue reset + kernel).
+// A work item is (instance, prefix).  Items sit in three queues, each sorted by decreasing cost: the widest instances are
+// run by a cluster of CTAs ("cluster team"), wide ones by a CTA ("block team"), narrow ones (R <= small_R) by one warp
+// ("warp team").  The kernel is persistent: every cluster first takes cluster items, then each of its CTAs block items,
+// then each warp warp items, with one atomic per item.  A team owns an arena of 2^R entries and a second table of the
+// same size in its slot, so a whole item runs without any grid-wide synchronisation.
+//
+// An item's steps run in passes of up to three (gsb_fuse.h), which read and write the table once: a thread takes a few
+// classes at a time through the pass's steps, and their values between two steps sit in shared-memory slots of its own.
+// Each step's code is compiled for its dataflow shape and member count (step_chunk).  The last pass of the prefix writes the
+// second table and the first pass of every suffix reads it, so the table that the suffixes share is neither saved nor
+// restored.  After a pass the team sums the written norm; the one-pass chain logic (power-of-two rescaling,
+// gsamp2.cpp:59-70) runs redundantly in every thread of the team.
+// Block size, the narrow-width threshold and CTAs per SM are chosen by an autotuner that times the actual batch; each
+// shape's launch is captured once as a CUDA graph (queue reset + kernel).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -21,59 +27,92 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <thread>
 #include <tuple>
 #include <vector>
 
 #include "gsb.h"
 #include "gsb_common.h"
+#include "gsb_fuse.h"
 #include "gsb_plan.h"
 #include "gsb_step.h"
 
 namespace gsb {
 
+namespace cg = cooperative_groups;
+
+// Shape of a step's dataflow: with m = 2 and every x = 1 term in the other output than its offset's x = 0 term, the host
+// orders the offsets so that the x = 0 terms of the first NTQ - H go to output 0 and those of the last H to output 1
+// (relabelling the outputs where that makes H <= NTQ / 2).  BK_ANY: everything else, with runtime tables.
+enum { BK_ANY = 0, BK_1_0, BK_2_0, BK_2_1, BK_4_0, BK_4_1, BK_4_2 };
+
+// One step inside a pass.  Every stage's values are numbered so that member j reads values ntq j + t; out[j][tau]: the
+// number of its outputs in the next stage (m j + tau in the last one).  Class sign: parity(class & lam) ^ bit j of mpar.
 struct BStep {
-    uint64_t g, rhoc, tq[4];
     double M[8];             // M[b][x] (re, im)
-    int nk, ntq, m, tk_off;
-    int tau0[4], tau1[4], par[4];
+    uint32_t lam, mpar;
+    int kind, nmem, ntq, m;
+    int tau0, tau1, par;     // bit t: offset t's x = 0 / x = 1 output, x = 1 sign
+    unsigned char out[16][2];
+    int pad;
 };
+
+// A pass of d steps: class p has base address XOR of col[j] over the bits of p; its value i of the first (last) stage
+// sits at base ^ zin[i] (zout[i]).  mid[s]: values of the stage after step s (s < d - 1), chunk: classes taken at a time.
+struct alignas(16) BPass {
+    int d, nb, chunk, mid[2];
+    uint32_t col[24], zin[32], zout[32];
+    BStep st[FUSE_MAX_STEPS];
+};
+static_assert(sizeof(BPass) % 16 == 0, "descriptors are copied in 16-byte words");
+// Slots of a thread: the values between two steps of a chunk's classes.  More classes per chunk spread a step's
+// descriptor loads over more work, fewer leave room for more CTAs: 512 instances of widths 7-20 in complex64 took 22.7,
+// 21.8 and 41 ms at 128, 256 and 512 B.
+constexpr int BATCH_SLOT_BYTES = 256;
+constexpr int BATCH_CLUSTER = 8;      // CTAs of a cluster team
+constexpr int BATCH_MAX_BLOCK = 512;
 
 struct BInst {
     int ns, R, K, n;
-    int step_off;            // first BStep
+    int pass_off, npass[2];  // first pass; passes of the prefix, of a suffix
     int64_t pre_off;         // prefix bits: [npre][K]
     int64_t suf_off;         // suffix bits: [npre][nsuf][ns - K]
     int64_t out_off;         // log2 Pr: [npre][nsuf]
 };
 
 struct BatchArgs {
-    const BStep *steps;
-    const uint64_t *tk;
+    const BPass *passes;
     const BInst *inst;
-    const int *items_big, *items_small;   // item = inst * npre + prefix
-    int n_big, n_small, npre, nsuf;
+    const int *items_wide, *items_big, *items_small;   // item = inst * npre + prefix
+    int n_wide, n_big, n_small, npre, nsuf;
     const int8_t *pre_bits, *suf_bits;
     double *log2p;
-    unsigned int *queues;    // [0] block-team queue, [1] warp-team queue
-    void *big_arena;         // per CTA: arena + snapshot of 2^big_R entries each
-    void *small_arena;       // per warp: arena + snapshot of 2^small_R entries each
-    int big_R, small_R;
+    unsigned int *queues;    // [0] block-team queue, [1] warp-team queue, [2] cluster-team queue
+    void *wide_arena;        // per cluster: two tables of 2^wide_R entries
+    void *big_arena;         // per CTA: two tables of 2^big_R entries
+    void *small_arena;       // per warp: two tables of 2^small_R entries
+    int wide_R, big_R, small_R;
 };
 
+// Teams.  sum() gives every thread the same total (fixed order) and is also the barrier between two passes: partial sums
+// alternate between two buffers, so a block needs one __syncthreads and a cluster one cluster barrier per pass.
 struct BlockTeam {
+    int buf = 0;
     __device__ int rank() const { return threadIdx.x; }
     __device__ int size() const { return blockDim.x; }
     __device__ int log2size() const { return __ffs((int)blockDim.x) - 1; }   // blockDim.x: a power of two
+    __device__ int local() const { return threadIdx.x; }     // threads that share this block's descriptor buffers
+    __device__ int nlocal() const { return blockDim.x; }
     __device__ void sync() const { __syncthreads(); }
-    __device__ double sum(double v) const {
-        __shared__ double red[32];
+    __device__ double sum(double v) {
+        __shared__ double red[2][BATCH_MAX_BLOCK / 32];
         v = warp_sum(v);
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-        __syncthreads();
-        if (lane == 0) red[w] = v;
+        const int nw = (int)(blockDim.x >> 5);
+        if ((threadIdx.x & 31) == 0) red[buf][threadIdx.x >> 5] = v;
         __syncthreads();
         double t = 0;
-        for (int i = 0; i < nw; i++) t += red[i];
+        for (int i = 0; i < nw; i++) t += red[buf][i];
+        buf ^= 1;
         return t;
     }
 };
@@ -82,6 +121,8 @@ struct WarpTeam {
     __device__ int rank() const { return threadIdx.x & 31; }
     __device__ int size() const { return 32; }
     __device__ int log2size() const { return 5; }
+    __device__ int local() const { return threadIdx.x & 31; }
+    __device__ int nlocal() const { return 32; }
     __device__ void sync() const { __syncwarp(); }
     __device__ double sum(double v) const {
         __syncwarp();
@@ -89,140 +130,288 @@ struct WarpTeam {
     }
 };
 
+// The CTAs of a cluster.
+struct ClusterTeam {
+    int buf = 0;
+    __device__ int rank() const { return (int)(cg::this_cluster().block_rank() * blockDim.x + threadIdx.x); }
+    __device__ int size() const { return (int)(cg::this_cluster().num_blocks() * blockDim.x); }
+    __device__ int log2size() const { return __ffs(size()) - 1; }
+    __device__ int local() const { return threadIdx.x; }
+    __device__ int nlocal() const { return blockDim.x; }
+    __device__ void sync() const { cg::this_cluster().sync(); }
+    __device__ double sum(double v) {
+        __shared__ double red[2][BATCH_MAX_BLOCK / 32], part[2][BATCH_CLUSTER];
+        cg::cluster_group cl = cg::this_cluster();
+        v = warp_sum(v);
+        const int nw = (int)(blockDim.x >> 5), nc = (int)cl.num_blocks();
+        if ((threadIdx.x & 31) == 0) red[buf][threadIdx.x >> 5] = v;
+        __syncthreads();
+        if ((int)threadIdx.x < nc) {   // thread i tells CTA i
+            double t = 0;
+            for (int i = 0; i < nw; i++) t += red[buf][i];
+            *cl.map_shared_rank(&part[buf][cl.block_rank()], (int)threadIdx.x) = t;
+        }
+        cl.sync();
+        double t = 0;
+        for (int i = 0; i < nc; i++) t += part[buf][i];
+        buf ^= 1;
+        return t;
+    }
+};
+
 template <typename E> struct ArithOf;
 template <> struct ArithOf<float2> { typedef float T; };
 template <> struct ArithOf<double2> { typedef double T; };
 
-__device__ __forceinline__ void ld_e(const float2 *m, uint64_t a, float &r, float &i) { const float2 v = m[a]; r = v.x; i = v.y; }
-__device__ __forceinline__ void ld_e(const double2 *m, uint64_t a, double &r, double &i) { const double2 v = m[a]; r = v.x; i = v.y; }
-__device__ __forceinline__ void st_e(float2 *m, uint64_t a, float r, float i) { m[a] = make_float2(r, i); }
-__device__ __forceinline__ void st_e(double2 *m, uint64_t a, double r, double i) { m[a] = make_double2(r, i); }
-__device__ __forceinline__ void ld_e(const float2 *m, uint64_t a, double &r, double &i) { const float2 v = m[a]; r = v.x; i = v.y; }
-__device__ __forceinline__ void st_e(float2 *m, uint64_t a, double r, double i) { m[a] = make_float2((float)r, (float)i); }
-
-__device__ __forceinline__ uint64_t bcoset_base(const uint64_t *tk, uint64_t c) {
-    uint64_t b = 0;
-    while (c) {
-        b ^= tk[__ffsll((long long)c) - 1];
-        c &= c - 1;
-    }
-    return b;
+__device__ __forceinline__ float2 mk2(float r, float i) { return make_float2(r, i); }
+__device__ __forceinline__ double2 mk2(double r, double i) { return make_double2(r, i); }
+__device__ __forceinline__ float signed_by(float x, int neg) { return __int_as_float(__float_as_int(x) ^ (neg << 31)); }
+__device__ __forceinline__ double signed_by(double x, int neg) {
+    return __hiloint2double(__double2hiint(x) ^ (neg << 31), __double2loint(x));
 }
 
-// The cosets of a step a team member visits: c = rank | (g << log2 team size) for the Gray codes g of the high bits,
-// so consecutive cosets differ in one high bit and the base is the member's fixed low part XOR one running value
-// (one XOR per coset instead of a loop over the bits of c).  f(c, base) is called for each.
-template <typename TM, typename F>
-__device__ __forceinline__ void team_cosets(const TM &tm, int nk, const uint64_t *tk, F f) {
-    const int ls = tm.log2size();
-    const uint64_t r = (uint64_t)tm.rank();
-    if (nk < ls && r >= (1ULL << nk)) return;
-    const uint64_t lo = bcoset_base(tk, r);
-    const uint64_t nh = nk > ls ? 1ULL << (nk - ls) : 1;
-    uint64_t hi = 0;
-    for (uint64_t n = 0; n < nh; n++) {
-        if (n) hi ^= tk[ls + __ffsll((long long)n) - 1];
-        f(r | ((n ^ (n >> 1)) << ls), lo ^ hi);
-    }
+// Classes n0 .. n0 + cn - 1 of a thread's walk: rank | (gray(n) << ls), the first one at `base` with index `cls`.
+struct Chunk {
+    uint32_t base, cls, n0, cn;
+    int ls;
+};
+__device__ __forceinline__ void chunk_next(const BPass &p, const Chunk &k, uint32_t n, uint32_t &base, uint32_t &cls) {
+    const int j = k.ls + __ffs((int)n) - 1;   // gray(n) = gray(n - 1) ^ 2^ctz(n)
+    base ^= p.col[j];
+    cls ^= 1u << j;
 }
 
-// One coset of step s: inputs already loaded (v), outputs stored, their squared norm returned.
-template <typename E, typename T, int NTQ>
-__device__ __forceinline__ T coset_out(const BStep &s, E *arena, uint64_t c, uint64_t base, const T (&vr)[NTQ],
-                                       const T (&vi)[NTQ], T m0r, T m0i, T m1r, T m1i) {
-    const int pc = __popcll(c & s.rhoc) & 1;
-    // x = 0 and signed x = 1 sums of the two outputs, in scalars (no runtime-indexed arrays)
-    T a0r = 0, a0i = 0, a1r = 0, a1i = 0, b0r = 0, b0i = 0, b1r = 0, b1i = 0;
+// What bounds the launch is the latency of the table reads (16 warps per SM; 27 % of the issue slots, a quarter of the HBM
+// peak), so reads are issued early.  Measured against single-step passes with generic code: 96 instances of widths 7-20
+// 12.0 -> 4.6 ms in complex64 and 17.7 -> 6.3 ms in complex128, 512 instances 46.2 -> 21.8 ms; fused passes with runtime
+// tables alone took 7.1 ms and 32 ms (3.3 times the instructions).  Twice the warps at 64 registers measured the same.
+//
+// A shaped step on the classes of a chunk.  FIRST reads the table, other steps
+// slots a..; LAST writes the table and returns the squared norm written, other steps slots b... NM: members, 0 for
+// a runtime count.  The step's offsets, signs and row stay in registers for the whole chunk.
+template <typename E, typename T, int NTQ, int H, int NM, bool FIRST, bool LAST>
+__device__ __noinline__ double step_chunk(const BPass &p, const BStep &s, const int8_t *bit, double scale, const E *in,
+                                          E *out, E *slots, int stride, int a, int b, const Chunk k) {
+    const double *M = s.M + 4 * bit[0];
+    const T m0r = (T)(scale * M[0]), m0i = (T)(scale * M[1]), m1r = (T)(scale * M[2]), m1i = (T)(scale * M[3]);
+    T sg[NTQ];
 #pragma unroll
-    for (int t = 0; t < NTQ; t++) {
-        T xr = vr[t], xi = vi[t];
-        if (s.tau0[t]) { a1r += xr; a1i += xi; } else { a0r += xr; a0i += xi; }
-        if ((pc ^ s.par[t]) & 1) { xr = -xr; xi = -xi; }
-        if (s.tau1[t]) { b1r += xr; b1i += xi; } else { b0r += xr; b0i += xi; }
-    }
-    const T r0 = m0r * a0r - m0i * a0i + m1r * b0r - m1i * b0i;
-    const T i0 = m0r * a0i + m0i * a0r + m1r * b0i + m1i * b0r;
-    st_e(arena, base, r0, i0);
-    T n = r0 * r0 + i0 * i0;
-    if (s.m == 2) {
-        const T r1 = m0r * a1r - m0i * a1i + m1r * b1r - m1i * b1i;
-        const T i1 = m0r * a1i + m0i * a1r + m1r * b1i + m1i * b1r;
-        st_e(arena, base ^ s.g, r1, i1);
-        n += r1 * r1 + i1 * i1;
-    }
-    return n;
-}
-
-// The write pass over the member's cosets (team_cosets' order), CPI cosets per iteration: every coset's inputs are
-// loaded before any output is stored (distinct cosets never share a slot, so this order is safe in place), which
-// multiplies the loads in flight of a latency-bound team.  Four cosets for complex64 (the big items' tables spill
-// from L2, and 4 cut the batch launch by 11 %); two for complex128, where four cost registers and ran 21 % slower.
-template <typename E, typename TM, int NTQ>
-__device__ double team_step_n(const TM &tm, const BStep &s, const uint64_t *tk, E *arena, int bit, double scale) {
-    typedef typename ArithOf<E>::T T;
-    constexpr int CPI = sizeof(E) == 8 ? 4 : 2;
-    const T m0r = (T)(scale * s.M[4 * bit + 0]), m0i = (T)(scale * s.M[4 * bit + 1]);
-    const T m1r = (T)(scale * s.M[4 * bit + 2]), m1i = (T)(scale * s.M[4 * bit + 3]);
+    for (int t = 0; t < NTQ; t++) sg[t] = (s.par >> t) & 1 ? (T)-1 : (T)1;
+    const uint32_t lam = s.lam, mpar = s.mpar;
+    constexpr int MU = NM ? NM : 1;
+    uint32_t zi[MU][NTQ], zo[MU][2];   // NM > 0: the members' offsets, in registers
+    if (NM)
+#pragma unroll
+        for (int j = 0; j < MU; j++) {
+            if (FIRST)
+#pragma unroll
+                for (int t = 0; t < NTQ; t++) zi[j][t] = p.zin[NTQ * j + t];
+#pragma unroll
+            for (int tau = 0; tau < 2; tau++) zo[j][tau] = LAST ? p.zout[2 * j + tau] : (uint32_t)(s.out[j][tau] * stride);
+        }
+    const int nm = NM ? NM : s.nmem, sin = NTQ * nm, sout = 2 * nm;
+    E *src = slots + a * stride, *dst = slots + b * stride;
+    uint32_t base = k.base, cls = k.cls;
     double nb = 0;
-    const int ls = tm.log2size();
-    const uint64_t r = (uint64_t)tm.rank();
-    if (!(s.nk < ls && r >= (1ULL << s.nk))) {
-        const uint64_t lo = bcoset_base(tk, r);
-        const uint64_t nh = s.nk > ls ? 1ULL << (s.nk - ls) : 1;   // a power of two
-        uint64_t hi = 0;
-        for (uint64_t n = 0; n < nh; n += CPI) {
-            // cosets n .. n + CPI - 1 (n a multiple of CPI): Gray step n + q flips high bit ctz(q); a bit is read
-            // only when that coset exists, so tk stays within the step's kept columns
-            if (n) hi ^= tk[ls + __ffsll((long long)n) - 1];
-            uint64_t h[CPI];
-            h[0] = hi;
+    // the next class's values in registers (complex64: up to 8; complex128 values took registers and ran 10 % slower)
+    constexpr bool UPFRONT = sizeof(E) == 8;
+    constexpr bool AHEAD = FIRST && NM > 0 && NM * NTQ <= 8 && sizeof(E) == 8;
+    E v[MU][NTQ], ahead[AHEAD ? MU : 1][NTQ];
+    auto load = [&](uint32_t at, E (&x)[MU][NTQ]) {
 #pragma unroll
-            for (int q = 1; q < CPI; q++) h[q] = n + (uint64_t)q < nh ? h[q - 1] ^ tk[ls + __ffs(q) - 1] : h[q - 1];
-            const int cnt = nh - n >= (uint64_t)CPI ? CPI : (int)(nh - n);
-            T vr[CPI][NTQ], vi[CPI][NTQ];
+        for (int j = 0; j < MU; j++)
 #pragma unroll
-            for (int q = 0; q < CPI; q++)
+            for (int t = 0; t < NTQ; t++) x[j][t] = in[at ^ zi[j][t]];
+    };
+    if constexpr (AHEAD) load(base, ahead);
+    for (uint32_t n = k.n0;;) {
+        const int cs = __popc(cls & lam);
+        T nn = 0;
+        auto member = [&](int j, const E (&v)[NTQ], const uint32_t (&oj)[2]) {
+            // x = 0 sums (X) and signed x = 1 sums (Z) of the two outputs
+            T Xr[2] = {0, 0}, Xi[2] = {0, 0}, Zr[2] = {0, 0}, Zi[2] = {0, 0};
 #pragma unroll
-                for (int t = 0; t < NTQ; t++) {
-                    if (q < cnt) ld_e(arena, (lo ^ h[q]) ^ s.tq[t], vr[q][t], vi[q][t]);
-                    else { vr[q][t] = 0; vi[q][t] = 0; }
+            for (int t = 0; t < NTQ; t++) {
+                const int o = t < NTQ - H ? 0 : 1;
+                const bool f = t == 0 || (H > 0 && t == NTQ - H);   // the first term of its sums
+                Xr[o] = f ? v[t].x : Xr[o] + v[t].x;
+                Xi[o] = f ? v[t].y : Xi[o] + v[t].y;
+                Zr[1 - o] = f ? sg[t] * v[t].x : fma(sg[t], v[t].x, Zr[1 - o]);
+                Zi[1 - o] = f ? sg[t] * v[t].y : fma(sg[t], v[t].y, Zi[1 - o]);
+            }
+            const int neg = (cs ^ (int)(mpar >> j)) & 1;
+            const T wr = signed_by(m1r, neg), wi = signed_by(m1i, neg);
+#pragma unroll
+            for (int tau = 0; tau < 2; tau++) {
+                T re, im;
+                if (H == 0 && tau == 0) {          // x = 0 terms only
+                    re = m0r * Xr[0] - m0i * Xi[0];
+                    im = m0r * Xi[0] + m0i * Xr[0];
+                } else if (H == 0) {               // x = 1 terms only
+                    re = wr * Zr[1] - wi * Zi[1];
+                    im = wr * Zi[1] + wi * Zr[1];
+                } else {
+                    re = m0r * Xr[tau] - m0i * Xi[tau] + wr * Zr[tau] - wi * Zi[tau];
+                    im = m0r * Xi[tau] + m0i * Xr[tau] + wr * Zi[tau] + wi * Zr[tau];
                 }
-            T nn = 0;
-#pragma unroll
-            for (int q = 0; q < CPI; q++)
-                if (q < cnt) {
-                    const uint64_t m = n + (uint64_t)q;
-                    nn += coset_out<E, T, NTQ>(s, arena, r | ((m ^ (m >> 1)) << ls), lo ^ h[q], vr[q], vi[q], m0r, m0i,
-                                               m1r, m1i);
+                if (LAST) {
+                    out[base ^ oj[tau]] = mk2(re, im);
+                    nn += re * re + im * im;
+                } else {
+                    dst[oj[tau]] = mk2(re, im);
                 }
-            nb += (double)nn;
-            hi = h[CPI - 1];
+            }
+        };
+        uint32_t nbase = base, ncls = cls;
+        const bool more = n + 1 < k.n0 + k.cn;
+        if (more) chunk_next(p, k, n + 1, nbase, ncls);
+        if constexpr (NM > 0) {
+            // every value of the class is loaded before any is used, and with AHEAD the next class's as well: a few dozen
+            // warps per SM have to cover the L2 and HBM latency
+            if constexpr (AHEAD) {
+#pragma unroll
+                for (int j = 0; j < MU; j++)
+#pragma unroll
+                    for (int t = 0; t < NTQ; t++) v[j][t] = ahead[j][t];
+                if (more) load(nbase, ahead);
+            } else if constexpr (FIRST && UPFRONT) {
+                load(base, v);
+            } else if constexpr (!FIRST) {
+#pragma unroll
+                for (int j = 0; j < MU; j++)
+#pragma unroll
+                    for (int t = 0; t < NTQ; t++) v[j][t] = src[(NTQ * j + t) * stride];
+            }
+#pragma unroll
+            for (int j = 0; j < NM; j++) {
+                if constexpr (FIRST && !UPFRONT)
+#pragma unroll
+                    for (int t = 0; t < NTQ; t++) v[j][t] = in[base ^ zi[j][t]];
+                member(j, v[j], zo[j]);
+            }
+        } else {
+            for (int j = 0; j < nm; j++) {
+#pragma unroll
+                for (int t = 0; t < NTQ; t++)
+                    v[0][t] = FIRST ? in[base ^ p.zin[NTQ * j + t]] : src[(NTQ * j + t) * stride];
+#pragma unroll
+                for (int tau = 0; tau < 2; tau++) zo[0][tau] = LAST ? p.zout[2 * j + tau] : (uint32_t)(s.out[j][tau] * stride);
+                member(j, v[0], zo[0]);
+            }
         }
+        nb += (double)nn;
+        n++;
+        if (!more) break;
+        base = nbase;
+        cls = ncls;
+        if (!FIRST) src += sin * stride;
+        if (!LAST) dst += sout * stride;
     }
-    tm.sync();
-    return tm.sum(nb);
+    return nb;
 }
 
-// One write pass of step s with bit `bit`, outputs scaled by `scale`; returns the written norm (to every thread).
-template <typename E, typename TM>
-__device__ double team_step(const TM &tm, const BStep &s, const uint64_t *tk, E *arena, int bit, double scale) {
-    switch (s.ntq) {
-        case 1: return team_step_n<E, TM, 1>(tm, s, tk, arena, bit, scale);
-        case 2: return team_step_n<E, TM, 2>(tm, s, tk, arena, bit, scale);
-        default: return team_step_n<E, TM, 4>(tm, s, tk, arena, bit, scale);
+// The same for any step (runtime tables; one or two outputs).
+template <typename E, typename T, bool FIRST, bool LAST>
+__device__ __noinline__ double step_chunk_any(const BPass &p, const BStep &s, const int8_t *bit, double scale, const E *in,
+                                              E *out, E *slots, int stride, int a, int b, const Chunk k) {
+    const double *M = s.M + 4 * bit[0];
+    const T m0r = (T)(scale * M[0]), m0i = (T)(scale * M[1]), m1r = (T)(scale * M[2]), m1i = (T)(scale * M[3]);
+    const int ntq = s.ntq, m = s.m, nm = s.nmem;
+    E *src = slots + a * stride, *dst = slots + b * stride;
+    uint32_t base = k.base, cls = k.cls;
+    double nb = 0;
+    for (uint32_t n = k.n0;;) {
+        T nn = 0;
+        for (int j = 0; j < nm; j++) {
+            T a0r = 0, a0i = 0, a1r = 0, a1i = 0, b0r = 0, b0i = 0, b1r = 0, b1i = 0;
+            for (int t = 0; t < ntq; t++) {
+                const E v = FIRST ? in[base ^ p.zin[ntq * j + t]] : src[(ntq * j + t) * stride];
+                if ((s.tau0 >> t) & 1) { a1r += v.x; a1i += v.y; } else { a0r += v.x; a0i += v.y; }
+                const T yr = signed_by(v.x, (s.par >> t) & 1), yi = signed_by(v.y, (s.par >> t) & 1);
+                if ((s.tau1 >> t) & 1) { b1r += yr; b1i += yi; } else { b0r += yr; b0i += yi; }
+            }
+            const int neg = (__popc(cls & s.lam) ^ (int)(s.mpar >> j)) & 1;
+            const T wr = signed_by(m1r, neg), wi = signed_by(m1i, neg);
+            for (int tau = 0; tau < m; tau++) {
+                const T xr = tau ? a1r : a0r, xi = tau ? a1i : a0i, zr = tau ? b1r : b0r, zi = tau ? b1i : b0i;
+                const T re = m0r * xr - m0i * xi + wr * zr - wi * zi, im = m0r * xi + m0i * xr + wr * zi + wi * zr;
+                if (LAST) {
+                    out[base ^ p.zout[m * j + tau]] = mk2(re, im);
+                    nn += re * re + im * im;
+                } else {
+                    dst[s.out[j][tau] * stride] = mk2(re, im);
+                }
+            }
+        }
+        nb += (double)nn;
+        if (++n >= k.n0 + k.cn) break;
+        chunk_next(p, k, n, base, cls);
+        if (!FIRST) src += ntq * nm * stride;
+        if (!LAST) dst += m * nm * stride;
     }
+    return nb;
 }
 
-// Live table before step s, in (coset, offset) order, to / from a compact buffer.
-template <typename E, typename TM>
-__device__ void team_copy(const TM &tm, const BStep &s, const uint64_t *tk, E *arena, E *snap, bool save) {
-    team_cosets(tm, s.nk, tk, [&](uint64_t c, uint64_t base) {
-        for (int t = 0; t < s.ntq; t++) {
-            if (save) snap[c * (uint64_t)s.ntq + (uint64_t)t] = arena[base ^ s.tq[t]];
-            else arena[base ^ s.tq[t]] = snap[c * (uint64_t)s.ntq + (uint64_t)t];
+template <typename E, typename T, bool FIRST, bool LAST>
+__device__ __forceinline__ double step_on(const BPass &p, const BStep &s, const int8_t *bit, double scale, const E *in, E *out,
+                                          E *slots, int stride, int a, int b, const Chunk &k) {
+#define GSB_BK(KIND, NTQ, H)                                                                                       \
+    case KIND:                                                                                                     \
+        switch (s.nmem) {                                                                                          \
+            case 1: return step_chunk<E, T, NTQ, H, 1, FIRST, LAST>(p, s, bit, scale, in, out, slots, stride, a, b, k); \
+            case 2: return step_chunk<E, T, NTQ, H, 2, FIRST, LAST>(p, s, bit, scale, in, out, slots, stride, a, b, k); \
+            case 4: return step_chunk<E, T, NTQ, H, 4, FIRST, LAST>(p, s, bit, scale, in, out, slots, stride, a, b, k); \
+            default: return step_chunk<E, T, NTQ, H, 0, FIRST, LAST>(p, s, bit, scale, in, out, slots, stride, a, b, k); \
         }
-    });
-    tm.sync();
+    switch (s.kind) {
+        GSB_BK(BK_1_0, 1, 0)
+        GSB_BK(BK_2_0, 2, 0)
+        GSB_BK(BK_2_1, 2, 1)
+        GSB_BK(BK_4_0, 4, 0)
+        GSB_BK(BK_4_1, 4, 1)
+        GSB_BK(BK_4_2, 4, 2)
+        default: return step_chunk_any<E, T, FIRST, LAST>(p, s, bit, scale, in, out, slots, stride, a, b, k);
+    }
+#undef GSB_BK
+}
+
+// One pass of a team from the table `in` to the table `out` (the same one, or the item's other one), the first step's
+// outputs scaled; returns the squared norm of this thread's outputs.
+template <typename E>
+__device__ __noinline__ double team_pass(const BPass &p, uint32_t r, int ls, const E *in, E *out, const int8_t *bits,
+                                         double scale, E *slots, int stride) {
+    typedef typename ArithOf<E>::T T;
+    if (p.nb < ls && r >= (1u << p.nb)) return 0;
+    Chunk k;
+    k.base = 0;
+    k.cls = r;
+    k.ls = ls;
+    for (int j = 0; j < min(p.nb, ls); j++)
+        if ((r >> j) & 1) k.base ^= p.col[j];
+    const uint32_t count = p.nb > ls ? 1u << (p.nb - ls) : 1;
+    k.cn = min(count, (uint32_t)p.chunk);   // powers of two
+    double nb = 0;
+    for (k.n0 = 0; k.n0 < count; k.n0 += k.cn) {
+        if (k.n0) {
+            // from the previous chunk's first class: gray(n0) ^ gray(n0 - cn) has the bits log2 cn - 1 (cn > 1) and above
+            const uint32_t f = k.n0 - k.cn, d = (k.n0 ^ (k.n0 >> 1)) ^ (f ^ (f >> 1));
+            for (uint32_t x = d; x; x &= x - 1) k.base ^= p.col[ls + __ffs((int)x) - 1];
+            k.cls ^= d << ls;
+        }
+        const int b1 = 0, b2 = (int)k.cn * p.mid[0];
+        if (p.d == 1) {
+            nb += step_on<E, T, true, true>(p, p.st[0], bits, scale, in, out, slots, stride, 0, 0, k);
+        } else {
+            step_on<E, T, true, false>(p, p.st[0], bits, scale, in, out, slots, stride, 0, b1, k);
+            if (p.d == 2) {
+                nb += step_on<E, T, false, true>(p, p.st[1], bits + 1, 1.0, in, out, slots, stride, b1, 0, k);
+            } else {
+                step_on<E, T, false, false>(p, p.st[1], bits + 1, 1.0, in, out, slots, stride, b1, b2, k);
+                nb += step_on<E, T, false, true>(p, p.st[2], bits + 2, 1.0, in, out, slots, stride, b2, 0, k);
+            }
+        }
+    }
+    return nb;
 }
 
 struct ChainState {
@@ -238,43 +427,98 @@ __device__ __forceinline__ void chain_update(ChainState &cs, double nb) {
         cs.dead = 1;
         return;
     }
-    int ex;
+    int ex = 0;
     frexp(nb, &ex);
     cs.ek = (ex - 1) >> 1;
     cs.scale = ldexp(1.0, -cs.ek);
 }
 
+// Passes a .. b - 1 of an instance with its bits (the first pass's step first): read from `first`, otherwise the arena,
+// the last one written to `last`, otherwise the arena.  desc: two descriptor buffers; the next pass's descriptor is
+// fetched during a pass.  Ends behind a team barrier (the last sum): tables complete, buffers free.
 template <typename E, typename TM>
-__device__ void run_item(const TM &tm, const BatchArgs &a, int item, E *arena, E *snap) {
+__device__ void run_passes(TM &tm, const BPass *passes, int a, int b, const int8_t *bits, const E *first, E *arena, E *last,
+                           BPass *desc, E *slots, int stride, ChainState &cs) {
+    constexpr int WORDS = (int)(sizeof(BPass) / 16), PER = (WORDS + 31) / 32;
+    const int l = tm.local(), nl = tm.nlocal();
+    for (int i = l; i < WORDS; i += nl) reinterpret_cast<int4 *>(desc)[i] = reinterpret_cast<const int4 *>(passes + a)[i];
+    tm.sync();
+    int k = 0;
+    for (int i = a; i < b; i++) {
+        const BPass &p = desc[(i - a) & 1];
+        int4 next[PER];
+        if (i + 1 < b)
+#pragma unroll
+            for (int q = 0; q < PER; q++)
+                if (l + q * nl < WORDS) next[q] = reinterpret_cast<const int4 *>(passes + i + 1)[l + q * nl];
+        const double nb = team_pass<E>(p, (uint32_t)tm.rank(), tm.log2size(), i == a ? first : arena,
+                                       i == b - 1 ? last : arena, bits + k, cs.scale, slots, stride);
+        k += p.d;
+        if (i + 1 < b)
+#pragma unroll
+            for (int q = 0; q < PER; q++)
+                if (l + q * nl < WORDS) reinterpret_cast<int4 *>(desc + ((i + 1 - a) & 1))[l + q * nl] = next[q];
+        chain_update(cs, tm.sum(nb));
+        if (cs.dead) break;
+    }
+}
+
+template <typename E, typename TM>
+__device__ void run_item(TM &tm, const BatchArgs &a, int item, E *arena, E *kept, BPass *desc, E *slots, int stride) {
     const int ii = item / a.npre, pre = item % a.npre;
     const BInst in = a.inst[ii];
-    const BStep *st = a.steps + in.step_off;
     const int8_t *pb = a.pre_bits + in.pre_off + (int64_t)pre * in.K;
-    if (tm.rank() == 0) st_e(arena, 0, 1.0, 0.0);
-    tm.sync();
+    if (tm.rank() == 0) arena[0] = mk2((typename ArithOf<E>::T)1, (typename ArithOf<E>::T)0);
     ChainState cs{1.0, 0.0, 1.0, 0, 0};
-    for (int k = 0; k < in.K && !cs.dead; k++) chain_update(cs, team_step(tm, st[k], a.tk + st[k].tk_off, arena, pb[k], cs.scale));
+    const int p0 = in.pass_off, p1 = p0 + in.npass[0], p2 = p1 + in.npass[1];
+    run_passes<E, TM>(tm, a.passes, p0, p1, pb, arena, arena, kept, desc, slots, stride, cs);
     const ChainState at_k = cs;
-    if (!cs.dead) team_copy(tm, st[in.K], a.tk + st[in.K].tk_off, arena, snap, true);
     const int nsuf_steps = in.ns - in.K;
     for (int sidx = 0; sidx < a.nsuf; sidx++) {
         cs = at_k;
         double lp = -INFINITY;
         if (!cs.dead) {
-            if (sidx > 0) team_copy(tm, st[in.K], a.tk + st[in.K].tk_off, arena, snap, false);
             const int8_t *sb = a.suf_bits + in.suf_off + ((int64_t)pre * a.nsuf + sidx) * nsuf_steps;
-            for (int k = in.K; k < in.ns && !cs.dead; k++)
-                chain_update(cs, team_step(tm, st[k], a.tk + st[k].tk_off, arena, sb[k - in.K], cs.scale));
+            run_passes<E, TM>(tm, a.passes, p1, p2, sb, kept, arena, arena, desc, slots, stride, cs);
             if (!cs.dead) lp = log2(cs.prev) + 2.0 * cs.lsc - in.n;
         }
         if (tm.rank() == 0) a.log2p[in.out_off + (int64_t)pre * a.nsuf + sidx] = lp;
     }
-    tm.sync();
 }
 
+// Dynamic shared memory of a block: two descriptors per warp (a block or cluster team uses the first two), then the
+// threads' slots.
+static size_t batch_smem(int block) {
+    return (size_t)(block / 32) * 2 * sizeof(BPass) + (size_t)BATCH_SLOT_BYTES * (size_t)block;
+}
+
+constexpr size_t BATCH_MAX_SMEM = (227 << 10) - 2048;   // dynamic, beside the teams' static sums
+
 template <typename E>
-__global__ void k_batch(const BatchArgs a) {
+__global__ void __launch_bounds__(BATCH_MAX_BLOCK) k_batch(const BatchArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int warps = (int)(blockDim.x >> 5), w = (int)(threadIdx.x >> 5);
+    BPass *desc = reinterpret_cast<BPass *>(smem);
+    E *slots = reinterpret_cast<E *>(smem + (size_t)warps * 2 * sizeof(BPass)) + threadIdx.x;
+    const int stride = (int)blockDim.x;
     __shared__ int s_item;
+    if (a.n_wide > 0) {
+        cg::cluster_group cl = cg::this_cluster();
+        const size_t wide = (size_t)1 << a.wide_R;
+        E *arena = reinterpret_cast<E *>(a.wide_arena) + (size_t)(blockIdx.x / cl.num_blocks()) * 2 * wide;
+        ClusterTeam ct;
+        for (;;) {
+            if (cl.block_rank() == 0 && threadIdx.x == 0) {
+                const int it = (int)atomicAdd(&a.queues[2], 1u);
+                for (unsigned r = 0; r < cl.num_blocks(); r++) *cl.map_shared_rank(&s_item, r) = it;
+            }
+            cl.sync();
+            const int it = s_item;
+            cl.sync();
+            if (it >= a.n_wide) break;
+            run_item<E, ClusterTeam>(ct, a, a.items_wide[it], arena, arena + wide, desc, slots, stride);
+        }
+    }
     const size_t big = (size_t)1 << a.big_R, small = (size_t)1 << a.small_R;
     E *arena = reinterpret_cast<E *>(a.big_arena) + (size_t)blockIdx.x * 2 * big;
     BlockTeam bt;
@@ -284,9 +528,8 @@ __global__ void k_batch(const BatchArgs a) {
         const int it = s_item;
         __syncthreads();
         if (it >= a.n_big) break;
-        run_item<E>(bt, a, a.items_big[it], arena, arena + big);
+        run_item<E, BlockTeam>(bt, a, a.items_big[it], arena, arena + big, desc, slots, stride);
     }
-    const int warps = (int)(blockDim.x >> 5), w = (int)(threadIdx.x >> 5);
     E *wa = reinterpret_cast<E *>(a.small_arena) + ((size_t)blockIdx.x * warps + (size_t)w) * 2 * small;
     WarpTeam wt;
     for (;;) {
@@ -294,7 +537,7 @@ __global__ void k_batch(const BatchArgs a) {
         if ((threadIdx.x & 31) == 0) it = (int)atomicAdd(&a.queues[1], 1u);
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= a.n_small) break;
-        run_item<E>(wt, a, a.items_small[it], wa, wa + small);
+        run_item<E, WarpTeam>(wt, a, a.items_small[it], wa, wa + small, desc + 2 * w, slots, stride);
     }
 }
 
@@ -309,11 +552,10 @@ struct BatchEngine {
     int prec = 64, dev = 0, sms = 0;
     size_t esize = 8;
     std::vector<HPlan> plans;
-    std::vector<BStep> h_steps;
-    std::vector<uint64_t> h_tk;
+    std::vector<int> K;             // prefix lengths that d_passes was made for
+    std::vector<int> pass_off, npass0, npass1;
     std::vector<double> cost;       // per instance: entries moved by one prefix + its suffixes (relative)
-    BStep *d_steps = nullptr;
-    uint64_t *d_tk = nullptr;
+    BPass *d_passes = nullptr;
     BInst *d_inst = nullptr;
     int *d_items = nullptr;
     int8_t *d_pre = nullptr, *d_suf = nullptr;
@@ -334,8 +576,7 @@ struct BatchEngine {
         cudaGetDevice(&prev);
         cudaSetDevice(dev);
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
-        cudaFree(d_steps);
-        cudaFree(d_tk);
+        cudaFree(d_passes);
         cudaFree(d_inst);
         cudaFree(d_items);
         cudaFree(d_pre);
@@ -368,27 +609,169 @@ struct gsb_batch {
     BatchEngine E;
 };
 
-// Lay out the items of a shape: wide instances to the block-team queue, narrow ones to the warp-team queue, each in
-// decreasing cost; size the team arenas.  Returns the device bytes the shape needs.
-static size_t shape_layout(const BatchEngine &E, const BatchShape &sh, std::vector<int> &big, std::vector<int> &small,
-                           int &big_R, int &small_R, int &grid) {
-    big.clear();
-    small.clear();
-    big_R = 0;
-    small_R = 0;
+// Items of a shape: the widest instances to the cluster-team queue, wide ones to the block-team queue, narrow ones to the
+// warp-team queue, each in decreasing cost, and the sizes of the team arenas.
+struct BatchLayout {
+    std::vector<int> wide, big, small;
+    int wide_R = 0, big_R = 0, small_R = 0, grid = 0;
+    size_t bytes = 0;
+};
+static BatchLayout shape_layout(const BatchEngine &E, const BatchShape &sh) {
+    BatchLayout L;
     std::vector<int> order(E.plans.size());
     for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
     std::sort(order.begin(), order.end(), [&](int x, int y) { return E.cost[(size_t)x] > E.cost[(size_t)y]; });
+    L.grid = E.sms * sh.per_sm / BATCH_CLUSTER * BATCH_CLUSTER;
+    // An item that would keep one CTA busy for longer than an even share of the whole batch goes to a cluster: a
+    // cluster spends part of its time on barriers, so it pays only where one CTA would be the batch's tail.  Thresholds of
+    // 1/4, 1/2, 1 and 2 shares took 5.6, 5.2, 4.7 and 5.6 ms on 96 instances of widths 7-20 (no clusters: 10 ms, the time of
+    // one width-20 item), 27.4, 24.4, 21.8 and 21.8 ms on 512, 2.4, 0.79, 0.80 and 0.80 ms on 200 of widths up to 15.
+    // Below width 15 a cluster's steps are barriers only (8 instances of width 12: 0.33 ms against 0.11 ms).
+    double total = 0;
+    for (double c : E.cost) total += c * E.npre;
+    const double share = total / L.grid;
     for (int i : order) {
         const int R = E.plans[(size_t)i].R;
-        auto &q = R <= sh.small_R ? small : big;
+        const bool small = R <= sh.small_R, wide = !small && R >= 15 && E.cost[(size_t)i] > share;
+        auto &q = small ? L.small : wide ? L.wide : L.big;
         for (int p = 0; p < E.npre; p++) q.push_back(i * E.npre + p);
-        if (R <= sh.small_R) small_R = std::max(small_R, R);
-        else big_R = std::max(big_R, R);
+        int &r = small ? L.small_R : wide ? L.wide_R : L.big_R;
+        r = std::max(r, R);
     }
-    grid = E.sms * sh.per_sm;
-    const size_t warps = (size_t)grid * (size_t)(sh.block / 32);
-    return E.esize * 2 * ((size_t)grid * ((size_t)1 << big_R) + warps * ((size_t)1 << small_R));
+    const size_t warps = (size_t)L.grid * (size_t)(sh.block / 32);
+    L.bytes = E.esize * 2 * ((L.wide.empty() ? 0 : (size_t)(L.grid / BATCH_CLUSTER) << L.wide_R) +
+                             ((size_t)L.grid << L.big_R) + (warps << L.small_R));
+    return L;
+}
+
+// The pass of steps gp.k0 .. gp.k0 + gp.d - 1; false when one class's values between the steps exceed `slots`.
+static bool make_pass(const HPlan &p, const GroupPlan &gp, int slots, BPass &g) {
+    memset(&g, 0, sizeof g);
+    int kept = 0;
+    for (int s = 0; s + 1 < gp.d; s++) kept += g.mid[s] = gp.stage_size[s + 1];
+    if (kept > slots || gp.nb > 24) return false;
+    g.d = gp.d;
+    g.nb = gp.nb;
+    g.chunk = 1;
+    while (g.chunk < 32 && 2 * g.chunk * kept <= slots) g.chunk *= 2;
+    std::vector<uint64_t> cols;
+    for (int j = 0; j < gp.L; j++) cols.push_back(1ULL << j);
+    cols.insert(cols.end(), gp.bhi.begin(), gp.bhi.end());
+    for (int j = 0; j < gp.nb; j++) g.col[j] = (uint32_t)cols[(size_t)j];
+    std::vector<int> number[FUSE_MAX_STEPS + 1];   // of the plan's stage values: member-major in the step that reads them
+    int perm[FUSE_MAX_STEPS][4], swp[FUSE_MAX_STEPS];
+    for (int s = 0; s < gp.d; s++) {
+        const HStep &hs = p.st[(size_t)(gp.k0 + s)];
+        const GroupPlan::Step &q = gp.step[s];
+        BStep &a = g.st[s];
+        bool shaped = q.m == 2;
+        int h = 0;
+        for (int t = 0; t < q.ntq; t++) {
+            shaped = shaped && hs.tau1[t] == 1 - hs.tau0[t];
+            h += hs.tau0[t];
+        }
+        swp[s] = shaped && 2 * h > q.ntq;
+        if (swp[s]) h = q.ntq - h;
+        int n = 0;
+        for (int out = 0; out < 2; out++)
+            for (int t = 0; t < q.ntq; t++)
+                if (!shaped ? out == 0 : (hs.tau0[t] ^ swp[s]) == out) perm[s][n++] = t;
+        a.kind = BK_ANY;
+        if (shaped && q.ntq == 1) a.kind = BK_1_0;
+        else if (shaped && q.ntq == 2) a.kind = h == 0 ? BK_2_0 : BK_2_1;
+        else if (shaped && q.ntq == 4) a.kind = h == 0 ? BK_4_0 : h == 1 ? BK_4_1 : BK_4_2;
+        a.nmem = q.nmem;
+        a.ntq = q.ntq;
+        a.m = q.m;
+        for (int b = 0; b < 2; b++)
+            for (int x = 0; x < 2; x++) {
+                a.M[4 * b + 2 * x] = hs.Mr[b][x];
+                a.M[4 * b + 2 * x + 1] = hs.Mi[b][x];
+            }
+        for (int t = 0; t < q.ntq; t++) {
+            a.tau0 |= (hs.tau0[perm[s][t]] ^ swp[s]) << t;
+            a.tau1 |= (hs.tau1[perm[s][t]] ^ swp[s]) << t;
+            a.par |= hs.par[perm[s][t]] << t;
+        }
+        for (int j = 0; j < gp.nb; j++)
+            a.lam |= (uint32_t)(__builtin_popcountll(cols[(size_t)j] & q.lambda) & 1) << j;
+        number[s].assign((size_t)gp.stage_size[s], 0);
+        for (int j = 0; j < q.nmem; j++) {
+            a.mpar |= (uint32_t)(q.mpar[j] & 1) << j;
+            for (int t = 0; t < q.ntq; t++) number[s][(size_t)q.in_idx[j][perm[s][t]]] = q.ntq * j + t;
+        }
+    }
+    for (int i = 0; i < gp.stage_size[0]; i++) g.zin[number[0][(size_t)i]] = (uint32_t)gp.z_in[(size_t)i];
+    for (int s = 0; s < gp.d; s++) {
+        const GroupPlan::Step &q = gp.step[s];
+        for (int j = 0; j < q.nmem; j++)
+            for (int tau = 0; tau < q.m; tau++) {
+                const int old = q.out_idx[j][tau ^ swp[s]];
+                if (s + 1 < gp.d) g.st[s].out[j][tau] = (unsigned char)number[s + 1][(size_t)old];
+                else g.zout[q.m * j + tau] = (uint32_t)gp.z_out[(size_t)old];
+            }
+    }
+    return true;
+}
+
+// Passes of steps k0 .. k1 - 1, each as long as its classes' slots allow.  A narrow instance is run by one warp by
+// default, and fusing leaves its lanes few classes with a long chain of work each: up to width 12 passes of several
+// steps have at least 2^8 classes (300 instances of widths up to 12: 0.63 ms with any number of classes, 0.43 at 2^5, 0.36
+// at 2^8).  Block and cluster teams are faster fused throughout (60 instances of widths 8-14: 0.27 against 0.33 ms).
+static bool passes_of(const HPlan &p, int k0, int k1, int slots, std::vector<BPass> &out) {
+    const int least = p.R <= 12 ? 8 : 0;
+    for (int k = k0; k < k1;) {
+        BPass g;
+        GroupPlan gp;
+        int d = std::min(FUSE_MAX_STEPS, k1 - k);
+        while (d > 0 && !(plan_group(p, k, d, 0, 24, gp) && (d == 1 || gp.nb >= least) && make_pass(p, gp, slots, g))) d--;
+        if (!d) return false;
+        out.push_back(g);
+        k += d;
+    }
+    return true;
+}
+
+// The pass lists for prefix lengths K (kept while they stay the same), made by the host's cores side by side: 17 us per
+// candidate pass, 20 passes per instance.
+static int batch_passes(BatchEngine &E, const int *K) {
+    const size_t n = E.plans.size();
+    if (E.K.size() == n && std::equal(E.K.begin(), E.K.end(), K)) return 0;
+    std::vector<std::vector<BPass>> got(n);
+    std::vector<int> pre(n, 0), bad(n, 0);
+    const int slots = BATCH_SLOT_BYTES / (int)E.esize;
+    const unsigned nt = std::max(1u, std::min({(unsigned)n, 16u, std::thread::hardware_concurrency()}));
+    auto work = [&](size_t t) {
+        for (size_t i = t; i < n; i += nt) {
+            const HPlan &p = E.plans[i];
+            bad[i] = !passes_of(p, 0, K[i], slots, got[i]);
+            pre[i] = (int)got[i].size();
+            bad[i] = bad[i] || !passes_of(p, K[i], p.ns, slots, got[i]);
+        }
+    };
+    std::vector<std::thread> th;
+    for (unsigned t = 1; t < nt; t++) th.emplace_back(work, t);
+    work(0);
+    for (std::thread &t : th) t.join();
+    std::vector<BPass> all;
+    E.pass_off.assign(n, 0);
+    E.npass0 = pre;
+    E.npass1.assign(n, 0);
+    for (size_t i = 0; i < n; i++) {
+        if (bad[i]) return fail(GSB_E_PLAN_LAYOUT, "instance " + std::to_string(i) + " does not fit the batch kernel's passes");
+        E.pass_off[i] = (int)all.size();
+        E.npass1[i] = (int)got[i].size() - pre[i];
+        all.insert(all.end(), got[i].begin(), got[i].end());
+    }
+    for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);   // they point at the old passes
+    E.graphs.clear();
+    cudaFree(E.d_passes);
+    E.d_passes = nullptr;
+    E.K.clear();
+    BT_CK(cudaMalloc(&E.d_passes, all.size() * sizeof(BPass)));
+    BT_CK(cudaMemcpy(E.d_passes, all.data(), all.size() * sizeof(BPass), cudaMemcpyHostToDevice));
+    E.K.assign(K, K + n);
+    return 0;
 }
 
 static int batch_graph(BatchEngine &E, const BatchShape &sh, cudaGraphExec_t *out) {
@@ -397,9 +780,8 @@ static int batch_graph(BatchEngine &E, const BatchShape &sh, cudaGraphExec_t *ou
         *out = it->second;
         return 0;
     }
-    std::vector<int> big, small;
-    int big_R, small_R, grid;
-    const size_t need = shape_layout(E, sh, big, small, big_R, small_R, grid);
+    const BatchLayout L = shape_layout(E, sh);
+    const size_t need = L.bytes;
     if (need > E.arena_bytes) {
         cudaFree(E.d_arena);
         E.d_arena = nullptr;
@@ -411,37 +793,56 @@ static int batch_graph(BatchEngine &E, const BatchShape &sh, cudaGraphExec_t *ou
     }
     cudaFree(E.d_items);
     E.d_items = nullptr;
-    std::vector<int> items(big);
-    items.insert(items.end(), small.begin(), small.end());
+    std::vector<int> items(L.wide);
+    items.insert(items.end(), L.big.begin(), L.big.end());
+    items.insert(items.end(), L.small.begin(), L.small.end());
     BT_CK(cudaMalloc(&E.d_items, std::max<size_t>(items.size(), 1) * sizeof(int)));
     if (!items.empty())
         BT_CK(cudaMemcpy(E.d_items, items.data(), items.size() * sizeof(int), cudaMemcpyHostToDevice));
     for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);   // items buffer changed
     E.graphs.clear();
     BatchArgs a;
-    a.steps = E.d_steps;
-    a.tk = E.d_tk;
+    a.passes = E.d_passes;
     a.inst = E.d_inst;
-    a.items_big = E.d_items;
-    a.items_small = E.d_items + big.size();
-    a.n_big = (int)big.size();
-    a.n_small = (int)small.size();
+    a.items_wide = E.d_items;
+    a.items_big = a.items_wide + L.wide.size();
+    a.items_small = a.items_big + L.big.size();
+    a.n_wide = (int)L.wide.size();
+    a.n_big = (int)L.big.size();
+    a.n_small = (int)L.small.size();
     a.npre = E.npre;
     a.nsuf = E.nsuf;
     a.pre_bits = E.d_pre;
     a.suf_bits = E.d_suf;
     a.log2p = E.d_out;
     a.queues = E.d_q;
-    a.big_arena = E.d_arena;
-    a.small_arena = static_cast<char *>(E.d_arena) + E.esize * 2 * (size_t)grid * ((size_t)1 << big_R);
-    a.big_R = big_R;
-    a.small_R = small_R;
+    char *mem = static_cast<char *>(E.d_arena);
+    a.wide_arena = mem;
+    if (a.n_wide) mem += E.esize * 2 * ((size_t)(L.grid / BATCH_CLUSTER) << L.wide_R);
+    a.big_arena = mem;
+    a.small_arena = mem + E.esize * 2 * ((size_t)L.grid << L.big_R);
+    a.wide_R = L.wide_R;
+    a.big_R = L.big_R;
+    a.small_R = L.small_R;
+    const size_t smem = batch_smem(sh.block);
+    const void *fn = E.prec == 128 ? (const void *)k_batch<double2> : (const void *)k_batch<float2>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)L.grid);
+    cfg.blockDim = dim3((unsigned)sh.block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = E.stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = BATCH_CLUSTER;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = a.n_wide ? 1 : 0;   // clusters only where an item needs one
     cudaGraph_t g = nullptr;
     BT_CK(cudaStreamBeginCapture(E.stream, cudaStreamCaptureModeThreadLocal));
-    cudaMemsetAsync(E.d_q, 0, 2 * sizeof(unsigned int), E.stream);
-    if (E.prec == 128) k_batch<double2><<<grid, sh.block, 0, E.stream>>>(a);
-    else k_batch<float2><<<grid, sh.block, 0, E.stream>>>(a);
-    cudaError_t e = cudaGetLastError();
+    cudaMemsetAsync(E.d_q, 0, 3 * sizeof(unsigned int), E.stream);
+    void *kargs[] = {&a};
+    const cudaError_t e0 = cudaLaunchKernelExC(&cfg, fn, kargs);
+    cudaError_t e = e0;
     cudaError_t e2 = cudaStreamEndCapture(E.stream, &g);
     if (e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -493,28 +894,7 @@ int gsb_batch_open(const char *const *texts, const size_t *lens, int ninst, int 
         double c = 0;
         for (int k = 0; k < p.ns; k++) {
             const HStep &s = p.st[(size_t)k];
-            BStep b;
-            memset(&b, 0, sizeof b);
-            b.nk = s.nk;
-            b.ntq = (int)s.tqs.size();
-            b.m = s.m;
-            b.g = s.m == 2 ? s.g : 0;
-            b.rhoc = s.rhoc;
-            for (int t = 0; t < b.ntq; t++) {
-                b.tq[t] = s.tqs[(size_t)t];
-                b.tau0[t] = s.tau0[t];
-                b.tau1[t] = s.tau1[t];
-                b.par[t] = s.par[t];
-            }
-            for (int bb = 0; bb < 2; bb++)
-                for (int x = 0; x < 2; x++) {
-                    b.M[4 * bb + 2 * x] = s.Mr[bb][x];
-                    b.M[4 * bb + 2 * x + 1] = s.Mi[bb][x];
-                }
-            b.tk_off = (int)E.h_tk.size();
-            for (int j = 0; j < s.nk; j++) E.h_tk.push_back(s.tk[(size_t)j]);
-            E.h_steps.push_back(b);
-            c += std::ldexp(1.0, s.nk) * (double)(b.ntq + b.m);
+            c += std::ldexp(1.0, s.nk) * (double)((int)s.tqs.size() + s.m);
         }
         E.cost.push_back(c);
     }
@@ -527,12 +907,9 @@ int gsb_batch_open(const char *const *texts, const size_t *lens, int ninst, int 
     } restore{prev};
     cudaDeviceGetAttribute(&E.sms, cudaDevAttrMultiProcessorCount, device);
     cudaError_t e = cudaStreamCreateWithFlags(&E.stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&E.d_steps, E.h_steps.size() * sizeof(BStep));
-    if (e == cudaSuccess) e = cudaMalloc(&E.d_tk, std::max<size_t>(E.h_tk.size(), 1) * sizeof(uint64_t));
-    if (e == cudaSuccess) e = cudaMalloc(&E.d_q, 2 * sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaMemcpy(E.d_steps, E.h_steps.data(), E.h_steps.size() * sizeof(BStep), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !E.h_tk.empty())
-        e = cudaMemcpy(E.d_tk, E.h_tk.data(), E.h_tk.size() * sizeof(uint64_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&E.d_q, 3 * sizeof(unsigned int));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BATCH_MAX_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BATCH_MAX_SMEM);
     if (e != cudaSuccess) {
         delete h;
         return fail(GSB_E_ALLOC, std::string("device allocation: ") + cudaGetErrorString(e));
@@ -553,7 +930,6 @@ int gsb_batch_set_strings(gsb_batch *h, const int *K, int npre, int nsuf, const 
     const int ninst = (int)E.plans.size();
     std::vector<BInst> inst((size_t)ninst);
     int64_t po = 0, so = 0, oo = 0;
-    int step_off = 0;
     for (int i = 0; i < ninst; i++) {
         const HPlan &p = E.plans[(size_t)i];
         if (K[i] < 1 || K[i] >= p.ns) return fail(GSB_E_USAGE, "prefix length must be in [1, ns) for instance " + std::to_string(i));
@@ -562,11 +938,9 @@ int gsb_batch_set_strings(gsb_batch *h, const int *K, int npre, int nsuf, const 
         b.R = p.R;
         b.K = K[i];
         b.n = p.n;
-        b.step_off = step_off;
         b.pre_off = po;
         b.suf_off = so;
         b.out_off = oo;
-        step_off += p.ns;
         po += (int64_t)npre * K[i];
         so += (int64_t)npre * nsuf * (p.ns - K[i]);
         oo += (int64_t)npre * nsuf;
@@ -583,6 +957,12 @@ int gsb_batch_set_strings(gsb_batch *h, const int *K, int npre, int nsuf, const 
         int p;
         ~Restore() { cudaSetDevice(p); }
     } restore{prev};
+    if (int rc = batch_passes(E, K)) return rc;
+    for (int i = 0; i < ninst; i++) {
+        inst[(size_t)i].pass_off = E.pass_off[(size_t)i];
+        inst[(size_t)i].npass[0] = E.npass0[(size_t)i];
+        inst[(size_t)i].npass[1] = E.npass1[(size_t)i];
+    }
     const bool resize = po != E.pre_total || so != E.suf_total || oo != E.out_total || npre != E.npre || nsuf != E.nsuf;
     if (resize) {
         for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);
@@ -682,9 +1062,8 @@ int gsb_batch_tune(gsb_batch *h, int reps, size_t max_bytes, int *block, int *sm
             for (int ps : {1, 2, 4}) {
                 if (blk * ps > 2048 || sr > maxR + 1 || blk > max_block) continue;
                 BatchShape sh{blk, sr, ps};
-                std::vector<int> big, small;
-                int bR, sR, grid;
-                if (shape_layout(E, sh, big, small, bR, sR, grid) > max_bytes) continue;
+                if (shape_layout(E, sh).bytes > max_bytes) continue;
+                if (batch_smem(blk) > BATCH_MAX_SMEM) continue;
                 E.shape = sh;
                 float ms = 0, tot = 0;
                 if (int rc = gsb_batch_run(h, out.data(), &ms)) return rc;
