@@ -723,7 +723,8 @@ static bool passes_of(const HPlan &p, int k0, int k1, int slots, std::vector<BPa
     for (int k = k0; k < k1;) {
         BPass g;
         GroupPlan gp;
-        int d = std::min(FUSE_MAX_STEPS, k1 - k);
+        int d = 1;   // a pass has at most the 2^nk cosets of each of its steps as classes
+        while (d < FUSE_MAX_STEPS && k + d < k1 && std::min(p.st[(size_t)k].nk, p.st[(size_t)(k + d)].nk) >= least) d++;
         while (d > 0 && !(plan_group(p, k, d, 0, 24, gp) && (d == 1 || gp.nb >= least) && make_pass(p, gp, slots, g))) d--;
         if (!d) return false;
         out.push_back(g);

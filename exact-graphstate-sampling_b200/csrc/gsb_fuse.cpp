@@ -2,30 +2,19 @@
 #include "gsb_fuse.h"
 
 #include <algorithm>
-#include <map>
 
 namespace gsb {
 
 namespace {
 
-// Subspace of GF(2)^64 with a pivot basis (pivot = leading bit).
-struct Sp {
-    uint64_t piv[64] = {0};
+// A subspace with the vectors that were added to it.
+struct Sp : Gf2Span {
     std::vector<uint64_t> basis;   // insertion order (elements() enumerates by doubling over it)
-    uint64_t reduce(uint64_t x) const {
-        for (int i = 63; i >= 0 && x; i--)
-            if (((x >> i) & 1) && piv[i]) x ^= piv[i];
-        return x;
-    }
     bool add(uint64_t x) {
-        const uint64_t r = reduce(x);
-        if (!r) return false;
-        piv[63 - __builtin_clzll(r)] = r;
+        if (!Gf2Span::add(x)) return false;
         basis.push_back(x);
         return true;
     }
-    bool contains(uint64_t x) const { return reduce(x) == 0; }
-    int dim() const { return (int)basis.size(); }
     std::vector<uint64_t> elements() const {
         std::vector<uint64_t> e{0};
         for (uint64_t b : basis) {
@@ -104,17 +93,18 @@ bool plan_group(const HPlan &p, int k0, int d, int min_L, int max_L, GroupPlan &
         for (int s = d - 1; s >= 0; s--)
             for (uint64_t z : std::vector<uint64_t>(Z[(size_t)s + 1].basis)) changed |= Z[(size_t)s].add(proj(s, z));
         for (int s = 0; s <= d; s++)
-            if (Z[(size_t)s].dim() > 5) return false;   // FUSE_MAX_STAGE = 32 values per class and stage
+            if (Z[(size_t)s].dim > 5) return false;   // FUSE_MAX_STAGE = 32 values per class and stage
     }
     if (changed) return false;
     // dataflow tables
-    for (int s = 0; s <= d; s++) gp.stage_size[s] = 1 << Z[(size_t)s].dim();
-    std::vector<std::map<uint64_t, int>> index((size_t)d + 1);
+    for (int s = 0; s <= d; s++) gp.stage_size[s] = 1 << Z[(size_t)s].dim;
     std::vector<std::vector<uint64_t>> elems((size_t)d + 1);
-    for (int s = 0; s <= d; s++) {
-        elems[(size_t)s] = Z[(size_t)s].elements();
-        for (size_t i = 0; i < elems[(size_t)s].size(); i++) index[(size_t)s][elems[(size_t)s][i]] = (int)i;
-    }
+    for (int s = 0; s <= d; s++) elems[(size_t)s] = Z[(size_t)s].elements();
+    auto number = [&](int s, uint64_t z) -> int {   // index of z in its stage (at most 32 values), -1: not one
+        const auto &e = elems[(size_t)s];
+        const auto it = std::find(e.begin(), e.end(), z);
+        return it == e.end() ? -1 : (int)(it - e.begin());
+    };
     for (int s = 0; s < d; s++) {
         const HStep &st = p.st[(size_t)(k0 + s)];
         GroupPlan::Step &gs = gp.step[s];
@@ -138,16 +128,16 @@ bool plan_group(const HPlan &p, int k0, int d, int min_L, int max_L, GroupPlan &
             const uint64_t y = members[(size_t)j];
             gs.mpar[j] = __builtin_popcountll(y & gs.lambda) & 1;
             for (int t = 0; t < gs.ntq; t++) {
-                auto it = index[(size_t)s].find(y ^ st.tqs[(size_t)t]);
-                if (it == index[(size_t)s].end()) return false;
-                gs.in_idx[j][t] = it->second;
-                seen_in[(size_t)it->second]++;
+                const int i = number(s, y ^ st.tqs[(size_t)t]);
+                if (i < 0) return false;
+                gs.in_idx[j][t] = i;
+                seen_in[(size_t)i]++;
             }
             for (int tau = 0; tau < st.m; tau++) {
-                auto it = index[(size_t)s + 1].find(tau ? (y ^ st.g) : y);
-                if (it == index[(size_t)s + 1].end()) return false;
-                gs.out_idx[j][tau] = it->second;
-                seen_out[(size_t)it->second]++;
+                const int i = number(s + 1, tau ? (y ^ st.g) : y);
+                if (i < 0) return false;
+                gs.out_idx[j][tau] = i;
+                seen_out[(size_t)i]++;
             }
         }
         for (int c : seen_in)
@@ -164,7 +154,7 @@ bool plan_group(const HPlan &p, int k0, int d, int min_L, int max_L, GroupPlan &
     Sp inter;
     for (uint64_t e : both.elements())
         if (L0.contains(e)) inter.add(e);
-    if (inter.dim() != Z[0].dim()) return false;
+    if (inter.dim != Z[0].dim) return false;
     // class-base space: columns every step of the group keeps, low unit vectors first
     std::vector<uint64_t> common;
     for (uint64_t a : p.st[(size_t)k0].tk) {
@@ -187,7 +177,7 @@ bool plan_group(const HPlan &p, int k0, int d, int min_L, int max_L, GroupPlan &
         if (a < (1ULL << L) && __builtin_popcountll(a) == 1) continue;   // already taken as a low unit vector
         if (acc.add(a)) gp.bhi.push_back(a);
     }
-    if (acc.dim() != L0.dim()) return false;
+    if (acc.dim != L0.dim) return false;
     gp.L = L;
     gp.nb = L + (int)gp.bhi.size();
     gp.z_in = elems[0];

@@ -66,25 +66,7 @@ std::string fmt(const char *f, int a, int b = 0) {
 
 }  // namespace
 
-int gf2_rank(const std::vector<uint64_t> &v) {
-    uint64_t piv[64] = {0};
-    int r = 0;
-    for (uint64_t x : v) {
-        for (int b = 63; b >= 0 && x; b--) {
-            if (!((x >> b) & 1)) continue;
-            if (!piv[b]) { piv[b] = x; r++; x = 0; break; }
-            x ^= piv[b];
-        }
-    }
-    return r;
-}
 
-bool gf2_in_span(const std::vector<uint64_t> &basis, uint64_t x) {
-    std::vector<uint64_t> v(basis);
-    int r = gf2_rank(v);
-    v.push_back(x);
-    return gf2_rank(v) == r;
-}
 
 int parse_plan_text(const char *text, size_t len, HPlan &p, std::string &err) {
     Tok t{text, text + len};
@@ -117,7 +99,7 @@ int parse_plan_text(const char *text, size_t len, HPlan &p, std::string &err) {
 
 int validate_plan(HPlan &p, std::string &err) {
     const uint64_t lim = p.R >= 64 ? ~0ULL : (1ULL << p.R);
-    std::vector<uint64_t> live{};   // basis of the live address space before the step; {0} = empty basis
+    Gf2Span live;   // the live address space before the step
     for (int k = 0; k < p.ns; k++) {
         HStep &s = p.st[(size_t)k];
         if (s.m != 1 && s.m != 2) { err = fmt("plan step %d: m = %d (must be 1 or 2)", k, s.m); return 7; }
@@ -151,34 +133,36 @@ int validate_plan(HPlan &p, std::string &err) {
             if (seen0 != 1 || seen1 != 1) { err = fmt("plan step %d: offset %d lacks exactly one x=0 and one x=1 term", k, (int)i); return 7; }
         }
         // read layout: Tkeep u basis(D) independent
-        std::vector<uint64_t> rd(s.tk);
-        std::vector<uint64_t> dbasis;
+        Gf2Span keep, rd;
+        bool independent = true;
+        for (uint64_t a : s.tk) independent = keep.add(a) && independent;
+        rd = keep;
+        Gf2Span offs;
         for (uint64_t a : d)
-            if (a && !gf2_in_span(dbasis, a)) dbasis.push_back(a);
-        rd.insert(rd.end(), dbasis.begin(), dbasis.end());
-        if (gf2_rank(rd) != (int)rd.size()) { err = fmt("plan step %d: coset slots are not disjoint (Tkeep and offsets dependent)", k); return 15; }
+            if (a && offs.add(a)) independent = rd.add(a) && independent;
+        if (!independent) { err = fmt("plan step %d: coset slots are not disjoint (Tkeep and offsets dependent)", k); return 15; }
         // the slots read must be exactly the live slots left by the previous step
-        if (rd.size() != live.size()) {
-            err = fmt("plan step %d reads a table of 2^%d entries", k, (int)rd.size()) + fmt("; the previous step left 2^%d", (int)live.size());
+        if (rd.dim != live.dim) {
+            err = fmt("plan step %d reads a table of 2^%d entries", k, rd.dim) + fmt("; the previous step left 2^%d", live.dim);
             return 15;
         }
-        for (uint64_t a : rd)
-            if (!gf2_in_span(live, a)) { err = fmt("plan step %d reads slots the previous step did not write", k); return 15; }
+        for (uint64_t a : rd.piv)
+            if (a && !live.contains(a)) { err = fmt("plan step %d reads slots the previous step did not write", k); return 15; }
         // write layout
-        std::vector<uint64_t> nl(s.tk);
+        Gf2Span nl = keep;
         if (s.m == 2) {
             if (s.g == 0) { err = fmt("plan step %d: m = 2 with g = 0", k); return 15; }
             if (d.size() > 1) {
                 if (!std::binary_search(d.begin(), d.end(), s.g)) { err = fmt("plan step %d: second output outside the coset's own slots", k); return 15; }
-            } else if (gf2_in_span(s.tk, s.g)) {
+            } else if (keep.contains(s.g)) {
                 err = fmt("plan step %d: growth slot g collides with a live slot", k);
                 return 15;
             }
-            nl.push_back(s.g);
+            nl.add(s.g);
         }
         live = nl;
     }
-    if (!live.empty()) { err = "the plan does not end with a single entry"; return 15; }
+    if (live.dim) { err = "the plan does not end with a single entry"; return 15; }
     return 0;
 }
 

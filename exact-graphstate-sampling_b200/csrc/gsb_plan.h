@@ -48,8 +48,34 @@ int parse_plan_text(const char *text, size_t len, HPlan &p, std::string &err);
 // Returns 0, GSB_E_PLAN_RANGE (7) or GSB_E_PLAN_LAYOUT (15).
 int validate_plan(HPlan &p, std::string &err);
 
-// GF(2) helpers on address vectors
-int gf2_rank(const std::vector<uint64_t> &v);
-bool gf2_in_span(const std::vector<uint64_t> &basis, uint64_t x);
+// Subspace of GF(2)^64 with a pivot basis (pivot = leading bit).
+struct Gf2Span {
+    uint64_t piv[64] = {0};
+    int dim = 0;
+    // x reduced by every pivot; looks at the set bits only
+    uint64_t reduce(uint64_t x) const {
+        for (uint64_t y = x; y;) {
+            const int i = 63 - __builtin_clzll(y);
+            if (piv[i]) { x ^= piv[i]; y ^= piv[i]; }
+            else y ^= 1ULL << i;
+        }
+        return x;
+    }
+    bool add(uint64_t x) {   // false: x was in the span
+        const uint64_t r = reduce(x);
+        if (!r) return false;
+        piv[63 - __builtin_clzll(r)] = r;
+        dim++;
+        return true;
+    }
+    bool contains(uint64_t x) const {
+        while (x) {
+            const uint64_t r = piv[63 - __builtin_clzll(x)];
+            if (!r) return false;
+            x ^= r;
+        }
+        return true;
+    }
+};
 
 }  // namespace gsb
