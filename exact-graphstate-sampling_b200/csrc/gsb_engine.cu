@@ -207,7 +207,7 @@ struct Engine {
     HPlan plan;
     int prec = 64, dev = 0, sms = 0;
     int arith = 32;                      // arithmetic of the complex64 wide-step kernels: 32 (FP32) or 64 (FP64)
-    int fuse_depth = 2;                  // chain mode: largest number of DP steps fused into one pass (1 = none)
+    int fuse_depth = 0;                  // chain mode: steps fused into one pass at most (1 = none; 0: modelled, chain_cover)
     std::vector<Op> chain_ops;           // 'chain' passes
     int hyb_K = 0;                       // gsb_set_hybrid_prefix: hybrid strings force their first hyb_K steps
     std::vector<Op> hyb_ops;             // fused 'chain' passes over those steps
@@ -353,7 +353,7 @@ struct Engine {
         c.tpb_log2 = L.tl;
         c.chunk_log2 = L.cl;
         c.nchunks = L.nchunks;
-        c.arena = arena;
+        c.arena = arena_stride();
         return c;
     }
 
@@ -366,7 +366,12 @@ struct Engine {
         while (2 * g * (unsigned)slots <= (unsigned)(SLOT_WAVES * cap)) g *= 2;
         return std::min((unsigned)grid, g);
     }
-    void *arena_mem() const { return slots == 1 ? mem : slot_mem; }
+    // The slots' arenas: the engine's own alone, or slot_mem's, or (two slots: half the memory to allocate) both.
+    void *arena_mem() const { return slots <= 2 ? mem : slot_mem; }
+    size_t arena_stride() const {
+        return slots == 2 ? (size_t)(((intptr_t)slot_mem - (intptr_t)mem) / (intptr_t)esize) : arena;
+    }
+    size_t slot_need(int nslots) const { return nslots == 1 ? 0 : (nslots == 2 ? 1 : (size_t)nslots) * arena * esize; }
 
     cudaError_t launch_step(int k, bool write, int driver, int k1, bool use_forced, bool use_unif) {
         const Launch &L = write ? lw[(size_t)k] : ln[(size_t)k];
@@ -477,8 +482,8 @@ struct Engine {
 
     cudaError_t launch_begin() {
         const int b = std::min(slots, 64);
-        if (prec == 128) k_begin<double2><<<slots / b, b, 0, stream>>>((double2 *)arena_mem(), st, arena);
-        else k_begin<float2><<<slots / b, b, 0, stream>>>((float2 *)arena_mem(), st, arena);
+        if (prec == 128) k_begin<double2><<<slots / b, b, 0, stream>>>((double2 *)arena_mem(), st, arena_stride());
+        else k_begin<float2><<<slots / b, b, 0, stream>>>((float2 *)arena_mem(), st, arena_stride());
         return cudaGetLastError();
     }
     cudaError_t launch_finish(int driver) {
@@ -567,13 +572,13 @@ struct Engine {
         const int key = kind << 16 | nslots;
         auto it = graphs.find(key);
         if (it != graphs.end()) { *out = it->second; return 0; }
-        if (nslots > 1 && (size_t)nslots * arena * esize > slot_bytes) {   // the slots' arenas, allocated on first use
+        if (slot_need(nslots) > slot_bytes) {   // the slots' arenas, allocated on first use
             GSB_CK(cudaStreamSynchronize(stream));
             for (auto kv = graphs.begin(); kv != graphs.end();)            // those that point at the old ones
                 if ((kv->first & 0xffff) > 1) { cudaGraphExecDestroy(kv->second); kv = graphs.erase(kv); }
                 else ++kv;
             free_slots();
-            if (alloc_slots((size_t)nslots * arena * esize) != cudaSuccess)
+            if (alloc_slots(slot_need(nslots)) != cudaSuccess)
                 return fail(GSB_E_ALLOC, "allocation of the slots' arenas failed");
         }
         const int driver = driver_of(kind);
@@ -690,10 +695,10 @@ static void apply_coeffs(Engine &E) {
             c.piv[b] = -1;
             c.br[b] = c.bi[b] = 0;
             c.cp[b] = 1;
-            if (f32 && std::max(n0, n1) > 0) {
+            if (std::max(n0, n1) > 0) {
                 const int pv = n0 >= n1 ? 0 : 1;
                 const std::complex<double> w(hs.Mr[b][pv], hs.Mi[b][pv]), o(hs.Mr[b][1 - pv], hs.Mi[b][1 - pv]);
-                const std::complex<double> beta = rnd(4 + b, o / w);
+                const std::complex<double> beta = f32 ? rnd(4 + b, o / w) : o / w;
                 c.piv[b] = pv;
                 c.br[b] = beta.real();
                 c.bi[b] = beta.imag();
@@ -960,7 +965,7 @@ static bool fill_group(Engine &E, const GroupPlan &gp, Op &op, int lcap = GROUP_
             a.c[b] = hs.Mr[b][0] * hs.Mr[b][0] + hs.Mi[b][0] * hs.Mi[b][0] + hs.Mr[b][1] * hs.Mr[b][1] +
                      hs.Mi[b][1] * hs.Mi[b][1];
             // factored form of a written complex64 step (FP32 arithmetic, compile-time shapes only)
-            const bool fact = kinds[s] != GK_ANY && cf.piv[b] >= 0;
+            const bool fact = kinds[s] != GK_ANY && cf.piv[b] >= 0;   // read by the factored builds only
             a.piv[b] = fact ? cf.piv[b] : -1;
             a.br[b] = fact ? cf.br[b] : 0;
             a.bi[b] = fact ? cf.bi[b] : 0;
@@ -1005,12 +1010,12 @@ static bool fill_group(Engine &E, const GroupPlan &gp, Op &op, int lcap = GROUP_
     // then are the same in every step).  By default the chain passes take it (complex64 chain 9.77 -> 9.29 ms per
     // string of pass time on the headline plan); the sampling passes measured even with it (18.88 vs 18.89 ms, some
     // passes faster, the folded ones 3 % slower), so there the autotuner times both.
-    const bool ws_ok = E.prec == 64 && E.arith == 32 && minb == 2 && L >= 9;
+    const bool ws_ok = minb == 2 && (E.prec == 64 ? E.arith == 32 && L >= 9 : L >= 8 && TR == 0);
     if (ws_req == 1 && !ws_ok) return false;
     const bool ws = ws_ok && (ws_req < 0 ? TR == 0 : ws_req == 1);
     op.ws = ws ? 1 : 0;
     op.threads = ws ? GROUP_NCT + 32 : GROUP_NCT;
-    if (E.prec == 128) op.fn = pick_group<double2, double>(op.d, op.tr);
+    if (E.prec == 128) op.fn = pick_group128(op.d, op.tr, ws);
     else if (E.arith == 64) op.fn = pick_group<float2, double>(op.d, op.tr);
     else if (minb == 3) op.fn = pick_group3(op.d, op.tr);
     else if (ws) op.fn = pick_group_ws(op.d, op.tr);
@@ -1067,7 +1072,7 @@ static bool ops_from_shapes(Engine &E, const std::vector<OpShape> &shapes, std::
 static void build_sample_ops(Engine &E) {
     E.sample_ops.clear();
     if (!E.sample_shapes.empty() && ops_from_shapes(E, E.sample_shapes, E.sample_ops)) return;
-    if (E.fuse_depth < 2) return;
+    if (E.fuse_depth == 1) return;
     const HPlan &p = E.plan;
     const int ns = p.ns;
     auto rof = [&](int k) { const HStep &h = p.st[(size_t)k]; return h.nk + (h.tqs.size() == 4 ? 2 : h.tqs.size() == 2 ? 1 : 0); };
@@ -1118,35 +1123,72 @@ static void build_sample_ops(Engine &E) {
     }
 }
 
-// Chain-mode pass list: wide steps fused greedily into groups of up to fuse_depth steps.
-// The fused 'chain' passes of steps 0 .. hyb_K - 1 (groups do not cross hyb_K), for hybrid strings whose first
-// hyb_K steps are forced.
-static void build_hyb_ops(Engine &E) {
-    E.hyb_ops.clear();
+// 'chain' passes of steps k0 .. k1 - 1.  With gsb_set_fusion's depth: wide steps fused greedily into groups of up to that
+// many.  By default: the cover with the least modelled time, entries moved over the rate of the pass's build.  The rates
+// are those of the n = 70, width-30 plan's passes (TB/s, complex64 / complex128, of a 6.5 peak): two steps 6.0 / 6.3 in the
+// warp-specialised build, 4.6 / 4.7 with a barrier per tile; three steps, which move a third less but are bound by issue,
+// 4.9 / 5.2 and 2.2 / 3.0.  A pass also costs about 8 us of latency, shared by the slots of a launch.  Per string at n = 70:
+// complex64 8.8 ms with pairs, 12.1 with greedy triples, 8.3 tuned; complex128 17.3, 18.3 and 16.1 ms.
+static void chain_cover(Engine &E, int k0, int k1, std::vector<Op> &ops) {
     const HPlan &p = E.plan;
-    for (int k = 0; k < E.hyb_K;) {
-        const HStep &hs = p.st[(size_t)k];
-        const int r = hs.nk + (hs.tqs.size() == 4 ? 2 : hs.tqs.size() == 2 ? 1 : 0);
-        bool done = false;
-        if (E.fuse_depth >= 2 && r >= GROUP_MIN_R) {
-            for (int d = std::min(std::min(E.fuse_depth, FUSE_MAX_STEPS), E.hyb_K - k); d >= 2 && !done; d--) {
-                GroupPlan gp;
-                if (!plan_group(p, k, d, 6, GROUP_MAX_L, gp)) continue;
-                Op op;
-                if (!fill_group(E, gp, op)) continue;
-                E.hyb_ops.push_back(op);
-                k += d;
-                done = true;
+    auto rof = [&](int k) { const HStep &h = p.st[(size_t)k]; return h.nk + (h.tqs.size() == 4 ? 2 : h.tqs.size() == 2 ? 1 : 0); };
+    auto single = [&](int k) {
+        Op op;
+        op.k0 = k;
+        op.d = 1;
+        op.entries = single_entries(p, k);
+        return op;
+    };
+    if (E.fuse_depth > 0) {
+        for (int k = k0; k < k1;) {
+            bool done = false;
+            if (E.fuse_depth >= 2 && rof(k) >= GROUP_MIN_R) {
+                for (int d = std::min({E.fuse_depth, FUSE_MAX_STEPS, k1 - k}); d >= 2 && !done; d--) {
+                    GroupPlan gp;
+                    if (!plan_group(p, k, d, 6, GROUP_MAX_L, gp)) continue;
+                    Op op;
+                    if (!fill_group(E, gp, op)) continue;
+                    ops.push_back(op);
+                    k += d;
+                    done = true;
+                }
+            }
+            if (!done) ops.push_back(single(k++));
+        }
+        return;
+    }
+    const double latency = 8e-6 * 6e12 / (double)E.esize / E.max_slots;   // of a launch, in entries at 6 TB/s
+    std::vector<double> cost((size_t)(k1 - k0) + 1, 0.0);
+    std::vector<Op> best((size_t)(k1 - k0));
+    for (int k = k1 - 1; k >= k0; k--) {
+        double &c = cost[(size_t)(k - k0)];
+        Op &pick = best[(size_t)(k - k0)];
+        pick = single(k);
+        // a step in a run shares the run's launch with its neighbours
+        c = pick.entries + (E.in_run(k) ? latency / 8 : latency) + cost[(size_t)(k + 1 - k0)];
+        if (rof(k) < GROUP_MIN_R) continue;
+        for (int d = 2; d <= std::min(FUSE_MAX_STEPS, k1 - k); d++) {
+            GroupPlan gp;
+            Op op;
+            if (!plan_group(p, k, d, 6, GROUP_MAX_L, gp) || !fill_group(E, gp, op)) continue;
+            const double rate = op.ws ? (d == 2 ? 1.0 : 0.82) : d == 2 ? 0.75 : E.prec == 64 ? 0.37 : 0.48;
+            const double t = op.entries / rate + latency + cost[(size_t)(k + d - k0)];
+            if (t < c) {
+                c = t;
+                pick = op;
             }
         }
-        if (!done) {
-            Op op;
-            op.k0 = k;
-            op.d = 1;
-            E.hyb_ops.push_back(op);
-            k++;
-        }
     }
+    for (int k = k0; k < k1;) {
+        ops.push_back(best[(size_t)(k - k0)]);
+        k += ops.back().d;
+    }
+}
+
+// The fused 'chain' passes of steps 0 .. hyb_K - 1, for hybrid strings whose first hyb_K steps are forced.
+static void build_hyb_ops(Engine &E) {
+    E.hyb_ops.clear();
+    chain_cover(E, 0, E.hyb_K, E.hyb_ops);
 }
 
 static void build_chain_ops(Engine &E) {
@@ -1154,32 +1196,7 @@ static void build_chain_ops(Engine &E) {
     build_sample_ops(E);
     E.chain_ops.clear();
     if (!E.chain_shapes.empty() && ops_from_shapes(E, E.chain_shapes, E.chain_ops)) return;
-    const HPlan &p = E.plan;
-    for (int k = 0; k < p.ns;) {
-        const HStep &hs = p.st[(size_t)k];
-        const int r = hs.nk + (hs.tqs.size() == 4 ? 2 : hs.tqs.size() == 2 ? 1 : 0);
-        bool done = false;
-        if (E.fuse_depth >= 2 && r >= GROUP_MIN_R) {
-            for (int d = std::min(E.fuse_depth, FUSE_MAX_STEPS); d >= 2 && !done; d--) {
-                GroupPlan gp;
-                if (!plan_group(p, k, d, 6, GROUP_MAX_L, gp)) continue;
-                Op op;
-                if (!fill_group(E, gp, op)) continue;
-                E.chain_ops.push_back(op);
-                k += d;
-                done = true;
-            }
-        }
-        if (!done) {
-            Op op;
-            op.k0 = k;
-            op.d = 1;
-            const double r1 = (double)(1ULL << r), r2 = (double)(1ULL << (hs.nk + (hs.m == 2 ? 1 : 0)));
-            op.entries = r1 + r2;
-            E.chain_ops.push_back(op);
-            k++;
-        }
-    }
+    chain_cover(E, 0, E.plan.ns, E.chain_ops);
 }
 
 static int open_plan(const char *text, size_t len, int precision, int device, gsb_engine **out) {
@@ -1911,8 +1928,8 @@ static int autotune(Engine &E, int mode, int reps) {
         const bool c64f = E.prec == 64 && E.arith == 32;
         for (int minb : {2, 3}) {
           if (minb == 3 && !c64f) continue;
-          for (int ws : {0, 1}) {   // the warp-specialised build: complex64 FP32, two CTAs per SM
-            if (ws && (minb != 2 || !c64f)) continue;
+          for (int ws : {0, 1}) {   // the warp-specialised build, two CTAs per SM
+            if (ws && minb != 2) continue;
             int lastL = -1;
             for (int lcap : {GROUP_MAX_L, GROUP_MAX_L - 1, GROUP_MAX_L - 2}) {
               OpShape sh;

@@ -750,7 +750,7 @@ __device__ __forceinline__ void group_cosets_f(const GroupArgs &ga, const GroupS
 #pragma unroll
                 for (int tau = 0; tau < 2; tau++) {
                     if (LAST) oo[tau] = TB ^ ga.ooff[j][tau];
-                    else oidx[tau] = gs.soff[j][tau];
+                    if (STS) oidx[tau] = gs.soff[j][tau];
                 }
                 member(io, oidx, oo, pc, pp ^ gs.mpar[j]);
             }
@@ -768,7 +768,7 @@ __device__ __forceinline__ void group_cosets_f(const GroupArgs &ga, const GroupS
 #pragma unroll
         for (int tau = 0; tau < 2; tau++) {
             if (LAST) oo[tau] = TB ^ ga.ooff[j][tau];
-            else oidx[tau] = gs.soff[j][tau];
+            if (STS) oidx[tau] = gs.soff[j][tau];
         }
         for (uint32_t g = g0; g < NG; g += gstride) {
             const uint32_t pc = (uint32_t)P * g;
@@ -1414,10 +1414,10 @@ __device__ __forceinline__ void group_trail64(const GroupArgs &ga, const GroupSt
     }
 }
 
-// A written step of a complex64 pass: the factored form when the step has a compile-time shape and a pivot (piv >= 0,
+// A written step of a factored pass: the factored form when the step has a compile-time shape and a pivot (piv >= 0,
 // GroupStepArgs::piv), else the general form with the scaled M row (w_r, w_i).
-template <typename T, bool SC, bool FIRST, bool LAST, bool STS, bool PK, bool UM = false>
-__device__ __forceinline__ void group_written64(const GroupArgs &ga, const GroupStepArgs &gs, float2 *__restrict__ mem,
+template <typename E, typename T, bool SC, bool FIRST, bool LAST, bool STS, bool PK, bool UM = false>
+__device__ __forceinline__ void group_written(const GroupArgs &ga, const GroupStepArgs &gs, E *__restrict__ mem,
                                                 const uint64_t TB, const int L, const uint32_t in, const uint32_t out,
                                                 const int piv, const T sc, const T br, const T bi,
                                                 const T (&w_r)[1][2], const T (&w_i)[1][2], T &nsum) {
@@ -1443,7 +1443,7 @@ __device__ __forceinline__ void group_written64(const GroupArgs &ga, const Group
         } else {
 // UM (warp-specialised passes): the common member counts 1, 2 and 4 at compile time
 #define GSB_GFN(NTQ_, H_, P_, NM_) \
-    group_cosets_f<float2, T, 2, NTQ_, H_, P_, SC, FIRST, LAST, STS, NM_>(ga, gs, mem, TB, L, in, out, sc, br, bi, nsum)
+    group_cosets_f<E, T, sizeof(E) == 8 ? 2 : 1, NTQ_, H_, P_, SC, FIRST, LAST, STS, NM_>(ga, gs, mem, TB, L, in, out, sc, br, bi, nsum)
 #define GSB_GF(NTQ_, H_, P_)                                             \
     do {                                                                 \
         if constexpr (UM) {                                              \
@@ -1478,7 +1478,7 @@ __device__ __forceinline__ void group_written64(const GroupArgs &ga, const Group
     }
     const uint32_t i1[1] = {in}, o1[1][1] = {{out}};
     T ns1[1][1] = {{0}};
-    group_cosets_any<float2, T, FIRST, LAST, STS, 1, 1, PK>(ga, gs, mem, TB, L, i1, o1, w_r, w_i, ns1);
+    group_cosets_any<E, T, FIRST, LAST, STS, 1, 1, PK>(ga, gs, mem, TB, L, i1, o1, w_r, w_i, ns1);
     nsum += ns1[0][0];
 }
 
@@ -1670,9 +1670,11 @@ __global__ void __launch_bounds__(WS ? GROUP_NCT + 32 : GROUP_NCT, MINB)
     // complex64 arena with FP32 arithmetic: the factored coefficients of each written step (pivot, beta with the
     // pass's scale, cp).  FP64 arithmetic (gsb_set_arith(64)) keeps the reference's complex64 arithmetic exactly:
     // full rotation, direct branch norms, the store the only rounding.
-    constexpr bool FACT = sizeof(E) == 8 && std::is_same<T, float>::value;
+    // Complex128 passes are factored as well, with exact coefficients: half the FP64 products per output.
+    constexpr bool C64F = sizeof(E) == 8 && std::is_same<T, float>::value;
+    constexpr bool FACT = C64F || sizeof(E) == 16;
     // folded sampling passes (GroupArgs::fold) exist only in the two-CTA build: the three-CTA register cap spills them
-    constexpr bool FOLD = FACT && PK && D == 2 && TR == 1 && MINB == 2;
+    constexpr bool FOLD = C64F && PK && D == 2 && TR == 1 && MINB == 2;
     static_assert(!WS || (FACT && MINB == 2), "warp-specialised build: complex64 FP32, two CTAs per SM");
     int fpiv[D];
     T fsc[D], fbr[D], fbi[D];
@@ -1698,7 +1700,7 @@ __global__ void __launch_bounds__(WS ? GROUP_NCT + 32 : GROUP_NCT, MINB)
     // reduced sums: the written steps' norms, then (TR) the trailing step's (n0, n1, 0, 0), or its shared sums
     // (A, B, Re C, Im C) when it takes the complex64 shared-sum form
     constexpr int ND = D + 4 * TR;
-    const bool trail_abc = FACT && TR == 1 && ga.st[D].kind != GK_ANY;
+    const bool trail_abc = C64F && TR == 1 && ga.st[D].kind != GK_ANY;
     double acc[ND];
 #pragma unroll
     for (int s = 0; s < ND; s++) acc[s] = 0;
@@ -1793,12 +1795,11 @@ __global__ void __launch_bounds__(WS ? GROUP_NCT + 32 : GROUP_NCT, MINB)
         // written steps: the first reads the input tile, the last writes the arena (and keeps its stage for the
         // trailing step); the input buffer is free once the first step is done: tile it + 2 goes there
         if constexpr (FACT) {
-            float2 *m64 = reinterpret_cast<float2 *>(mem);
             if (D == 1)
-                group_written64<T, true, true, true, TR == 1, PK, WS && !PK>(ga, ga.st[0], m64, TB, L, tin[0], sm.mid[1], fpiv[0],
+                group_written<E, T, true, true, true, TR == 1, PK, WS && !PK>(ga, ga.st[0], mem, TB, L, tin[0], sm.mid[1], fpiv[0],
                                                                  fsc[0], fbr[0], fbi[0], w[0], wj[0], ns[0][0][0]);
             else
-                group_written64<T, true, true, false, true, PK, WS && !PK>(ga, ga.st[0], m64, TB, L, tin[0], sm.mid[1], fpiv[0],
+                group_written<E, T, true, true, false, true, PK, WS && !PK>(ga, ga.st[0], mem, TB, L, tin[0], sm.mid[1], fpiv[0],
                                                                fsc[0], fbr[0], fbi[0], w[0], wj[0], ns[0][0][0]);
         } else if (D == 1) {
             group_cosets_any<E, T, true, true, TR == 1, 1, 1, PK>(ga, ga.st[0], mem, TB, L, tin, m1o, w[0], wj[0], ns[0]);
@@ -1819,24 +1820,23 @@ __global__ void __launch_bounds__(WS ? GROUP_NCT + 32 : GROUP_NCT, MINB)
             issued++;
         }
         if constexpr (FACT) {
-            float2 *m64 = reinterpret_cast<float2 *>(mem);
             if (FOLD && ga.fold) {   // the written stage is not kept: the trailing step folds it
-                group_written64<T, false, false, true, false, PK, WS && !PK>(ga, ga.st[1], m64, TB, L, sm.mid[1], 0u,
+                group_written<E, T, false, false, true, false, PK, WS && !PK>(ga, ga.st[1], mem, TB, L, sm.mid[1], 0u,
                                                                  fpiv[D > 1 ? 1 : 0], fsc[D > 1 ? 1 : 0],
                                                                  fbr[D > 1 ? 1 : 0], fbi[D > 1 ? 1 : 0],
                                                                  w[D > 1 ? 1 : 0], wj[D > 1 ? 1 : 0], ns[D > 1 ? 1 : 0][0][0]);
             } else if (D == 2) {
-                group_written64<T, false, false, true, TR == 1, PK, WS && !PK>(ga, ga.st[1], m64, TB, L, sm.mid[1], sm.mid[2],
+                group_written<E, T, false, false, true, TR == 1, PK, WS && !PK>(ga, ga.st[1], mem, TB, L, sm.mid[1], sm.mid[2],
                                                                    fpiv[D > 1 ? 1 : 0], fsc[D > 1 ? 1 : 0],
                                                                    fbr[D > 1 ? 1 : 0], fbi[D > 1 ? 1 : 0],
                                                                    w[D > 1 ? 1 : 0], wj[D > 1 ? 1 : 0], ns[D > 1 ? 1 : 0][0][0]);
             } else if (D == 3) {
-                group_written64<T, false, false, false, true, PK, WS && !PK>(ga, ga.st[1], m64, TB, L, sm.mid[1], sm.mid[2],
+                group_written<E, T, false, false, false, true, PK, WS && !PK>(ga, ga.st[1], mem, TB, L, sm.mid[1], sm.mid[2],
                                                                  fpiv[D > 1 ? 1 : 0], fsc[D > 1 ? 1 : 0],
                                                                  fbr[D > 1 ? 1 : 0], fbi[D > 1 ? 1 : 0],
                                                                  w[D > 1 ? 1 : 0], wj[D > 1 ? 1 : 0], ns[D > 1 ? 1 : 0][0][0]);
                 if constexpr (!WS) __syncthreads();
-                group_written64<T, false, false, true, false, PK, WS && !PK>(ga, ga.st[2], m64, TB, L, sm.mid[2], 0u,
+                group_written<E, T, false, false, true, false, PK, WS && !PK>(ga, ga.st[2], mem, TB, L, sm.mid[2], 0u,
                                                                  fpiv[D > 2 ? 2 : 0], fsc[D > 2 ? 2 : 0],
                                                                  fbr[D > 2 ? 2 : 0], fbi[D > 2 ? 2 : 0],
                                                                  w[D > 2 ? 2 : 0], wj[D > 2 ? 2 : 0], ns[D > 2 ? 2 : 0][0][0]);
@@ -1861,9 +1861,9 @@ __global__ void __launch_bounds__(WS ? GROUP_NCT + 32 : GROUP_NCT, MINB)
                 }
             }
             if (done) {
-            } else if (FACT && trail_abc)
-                group_trail64<E, T, PK>(ga, ga.st[D], TB, L, tmid[0], tabc);
-            else
+            } else if (trail_abc) {
+                if constexpr (C64F) group_trail64<E, T, PK>(ga, ga.st[D], TB, L, tmid[0], tabc);
+            } else
                 group_cosets_any<E, T, false, false, false, 1, 2, PK>(ga, ga.st[D], mem, TB, L, tmid, none2, tr_r, tr_i, nt);
         }
         if constexpr (!WS) __syncthreads();

@@ -1,4 +1,4 @@
-// The complex64 FP32 fused-pass kernels (k_group<float2, float, ...>) are instantiated in translation units of their
+// The complex64 FP32 and the complex128 fused-pass kernels are instantiated in translation units of their
 // own, so the library's objects compile in parallel; these return their addresses for cudaLaunchKernel.
 #pragma once
 
@@ -9,5 +9,6 @@ void *pick_group_ws(int d, int tr);    // warp-specialised, tiles of 2^9 classes
 void *pick_group_ws_three();           // the same, three steps (gsb_group_ws3.cu)
 void *pick_group_ws_trailing(int d);   // the same with a trailing step, tr = 1 (gsb_group_wst.cu)
 void *pick_group3(int d, int tr);      // three CTAs per SM (gsb_group3.cu)
+void *pick_group128(int d, int tr, bool ws);   // complex128 (gsb_group128.cu)
 
 }  // namespace gsb

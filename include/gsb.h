@@ -113,8 +113,9 @@ int gsb_synchronize(gsb_engine *e);
  * e.g. a framework's current stream, so events recorded there bracket the engine's kernels. */
 int gsb_set_stream(gsb_engine *e, void *cuda_stream);
 /* 'chain' mode fuses runs of up to `depth` consecutive wide steps (tables of >= 2^12 entries) into one pass over
- * the arena: the intermediate tables of a group live in shared-memory tiles only.  depth 1 disables fusion;
- * default 2.  Results are those of the unfused steps up to rounding. */
+ * the arena: the intermediate tables of a group live in shared-memory tiles only.  depth 1 disables fusion; without
+ * this call the library picks passes of one to three steps by their modelled time.  Results are those of the unfused
+ * steps up to rounding. */
 int gsb_set_fusion(gsb_engine *e, int depth);
 /* Autotune the pass lists on this device: every candidate pass (one step; 2 or 3 fused steps; for sampling with or
  * without the next step's branch norms; tiles of up to 2^8, 2^9 or 2^10 classes) is timed alone with CUDA events,

@@ -1,6 +1,6 @@
 """Calls that carry several strings or samples per launch (slots): every mode against the oracle, at string counts
-around the slot counts (1, 2, 3, one more than a power of two) and at widths from a single small run (width 6) over
-fused passes (width 16) to the one-slot arenas; zero-probability strings beside live ones; and the fused passes'
+around the slot counts (1, 2, 3, one more than a power of two) and at widths from a single small run (width 6) to
+fused passes of two and three steps (width 18); zero-probability strings beside live ones; and the fused passes'
 bounded wait running out in several slots at once."""
 import os
 import tempfile
@@ -30,7 +30,7 @@ def instances():
 
 
 @pytest.mark.parametrize("prec", [128, 64])
-@pytest.mark.parametrize("n,count", [(18, 1), (18, 2), (18, 67), (29, 5), (33, 3), (38, 1), (38, 2), (38, 9)])
+@pytest.mark.parametrize("n,count", [(18, 1), (18, 2), (18, 67), (29, 5), (33, 3), (38, 1), (38, 2), (38, 9), (44, 3)])
 def test_counts_against_oracle(instances, n, count, prec):
     import gsb
     import workloads
