@@ -226,6 +226,8 @@ struct Engine {
     double *d_unif = nullptr, *d_cond = nullptr, *d_logp = nullptr, *d_aux = nullptr;
     void *d_dump = nullptr;
     size_t dump_bytes = 0;
+    void *d_small = nullptr;             // gsb_resume: slice descriptors
+    size_t small_bytes = 0;
     std::vector<StepArgs> args;
     // runs of small steps (gsb_run.cuh): maximal parts of consecutive steps, and each step's part (-1: none)
     struct RunPart {
@@ -248,6 +250,7 @@ struct Engine {
     size_t slot_bytes = 0;
     cudaMemPool_t slot_pool = nullptr;
     std::map<void *, int> occ;
+    std::map<std::pair<void *, size_t>, int> group_occ;
     // complex128 re-evaluation of unlikely strings (gsb_set_guard): the engine that re-evaluates this one's strings
     // whose log2 Pr + ns < guard_lx, and the engine this one re-evaluates for
     Engine *guard = nullptr, *guarded = nullptr;
@@ -281,6 +284,7 @@ struct Engine {
         cudaFree(d_logp);
         cudaFree(d_aux);
         cudaFree(d_dump);
+        cudaFree(d_small);
         if (own_stream) cudaStreamDestroy(own_stream);
     }
 
@@ -298,6 +302,18 @@ struct Engine {
         if (e != cudaSuccess) { cudaGetLastError(); slot_mem = nullptr; return e; }
         slot_bytes = bytes;
         return e;
+    }
+
+    // CTAs per SM of a fused pass, 0 when its kernel cannot be set up; asked once per kernel and size (the covers of a
+    // plan's steps try some hundred passes).
+    int group_occupancy(void *fn, int threads, size_t smem) {
+        const auto key = std::make_pair(fn, smem);
+        const auto it = group_occ.find(key);
+        if (it != group_occ.end()) return it->second;
+        int nb = 0;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GROUP_SMEM_BUDGET) != cudaSuccess) nb = 0;
+        else if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem) != cudaSuccess || nb < 1) nb = 1;
+        return group_occ[key] = nb;
     }
 
     int occupancy(void *fn, int block) {
@@ -1020,10 +1036,8 @@ static bool fill_group(Engine &E, const GroupPlan &gp, Op &op, int lcap = GROUP_
     else if (minb == 3) op.fn = pick_group3(op.d, op.tr);
     else if (ws) op.fn = pick_group_ws(op.d, op.tr);
     else op.fn = pick_group_f32(op.d, op.tr);
-    if (cudaFuncSetAttribute(op.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GROUP_SMEM_BUDGET) != cudaSuccess)
-        return false;
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, op.fn, op.threads, op.smem) != cudaSuccess || nb < 1) nb = 1;
+    const int nb = E.group_occupancy(op.fn, op.threads, op.smem);
+    if (nb < 1) return false;
     op.cap = nb * E.sms;
     op.grid = (int)std::min<uint64_t>(op.ntiles, (uint64_t)op.cap);
     op.entries = gp.entries_moved;
@@ -1682,19 +1696,32 @@ int gsb_resume(gsb_engine *e, const int8_t *forced, int K, uint64_t seed, int64_
         dptr[(size_t)s] = (const char *)E->d_dump + tbytes * (size_t)s;
         GSB_CK(cudaMemcpyAsync((void *)dptr[(size_t)s], dumps[s], tbytes, cudaMemcpyHostToDevice, E->stream));
     }
-    void *small = nullptr;
-    const size_t sbytes = (size_t)nslices * (8 + 8 + 8 + 16);
-    GSB_CK(cudaMallocAsync(&small, sbytes, E->stream));
-    char *sp = (char *)small;
-    GSB_CK(cudaMemcpyAsync(sp, dptr.data(), (size_t)nslices * 8, cudaMemcpyHostToDevice, E->stream));
-    GSB_CK(cudaMemcpyAsync(sp + (size_t)nslices * 8, f.data(), (size_t)nslices * 8, cudaMemcpyHostToDevice, E->stream));
-    GSB_CK(cudaMemcpyAsync(sp + (size_t)nslices * 16, cs.data(), (size_t)nslices * 8, cudaMemcpyHostToDevice, E->stream));
-    GSB_CK(cudaMemcpyAsync(sp + (size_t)nslices * 24, tperm.data(), (size_t)nslices * 16, cudaMemcpyHostToDevice, E->stream));
+    // the slices' pointers, scales and translations: one copy into a buffer that the engine keeps (an allocation from the
+    // device's default pool and its release cost 0.4 ms a call, more than the kernels of a width-16 resume)
+    const size_t ns8 = (size_t)nslices * 8;
+    std::vector<char> small(5 * ns8);
+    memcpy(small.data(), dptr.data(), ns8);
+    memcpy(small.data() + ns8, f.data(), ns8);
+    memcpy(small.data() + 2 * ns8, cs.data(), ns8);
+    memcpy(small.data() + 3 * ns8, tperm.data(), 2 * ns8);
+    if (E->small_bytes < small.size()) {
+        cudaFree(E->d_small);
+        E->d_small = nullptr;
+        E->small_bytes = 0;
+        if (cudaMalloc(&E->d_small, small.size()) != cudaSuccess) {
+            cudaGetLastError();
+            E->d_small = nullptr;
+            return fail(GSB_E_ALLOC, "allocation of the slice descriptors failed");
+        }
+        E->small_bytes = small.size();
+    }
+    GSB_CK(cudaMemcpyAsync(E->d_small, small.data(), small.size(), cudaMemcpyHostToDevice, E->stream));
+    const char *sp = (const char *)E->d_small;
     ResumeArgs ra;
     ra.dumps = (const void *const *)sp;
-    ra.f = (const double *)(sp + (size_t)nslices * 8);
-    ra.cshift = (const uint64_t *)(sp + (size_t)nslices * 16);
-    ra.tperm = (const int *)(sp + (size_t)nslices * 24);
+    ra.f = (const double *)(sp + ns8);
+    ra.cshift = (const uint64_t *)(sp + 2 * ns8);
+    ra.tperm = (const int *)(sp + 3 * ns8);
     ra.nsl = nslices;
     ra.ntq = ntq;
     ra.K = K;
@@ -1729,7 +1756,6 @@ int gsb_resume(gsb_engine *e, const int8_t *forced, int K, uint64_t seed, int64_
         GSB_CK(cudaMemcpyAsync(hb.data(), E->d_bits, (size_t)ns, cudaMemcpyDeviceToHost, E->stream));
         GSB_CK(cudaMemcpyAsync(hc.data(), E->d_cond, (size_t)ns * 8, cudaMemcpyDeviceToHost, E->stream));
     }
-    GSB_CK(cudaFreeAsync(small, E->stream));
     GSB_CK(cudaStreamSynchronize(E->stream));
     for (int k = 0; k < ns; k++) bits[k] = k < K ? forced[k] : hb[(size_t)k];
     if (cond)
