@@ -15,7 +15,6 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
-#include <mutex>
 #include <random>
 #include <string>
 #include <tuple>
@@ -160,49 +159,6 @@ static uint32_t group_smem_bytes(int D, int TR, const int (&ssz)[4], int L, bool
     return D == 3 ? group_smem<E, T, 3, 0>(ssz, L).total : group_smem<E, T, 2, 0>(ssz, L).total;
 }
 
-// Device memory of the slots' arenas.  cudaMalloc and cudaFree cost about 25 us per MB here, more than a whole call
-// on a fresh engine (50 samples of width 19: 1.4 ms, 13 ms with 512 MB to allocate), so the arenas come from a CUDA
-// memory pool per device (stream ordered, safe with several threads) that keeps at most SLOT_BYTES of freed memory for
-// the next engine and returns it when the last engine that used it closes.
-class SlotPool {
-    struct Dev {
-        cudaMemPool_t pool = nullptr;
-        int users = 0;
-    };
-    std::mutex mu;
-    std::map<int, Dev> devs;
-
-public:
-    static SlotPool &get() {
-        static SlotPool *p = new SlotPool();   // never destroyed: engines may close while the process exits
-        return *p;
-    }
-    cudaError_t open(int dev, cudaMemPool_t *pool) {
-        std::lock_guard<std::mutex> lock(mu);
-        Dev &d = devs[dev];
-        if (!d.pool) {
-            cudaMemPoolProps props;
-            memset(&props, 0, sizeof props);
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            cudaError_t e = cudaMemPoolCreate(&d.pool, &props);
-            if (e != cudaSuccess) { d.pool = nullptr; return e; }
-            uint64_t keep = SLOT_BYTES;
-            e = cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-            if (e != cudaSuccess) return e;
-        }
-        d.users++;
-        *pool = d.pool;
-        return cudaSuccess;
-    }
-    void close(int dev) {
-        std::lock_guard<std::mutex> lock(mu);
-        Dev &d = devs[dev];
-        if (--d.users == 0) cudaMemPoolTrimTo(d.pool, 0);
-    }
-};
-
 struct Engine {
     HPlan plan;
     int prec = 64, dev = 0, sms = 0;
@@ -237,8 +193,8 @@ struct Engine {
     std::vector<RunPart> parts;
     std::vector<int> part_of;
     std::vector<RunStep> rsteps;
-    RunStep *d_rs = nullptr;             // device copies, read by the runs
-    StepArgs *d_args = nullptr;          // args, then a one-entry table
+    StepArgs *d_args = nullptr;          // device copies, read by the runs: args and a one-entry table,
+    RunStep *d_rs = nullptr;             // then rsteps (one allocation)
     bool args_dirty = true;              // args changed since the device copies were last written
     std::vector<Launch> lw, ln;
     std::map<int, cudaGraphExec_t> graphs;   // key: graph kind << 16 | slots
@@ -248,7 +204,6 @@ struct Engine {
     int used_slots = 1;                  // slots of the launches queued since the device's error flags were read
     void *slot_mem = nullptr;            // the arenas of launches that carry several items
     size_t slot_bytes = 0;
-    cudaMemPool_t slot_pool = nullptr;
     std::map<void *, int> occ;
     std::map<std::pair<void *, size_t>, int> group_occ;
     // complex128 re-evaluation of unlikely strings (gsb_set_guard): the engine that re-evaluates this one's strings
@@ -270,11 +225,9 @@ struct Engine {
         if (guarded) guarded->guard = nullptr;
         DevGuard g(dev);
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
-        cudaFree(mem);   // waits for the device, so nothing queued uses the slots' arenas any more
-        free_slots();
-        if (slot_pool) SlotPool::get().close(dev);
+        cudaFree(mem);
+        cudaFree(slot_mem);
         cudaFree(d_args);
-        cudaFree(d_rs);
         cudaFree(st);
         cudaFree(partials);
         cudaFree(d_forced);
@@ -286,22 +239,6 @@ struct Engine {
         cudaFree(d_dump);
         cudaFree(d_small);
         if (own_stream) cudaStreamDestroy(own_stream);
-    }
-
-    void free_slots() {
-        if (!slot_mem) return;
-        cudaFreeAsync(slot_mem, own_stream);
-        cudaStreamSynchronize(own_stream);
-        slot_mem = nullptr;
-        slot_bytes = 0;
-    }
-    cudaError_t alloc_slots(size_t bytes) {
-        cudaError_t e = slot_pool ? cudaSuccess : SlotPool::get().open(dev, &slot_pool);
-        if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&slot_mem, bytes, slot_pool, own_stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(own_stream);
-        if (e != cudaSuccess) { cudaGetLastError(); slot_mem = nullptr; return e; }
-        slot_bytes = bytes;
-        return e;
     }
 
     // CTAs per SM of a fused pass, 0 when its kernel cannot be set up; asked once per kernel and size (the covers of a
@@ -593,9 +530,16 @@ struct Engine {
             for (auto kv = graphs.begin(); kv != graphs.end();)            // those that point at the old ones
                 if ((kv->first & 0xffff) > 1) { cudaGraphExecDestroy(kv->second); kv = graphs.erase(kv); }
                 else ++kv;
-            free_slots();
-            if (alloc_slots(slot_need(nslots)) != cudaSuccess)
+            cudaFree(slot_mem);
+            slot_mem = nullptr;
+            slot_bytes = 0;
+            const size_t bytes = slot_need(nslots);
+            if (cudaMalloc(&slot_mem, bytes) != cudaSuccess) {
+                cudaGetLastError();
+                slot_mem = nullptr;
                 return fail(GSB_E_ALLOC, "allocation of the slots' arenas failed");
+            }
+            slot_bytes = bytes;
         }
         const int driver = driver_of(kind);
         const bool use_forced = kind != 2, use_unif = kind >= 2;
@@ -845,8 +789,9 @@ static int make_args(Engine &E) {
     maxgrid = std::max(maxgrid, E.max_slots > 1 ? std::max((size_t)E.sms * 8 * SLOT_WAVES, (size_t)E.max_slots)
                                                 : (size_t)E.sms * 8);
     GSB_CK(cudaMalloc(&E.partials, maxgrid * PARTIAL_SUMS * sizeof(double)));
-    GSB_CK(cudaMalloc(&E.d_args, ((size_t)p.ns + 1) * sizeof(StepArgs)));
-    GSB_CK(cudaMalloc(&E.d_rs, std::max<size_t>(E.rsteps.size(), 1) * sizeof(RunStep)));
+    const size_t sa_bytes = ((size_t)p.ns + 1) * sizeof(StepArgs);   // one allocation: each costs 0.3 ms
+    GSB_CK(cudaMalloc(&E.d_args, sa_bytes + E.rsteps.size() * sizeof(RunStep)));
+    E.d_rs = reinterpret_cast<RunStep *>(reinterpret_cast<char *>(E.d_args) + sa_bytes);
     StepArgs end;
     memset(&end, 0, sizeof end);
     end.ntq = 1;
