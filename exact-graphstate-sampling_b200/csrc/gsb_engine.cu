@@ -113,11 +113,12 @@ static_assert(sizeof(GroupArgs) + sizeof(void *) + sizeof(Ctx) <= 4096, "fused-p
 
 // Items per launch (slots, gsb_kernels.cuh): at most MAX_SLOTS, with arenas of at most SLOT_BYTES together.  The bound
 // is well above the 126 MB L2: the narrow steps at both ends of an item cost time, not bandwidth, and more items
-// share it.  50 strings of width 19, complex128 'chain', at 64 / 128 / 256 / 512 MB: 1.91 / 1.36 / 0.91 / 0.78 ms (one at a
-// time: 14 ms); 9 strings of width 24, complex64: 3.06 / 2.30 / 1.82 / 1.57 ms.  Blocks of a launch: SLOT_WAVES rounds of
-// what the device holds; 1 and 2 measured alike, 4 was 10 % slower at width 19.
+// share it.  At 256 MB / 512 MB / 1 GB / 2 GB: 9 strings of width 24 in complex64 1.69 / 1.50 / 1.06 / 1.06 ms, 12 hybrid
+// proposals of width 25 4.98 / 3.90 / 3.58 / 3.57 ms, 8 complex128 strings 5.38 / 4.60 / 4.08 / 3.85 ms, 50 samples of width 19
+// in complex128 1.56 / 1.41 / 1.42 / 1.42 ms.  Blocks of a launch: SLOT_WAVES rounds of what the device holds; 1 and 2
+// measured alike, 4 was 10 % slower at width 19.
 constexpr int MAX_SLOTS = 1024, SLOT_WAVES = 2;
-constexpr size_t SLOT_BYTES = (size_t)512 << 20;
+constexpr size_t SLOT_BYTES = (size_t)1024 << 20;
 
 struct Op {
     int k0 = 0, d = 1, tr = 0, lcap = 0;   // lcap: the tile-size cap the pass was built with (fused passes)
