@@ -49,13 +49,20 @@ struct GradCtx {
     int ns;
 };
 
-// One step inside a pass: member j of a class reads values in[j][t] of its stage and writes values out[j][tau] of the
-// next one; its class sign is parity(class & lam) ^ mpar[j].
+// Shape of a step's dataflow: with m = 2 and every x = 1 term in the other output than its offset's x = 0 term, the host
+// orders the offsets so that the x = 0 terms of the first NTQ - H go to output 0 and those of the last H to output 1
+// (relabelling the outputs where that makes H <= NTQ / 2).  RK_ANY: everything else, with runtime tables.
+enum { RK_ANY = 0, RK_1_0, RK_2_0, RK_2_1, RK_4_0, RK_4_1, RK_4_2 };
+
+// One step inside a pass.  Every stage's values are numbered so that member j reads values ntq j + t; out[j][tau]: the
+// number of its outputs in the next stage (m j + tau in the last one).  Class sign: parity(class & lam) ^ bit j of mpar.
 struct GradStep {
-    int k, nmem, ntq, m;
-    int tau0, tau1, par;     // bit t: offset t's x = 0 / x = 1 output, x = 1 sign
+    int k, kind, nmem, ntq, m;
+    int tau0, tau1;          // bit t: offset t's x = 0 / x = 1 output
+    uint32_t mpar;
+    double sg[4];            // sign of offset t's x = 1 term
     uint64_t lam;
-    unsigned char in[16][4], out[16][2], mpar[16];
+    unsigned char out[16][2];
 };
 
 // A pass: 2^nb classes; class p has index XOR of cin[j] (cout[j]) over the bits of p in the table read (written), and
@@ -126,72 +133,157 @@ __device__ __forceinline__ MRow step_row(const GradStep &s, const GradCtx &g) {
 // This thread's slot i.
 __device__ __forceinline__ double2 &slot(double2 *sh, int i) { return sh[i * GRAD_THREADS + (int)threadIdx.x]; }
 
-// Coset sums of a member: X[tau] of the x = 0 terms, Z[tau] of the x = 1 terms with their term signs.
+// Member j's values, inputs in slots a..
 template <int NTQ>
+__device__ __forceinline__ void member_values(double2 *sh, int a, int j, double2 (&v)[NTQ]) {
+#pragma unroll
+    for (int t = 0; t < NTQ; t++) v[t] = slot(sh, a + NTQ * j + t);
+}
+
+// Coset sums of a shaped member: X[tau] of the x = 0 terms, Z[tau] of the signed x = 1 terms (H = 0: X[0] and Z[1] only).
+template <int NTQ, int H>
 __device__ __forceinline__ void member_sums(const GradStep &s, const double2 (&v)[NTQ], double2 (&X)[2], double2 (&Z)[2]) {
-    X[0] = X[1] = Z[0] = Z[1] = make_double2(0, 0);
 #pragma unroll
     for (int t = 0; t < NTQ; t++) {
-        if ((s.tau0 >> t) & 1) X[1] = cadd(X[1], v[t]);
-        else X[0] = cadd(X[0], v[t]);
-        const double2 w = csign(v[t], (s.par >> t) & 1);
-        if ((s.tau1 >> t) & 1) Z[1] = cadd(Z[1], w);
-        else Z[0] = cadd(Z[0], w);
+        const int o = t < NTQ - H ? 0 : 1;
+        const bool first = t == 0 || (H > 0 && t == NTQ - H);
+        X[o] = first ? v[t] : cadd(X[o], v[t]);
+        Z[1 - o] = first ? make_double2(s.sg[t] * v[t].x, s.sg[t] * v[t].y)
+                         : make_double2(fma(s.sg[t], v[t].x, Z[1 - o].x), fma(s.sg[t], v[t].y, Z[1 - o].y));
     }
 }
 
-// A step forward on one class: values in slots a.. to f(index, value).
-template <int NTQ, typename F>
+// A shaped step forward on one class: values in slots a.., output tau of member j to f(j, tau, value).  NM: members, 0
+// for a runtime count; known counts leave every index a constant.
+template <int NTQ, int H, int NM, typename F>
 __device__ __forceinline__ void class_fwd(const GradStep &s, const MRow &m, double2 *sh, int a, int cpar, F f) {
-    for (int j = 0; j < s.nmem; j++) {
+    auto member = [&](int j) {
         double2 v[NTQ], X[2], Z[2];
+        member_values<NTQ>(sh, a, j, v);
+        member_sums<NTQ, H>(s, v, X, Z);
+        const double2 m1 = csign(m.m1, (cpar ^ (int)(s.mpar >> j)) & 1);
+        f(j, 0, H == 0 ? cmul(m.m0, X[0]) : cfma(m.m0, X[0], cmul(m1, Z[0])));
+        f(j, 1, H == 0 ? cmul(m1, Z[1]) : cfma(m.m0, X[1], cmul(m1, Z[1])));
+    };
+    if constexpr (NM > 0) {
 #pragma unroll
-        for (int t = 0; t < NTQ; t++) v[t] = slot(sh, a + s.in[j][t]);
-        member_sums<NTQ>(s, v, X, Z);
-        const double2 m1 = csign(m.m1, (cpar ^ s.mpar[j]) & 1);
-        f(s.out[j][0], cfma(m.m0, X[0], cmul(m1, Z[0])));
-        if (s.m == 2) f(s.out[j][1], cfma(m.m0, X[1], cmul(m1, Z[1])));
+        for (int j = 0; j < NM; j++) member(j);
+    } else {
+        for (int j = 0; j < s.nmem; j++) member(j);
     }
 }
 
-// A step in reverse on one class: inputs in slots a.., lambda of its outputs in slots l..; lambda of its inputs to
-// f(index, value), the sums for dZ/dM to acc.
-template <int NTQ, typename F>
-__device__ __forceinline__ void class_bwd(const GradStep &s, const MRow &m, double2 *sh, int a, int l, int cpar,
-                                          double2 (&acc)[2], F f) {
-    for (int j = 0; j < s.nmem; j++) {
+// A shaped step in reverse on one class: inputs in slots a.., lambda of output tau of member j in slot lam(j, tau);
+// lambda of its offset t to f(j, t, value), the sums for dZ/dM to acc.
+template <int NTQ, int H, int NM, typename L, typename F>
+__device__ __forceinline__ void class_bwd(const GradStep &s, const MRow &m, double2 *sh, int a, int cpar, double2 (&acc)[2],
+                                          L lam, F f) {
+    auto member = [&](int j) {
         double2 v[NTQ], X[2], Z[2];
-#pragma unroll
-        for (int t = 0; t < NTQ; t++) v[t] = slot(sh, a + s.in[j][t]);
-        const double2 l0 = slot(sh, l + s.out[j][0]);
-        const double2 l1 = s.m == 2 ? slot(sh, l + s.out[j][1]) : make_double2(0, 0);
-        member_sums<NTQ>(s, v, X, Z);
-        const int cs = (cpar ^ s.mpar[j]) & 1;
-        acc[0] = cfma(l0, X[0], cfma(l1, X[1], acc[0]));
-        acc[1] = cadd(acc[1], csign(cfma(l0, Z[0], cmul(l1, Z[1])), cs));
+        member_values<NTQ>(sh, a, j, v);
+        const double2 l0 = slot(sh, lam(j, 0)), l1 = slot(sh, lam(j, 1));
+        member_sums<NTQ, H>(s, v, X, Z);
+        const int cs = (cpar ^ (int)(s.mpar >> j)) & 1;
         const double2 m1 = csign(m.m1, cs);
-        const double2 a0 = cmul(m.m0, l0), a1 = cmul(m.m0, l1), b0 = cmul(m1, l0), b1 = cmul(m1, l1);
+        double2 p[2], q[2];   // m0 lambda and m1 lambda of the outputs that x = 0 / x = 1 terms reach
+        if (H == 0) {
+            acc[0] = cfma(l0, X[0], acc[0]);
+            acc[1] = cfma(csign(l1, cs), Z[1], acc[1]);
+            p[0] = cmul(m.m0, l0);
+            q[1] = cmul(m1, l1);
+        } else {
+            acc[0] = cfma(l0, X[0], cfma(l1, X[1], acc[0]));
+            acc[1] = cfma(csign(l0, cs), Z[0], cfma(csign(l1, cs), Z[1], acc[1]));
+            p[0] = cmul(m.m0, l0);
+            p[1] = cmul(m.m0, l1);
+            q[0] = cmul(m1, l0);
+            q[1] = cmul(m1, l1);
+        }
 #pragma unroll
         for (int t = 0; t < NTQ; t++) {
-            const double2 x = (s.tau0 >> t) & 1 ? a1 : a0, y = (s.tau1 >> t) & 1 ? b1 : b0;
-            f(s.in[j][t], cadd(x, csign(y, (s.par >> t) & 1)));
+            const int o = t < NTQ - H ? 0 : 1;
+            f(j, t, make_double2(fma(s.sg[t], q[1 - o].x, p[o].x), fma(s.sg[t], q[1 - o].y, p[o].y)));
+        }
+    };
+    if constexpr (NM > 0) {
+#pragma unroll
+        for (int j = 0; j < NM; j++) member(j);
+    } else {
+        for (int j = 0; j < s.nmem; j++) member(j);
+    }
+}
+
+// Any step: runtime offsets and outputs (one or two).
+template <typename F>
+__device__ __forceinline__ void class_fwd_any(const GradStep &s, const MRow &m, double2 *sh, int a, int cpar, F f) {
+    for (int j = 0; j < s.nmem; j++) {
+        double2 X[2], Z[2];
+        X[0] = X[1] = Z[0] = Z[1] = make_double2(0, 0);
+        for (int t = 0; t < s.ntq; t++) {
+            const double2 v = slot(sh, a + s.ntq * j + t), w = make_double2(s.sg[t] * v.x, s.sg[t] * v.y);
+            if ((s.tau0 >> t) & 1) X[1] = cadd(X[1], v);
+            else X[0] = cadd(X[0], v);
+            if ((s.tau1 >> t) & 1) Z[1] = cadd(Z[1], w);
+            else Z[0] = cadd(Z[0], w);
+        }
+        const double2 m1 = csign(m.m1, (cpar ^ (int)(s.mpar >> j)) & 1);
+        f(j, 0, cfma(m.m0, X[0], cmul(m1, Z[0])));
+        if (s.m == 2) f(j, 1, cfma(m.m0, X[1], cmul(m1, Z[1])));
+    }
+}
+template <typename L, typename F>
+__device__ __forceinline__ void class_bwd_any(const GradStep &s, const MRow &m, double2 *sh, int a, int cpar, double2 (&acc)[2],
+                                              L lam, F f) {
+    for (int j = 0; j < s.nmem; j++) {
+        const double2 l0 = slot(sh, lam(j, 0)), l1 = s.m == 2 ? slot(sh, lam(j, 1)) : make_double2(0, 0);
+        const int cs = (cpar ^ (int)(s.mpar >> j)) & 1;
+        const double2 m1 = csign(m.m1, cs), s0 = csign(l0, cs), s1 = csign(l1, cs);
+        const double2 p0 = cmul(m.m0, l0), p1 = cmul(m.m0, l1), q0 = cmul(m1, l0), q1 = cmul(m1, l1);
+        for (int t = 0; t < s.ntq; t++) {
+            const double2 v = slot(sh, a + s.ntq * j + t), w = make_double2(s.sg[t] * v.x, s.sg[t] * v.y);
+            const bool u0 = (s.tau0 >> t) & 1, u1 = (s.tau1 >> t) & 1;
+            acc[0] = cfma(u0 ? l1 : l0, v, acc[0]);
+            acc[1] = cfma(u1 ? s1 : s0, w, acc[1]);
+            const double2 p = u0 ? p1 : p0, q = u1 ? q1 : q0;
+            f(j, t, make_double2(fma(s.sg[t], q.x, p.x), fma(s.sg[t], q.y, p.y)));
         }
     }
 }
 
+#define GSB_RK(KIND, CALL, NTQ, H)                  \
+    case KIND:                                      \
+        switch (s.nmem) {                           \
+            case 1: CALL(NTQ, H, 1); break;         \
+            case 2: CALL(NTQ, H, 2); break;         \
+            case 4: CALL(NTQ, H, 4); break;         \
+            default: CALL(NTQ, H, 0); break;        \
+        }                                           \
+        break;
+#define GSB_RKS(CALL, ANY)                          \
+    switch (s.kind) {                               \
+        GSB_RK(RK_1_0, CALL, 1, 0)                  \
+        GSB_RK(RK_2_0, CALL, 2, 0)                  \
+        GSB_RK(RK_2_1, CALL, 2, 1)                  \
+        GSB_RK(RK_4_0, CALL, 4, 0)                  \
+        GSB_RK(RK_4_1, CALL, 4, 1)                  \
+        GSB_RK(RK_4_2, CALL, 4, 2)                  \
+        default: ANY;                               \
+    }
 template <typename F>
-__device__ __forceinline__ void class_fwd_any(const GradStep &s, const MRow &m, double2 *sh, int a, int cpar, F f) {
-    if (s.ntq == 4) class_fwd<4>(s, m, sh, a, cpar, f);
-    else if (s.ntq == 2) class_fwd<2>(s, m, sh, a, cpar, f);
-    else class_fwd<1>(s, m, sh, a, cpar, f);
+__device__ __forceinline__ void step_fwd(const GradStep &s, const MRow &m, double2 *sh, int a, int cpar, F f) {
+#define GSB_CALL(NTQ, H, NM) class_fwd<NTQ, H, NM>(s, m, sh, a, cpar, f)
+    GSB_RKS(GSB_CALL, class_fwd_any(s, m, sh, a, cpar, f))
+#undef GSB_CALL
 }
-template <typename F>
-__device__ __forceinline__ void class_bwd_any(const GradStep &s, const MRow &m, double2 *sh, int a, int l, int cpar,
-                                              double2 (&acc)[2], F f) {
-    if (s.ntq == 4) class_bwd<4>(s, m, sh, a, l, cpar, acc, f);
-    else if (s.ntq == 2) class_bwd<2>(s, m, sh, a, l, cpar, acc, f);
-    else class_bwd<1>(s, m, sh, a, l, cpar, acc, f);
+template <typename L, typename F>
+__device__ __forceinline__ void step_bwd(const GradStep &s, const MRow &m, double2 *sh, int a, int cpar, double2 (&acc)[2],
+                                         L lam, F f) {
+#define GSB_CALL(NTQ, H, NM) class_bwd<NTQ, H, NM>(s, m, sh, a, cpar, acc, lam, f)
+    GSB_RKS(GSB_CALL, class_bwd_any(s, m, sh, a, cpar, acc, lam, f))
+#undef GSB_CALL
 }
+#undef GSB_RKS
+#undef GSB_RK
 
 __global__ void k_gr_begin(double2 *T, size_t stride) { T[blockIdx.y * stride] = make_double2(1.0, 0.0); }
 
@@ -210,18 +302,18 @@ __global__ void __launch_bounds__(GRAD_THREADS) k_gr_fwd(const GradPass g, const
         copies_landed();
         const uint64_t p = w.p;
         const uint32_t o = w.out;
+        const int s1 = g.ssz[0], om = g.st[D - 1].m;
+        auto store = [&](int j, int tau, double2 v) { out[o ^ g.zout[om * j + tau]] = v; };
         if (D == 1) {
-            class_fwd_any(g.st[0], ma, sh, 0, __popcll(p & g.st[0].lam), [&](int i, double2 v) { out[o ^ g.zout[i]] = v; });
+            step_fwd(g.st[0], ma, sh, 0, __popcll(p & g.st[0].lam), store);
         } else {
-            const int s1 = g.ssz[0];
-            class_fwd_any(g.st[0], ma, sh, 0, __popcll(p & g.st[0].lam), [&](int i, double2 v) { slot(sh, s1 + i) = v; });
+            step_fwd(g.st[0], ma, sh, 0, __popcll(p & g.st[0].lam),
+                     [&](int j, int tau, double2 v) { slot(sh, s1 + g.st[0].out[j][tau]) = v; });
         }
         w.next(g);   // the first stage is done: the next class's values arrive while the second step runs
         if (w.more())
             for (int i = 0; i < g.ssz[0]; i++) copy16(&slot(sh, i), in + (w.in ^ g.zin[i]));
-        if (D == 2)
-            class_fwd_any(g.st[1], mb, sh, g.ssz[0], __popcll(p & g.st[D - 1].lam),
-                          [&](int i, double2 v) { out[o ^ g.zout[i]] = v; });
+        if (D == 2) step_fwd(g.st[D - 1], mb, sh, s1, __popcll(p & g.st[D - 1].lam), store);
     }
 }
 
@@ -235,9 +327,10 @@ __global__ void k_gr_final(const double2 *T, size_t t_stride, double2 *Lam, size
 __global__ void k_gr_next(int *item, int bs) { *item += bs; }
 __global__ void k_gr_set_item(int *item, int v) { *item = v; }
 
-// Measured on the width-20 workload (128 strings, loss and gradient): 23.1 -> 9.6 ms a call with both sweeps in two-step
-// passes.  The widest reverse pass moves 1.3 GB in 0.34 ms and is bound by issue (65 % of the slots, 900 instructions per
-// class of four values); five blocks per SM (96 registers, no spills) took 4 % off against four, six and eight spill.
+// Measured on the width-20 workload (128 strings, loss and gradient): 23.1 -> 9.4 ms a call with both sweeps in two-step
+// passes and runtime tables (the widest reverse pass bound by issue: 900 instructions per class of four values, 0.34 ms for
+// 1.3 GB), 8.4 ms with each step's code compiled for its shape and member count (470 instructions, 0.24 ms, 5.4 TB/s: the
+// reads of T and lambda).  Five blocks per SM (96 registers) took 4 % off against four; six and eight spill.
 //
 // Reverse pass: lambda after the pass (`lo`) and the table before it (T) to lambda before it (`li`), and
 // dZ/dM_k[b_k][x] of its steps.  Deterministic reduction: per-block partials, the last block sums them in block order
@@ -264,15 +357,18 @@ __global__ void __launch_bounds__(GRAD_THREADS, 5) k_gr_bwd(const GradPass g, co
         copies_landed();
         const int pa = __popcll(w.p & g.st[0].lam);
         const uint32_t in = w.in;
-        auto store = [&](int i, double2 v) { li[in ^ g.zin[i]] = v; };
+        const int na = g.st[0].ntq, nb = g.st[D - 1].ntq, om = g.st[D - 1].m;
+        auto store = [&](int j, int t, double2 v) { li[in ^ g.zin[na * j + t]] = v; };
+        auto after = [&](int j, int tau) { return s2 + om * j + tau; };
         if (D == 1) {
-            class_bwd_any(g.st[0], ma, sh, 0, s2, pa, acc[0], store);
+            step_bwd(g.st[0], ma, sh, 0, pa, acc[0], after, store);
         } else {
-            // a stage-1 slot holds the step's input until the member that reads it, then its lambda
-            auto keep = [&](int i, double2 v) { slot(sh, s1 + i) = v; };
-            class_fwd_any(g.st[0], ma, sh, 0, pa, keep);
-            class_bwd_any(g.st[D - 1], mb, sh, s1, s2, __popcll(w.p & g.st[D - 1].lam), acc[D - 1], keep);
-            class_bwd_any(g.st[0], ma, sh, 0, s1, pa, acc[0], store);
+            // a stage-1 slot holds the second step's input until the member that reads it, then its lambda
+            auto mid = [&](int j, int tau) { return s1 + g.st[0].out[j][tau]; };
+            step_fwd(g.st[0], ma, sh, 0, pa, [&](int j, int tau, double2 v) { slot(sh, mid(j, tau)) = v; });
+            step_bwd(g.st[D - 1], mb, sh, s1, __popcll(w.p & g.st[D - 1].lam), acc[D - 1], after,
+                     [&](int j, int t, double2 v) { slot(sh, s1 + nb * j + t) = v; });
+            step_bwd(g.st[0], ma, sh, 0, pa, acc[0], mid, store);
         }
     }
     __shared__ double red[4 * D][GRAD_THREADS / 32];
@@ -356,28 +452,54 @@ static bool make_pass(const HPlan &p, const GroupPlan &gp, GradPass &g) {
         g.cin[j] = before(cols[(size_t)j]);
         g.cout[j] = after(cols[(size_t)j]);
     }
-    for (int i = 0; i < gp.stage_size[0]; i++) g.zin[i] = before(gp.z_in[(size_t)i]);
-    for (int i = 0; i < gp.stage_size[gp.d]; i++) g.zout[i] = after(gp.z_out[(size_t)i]);
+    std::vector<int> number[3];   // of the plan's stage values: member-major in the step that reads them
+    int perm[2][4], swp[2];
     for (int s = 0; s < gp.d; s++) {
         const HStep &hs = p.st[(size_t)(gp.k0 + s)];
         const GroupPlan::Step &q = gp.step[s];
         GradStep &a = g.st[s];
+        bool shaped = q.m == 2;
+        int h = 0;
+        for (int t = 0; t < q.ntq; t++) {
+            shaped = shaped && hs.tau1[t] == 1 - hs.tau0[t];
+            h += hs.tau0[t];
+        }
+        swp[s] = shaped && 2 * h > q.ntq;
+        if (swp[s]) h = q.ntq - h;
+        int n = 0;
+        for (int out = 0; out < 2; out++)
+            for (int t = 0; t < q.ntq; t++)
+                if (!shaped ? out == 0 : (hs.tau0[t] ^ swp[s]) == out) perm[s][n++] = t;
+        a.kind = RK_ANY;
+        if (shaped && q.ntq == 1) a.kind = RK_1_0;
+        else if (shaped && q.ntq == 2) a.kind = h == 0 ? RK_2_0 : RK_2_1;
+        else if (shaped && q.ntq == 4) a.kind = h == 0 ? RK_4_0 : h == 1 ? RK_4_1 : RK_4_2;
         a.k = gp.k0 + s;
         a.nmem = q.nmem;
         a.ntq = q.ntq;
         a.m = q.m;
         for (int t = 0; t < q.ntq; t++) {
-            a.tau0 |= hs.tau0[t] << t;
-            a.tau1 |= hs.tau1[t] << t;
-            a.par |= hs.par[t] << t;
+            a.tau0 |= (hs.tau0[perm[s][t]] ^ swp[s]) << t;
+            a.tau1 |= (hs.tau1[perm[s][t]] ^ swp[s]) << t;
+            a.sg[t] = hs.par[perm[s][t]] ? -1.0 : 1.0;
         }
         for (int j = 0; j < gp.nb; j++)
             a.lam |= (uint64_t)(__builtin_popcountll(cols[(size_t)j] & q.lambda) & 1) << j;
+        number[s].assign((size_t)gp.stage_size[s], 0);
         for (int j = 0; j < q.nmem; j++) {
-            for (int t = 0; t < q.ntq; t++) a.in[j][t] = (unsigned char)q.in_idx[j][t];
-            for (int tau = 0; tau < q.m; tau++) a.out[j][tau] = (unsigned char)q.out_idx[j][tau];
-            a.mpar[j] = (unsigned char)q.mpar[j];
+            a.mpar |= (uint32_t)(q.mpar[j] & 1) << j;
+            for (int t = 0; t < q.ntq; t++) number[s][(size_t)q.in_idx[j][perm[s][t]]] = q.ntq * j + t;
         }
+    }
+    for (int i = 0; i < gp.stage_size[0]; i++) g.zin[number[0][(size_t)i]] = before(gp.z_in[(size_t)i]);
+    for (int s = 0; s < gp.d; s++) {
+        const GroupPlan::Step &q = gp.step[s];
+        for (int j = 0; j < q.nmem; j++)
+            for (int tau = 0; tau < q.m; tau++) {
+                const int old = q.out_idx[j][tau ^ swp[s]];
+                if (s + 1 < gp.d) g.st[s].out[j][tau] = (unsigned char)number[s + 1][(size_t)old];
+                else g.zout[q.m * j + tau] = after(gp.z_out[(size_t)old]);
+            }
     }
     return true;
 }
