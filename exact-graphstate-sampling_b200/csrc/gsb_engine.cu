@@ -355,8 +355,9 @@ struct Engine {
         ra.aux = d_aux;
         int nk = 0;
         for (int k = k0; k < k1; k++) nk = std::max(nk, args[(size_t)k].nk);
-        // four cosets of the widest step per thread, at least a warp and at most 512 threads
-        const unsigned T = 1u << std::min(9, std::max(5, nk - 2));
+        // two cosets of the widest step per thread where bits are drawn (their sums then stay in registers), else four; at
+        // least a warp and at most 512 threads
+        const unsigned T = 1u << std::min(9, std::max(5, nk - (norm ? 1 : 2)));
         Ctx c = ctx(driver, k_end, Launch(), use_forced, use_unif);
         void *memp = arena_mem();
         void *kargs[] = {&ra, &memp, &c};

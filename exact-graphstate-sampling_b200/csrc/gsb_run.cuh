@@ -4,7 +4,7 @@
 // their own, or as steps over the arena in global memory, they are bound by latency alone: the arena version of this
 // kernel took 2.5 us per step (two block barriers around scalar work in one thread, and dependent loads of the
 // descriptor, the state and the table), 54 us for each end of a 'chain' string at width 19 (now 40 for 64 strings side by
-// side), 115 us for a 20-step 'prob' (now 77; both cold), and a call of 1024 strings at n = 20 0.53 ms (now 0.12).  What
+// side), 115 us for a 20-step 'prob' (now 65; both cold), and a call of 1024 strings at n = 20 0.53 ms (now 0.11).  What
 // is left is the latency of FP64 sums, shuffles and instruction fetches, step after step.  Here
 //   * the live table sits in shared memory in compact coordinates: the addresses that the run's steps touch span a
 //     subspace of dimension D <= RUN_DIM, the host picks a basis of it (the widest step's columns first, so that its
@@ -154,6 +154,93 @@ __device__ __forceinline__ void run_pass(const RunStep &s, E *tab, int bv, doubl
     else run_pass_n<E, 1, WRITE>(s, tab, bv, sc, sum);
 }
 
+// A step whose bit is drawn from its branch norms, with at most two cosets per thread: the cosets' sums stay in registers
+// between the norms and the write, which then reads nothing and forms no sums again (one prob at n = 20: 74 -> 67 us a
+// call, 100 samples 155 -> 148).
+struct CosetSums {
+    double x[2][2], z[2][2];   // [tau][re, im]: x = 0 and signed x = 1 sums
+    uint32_t base;
+};
+template <typename E, int NTQ>
+__device__ __forceinline__ void coset_sums(const RunStep &s, const E *tab, uint32_t per, CosetSums (&c)[2]) {
+    const uint32_t T = blockDim.x, tid = threadIdx.x;
+    const int lt = __ffs((int)T) - 1;
+    uint32_t lo = 0;
+#pragma unroll
+    for (int j = 0; j < 9; j++)
+        if ((tid >> j) & 1) lo ^= s.tk[j];
+    const int plo = __popc(tid & s.rhoc);
+    E v[2][NTQ];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        if ((uint32_t)u >= per) break;
+        c[u].base = u ? lo ^ s.tk[lt] : lo;
+#pragma unroll
+        for (int t = 0; t < NTQ; t++) v[u][t] = tab[c[u].base ^ s.tq[t]];
+    }
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        if ((uint32_t)u >= per) break;
+        const int pc = plo ^ (u ? (int)(s.rhoc >> lt) : 0);
+#pragma unroll
+        for (int tau = 0; tau < 2; tau++) c[u].x[tau][0] = c[u].x[tau][1] = c[u].z[tau][0] = c[u].z[tau][1] = 0;
+#pragma unroll
+        for (int t = 0; t < NTQ; t++) {
+            const double xr = (double)v[u][t].x, xi = (double)v[u][t].y;
+            if ((s.tau0 >> t) & 1) { c[u].x[1][0] += xr; c[u].x[1][1] += xi; }
+            else { c[u].x[0][0] += xr; c[u].x[0][1] += xi; }
+            const int neg = (pc ^ (s.par >> t)) & 1;
+            const double yr = flip_sign(xr, neg), yi = flip_sign(xi, neg);
+            if ((s.tau1 >> t) & 1) { c[u].z[1][0] += yr; c[u].z[1][1] += yi; }
+            else { c[u].z[0][0] += yr; c[u].z[0][1] += yi; }
+        }
+    }
+}
+template <typename E>
+__device__ __forceinline__ void coset_sums_any(const RunStep &s, const E *tab, uint32_t per, CosetSums (&c)[2]) {
+    if (s.ntq == 4) coset_sums<E, 4>(s, tab, per, c);
+    else if (s.ntq == 2) coset_sums<E, 2>(s, tab, per, c);
+    else coset_sums<E, 1>(s, tab, per, c);
+}
+// Output tau of a coset under row b, times sc.
+__device__ __forceinline__ void coset_out(const RunStep &s, const CosetSums &c, int b, int tau, double sc, double &r, double &i) {
+    const double m0r = s.M[b][0][0], m0i = s.M[b][0][1], m1r = s.M[b][1][0], m1i = s.M[b][1][1];
+    const double xr = c.x[tau][0], xi = c.x[tau][1], zr = c.z[tau][0], zi = c.z[tau][1];
+    r = (m0r * xr - m0i * xi + m1r * zr - m1i * zi) * sc;
+    i = (m0r * xi + m0i * xr + m1r * zi + m1i * zr) * sc;
+}
+__device__ __forceinline__ void coset_norms(const RunStep &s, uint32_t per, const CosetSums (&c)[2], double (&sum)[2]) {
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        if ((uint32_t)u >= per) break;
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+#pragma unroll
+            for (int tau = 0; tau < 2; tau++) {
+                if (tau >= s.m) break;
+                double r, i;
+                coset_out(s, c[u], b, tau, 1.0, r, i);
+                sum[b] += r * r + i * i;
+            }
+    }
+}
+template <typename E>
+__device__ __forceinline__ void coset_write(const RunStep &s, E *tab, uint32_t per, const CosetSums (&c)[2], int bv, double sc,
+                                            double (&sum)[2]) {
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        if ((uint32_t)u >= per) break;
+#pragma unroll
+        for (int tau = 0; tau < 2; tau++) {
+            if (tau >= s.m) break;
+            double r, i;
+            coset_out(s, c[u], bv, tau, sc, r, i);
+            store_entry(tab + (tau ? c[u].base ^ s.g : c[u].base), r, i);
+            sum[0] += r * r + i * i;
+        }
+    }
+}
+
 // Shared memory of a run: the table, two step descriptors, the warp sums, and per step two saved scalars, the uniform
 // and the bit.
 inline size_t run_smem(int dim, int nsteps, size_t esize) {
@@ -222,6 +309,10 @@ __global__ void __launch_bounds__(RUN_THREADS) k_run(const RunArgs ra, E *__rest
         if (tid < WORDS) next = reinterpret_cast<const uint64_t *>(ra.rs + k + 1)[tid];
         double sum[2] = {0, 0};
         const int f = bit[k];
+        const uint32_t N = 1u << s.nk;
+        const bool pair = N <= 2u * (uint32_t)T;   // at most two cosets per thread
+        const uint32_t per = (uint32_t)tid >= N ? 0 : N > (uint32_t)T ? 2 : 1;
+        CosetSums c[2];
         if (cx.driver == DRV_CHAIN1) {
             run_pass<true>(s, tab, f, sc, sum);
             if (tid < WORDS) reinterpret_cast<uint64_t *>(steps + ((k + 1) & 1))[tid] = next;
@@ -236,7 +327,12 @@ __global__ void __launch_bounds__(RUN_THREADS) k_run(const RunArgs ra, E *__rest
             ek = (ex - 1) >> 1;
             sc = ldexp(1.0, -ek);
         } else if (cx.driver == DRV_CHAIN) {
-            run_pass<false>(s, tab, 0, 1.0, sum);
+            if (pair) {
+                coset_sums_any(s, tab, per, c);
+                coset_norms(s, per, c, sum);
+            } else {
+                run_pass<false>(s, tab, 0, 1.0, sum);
+            }
             run_sum<2>(sum, red, buf);
             n0 = sum[0];
             n1 = sum[1];
@@ -247,7 +343,8 @@ __global__ void __launch_bounds__(RUN_THREADS) k_run(const RunArgs ra, E *__rest
             if (!(pb > 0)) { died = k; break; }
             sc = rsqrt(bv ? n1 : n0);
             sum[0] = 0;
-            run_pass<true>(s, tab, bv, sc, sum);
+            if (pair) coset_write(s, tab, per, c, bv, sc, sum);
+            else run_pass<true>(s, tab, bv, sc, sum);
             if (tid < WORDS) reinterpret_cast<uint64_t *>(steps + ((k + 1) & 1))[tid] = next;
             if (k + 1 < n || ra.finish) {
                 __syncthreads();
@@ -258,15 +355,22 @@ __global__ void __launch_bounds__(RUN_THREADS) k_run(const RunArgs ra, E *__rest
             }
         } else {   // DRV_HYBRID
             if (f >= 0) bv = f;
-            if (f < 0 && ra.norm) {
-                run_pass<false>(s, tab, 0, 1.0, sum);
+            const bool drawn = f < 0 && ra.norm;
+            if (drawn) {
+                if (pair) {
+                    coset_sums_any(s, tab, per, c);
+                    coset_norms(s, per, c, sum);
+                } else {
+                    run_pass<false>(s, tab, 0, 1.0, sum);
+                }
                 run_sum<2>(sum, red, buf);
                 n0 = sum[0];
                 n1 = sum[1];
                 bv = un[k] < n1 / (n0 + n1);
                 sum[0] = 0;
             }
-            run_pass<true>(s, tab, bv, rsqrt(prev), sum);
+            if (drawn && pair) coset_write(s, tab, per, c, bv, rsqrt(prev), sum);
+            else run_pass<true>(s, tab, bv, rsqrt(prev), sum);
             if (tid < WORDS) reinterpret_cast<uint64_t *>(steps + ((k + 1) & 1))[tid] = next;
             double nb[1] = {sum[0]};
             run_sum<1>(nb, red, buf);
