@@ -166,6 +166,7 @@ struct Engine {
     int arith = 32;                      // arithmetic of the complex64 wide-step kernels: 32 (FP32) or 64 (FP64)
     int fuse_depth = 0;                  // chain mode: steps fused into one pass at most (1 = none; 0: modelled, chain_cover)
     std::vector<Op> chain_ops;           // 'chain' passes
+    bool prob_by_chain = false;          // 'prob' strings run the 'chain' passes (conserves)
     int hyb_K = 0;                       // gsb_set_hybrid_prefix: hybrid strings force their first hyb_K steps
     std::vector<Op> hyb_ops;             // fused 'chain' passes over those steps
     std::vector<Op> sample_ops;          // 'prob' / 'sample' passes (build_sample_ops)
@@ -622,12 +623,36 @@ static std::complex<double> round_diffused(std::complex<double> v, double &cum) 
     return best;
 }
 
+// Whether every step's branch norms add up to twice the table's norm: its M is unitary, and the map from a coset's values
+// to its x = 0 and signed x = 1 sums is sqrt(2) times an isometry (true of every plan of a graph state, since the
+// probabilities of a bit's two values add up to the prefix's).  Then the normalised two-pass chain's n_b / (n_0 + n_1) is
+// the one-pass chain's n_b / (2 |T|^2), and 'prob' needs no branch norms: its strings run the 'chain' passes.
+static bool conserves(const HPlan &p) {
+    for (const HStep &s : p.st) {
+        const std::complex<double> a(s.Mr[0][0], s.Mi[0][0]), b(s.Mr[0][1], s.Mi[0][1]), c(s.Mr[1][0], s.Mi[1][0]),
+            d(s.Mr[1][1], s.Mi[1][1]);
+        const double eps = 1e-14;   // of a conditional, far below complex128's accumulated rounding of a string
+        if (!(std::fabs(std::norm(a) + std::norm(c) - 1) <= eps && std::fabs(std::norm(b) + std::norm(d) - 1) <= eps &&
+              std::abs(std::conj(a) * b + std::conj(c) * d) <= eps))
+            return false;
+        for (size_t t = 0; t < s.tqs.size(); t++)
+            for (size_t u = t + 1; u < s.tqs.size(); u++) {
+                int g = s.tau0[t] == s.tau0[u];
+                if (s.tau1[t] == s.tau1[u]) g += (s.par[t] ^ s.par[u]) & 1 ? -1 : 1;
+                if (g) return false;
+            }
+    }
+    return true;
+}
+
 // The coefficients a complex64 engine with FP32 arithmetic uses: M entries (single-step kernels, the fused passes'
 // general shape) and, per bit, the factored step's pivot (the larger of the row's two entries), its ratio
 // beta = M[b][1-piv] / M[b][piv] and cp = |M[b][piv]|^2 (exact), all rounded by round_diffused in step order.
 // Other engines use the plan's M as it is (FP64 arithmetic, or complex128).
+static bool conserves(const HPlan &p);
 static void apply_coeffs(Engine &E) {
     const HPlan &p = E.plan;
+    E.prob_by_chain = conserves(p);
     const bool f32 = E.prec == 64 && E.arith == 32;
     E.c32.assign((size_t)p.ns, Engine::Coef32());
     // running sums of Re d per (role, exact value): roles 0-3 the M entries [b][x], 4-5 the ratios of bit b
@@ -1205,7 +1230,7 @@ static int open_plan(const char *text, size_t len, int precision, int device, gs
     if ((e = cudaMalloc(&E->d_unif, cap * ns * 8)) != cudaSuccess) return cuda_fail(e, "buffers");
     if ((e = cudaMalloc(&E->d_cond, cap * ns * 8)) != cudaSuccess) return cuda_fail(e, "buffers");
     if ((e = cudaMalloc(&E->d_logp, cap * 8)) != cudaSuccess) return cuda_fail(e, "buffers");
-    if ((e = cudaMalloc(&E->d_aux, cap * 8)) != cudaSuccess) return cuda_fail(e, "buffers");
+    if ((e = cudaMalloc(&E->d_aux, cap * 16)) != cudaSuccess) return cuda_fail(e, "buffers");
     if ((e = cudaMemsetAsync(E->d_forced, 0, cap * ns, E->stream)) != cudaSuccess) return cuda_fail(e, "buffers");
     rc = make_args(*E);
     if (rc) { std::string m = g_err; delete E; return fail(rc, m); }
@@ -1343,6 +1368,39 @@ static int forced_batch(Engine *E, int kind, const int8_t *bits, int64_t nstr, d
     return 0;
 }
 
+// 'prob' strings (log2 Pr), by the 'chain' passes where the plan conserves probability.  The two-pass chain ends a string
+// as impossible where 1 - p rounds to 0; the one-pass chain leaves rounding noise there, so strings with a conditional
+// below PROB_FLOOR (no possible branch of a circuit comes near it) run the two passes as well.
+constexpr double PROB_FLOOR = 1.0 / ((uint64_t)1 << 40);
+static int prob_batch(Engine *E, const int8_t *bits, int64_t nstr, double *log2p) {
+    if (!E->prob_by_chain) return forced_batch(E, 1, bits, nstr, log2p, nullptr);
+    const int ns = E->plan.ns;
+    std::vector<double> got(2 * (size_t)std::min<int64_t>(nstr, E->cap));   // per string: log2 Pr, least conditional
+    std::vector<int64_t> idx;
+    for (int64_t off = 0; off < nstr; off += E->cap) {
+        const int64_t nb = std::min<int64_t>(E->cap, nstr - off);
+        if (ns) GSB_CK(cudaMemcpyAsync(E->d_forced, bits + off * ns, (size_t)(nb * ns), cudaMemcpyHostToDevice, E->stream));
+        int rc = E->run_graph_items(0, nb);
+        if (rc) return rc;
+        k_least_cond<<<(unsigned)nb, 32, 0, E->stream>>>(E->d_cond, ns, E->d_logp, E->d_aux);
+        GSB_CK(cudaGetLastError());
+        GSB_CK(cudaMemcpyAsync(got.data(), E->d_aux, (size_t)nb * 16, cudaMemcpyDeviceToHost, E->stream));
+        GSB_CK(cudaStreamSynchronize(E->stream));
+        if ((rc = check_device(E))) return rc;
+        for (int64_t i = 0; i < nb; i++) {
+            log2p[off + i] = got[(size_t)(2 * i)];
+            if (!(got[(size_t)(2 * i + 1)] >= PROB_FLOOR)) idx.push_back(off + i);
+        }
+    }
+    if (idx.empty()) return 0;
+    std::vector<int8_t> b(idx.size() * (size_t)std::max(ns, 1));
+    std::vector<double> lp(idx.size());
+    for (size_t j = 0; j < idx.size(); j++) memcpy(b.data() + j * (size_t)ns, bits + idx[j] * ns, (size_t)ns);
+    if (int rc = forced_batch(E, 1, b.data(), (int64_t)idx.size(), lp.data(), nullptr)) return rc;
+    for (size_t j = 0; j < idx.size(); j++) log2p[idx[j]] = lp[j];
+    return 0;
+}
+
 // ---- complex128 guard (gsb_set_guard) ----
 // A complex64 log2 Pr carries a rounding error that grows as 1 / sqrt(Pr 2^ns) (the table's rounding is absolute
 // in units of its norm, and an unlikely string's amplitude is a small remainder of it); strings below the guard's
@@ -1367,7 +1425,8 @@ static int guard_host(Engine *E, int kind, const int8_t *bits, int64_t nstr, dou
     Engine *G = E->guard;
     {
         DevGuard g(G->dev);
-        int rc = forced_batch(G, kind, b.data(), (int64_t)m, lp.data(), cond ? cd.data() : nullptr);
+        int rc = kind == 1 ? prob_batch(G, b.data(), (int64_t)m, lp.data())
+                           : forced_batch(G, kind, b.data(), (int64_t)m, lp.data(), cond ? cd.data() : nullptr);
         if (rc) return rc;
     }
     for (size_t j = 0; j < m; j++) {
@@ -1435,7 +1494,7 @@ int gsb_prob(gsb_engine *e, const int8_t *bits, int64_t nstr, double *log2p) {
     DevGuard g(E->dev);
     int rc = check_bits(bits, nstr, E->plan.ns, false);
     if (rc) return rc;
-    if ((rc = forced_batch(E, 1, bits, nstr, log2p, nullptr))) return rc;
+    if ((rc = prob_batch(E, bits, nstr, log2p))) return rc;
     return guard_host(E, 1, bits, nstr, log2p, nullptr);
 }
 

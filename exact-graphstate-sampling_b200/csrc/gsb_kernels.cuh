@@ -653,6 +653,18 @@ static __global__ void k_set_item(DevState *st, int first, int nitems) {
     st[slot].nitems = nitems;
 }
 
+// Each item's log2 Pr and the least conditional of its row (one warp each; 0 for a NaN among them), as pairs.
+static __global__ void k_least_cond(const double *cond, int ns, const double *logp, double *out) {
+    const double *c = cond + (size_t)blockIdx.x * (size_t)ns;
+    double v = 1;
+    for (int k = (int)threadIdx.x; k < ns; k += 32) v = c[k] >= v ? v : c[k] == c[k] ? c[k] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (threadIdx.x == 0) {
+        out[2 * blockIdx.x] = logp[blockIdx.x];
+        out[2 * blockIdx.x + 1] = v;
+    }
+}
+
 // Hybrid item whose first K steps are forced and ran as 'chain' passes (DRV_CHAIN1): from here on the run_steps
 // conventions (gsamp2.cpp:77-98).  The stored table is the true one times 2^-lsc, which is run_steps' logscale;
 // log2 Pr of the prefix is log2 |table|^2 + 2 lsc - K.  The forced bits of the prefix go to the output row.

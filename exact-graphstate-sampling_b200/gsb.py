@@ -224,7 +224,7 @@ class Engine:
 
     # --- modes ---
     def prob(self, strings):
-        """'prob': log2 Pr of each string (two passes per step)."""
+        """'prob': log2 Pr of each string (two passes per step, or one where every step conserves probability)."""
         b = as_bits(strings, self.ns)
         out = np.zeros(len(b), np.float64)
         if len(b):

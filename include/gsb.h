@@ -68,7 +68,8 @@ int gsb_info(const gsb_engine *e, int *n, int *nsteps, int *R, int *precision);
 /* qubit (vertex) of each step, nsteps entries */
 int gsb_step_vertices(const gsb_engine *e, int *out);
 
-/* 'prob': log2 Pr of each string, normalised two-pass chain (gsamp2.cpp:39-55, 217-223). */
+/* 'prob': log2 Pr of each string, the normalised two-pass chain's (gsamp2.cpp:39-55, 217-223).  Where every step conserves
+ * probability (M unitary, as in every plan of a circuit) the one-pass chain gives the same number and is what runs. */
 int gsb_prob(gsb_engine *e, const int8_t *bits, int64_t nstr, double *log2p);
 
 /* 'chain': one pass per step; log2 Pr and every conditional Pr(b_k | b_1..b_{k-1}) (gsamp2.cpp:56-70, 217-222).
