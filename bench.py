@@ -594,6 +594,11 @@ def _form_line(form, metric, value, unit, hib, extra, emit=True):
     return d
 
 
+def _pair_entries(steps, reads=1):
+    """Table entries of a sweep over `steps` in passes of two: `reads` tables read and one written per pass."""
+    return sum(reads * (1 << steps[i]["r"]) + (1 << steps[min(i + 1, len(steps) - 1)]["rn"]) for i in range(0, len(steps), 2))
+
+
 def run_form_batch(args, emit=True):
     """Batched uneven workload: one persistent launch over all (instance, prefix) items."""
     import numpy as np
@@ -623,19 +628,16 @@ def run_form_batch(args, emit=True):
     fin = np.isfinite(lp128)
     d = np.abs(lp - lp128)[fin]
     nstr = lp.size
-    # algorithmic bytes: per item one prefix sweep plus nsuf suffix sweeps (one write pass per step), the
-    # snapshot and its restores
+    # algorithmic bytes: per item one prefix sweep plus nsuf suffix sweeps, in passes of two steps that read and write
+    # the table once (the kernel fuses up to three where a class's values fit, and none on narrow tables)
     E = 8
     byt = 0
     for w, K in zip(bw["instances"], bw["K"]):
         st = w["steps"]
-        pre = sum((1 << s["r"]) + (1 << s["rn"]) for s in st[:K])
-        suf = sum((1 << s["r"]) + (1 << s["rn"]) for s in st[K:])
-        snap = 1 << st[K]["r"]
-        byt += 16 * E * (pre + 4 * suf + 2 * snap + 3 * 2 * snap)
+        byt += 16 * E * (_pair_entries(st[:K]) + 4 * _pair_entries(st[K:]))
     peak, kind = peaks()
     l2 = max(gsb.probe_l2_copy(mib=mib) for mib in (16, 24, 32))
-    # working set of the items in flight: each CTA team holds one wide item's arena and snapshot (2 x 2^R x E)
+    # working set of the items in flight: each CTA team holds one wide item's two tables (2 x 2^R x E)
     wide = [1 << r for r in widths if r > small_R] or [0]
     working_set = min(len(wide), per_sm * 148) * 2 * E * float(np.mean(wide))
     l2_bytes = 126e6
@@ -656,8 +658,8 @@ def run_form_batch(args, emit=True):
                    "roofline": roof_l2 if working_set <= l2_bytes else roof_hbm,
                    "roofline_other": roof_hbm if working_set <= l2_bytes else roof_l2,
                    "working_set_bytes": working_set,
-                   "roofline_choice": "the L2 line when the wide items in flight (one per CTA team: arena and "
-                                      "snapshot) fit the 126 MB L2, else the HBM line",
+                   "roofline_choice": "the L2 line when the wide items in flight (one per CTA team: two tables) "
+                                      "fit the 126 MB L2, else the HBM line",
                    "orders": args.batch_order,
                    "host_planning_s": t_plan, "steps": args.steps, "warmup": args.warmup,
                }, emit=emit)
@@ -690,12 +692,10 @@ def run_form_grad(args, emit=True):
         if i >= max(3, args.warmup):
             times.append(time.perf_counter() - t0)
     t = statistics.median(times)
-    # algorithmic bytes of the sweep (complex128): per string, every step's forward pass twice (the sweep and the
-    # recompute of its checkpoint segment: read 2^r, write 2^r') and its reverse pass (read the step's input table and
-    # lambda_{k+1}, write lambda_k: 2^r + 2^r' + 2^r); the time is the whole loss + gradient, host work included
-    fwd = sum((1 << s["r"]) + (1 << s["rn"]) for s in w["steps"])
-    bwd = sum(2 * (1 << s["r"]) + (1 << s["rn"]) for s in w["steps"])
-    byt = 16.0 * len(bits) * (2 * fwd + bwd)
+    # algorithmic bytes of the sweep (complex128): per string and pass of two steps, forward (read the table before,
+    # write the one after) and reverse (read the table before and lambda after, write lambda before); the time is the
+    # whole loss + gradient, host work included
+    byt = 16.0 * len(bits) * (_pair_entries(w["steps"]) + _pair_entries(w["steps"], reads=2))
     peak, kind = peaks()
     sweep.close()
     return _form_line("grad", "s per loss+gradient, n=48 rotation layer, 2048 exact targets", t, "s", False, {
