@@ -1634,10 +1634,12 @@ int gsb_prefix(gsb_engine *e, const int8_t *forced, int K, void *dump, double *l
     Engine::Seq q;
     GSB_CK(E->enqueue_steps(q, 0, Kr, DRV_HYBRID, Kr, false, true, false, false));
     GSB_CK(E->seq_begin(q));   // K = 0
+    size_t bytes = 0;
     if (dump) {   // dump == NULL: only the prefix probability (a marginal) is wanted
         int nk, ntq;
         gsb_dump_shape(e, K, &nk, &ntq);
-        const size_t nent = ((size_t)1 << nk) * (size_t)ntq, bytes = nent * E->esize;
+        const size_t nent = ((size_t)1 << nk) * (size_t)ntq;
+        bytes = nent * E->esize;
         int rc = ensure_dump(E, bytes);
         if (rc) return rc;
         StepArgs a = dump_args(E, K);
@@ -1650,6 +1652,9 @@ int gsb_prefix(gsb_engine *e, const int8_t *forced, int K, void *dump, double *l
     DevState hs;
     GSB_CK(cudaMemcpyAsync(&hs, E->st, sizeof hs, cudaMemcpyDeviceToHost, E->stream));
     GSB_CK(cudaStreamSynchronize(E->stream));
+    // A prefix of probability 0 leaves zeros.  The arena does not hold them: a run stops at the step that ends the item
+    // without writing its table back, and no later step writes the entries it would have added.
+    if (dump && hs.dead) memset(dump, 0, bytes);
     if (logscale) *logscale = hs.logscale;
     if (log2p_prefix) *log2p_prefix = hs.logp;
     return 0;
