@@ -302,6 +302,8 @@ __global__ void __launch_bounds__(RUN_THREADS) k_run(const RunArgs ra, E *__rest
         __syncthreads();
     }
 
+    // An item dies where a branch has probability 0, not where a norm is not a number: a NaN goes on to the results, as the
+    // epilogues of the wide steps let it.
     int buf = 0, died = -1;
     for (int k = 0; k < n; k++) {
         const RunStep &s = steps[k & 1];
@@ -321,7 +323,7 @@ __global__ void __launch_bounds__(RUN_THREADS) k_run(const RunArgs ra, E *__rest
             if (tid == 0) { va[k] = ldexp(nb[0], 2 * ek); vb[k] = 2 * prev; }
             lsc += ek;
             prev = nb[0];
-            if (!(prev > 0)) { died = k; break; }
+            if (prev <= 0) { died = k; break; }
             int ex;
             frexp(prev, &ex);
             ek = (ex - 1) >> 1;
@@ -340,7 +342,7 @@ __global__ void __launch_bounds__(RUN_THREADS) k_run(const RunArgs ra, E *__rest
             bv = f >= 0 ? f : un[k] < p1;
             const double pb = bv ? p1 : 1 - p1;
             if (tid == 0) { va[k] = pb; bit[k] = (int8_t)bv; }
-            if (!(pb > 0)) { died = k; break; }
+            if (pb <= 0) { died = k; break; }
             sc = rsqrt(bv ? n1 : n0);
             sum[0] = 0;
             if (pair) coset_write(s, tab, per, c, bv, sc, sum);
@@ -376,7 +378,7 @@ __global__ void __launch_bounds__(RUN_THREADS) k_run(const RunArgs ra, E *__rest
             run_sum<1>(nb, red, buf);
             if (tid == 0) { va[k] = nb[0] / 2; vb[k] = prev; bit[k] = (int8_t)bv; }
             prev = nb[0];
-            if (!(prev > 0)) { died = k; break; }
+            if (prev <= 0) { died = k; break; }
         }
     }
     __syncthreads();
