@@ -494,12 +494,12 @@ struct Engine {
         return q.dry ? cudaSuccess : launch_finish(driver);
     }
 
-    // Launches of one item (mode 0: 'chain', else 'prob' / 'sample').
+    // Launches of one item (mode 0: 'chain', 1: the sampling passes, else 'hybrid').
     int64_t item_launches(int mode) {
         if (whole()) return 1;
         Seq q;
         q.dry = true;
-        enqueue_item(mode == 0 ? DRV_CHAIN1 : DRV_CHAIN, true, false, q);
+        enqueue_item(mode == 0 ? DRV_CHAIN1 : mode == 1 ? DRV_CHAIN : DRV_HYBRID, true, false, q);
         return q.launches;
     }
 
