@@ -755,22 +755,29 @@ static int batch_passes(BatchEngine &E, const int *K) {
     work(0);
     for (std::thread &t : th) t.join();
     std::vector<BPass> all;
-    E.pass_off.assign(n, 0);
-    E.npass0 = pre;
-    E.npass1.assign(n, 0);
+    std::vector<int> off(n, 0), suf(n, 0);
     for (size_t i = 0; i < n; i++) {
         if (bad[i]) return fail(GSB_E_PLAN_LAYOUT, "instance " + std::to_string(i) + " does not fit the batch kernel's passes");
-        E.pass_off[i] = (int)all.size();
-        E.npass1[i] = (int)got[i].size() - pre[i];
+        off[i] = (int)all.size();
+        suf[i] = (int)got[i].size() - pre[i];
         all.insert(all.end(), got[i].begin(), got[i].end());
+    }
+    // until the new table is on the device the engine keeps the old one, with the offsets that belong to it
+    BPass *d = nullptr;
+    cudaError_t e = cudaMalloc(&d, all.size() * sizeof(BPass));
+    if (e == cudaSuccess) e = cudaMemcpy(d, all.data(), all.size() * sizeof(BPass), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(d);
+        return fail(GSB_E_CUDA, std::string("the batch's pass table: ") + cudaGetErrorString(e));
     }
     for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);   // they point at the old passes
     E.graphs.clear();
     cudaFree(E.d_passes);
-    E.d_passes = nullptr;
-    E.K.clear();
-    BT_CK(cudaMalloc(&E.d_passes, all.size() * sizeof(BPass)));
-    BT_CK(cudaMemcpy(E.d_passes, all.data(), all.size() * sizeof(BPass), cudaMemcpyHostToDevice));
+    E.d_passes = d;
+    E.pass_off.swap(off);
+    E.npass0.swap(pre);
+    E.npass1.swap(suf);
     E.K.assign(K, K + n);
     return 0;
 }
@@ -964,7 +971,8 @@ int gsb_batch_set_strings(gsb_batch *h, const int *K, int npre, int nsuf, const 
         inst[(size_t)i].npass[0] = E.npass0[(size_t)i];
         inst[(size_t)i].npass[1] = E.npass1[(size_t)i];
     }
-    const bool resize = po != E.pre_total || so != E.suf_total || oo != E.out_total || npre != E.npre || nsuf != E.nsuf;
+    // no d_inst (the last of the buffers): none yet, or a call that found no memory for them
+    const bool resize = !E.d_inst || po != E.pre_total || so != E.suf_total || oo != E.out_total || npre != E.npre || nsuf != E.nsuf;
     if (resize) {
         for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);
         E.graphs.clear();

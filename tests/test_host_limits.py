@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import fake_runtime
-from fake_runtime import LAUNCHES
+from fake_runtime import LAUNCHES, NULL_TABLES
 
 
 @pytest.fixture
@@ -46,3 +46,35 @@ def test_launches_per_item(fake, n, prefix, prec):
             hybrid = eng.launches_per_item(2)
             eng.set_fusion(1)
             assert hybrid == eng.launches_per_item(1) == eng.launches_per_item(2)
+
+
+def batch_strings(plans, K, npre=2, nsuf=2):
+    ns = [int(p.split()[1]) for p in plans]
+    return [K] * len(plans), [np.zeros((npre, K), np.int8)] * len(plans), \
+        [np.zeros((npre, nsuf, n - K), np.int8) for n in ns]
+
+
+def test_batch_without_room_for_other_strings(fake):
+    """A set_strings that runs out of memory at any of its allocations leaves a batch that runs the strings it had, or says
+    that it has none, never one whose launch has no pass table; and that takes new strings once there is room."""
+    gsb, dev = fake
+    plans = [plan(n) for n in (18, 24)]
+    b = gsb.Batch(plans)
+    failed = 0
+    for room in (0, 1 << 8, 1 << 10, 1 << 12, 1 << 14, 1 << 15, 1 << 16, 1 << 17):
+        b.set_strings(*batch_strings(plans, 8))
+        b.run()
+        dev.fake_set_capacity(dev.fake_used() + room if room else 0)
+        try:
+            b.set_strings(*batch_strings(plans, 9, npre=64, nsuf=16))
+        except gsb.GsbError:
+            failed += 1
+        dev.fake_set_capacity(1 << 40)
+        try:
+            b.run()
+        except gsb.GsbError as e:
+            assert "no strings set" in str(e)
+        assert dev.fake_count(NULL_TABLES) == 0
+    assert failed > 3
+    b.close()
+    assert dev.fake_used() == 0
