@@ -23,9 +23,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <map>
+#include <new>
 #include <string>
 #include <thread>
 #include <tuple>
@@ -742,17 +745,26 @@ static int batch_passes(BatchEngine &E, const int *K) {
     std::vector<int> pre(n, 0), bad(n, 0);
     const int slots = BATCH_SLOT_BYTES / (int)E.esize;
     const unsigned nt = std::max(1u, std::min({(unsigned)n, 16u, std::thread::hardware_concurrency()}));
-    auto work = [&](size_t t) {
-        for (size_t i = t; i < n; i += nt) {
-            const HPlan &p = E.plans[i];
-            bad[i] = !passes_of(p, 0, K[i], slots, got[i]);
-            pre[i] = (int)got[i].size();
-            bad[i] = bad[i] || !passes_of(p, K[i], p.ns, slots, got[i]);
+    std::atomic<size_t> next{0};
+    auto work = [&] {
+        for (size_t i; (i = next++) < n;) {
+            try {
+                const HPlan &p = E.plans[i];
+                bad[i] = !passes_of(p, 0, K[i], slots, got[i]);
+                pre[i] = (int)got[i].size();
+                bad[i] = bad[i] || !passes_of(p, K[i], p.ns, slots, got[i]);
+            } catch (const std::bad_alloc &) {
+                bad[i] = 2;
+            }
         }
     };
     std::vector<std::thread> th;
-    for (unsigned t = 1; t < nt; t++) th.emplace_back(work, t);
-    work(0);
+    th.reserve(nt);
+    try {
+        for (unsigned t = 1; t < nt; t++) th.emplace_back(work);
+    } catch (const std::exception &) {   // no more threads: those there are, and this one, take all instances
+    }
+    work();
     for (std::thread &t : th) t.join();
     std::vector<BPass> all;
     std::vector<int> off(n, 0), suf(n, 0);

@@ -1,5 +1,9 @@
 """The library's host code where a device or a system runs short, on a CUDA runtime that runs nothing (fake_runtime.py): what
 it launches, allocates and reports, not what the kernels compute."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -78,3 +82,27 @@ def test_batch_without_room_for_other_strings(fake):
     assert failed > 3
     b.close()
     assert dev.fake_used() == 0
+
+
+def test_batch_without_threads(fake, tmp_path):
+    """Pass lists are made by several threads where the system has them, and by the caller alone where it has none."""
+    lib = str(tmp_path / "no_threads.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", lib, os.path.join(fake_runtime.HERE, "fake_cuda", "no_threads.c")], check=True)
+    texts = tmp_path / "plan.txt"
+    texts.write_text(plan(18))
+    run = """
+import ctypes, sys
+lib = ctypes.CDLL(sys.argv[1])
+text = open(sys.argv[2], "rb").read()
+n, K = 40, 8
+ns = int(text.split()[1])
+h = ctypes.c_void_p()
+assert lib.gsb_batch_open((ctypes.c_char_p * n)(*[text] * n), (ctypes.c_size_t * n)(*[len(text)] * n), n, 64, 0, ctypes.byref(h)) == 0
+zeros = (ctypes.c_int8 * (n * ns))()
+assert lib.gsb_batch_set_strings(h, (ctypes.c_int * n)(*[K] * n), 1, 1, zeros, zeros) == 0
+out = (ctypes.c_double * n)()
+assert lib.gsb_batch_run(h, out, None) == 0
+"""
+    r = subprocess.run([sys.executable, "-c", run, fake_runtime.LIB, str(texts)], env=dict(os.environ, LD_PRELOAD=lib),
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
