@@ -811,6 +811,8 @@ static int batch_graph(BatchEngine &E, const BatchShape &sh, cudaGraphExec_t *ou
         BT_CK(cudaMalloc(&E.d_arena, need));
         E.arena_bytes = need;
     }
+    for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);   // they point at the old items
+    E.graphs.clear();
     cudaFree(E.d_items);
     E.d_items = nullptr;
     std::vector<int> items(L.wide);
@@ -819,8 +821,6 @@ static int batch_graph(BatchEngine &E, const BatchShape &sh, cudaGraphExec_t *ou
     BT_CK(cudaMalloc(&E.d_items, std::max<size_t>(items.size(), 1) * sizeof(int)));
     if (!items.empty())
         BT_CK(cudaMemcpy(E.d_items, items.data(), items.size() * sizeof(int), cudaMemcpyHostToDevice));
-    for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);   // items buffer changed
-    E.graphs.clear();
     BatchArgs a;
     a.passes = E.d_passes;
     a.inst = E.d_inst;

@@ -10,7 +10,14 @@ namespace {
 std::map<void *, size_t> blocks;
 size_t used = 0, capacity = (size_t)1 << 40, largest = 0;
 long mallocs = 0, failed = 0, launches = 0, attributes = 0, null_arguments = 0;
-char handle;   // what every stream, event and graph points at
+char handle;   // what every stream and event points at
+// A graph remembers the device buffers that its batched launch was given (the first three arguments: passes, instances,
+// items); a replay after one of them was freed is counted.
+struct Graph {
+    void *buf[3];
+};
+Graph captured;
+long stale = 0;
 cudaError_t last = cudaSuccess;
 }  // namespace
 
@@ -20,10 +27,10 @@ extern "C" {
 void fake_set_capacity(size_t bytes) { capacity = bytes; }
 size_t fake_used(void) { return used; }
 long fake_count(int what) {
-    return what == 0 ? mallocs : what == 1 ? failed : what == 2 ? launches : what == 3 ? attributes : null_arguments;
+    return what == 0 ? mallocs : what == 1 ? failed : what == 2 ? launches : what == 3 ? attributes : what == 4 ? null_arguments : stale;
 }
 size_t fake_largest(void) { return largest; }
-void fake_reset(void) { mallocs = failed = launches = attributes = null_arguments = 0, largest = 0; }
+void fake_reset(void) { mallocs = failed = launches = attributes = null_arguments = stale = 0, largest = 0; }
 
 cudaError_t cudaMalloc(void **p, size_t n) {
     mallocs++;
@@ -88,12 +95,30 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = (cudaStr
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize(void) { return cudaSuccess; }
-cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
-cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) { *g = (cudaGraph_t)&handle; return cudaSuccess; }
-cudaError_t cudaGraphInstantiate(cudaGraphExec_t *x, cudaGraph_t, unsigned long long) { *x = (cudaGraphExec_t)&handle; return cudaSuccess; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
-cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
+    captured = Graph();
+    return cudaSuccess;
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) {
+    *g = (cudaGraph_t) new Graph(captured);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t *x, cudaGraph_t g, unsigned long long) {
+    *x = (cudaGraphExec_t) new Graph(*(Graph *)g);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t) {
+    for (void *b : ((Graph *)x)->buf) stale += b && !blocks.count(b);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t g) {
+    delete (Graph *)g;
+    return cudaSuccess;
+}
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) {
+    delete (Graph *)x;
+    return cudaSuccess;
+}
 cudaError_t cudaEventCreate(cudaEvent_t *e) { *e = (cudaEvent_t)&handle; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
@@ -117,6 +142,7 @@ cudaError_t cudaLaunchKernel(const void *, dim3, dim3, void **args, size_t, cuda
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **args) {
     if (!*(void **)args[0]) null_arguments++;   // the batched launch: its first argument is the pass table
+    memcpy(captured.buf, args[0], sizeof captured.buf);
     return cudaLaunchKernel(f, c->gridDim, c->blockDim, args, c->dynamicSmemBytes, c->stream);
 }
 

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import fake_runtime
-from fake_runtime import LAUNCHES, NULL_TABLES
+from fake_runtime import LAUNCHES, NULL_TABLES, STALE_REPLAYS
 
 
 @pytest.fixture
@@ -106,3 +106,33 @@ assert lib.gsb_batch_run(h, out, None) == 0
     r = subprocess.run([sys.executable, "-c", run, fake_runtime.LIB, str(texts)], env=dict(os.environ, LD_PRELOAD=lib),
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+
+
+def test_batch_without_room_for_another_shape(fake):
+    """A shape whose item lists or arenas find no memory leaves no graph behind that points at freed ones."""
+    gsb, dev = fake
+    plans = [plan(n) for n in (18, 24)]
+    b = gsb.Batch(plans)
+    b.set_strings(*batch_strings(plans, 8))
+    small, large = (128, 12, 1), (128, 12, 4)
+    b.set_shape(*large)
+    b.run()
+    b.set_shape(*small)          # the arenas of the larger shape serve it
+    b.run()
+    dev.fake_set_capacity(0)
+    b.set_shape(*large)
+    with pytest.raises(gsb.GsbError):
+        b.run()
+    b.set_shape(*small)
+    try:
+        b.run()
+    except gsb.GsbError:
+        pass
+    assert dev.fake_count(STALE_REPLAYS) == 0
+    dev.fake_set_capacity(1 << 40)
+    for shape in (small, large):
+        b.set_shape(*shape)
+        b.run()
+    assert dev.fake_count(STALE_REPLAYS) == dev.fake_count(NULL_TABLES) == 0
+    b.close()
+    assert dev.fake_used() == 0
