@@ -36,6 +36,8 @@ static thread_local std::string g_err;
 
 int fail(int code, const std::string &msg) {
     g_err = msg;
+    // an error that a call reports is not found again by the next one's check of its launches
+    if (code == GSB_E_CUDA || code == GSB_E_ALLOC) cudaGetLastError();
     return code;
 }
 

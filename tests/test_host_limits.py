@@ -136,3 +136,28 @@ def test_batch_without_room_for_another_shape(fake):
     assert dev.fake_count(STALE_REPLAYS) == dev.fake_count(NULL_TABLES) == 0
     b.close()
     assert dev.fake_used() == 0
+
+
+def test_errors_that_were_reported_do_not_come_back(fake):
+    """An allocation that failed is its own call's error, not that of the next call whose launches are checked."""
+    gsb, dev = fake
+    plans = [plan(36), plan(24)]
+    with gsb.Engine.from_text(plans[0], precision=128) as eng:
+        line = np.zeros((1, eng.ns), np.int8)
+
+        def without_room(call):
+            dev.fake_set_capacity(0)
+            with pytest.raises(gsb.GsbError):
+                call()
+            dev.fake_set_capacity(1 << 40)
+            eng.prob(line)
+        eng.prob(line)
+        b = gsb.Batch(plans)
+        without_room(lambda: b.set_strings(*batch_strings(plans, 8)))
+        b.set_strings(*batch_strings(plans, 8))
+        without_room(b.run)
+        without_room(lambda: gsb.Batch(plans))
+        without_room(lambda: gsb.Engine.from_text(plans[1]))
+        without_room(lambda: gsb.GradSweep(plans[1]))
+        without_room(lambda: gsb.dp_extend(np.ones(1, complex), 0, 0, 0, [], [], [1, 0, 1, 0]))
+        b.close()
