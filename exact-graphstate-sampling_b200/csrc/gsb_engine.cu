@@ -204,6 +204,7 @@ struct Engine {
     std::map<int, cudaGraphExec_t> graphs;   // key: graph kind << 16 | slots
     size_t arena = 0;                    // entries of an arena
     int max_slots = 1;                   // items per launch at most (a power of two, MAX_SLOTS and SLOT_BYTES)
+    int slot_limit = 1;                  // max_slots, or as many as the device's free memory allowed when it ran out
     int slots = 1;                       // items carried by the launches being queued
     int used_slots = 1;                  // slots of the launches queued since the device's error flags were read
     void *slot_mem = nullptr;            // the arenas of launches that carry several items
@@ -582,9 +583,12 @@ struct Engine {
         }
         cudaGraphExec_t ex;
         int s = 1;
-        while (s < max_slots && s < n) s *= 2;
+        while (s < slot_limit && s < n) s *= 2;
         int rc = graph(kind, s, &ex);
-        if (rc == GSB_E_ALLOC) rc = graph(kind, s = 1, &ex);   // no room for more than the engine's own arena
+        while (rc == GSB_E_ALLOC && s > 1) {   // no room for so many arenas: as many as fit, from now on
+            slot_limit = s /= 2;
+            rc = graph(kind, s, &ex);
+        }
         if (rc) return rc;
         used_slots = std::max(used_slots, s);
         const int b = std::min(s, 64);
@@ -814,6 +818,7 @@ static int make_args(Engine &E) {
     }
     build_runs(E);
     if (E.whole()) E.max_slots = 1;   // its items need no slots
+    E.slot_limit = E.max_slots;
     // a launch of several slots: one block each, or blocks of 256 threads (8 per SM) in at most SLOT_WAVES rounds
     maxgrid = std::max(maxgrid, E.max_slots > 1 ? std::max((size_t)E.sms * 8 * SLOT_WAVES, (size_t)E.max_slots)
                                                 : (size_t)E.sms * 8);

@@ -17,7 +17,7 @@ struct Graph {
     void *buf[3];
 };
 Graph captured;
-long stale = 0;
+long stale = 0, replays = 0;
 cudaError_t last = cudaSuccess;
 }  // namespace
 
@@ -27,10 +27,10 @@ extern "C" {
 void fake_set_capacity(size_t bytes) { capacity = bytes; }
 size_t fake_used(void) { return used; }
 long fake_count(int what) {
-    return what == 0 ? mallocs : what == 1 ? failed : what == 2 ? launches : what == 3 ? attributes : what == 4 ? null_arguments : stale;
+    return what == 0 ? mallocs : what == 1 ? failed : what == 2 ? launches : what == 3 ? attributes : what == 4 ? null_arguments : what == 5 ? stale : replays;
 }
 size_t fake_largest(void) { return largest; }
-void fake_reset(void) { mallocs = failed = launches = attributes = null_arguments = stale = 0, largest = 0; }
+void fake_reset(void) { mallocs = failed = launches = attributes = null_arguments = stale = replays = 0, largest = 0; }
 
 cudaError_t cudaMalloc(void **p, size_t n) {
     mallocs++;
@@ -108,6 +108,7 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t *x, cudaGraph_t g, unsigned lon
     return cudaSuccess;
 }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t) {
+    replays++;
     for (void *b : ((Graph *)x)->buf) stale += b && !blocks.count(b);
     return cudaSuccess;
 }

@@ -56,4 +56,4 @@ def load():
     return gsb, dev
 
 
-MALLOCS, FAILED, LAUNCHES, ATTRIBUTES, NULL_TABLES, STALE_REPLAYS = range(6)
+MALLOCS, FAILED, LAUNCHES, ATTRIBUTES, NULL_TABLES, STALE_REPLAYS, REPLAYS = range(7)

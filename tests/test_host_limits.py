@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import fake_runtime
-from fake_runtime import LAUNCHES, NULL_TABLES, STALE_REPLAYS
+from fake_runtime import FAILED, LAUNCHES, MALLOCS, NULL_TABLES, REPLAYS, STALE_REPLAYS
 
 
 @pytest.fixture
@@ -161,3 +161,29 @@ def test_errors_that_were_reported_do_not_come_back(fake):
         without_room(lambda: gsb.GradSweep(plans[1]))
         without_room(lambda: gsb.dp_extend(np.ones(1, complex), 0, 0, 0, [], [], [1, 0, 1, 0]))
         b.close()
+
+
+@pytest.mark.parametrize("prec", [128, 64])
+@pytest.mark.parametrize("room", [0, 1, 2, 5, 31, 64])
+def test_slots_where_arenas_do_not_fit(fake, room, prec):
+    """A call of 100 strings on a device with room for `room` arenas beside the engine's: as many slots as fit (two slots take
+    one arena more, the engine's own being one of them), found once, with a call of few strings before and after it."""
+    gsb, dev = fake
+    text = plan(36)
+    arena = (16 if prec == 128 else 8) << int(text.split()[2])
+    slots = max([1] + [s for s in (2, 4, 8, 16, 32, 64) if (1 if s == 2 else s) <= room])
+    with gsb.Engine.from_text(text, precision=prec) as eng:
+        few, many = np.zeros((min(slots, 4), eng.ns), np.int8), np.zeros((100, eng.ns), np.int8)
+        eng.chain(few)
+        small = dev.fake_used()
+        dev.fake_set_capacity(small + max(0, room - (0 if slots == 1 else 1 if len(few) == 2 else len(few))) * arena)
+        dev.fake_reset()
+        eng.chain(many)
+        tried = dev.fake_count(FAILED)
+        assert dev.fake_count(REPLAYS) == -(-100 // slots)
+        dev.fake_reset()
+        for _ in range(2):
+            eng.chain(many)
+            eng.chain(few)
+        assert dev.fake_count(FAILED) == dev.fake_count(MALLOCS) == 0 and tried <= 7
+        assert dev.fake_count(REPLAYS) == 2 * (-(-100 // slots) + 1)
