@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <exception>
 #include <map>
@@ -566,6 +567,7 @@ struct BatchEngine {
     unsigned int *d_q = nullptr;
     void *d_arena = nullptr;
     size_t arena_bytes = 0;
+    size_t limit = SIZE_MAX;        // of the arenas' bytes, where clusters can be done without (shape_layout)
     int npre = 0, nsuf = 0;
     int64_t pre_total = 0, suf_total = 0, out_total = 0;
     std::vector<BInst> h_inst;
@@ -619,7 +621,7 @@ struct BatchLayout {
     int wide_R = 0, big_R = 0, small_R = 0, grid = 0;
     size_t bytes = 0;
 };
-static BatchLayout shape_layout(const BatchEngine &E, const BatchShape &sh) {
+static BatchLayout team_layout(const BatchEngine &E, const BatchShape &sh, bool clusters) {
     BatchLayout L;
     std::vector<int> order(E.plans.size());
     for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
@@ -635,7 +637,7 @@ static BatchLayout shape_layout(const BatchEngine &E, const BatchShape &sh) {
     const double share = total / L.grid;
     for (int i : order) {
         const int R = E.plans[(size_t)i].R;
-        const bool small = R <= sh.small_R, wide = !small && R >= 15 && E.cost[(size_t)i] > share;
+        const bool small = R <= sh.small_R, wide = clusters && !small && R >= 15 && E.cost[(size_t)i] > share;
         auto &q = small ? L.small : wide ? L.wide : L.big;
         for (int p = 0; p < E.npre; p++) q.push_back(i * E.npre + p);
         int &r = small ? L.small_R : wide ? L.wide_R : L.big_R;
@@ -644,6 +646,17 @@ static BatchLayout shape_layout(const BatchEngine &E, const BatchShape &sh) {
     const size_t warps = (size_t)L.grid * (size_t)(sh.block / 32);
     L.bytes = E.esize * 2 * ((L.wide.empty() ? 0 : (size_t)(L.grid / BATCH_CLUSTER) << L.wide_R) +
                              ((size_t)L.grid << L.big_R) + (warps << L.small_R));
+    return L;
+}
+
+// Cluster teams have arenas of their own beside those of the block teams, which need no less where a second instance of the
+// same width is left to them: within E.limit, or else the block teams take every wide instance if that needs less.
+static BatchLayout shape_layout(const BatchEngine &E, const BatchShape &sh) {
+    BatchLayout L = team_layout(E, sh, true);
+    if (L.bytes > E.limit && !L.wide.empty()) {
+        BatchLayout B = team_layout(E, sh, false);
+        if (B.bytes < L.bytes) L = B;
+    }
     return L;
 }
 
@@ -800,16 +813,26 @@ static int batch_graph(BatchEngine &E, const BatchShape &sh, cudaGraphExec_t *ou
         *out = it->second;
         return 0;
     }
-    const BatchLayout L = shape_layout(E, sh);
-    const size_t need = L.bytes;
-    if (need > E.arena_bytes) {
+    BatchLayout L = shape_layout(E, sh);
+    if (L.bytes > E.arena_bytes) {
         cudaFree(E.d_arena);
         E.d_arena = nullptr;
         E.arena_bytes = 0;
         for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);   // they point at the old arena
         E.graphs.clear();
-        BT_CK(cudaMalloc(&E.d_arena, need));
-        E.arena_bytes = need;
+        cudaError_t e = cudaMalloc(&E.d_arena, L.bytes);
+        if (e == cudaErrorMemoryAllocation) {   // no room for the cluster teams' arenas: without them, from now on
+            E.limit = L.bytes - 1;
+            const size_t tried = L.bytes;
+            L = shape_layout(E, sh);
+            if (L.bytes < tried) {
+                cudaGetLastError();
+                e = cudaMalloc(&E.d_arena, L.bytes);
+            }
+        }
+        if (e != cudaSuccess) E.d_arena = nullptr;
+        BT_CK(e);
+        E.arena_bytes = L.bytes;
     }
     for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);   // they point at the old items
     E.graphs.clear();
@@ -1075,6 +1098,7 @@ int gsb_batch_tune(gsb_batch *h, int reps, size_t max_bytes, int *block, int *sm
     if (!E.d_out) return fail(GSB_E_STATE, "no strings set (gsb_batch_set_strings)");
     std::vector<double> out((size_t)std::max<int64_t>(E.out_total, 1));
     float best = 1e30f;
+    E.limit = max_bytes;
     BatchShape bs = E.shape;
     const int maxR = E.max_R();
     const int max_block = batch_max_block(E);   // shapes the kernel cannot launch are skipped

@@ -20,9 +20,9 @@ def fake():
     dev.fake_set_capacity(1 << 40)
 
 
-def plan(n):
+def plan(n, seed=11):
     import workloads
-    return workloads.matching_instance(n, n, 11, 8, 20000)["plan"]
+    return workloads.matching_instance(n, n, seed, 8, 20000)["plan"]
 
 
 @pytest.mark.parametrize("prec", [128, 64])
@@ -187,3 +187,30 @@ def test_slots_where_arenas_do_not_fit(fake, room, prec):
             eng.chain(few)
         assert dev.fake_count(FAILED) == dev.fake_count(MALLOCS) == 0 and tried <= 7
         assert dev.fake_count(REPLAYS) == 2 * (-(-100 // slots) + 1)
+
+
+@pytest.mark.parametrize("prec", [128, 64])
+def test_batch_without_room_for_cluster_arenas(fake, prec):
+    """Cluster teams have arenas beside those of the block teams. Without room for both, or above the tuner's bound, the wide
+    instances go to block teams."""
+    gsb, dev = fake
+    # one instance of width 15 whose cost is above an even share of the batch, 300 of the same width below it: both kinds of
+    # teams have arenas of 2^15 entries
+    plans = [plan(38, 5)] * 300 + [plan(39, 3)]
+    assert {p.split()[2] for p in plans} == {"15"}
+    b = gsb.Batch(plans, precision=prec)
+    b.set_strings(*batch_strings(plans, 8, 1, 1))
+    b.run()
+    both, with_clusters = dev.fake_largest(), dev.fake_used()
+    b.close()
+    assert dev.fake_used() == 0
+    b = gsb.Batch(plans, precision=prec)
+    b.set_strings(*batch_strings(plans, 8, 1, 1))
+    dev.fake_reset()
+    dev.fake_set_capacity(with_clusters - (1 << 20))
+    b.run()
+    assert dev.fake_largest() < both
+    dev.fake_reset()
+    b.run()
+    assert dev.fake_count(MALLOCS) == 0
+    b.close()
