@@ -869,6 +869,8 @@ static int batch_graph(BatchEngine &E, const BatchShape &sh, cudaGraphExec_t *ou
     a.small_R = L.small_R;
     const size_t smem = batch_smem(sh.block);
     const void *fn = E.prec == 128 ? (const void *)k_batch<double2> : (const void *)k_batch<float2>;
+    // asked for here and not in an open, which would load both precisions' kernels
+    BT_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BATCH_MAX_SMEM));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)L.grid);
     cfg.blockDim = dim3((unsigned)sh.block);
@@ -951,8 +953,6 @@ int gsb_batch_open(const char *const *texts, const size_t *lens, int ninst, int 
     cudaDeviceGetAttribute(&E.sms, cudaDevAttrMultiProcessorCount, device);
     cudaError_t e = cudaStreamCreateWithFlags(&E.stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&E.d_q, 3 * sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BATCH_MAX_SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BATCH_MAX_SMEM);
     if (e != cudaSuccess) {
         delete h;
         return fail(GSB_E_ALLOC, std::string("device allocation: ") + cudaGetErrorString(e));

@@ -162,6 +162,8 @@ static uint32_t group_smem_bytes(int D, int TR, const int (&ssz)[4], int L, bool
     return D == 3 ? group_smem<E, T, 3, 0>(ssz, L).total : group_smem<E, T, 2, 0>(ssz, L).total;
 }
 
+constexpr int RUN_MAX_STEPS = 1024;   // saved scalars of a run in shared memory: 25 B per step
+
 struct Engine {
     HPlan plan;
     int prec = 64, dev = 0, sms = 0;
@@ -517,9 +519,24 @@ struct Engine {
                         r.M[b][x][0] = args[(size_t)k].Mr[b][x];
                         r.M[b][x][1] = args[(size_t)k].Mi[b][x];
                     }
-        GSB_CK(cudaMemcpyAsync(d_args, args.data(), args.size() * sizeof(StepArgs), cudaMemcpyHostToDevice, stream));
-        GSB_CK(cudaMemcpyAsync(d_rs, rsteps.data(), rsteps.size() * sizeof(RunStep), cudaMemcpyHostToDevice, stream));
+        // args, the entry after the last step (an empty table) and rsteps, as the device holds them
+        const size_t na = args.size() * sizeof(StepArgs), nr = rsteps.size() * sizeof(RunStep);
+        StepArgs end;
+        memset(&end, 0, sizeof end);
+        end.ntq = 1;
+        std::vector<char> all(na + sizeof end + nr);
+        if (na) memcpy(all.data(), args.data(), na);
+        memcpy(all.data() + na, &end, sizeof end);
+        if (nr) memcpy(all.data() + na + sizeof end, rsteps.data(), nr);
+        GSB_CK(cudaMemcpyAsync(d_args, all.data(), all.size(), cudaMemcpyHostToDevice, stream));
         GSB_CK(cudaStreamSynchronize(stream));
+        // Asked for here and not in an open, which would load the kernel, and only where a run needs it: engines of narrow
+        // plans never do.
+        size_t most = 0;
+        for (const RunPart &p : parts) most = std::max(most, run_smem(p.dim, p.k1 - p.k0, esize));
+        if (most > 48 * 1024)
+            GSB_CK(cudaFuncSetAttribute(run_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)run_smem(RUN_DIM, RUN_MAX_STEPS, sizeof(double2))));
         args_dirty = false;
         return 0;
     }
@@ -730,7 +747,6 @@ struct Coords {
 
 // Parts of consecutive steps whose columns span at most 2^RUN_DIM addresses, each as long as it can be, with their steps
 // in compact coordinates.  Every step of at most 2^10 cosets fits one (its columns span nk + 2 dimensions at most).
-constexpr int RUN_MAX_STEPS = 1024;   // saved scalars of a run in shared memory: 25 B per step
 static void build_runs(Engine &E) {
     const int ns = E.plan.ns;
     E.parts.clear();
@@ -826,13 +842,7 @@ static int make_args(Engine &E) {
     const size_t sa_bytes = ((size_t)p.ns + 1) * sizeof(StepArgs);   // one allocation: each costs 0.3 ms
     GSB_CK(cudaMalloc(&E.d_args, sa_bytes + E.rsteps.size() * sizeof(RunStep)));
     E.d_rs = reinterpret_cast<RunStep *>(reinterpret_cast<char *>(E.d_args) + sa_bytes);
-    StepArgs end;
-    memset(&end, 0, sizeof end);
-    end.ntq = 1;
-    GSB_CK(cudaMemcpy(E.d_args + p.ns, &end, sizeof end, cudaMemcpyHostToDevice));
     E.args_dirty = true;
-    GSB_CK(cudaFuncSetAttribute(E.run_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)run_smem(RUN_DIM, RUN_MAX_STEPS, sizeof(double2))));
     return 0;
 }
 

@@ -573,16 +573,37 @@ struct GradEngine {
         *stride = (size_t)(q - 1) * seg_stride;
         return d_seg + (i % (size_t)q - 1) * seg_stride;
     }
+    static size_t fwd_smem(const GradPass &g) { return (size_t)(g.ssz[0] + (g.d == 2 ? g.ssz[1] : 0)) * 16 * GRAD_THREADS; }
+    static size_t bwd_smem(const GradPass &g) {
+        return (size_t)(g.ssz[0] + g.ssz[1] + (g.d == 2 ? g.ssz[2] : 0)) * 16 * GRAD_THREADS;
+    }
+    // Kernels whose passes need more shared memory than a launch has by default; asked for before the first sweep and not in
+    // an open, which would load the kernels.
+    cudaError_t allow_smem() const {
+        const int most = GRAD_MAX_VALUES * 16 * GRAD_THREADS;   // of the largest pass
+        cudaError_t e = cudaSuccess;
+        for (int d = 1; d <= 2; d++) {
+            size_t f = 0, b = 0;
+            for (const GradPass &g : passes)
+                if (g.d == d) { f = std::max(f, fwd_smem(g)); b = std::max(b, bwd_smem(g)); }
+            const void *fk = d == 2 ? (const void *)k_gr_fwd<2> : (const void *)k_gr_fwd<1>;
+            const void *bk = d == 2 ? (const void *)k_gr_bwd<2> : (const void *)k_gr_bwd<1>;
+            // the reverse pass's static sums count too
+            if (e == cudaSuccess && f > 47 * 1024) e = cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+            if (e == cudaSuccess && b > 47 * 1024) e = cudaFuncSetAttribute(bk, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        }
+        return e;
+    }
     cudaError_t fwd(size_t i, const double2 *in, size_t is, double2 *out, size_t os) {
         const GradPass &g = passes[i];
-        const size_t sm = (size_t)(g.ssz[0] + (g.d == 2 ? g.ssz[1] : 0)) * 16 * GRAD_THREADS;
+        const size_t sm = fwd_smem(g);
         if (g.d == 2) k_gr_fwd<2><<<grid_of(g), GRAD_THREADS, sm, stream>>>(g, in, is, out, os, ctx());
         else k_gr_fwd<1><<<grid_of(g), GRAD_THREADS, sm, stream>>>(g, in, is, out, os, ctx());
         return cudaGetLastError();
     }
     cudaError_t bwd(size_t i, const double2 *T, size_t ts, const double2 *lo, double2 *li) {
         const GradPass &g = passes[i];
-        const size_t sm = (size_t)(g.ssz[0] + g.ssz[1] + (g.d == 2 ? g.ssz[2] : 0)) * 16 * GRAD_THREADS;
+        const size_t sm = bwd_smem(g);
         if (g.d == 2)
             k_gr_bwd<2><<<grid_of(g), GRAD_THREADS, sm, stream>>>(g, T, ts, lo, li, seg_stride, ctx(), partials, d_counter,
                                                                   d_grad);
@@ -727,10 +748,6 @@ int gsb_grad_open_text(const char *text, size_t len, int device, int every, gsb_
     if (e == cudaSuccess) e = cudaMalloc(&E.d_item, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&E.d_counter, bs * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMemsetAsync(E.d_counter, 0, bs * sizeof(unsigned int), E.stream);
-    const int most = GRAD_MAX_VALUES * 16 * GRAD_THREADS;   // shared memory of the largest pass
-    for (const void *f : {(const void *)k_gr_fwd<1>, (const void *)k_gr_fwd<2>, (const void *)k_gr_bwd<1>,
-                          (const void *)k_gr_bwd<2>})
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e == cudaSuccess) e = cudaStreamSynchronize(E.stream);
     if (e != cudaSuccess) {
         delete h;
@@ -761,6 +778,7 @@ int gsb_grad_run(gsb_grad *h, const double *M, const int8_t *bits, int64_t nstr,
     } restore{prev};
     GR_CK(cudaMemcpyAsync(E.d_M, M, (size_t)ns * 8 * sizeof(double), cudaMemcpyHostToDevice, E.stream));
     if (!E.graph) {
+        GR_CK(E.allow_smem());
         cudaGraph_t gr = nullptr;
         GR_CK(cudaStreamBeginCapture(E.stream, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = E.enqueue();

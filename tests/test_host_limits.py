@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import fake_runtime
-from fake_runtime import FAILED, LAUNCHES, MALLOCS, NULL_TABLES, REPLAYS, STALE_REPLAYS
+from fake_runtime import ATTRIBUTES, FAILED, LAUNCHES, MALLOCS, NULL_TABLES, REPLAYS, STALE_REPLAYS
 
 
 @pytest.fixture
@@ -214,3 +214,36 @@ def test_batch_without_room_for_cluster_arenas(fake, prec):
     b.run()
     assert dev.fake_count(MALLOCS) == 0
     b.close()
+
+
+@pytest.mark.parametrize("prec", [128, 64])
+def test_opens_load_no_kernel(fake, prec):
+    """Asking for a kernel's attributes loads it. An open of a narrow engine, a batch or a gradient sweep leaves that to the
+    first call, and an engine whose runs fit the default shared memory never asks."""
+    gsb, dev = fake
+    text = plan(24)
+    with gsb.Engine.from_text(text, precision=prec) as eng:
+        assert dev.fake_count(ATTRIBUTES) == 0
+        eng.prob(np.zeros((1, eng.ns), np.int8))
+        assert dev.fake_count(ATTRIBUTES) == 0
+    b = gsb.Batch([text], precision=prec)
+    g = gsb.GradSweep(text)
+    assert dev.fake_count(ATTRIBUTES) == 0
+    b.set_strings(*batch_strings([text], 8))
+    b.run()
+    assert dev.fake_count(ATTRIBUTES) == 1
+    b.close()
+    g.close()
+
+
+@pytest.mark.parametrize("prec", [128, 64])
+def test_runs_that_need_shared_memory_ask_for_it(fake, prec):
+    """A run over 2^12 entries of complex128 needs 64 KB; of complex64, 32 KB."""
+    gsb, dev = fake
+    text = plan(36)
+    with gsb.Engine.from_text(text, precision=prec) as eng:
+        opened = dev.fake_count(ATTRIBUTES)
+        line = np.zeros((1, eng.ns), np.int8)
+        eng.chain(line)
+        eng.chain(line)
+        assert dev.fake_count(ATTRIBUTES) == opened + (1 if prec == 128 else 0)
