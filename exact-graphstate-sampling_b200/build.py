@@ -20,9 +20,9 @@ CLI128 = os.path.join(HERE, "gsb2_c128")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall"]
-# the complex64 FP32 fused passes sit in translation units of their own (gsb_group_*.cu): the largest objects, compiled
-# in parallel with the rest
-LIB_SOURCES = ["gsb_engine.cu", "gsb_group_ws.cu", "gsb_group_ws3.cu", "gsb_group_wst.cu", "gsb_group_f32.cu", "gsb_group3.cu", "gsb_group128.cu",
+# the complex64 FP32 and complex128 fused passes sit in translation units of their own (gsb_group*.cu): the largest objects,
+# compiled in parallel with the rest, each once for launches of one item and once (GSB_SLOTS) for launches of several
+LIB_SOURCES = ["gsb_group_ws3.cu", "gsb_engine.cu", "gsb_group_ws.cu", "gsb_group_wst.cu", "gsb_group_f32.cu", "gsb_group3.cu", "gsb_group128.cu",
                "gsb_dp.cu", "gsb_grad.cu", "gsb_batch.cu", "gsb_probe.cu", "gsb_plan.cpp", "gsb_order.cpp", "gsb_fuse.cpp"]
 LIB_DEPS = LIB_SOURCES + ["gsb_kernels.cuh", "gsb_run.cuh", "gsb_group.cuh", "gsb_step.h", "gsb_plan.h", "gsb_common.h", "gsb_fuse.h",
                           "gsb_pick.h"]
@@ -56,12 +56,17 @@ def build(force=False, verbose_ptxas=False):
         cmds, objs = [], []
         headers = [d for d in deps if not d.endswith((".cu", ".cpp"))]
         only_engine = os.path.join(CSRC, "gsb_run.cuh")
+        units = []
         for f in LIB_SOURCES:
-            obj = os.path.join(objdir, f + ".o")
+            units.append((f, f + ".o", []))
+            if f.startswith("gsb_group"):
+                units.append((f, f + ".slots.o", ["-DGSB_SLOTS=1"]))
+        for f, name, defines in units:
+            obj = os.path.join(objdir, name)
             objs.append(obj)
             if not force and not verbose_ptxas and not _stale(obj, [os.path.join(CSRC, f)] + [h for h in headers if h != only_engine or f == "gsb_engine.cu"]):
                 continue
-            cmds.append([_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose_ptxas else []) +
+            cmds.append([_nvcc()] + NVCC_FLAGS + defines + (["-Xptxas", "-v"] if verbose_ptxas else []) +
                         ["-c", "-I" + INCLUDE, "-I" + CSRC, "-o", obj, os.path.join(CSRC, f)])
         with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(len(cmds), os.cpu_count() or 1))) as ex:
             list(ex.map(_run, cmds))

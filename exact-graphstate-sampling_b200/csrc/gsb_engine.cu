@@ -102,10 +102,19 @@ static void *pick_wide(int prec, int ntq, int m, bool write, bool fp32) {
     return m == 2 ? pick_wide128<1, 2>(write) : pick_wide128<1, 1>(write);
 }
 
-template <typename E, typename T>
+template <typename E, typename T, bool SLOTS>
 static void *pick_group(int d, int tr) {
-    if (tr) return d == 2 ? (void *)k_group<E, T, 2, 1> : (void *)k_group<E, T, 1, 1>;
-    return d == 3 ? (void *)k_group<E, T, 3, 0> : (void *)k_group<E, T, 2, 0>;
+    if (tr) return d == 2 ? (void *)k_group<E, T, 2, 1, SLOTS> : (void *)k_group<E, T, 1, 1, SLOTS>;
+    return d == 3 ? (void *)k_group<E, T, 3, 0, SLOTS> : (void *)k_group<E, T, 2, 0, SLOTS>;
+}
+
+// The fused pass's kernel for launches of one item (SLOTS = false) or of several.
+template <bool SLOTS>
+static void *pick_fused(int prec, int arith, int minb, bool ws, int d, int tr) {
+    if (prec == 128) return pick_group128<SLOTS>(d, tr, ws);
+    if (arith == 64) return pick_group<float2, double, SLOTS>(d, tr);
+    if (minb == 3) return pick_group3<SLOTS>(d, tr);
+    return ws ? pick_group_ws<SLOTS>(d, tr) : pick_group_f32<SLOTS>(d, tr);
 }
 
 // One pass of an item: a single step (group == false: norm pass + write pass when sampling) or a fused group that
@@ -130,8 +139,8 @@ struct Op {
     bool group = false;
     bool norm_first = false;  // sampling: a norm pass of step k0 runs first (its bit has no other source)
     GroupArgs ga;
-    void *fn = nullptr;
-    int grid = 1, cap = 1;    // blocks of one item; blocks the device holds at once
+    void *fn = nullptr, *fn_slots = nullptr;   // kernels of launches that carry one item, and several
+    int grid = 1;             // blocks of one item alone
     size_t smem = 0;
     unsigned int ntiles = 0;
     double entries = 0;       // entries read + written by the pass (the norm pass not included)
@@ -259,6 +268,9 @@ struct Engine {
         else if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem) != cudaSuccess || nb < 1) nb = 1;
         return group_occ[key] = nb;
     }
+
+    // Blocks the device holds of a fused pass's kernel for several items, set up on first use.
+    int slots_capacity(const Op &op) { return std::max(1, group_occupancy(op.fn_slots, op.threads, op.smem)) * sms; }
 
     int occupancy(void *fn, int block) {
         auto it = occ.find(fn);
@@ -466,7 +478,9 @@ struct Engine {
         ga.withhold_loads = withhold_loads;
         void *memp = arena_mem();
         void *kargs[] = {&ga, &memp, &c};
-        return cudaLaunchKernel(op.fn, dim3(slot_grid(op.grid, op.cap), (unsigned)slots), dim3((unsigned)op.threads), kargs,
+        if (slots == 1) return cudaLaunchKernel(op.fn, dim3((unsigned)op.grid), dim3((unsigned)op.threads), kargs, op.smem, stream);
+        const int cap = slots_capacity(op);
+        return cudaLaunchKernel(op.fn_slots, dim3(slot_grid(op.grid, cap), (unsigned)slots), dim3((unsigned)op.threads), kargs,
                                 op.smem, stream);
     }
 
@@ -567,6 +581,9 @@ struct Engine {
         const int driver = driver_of(kind);
         const bool use_forced = kind != 2, use_unif = kind >= 2;
         if (int rc = upload()) return rc;
+        if (nslots > 1)   // the kernels for several items are loaded before the capture
+            for (const Op &op : kind == 0 ? chain_ops : kind == 3 ? hyb_ops : sample_ops)
+                if (op.group) slots_capacity(op);
         cudaGraph_t g = nullptr;
         GSB_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         slots = nslots;
@@ -1020,15 +1037,11 @@ static bool fill_group(Engine &E, const GroupPlan &gp, Op &op, int lcap = GROUP_
     const bool ws = ws_ok && (ws_req < 0 ? TR == 0 : ws_req == 1);
     op.ws = ws ? 1 : 0;
     op.threads = ws ? GROUP_NCT + 32 : GROUP_NCT;
-    if (E.prec == 128) op.fn = pick_group128(op.d, op.tr, ws);
-    else if (E.arith == 64) op.fn = pick_group<float2, double>(op.d, op.tr);
-    else if (minb == 3) op.fn = pick_group3(op.d, op.tr);
-    else if (ws) op.fn = pick_group_ws(op.d, op.tr);
-    else op.fn = pick_group_f32(op.d, op.tr);
+    op.fn = pick_fused<false>(E.prec, E.arith, minb, ws, op.d, op.tr);
+    op.fn_slots = pick_fused<true>(E.prec, E.arith, minb, ws, op.d, op.tr);
     const int nb = E.group_occupancy(op.fn, op.threads, op.smem);
     if (nb < 1) return false;
-    op.cap = nb * E.sms;
-    op.grid = (int)std::min<uint64_t>(op.ntiles, (uint64_t)op.cap);
+    op.grid = (int)std::min<uint64_t>(op.ntiles, (uint64_t)(nb * E.sms));
     op.entries = gp.entries_moved;
     return true;
 }

@@ -1622,11 +1622,15 @@ __host__ __device__ inline GroupSmem group_smem(const int (&ssz)[4], int L, bool
 // load-issuing warp.  From 2^9 classes a step thread handles the same class pairs in every step of the pass, so the
 // stages between steps are private to it and need no barrier; the input buffers are handed over by mbarriers (loads
 // landed / every step warp done reading), so the step warps do not wait for one another within or between tiles.
-template <typename E, typename T, int D, int TR, int MINB = 2, bool WS = false>
+// SLOTS: builds for launches that carry several items.  Computed pointers to the slot's arena, state and partials cost
+// registers or spills (three-step warp-specialised passes 32 -> 48 bytes, <1, 1> 100 -> 102 registers); with them as kernel
+// parameters one item of width 30 is faster: 'chain' 8.39 -> 8.19 ms in complex64 and 15.8 -> 15.4 ms in complex128, a
+// complex64 sample 17.3 -> 17.2 ms.
+template <typename E, typename T, int D, int TR, bool SLOTS, int MINB = 2, bool WS = false>
 __global__ void __launch_bounds__(WS ? GROUP_NCT + 32 : GROUP_NCT, MINB)
     k_group(const GroupArgs ga, E *__restrict__ mem, const Ctx c0) {
-    const Ctx cx = slot_ctx(c0);
-    mem += (size_t)blockIdx.y * cx.arena;
+    const Ctx cx = SLOTS ? slot_ctx(c0) : c0;
+    if (SLOTS) mem += (size_t)blockIdx.y * cx.arena;
     DevState *st = cx.st;
     if (*(volatile int *)&st->dead) return;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1675,7 +1679,7 @@ __global__ void __launch_bounds__(WS ? GROUP_NCT + 32 : GROUP_NCT, MINB)
     constexpr bool FACT = C64F || sizeof(E) == 16;
     // folded sampling passes (GroupArgs::fold) exist only in the two-CTA build: the three-CTA register cap spills them
     constexpr bool FOLD = C64F && PK && D == 2 && TR == 1 && MINB == 2;
-    static_assert(!WS || (FACT && MINB == 2), "warp-specialised build: complex64 FP32, two CTAs per SM");
+    static_assert(!WS || (FACT && MINB == 2), "warp-specialised build: factored passes, two CTAs per SM");
     int fpiv[D];
     T fsc[D], fbr[D], fbi[D];
     double fcp[D];

@@ -5,10 +5,10 @@
 
 namespace gsb {
 
-void *pick_group128(int d, int tr, bool ws) {
-    if (tr) return d == 2 ? (void *)k_group<double2, double, 2, 1> : (void *)k_group<double2, double, 1, 1>;
-    if (ws) return d == 3 ? (void *)k_group<double2, double, 3, 0, 2, true> : (void *)k_group<double2, double, 2, 0, 2, true>;
-    return d == 3 ? (void *)k_group<double2, double, 3, 0> : (void *)k_group<double2, double, 2, 0>;
+template <> void *pick_group128<GSB_SLOTS>(int d, int tr, bool ws) {
+    if (tr) return d == 2 ? (void *)k_group<double2, double, 2, 1, GSB_SLOTS> : (void *)k_group<double2, double, 1, 1, GSB_SLOTS>;
+    if (ws) return d == 3 ? (void *)k_group<double2, double, 3, 0, GSB_SLOTS, 2, true> : (void *)k_group<double2, double, 2, 0, GSB_SLOTS, 2, true>;
+    return d == 3 ? (void *)k_group<double2, double, 3, 0, GSB_SLOTS> : (void *)k_group<double2, double, 2, 0, GSB_SLOTS>;
 }
 
 }  // namespace gsb

@@ -4,9 +4,9 @@
 
 namespace gsb {
 
-void *pick_group3(int d, int tr) {
-    if (tr) return d == 2 ? (void *)k_group<float2, float, 2, 1, 3> : (void *)k_group<float2, float, 1, 1, 3>;
-    return d == 3 ? (void *)k_group<float2, float, 3, 0, 3> : (void *)k_group<float2, float, 2, 0, 3>;
+template <> void *pick_group3<GSB_SLOTS>(int d, int tr) {
+    if (tr) return d == 2 ? (void *)k_group<float2, float, 2, 1, GSB_SLOTS, 3> : (void *)k_group<float2, float, 1, 1, GSB_SLOTS, 3>;
+    return d == 3 ? (void *)k_group<float2, float, 3, 0, GSB_SLOTS, 3> : (void *)k_group<float2, float, 2, 0, GSB_SLOTS, 3>;
 }
 
 }  // namespace gsb

@@ -5,9 +5,9 @@
 
 namespace gsb {
 
-void *pick_group_ws(int d, int tr) {
-    if (tr) return pick_group_ws_trailing(d);
-    return d == 3 ? pick_group_ws_three() : (void *)k_group<float2, float, 2, 0, 2, true>;
+template <> void *pick_group_ws<GSB_SLOTS>(int d, int tr) {
+    if (tr) return pick_group_ws_trailing<GSB_SLOTS>(d);
+    return d == 3 ? pick_group_ws_three<GSB_SLOTS>() : (void *)k_group<float2, float, 2, 0, GSB_SLOTS, 2, true>;
 }
 
 }  // namespace gsb

@@ -4,6 +4,6 @@
 
 namespace gsb {
 
-void *pick_group_ws_three() { return (void *)k_group<float2, float, 3, 0, 2, true>; }
+template <> void *pick_group_ws_three<GSB_SLOTS>() { return (void *)k_group<float2, float, 3, 0, GSB_SLOTS, 2, true>; }
 
 }  // namespace gsb

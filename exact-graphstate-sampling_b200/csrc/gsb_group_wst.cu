@@ -5,8 +5,8 @@
 
 namespace gsb {
 
-void *pick_group_ws_trailing(int d) {
-    return d == 2 ? (void *)k_group<float2, float, 2, 1, 2, true> : (void *)k_group<float2, float, 1, 1, 2, true>;
+template <> void *pick_group_ws_trailing<GSB_SLOTS>(int d) {
+    return d == 2 ? (void *)k_group<float2, float, 2, 1, GSB_SLOTS, 2, true> : (void *)k_group<float2, float, 1, 1, GSB_SLOTS, 2, true>;
 }
 
 }  // namespace gsb

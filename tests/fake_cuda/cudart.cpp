@@ -17,7 +17,8 @@ struct Graph {
     void *buf[3];
 };
 Graph captured;
-long stale = 0, replays = 0;
+long stale = 0, replays = 0, fused_one = 0, fused_several = 0, fused_wrong = 0;
+char kernel_one, kernel_several;   // the fused passes' kernels for launches of one item, and of several
 cudaError_t last = cudaSuccess;
 }  // namespace
 
@@ -27,10 +28,11 @@ extern "C" {
 void fake_set_capacity(size_t bytes) { capacity = bytes; }
 size_t fake_used(void) { return used; }
 long fake_count(int what) {
-    return what == 0 ? mallocs : what == 1 ? failed : what == 2 ? launches : what == 3 ? attributes : what == 4 ? null_arguments : what == 5 ? stale : replays;
+    return what == 0 ? mallocs : what == 1 ? failed : what == 2 ? launches : what == 3 ? attributes : what == 4 ? null_arguments : what == 5 ? stale : what == 6 ? replays : what == 7 ? fused_one
+         : what == 8 ? fused_several : fused_wrong;
 }
 size_t fake_largest(void) { return largest; }
-void fake_reset(void) { mallocs = failed = launches = attributes = null_arguments = stale = replays = 0, largest = 0; }
+void fake_reset(void) { mallocs = failed = launches = attributes = null_arguments = stale = replays = fused_one = fused_several = fused_wrong = 0, largest = 0; }
 
 cudaError_t cudaMalloc(void **p, size_t n) {
     mallocs++;
@@ -136,9 +138,11 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const
     *n = 2;
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void *, dim3, dim3, void **args, size_t, cudaStream_t) {
-    (void)args;
+cudaError_t cudaLaunchKernel(const void *f, dim3 grid, dim3, void **, size_t, cudaStream_t) {
     launches++;
+    fused_one += f == &kernel_one;
+    fused_several += f == &kernel_several;
+    fused_wrong += (f == &kernel_one && grid.y != 1) || (f == &kernel_several && grid.y < 2);
     return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **args) {
@@ -172,8 +176,17 @@ cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *sm, void *st) {
 
 // the fused passes' kernels are picked in translation units of their own, which are left out
 namespace gsb {
-void *pick_group_f32(int, int) { return &handle; }
-void *pick_group3(int, int) { return &handle; }
-void *pick_group_ws(int, int) { return &handle; }
-void *pick_group128(int, int, bool) { return &handle; }
+static void *fused(bool several) { return several ? &kernel_several : &kernel_one; }
+template <bool S> void *pick_group_f32(int, int) { return fused(S); }
+template <bool S> void *pick_group3(int, int) { return fused(S); }
+template <bool S> void *pick_group_ws(int, int) { return fused(S); }
+template <bool S> void *pick_group128(int, int, bool) { return fused(S); }
+template void *pick_group_f32<false>(int, int);
+template void *pick_group_f32<true>(int, int);
+template void *pick_group3<false>(int, int);
+template void *pick_group3<true>(int, int);
+template void *pick_group_ws<false>(int, int);
+template void *pick_group_ws<true>(int, int);
+template void *pick_group128<false>(int, int, bool);
+template void *pick_group128<true>(int, int, bool);
 }  // namespace gsb

@@ -56,4 +56,5 @@ def load():
     return gsb, dev
 
 
-MALLOCS, FAILED, LAUNCHES, ATTRIBUTES, NULL_TABLES, STALE_REPLAYS, REPLAYS = range(7)
+(MALLOCS, FAILED, LAUNCHES, ATTRIBUTES, NULL_TABLES, STALE_REPLAYS, REPLAYS, FUSED_ONE, FUSED_SEVERAL,
+ FUSED_WRONG) = range(10)

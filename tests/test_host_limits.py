@@ -8,7 +8,8 @@ import numpy as np
 import pytest
 
 import fake_runtime
-from fake_runtime import ATTRIBUTES, FAILED, LAUNCHES, MALLOCS, NULL_TABLES, REPLAYS, STALE_REPLAYS
+from fake_runtime import (ATTRIBUTES, FAILED, FUSED_ONE, FUSED_SEVERAL, FUSED_WRONG, LAUNCHES, MALLOCS, NULL_TABLES, REPLAYS,
+                          STALE_REPLAYS)
 
 
 @pytest.fixture
@@ -247,3 +248,18 @@ def test_runs_that_need_shared_memory_ask_for_it(fake, prec):
         eng.chain(line)
         eng.chain(line)
         assert dev.fake_count(ATTRIBUTES) == opened + (1 if prec == 128 else 0)
+
+
+@pytest.mark.parametrize("prec", [128, 64])
+@pytest.mark.parametrize("count", [1, 2, 3, 100])
+def test_fused_kernels_by_items(fake, count, prec):
+    """Launches of one item take the kernels whose pointers are parameters, launches of several those that compute them."""
+    gsb, dev = fake
+    with gsb.Engine.from_text(plan(44), precision=prec) as eng:
+        lines = np.zeros((count, eng.ns), np.int8)
+        eng.set_hybrid_prefix(eng.ns - 4)
+        for call in (lambda: eng.chain(lines), lambda: eng.sample(count, 1), lambda: eng.hybrid(lines, 1)):
+            dev.fake_reset()
+            call()
+            one, several = dev.fake_count(FUSED_ONE), dev.fake_count(FUSED_SEVERAL)
+            assert (one > 0, several > 0) == (count == 1, count > 1) and dev.fake_count(FUSED_WRONG) == 0
