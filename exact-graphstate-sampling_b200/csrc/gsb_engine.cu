@@ -557,19 +557,25 @@ struct Engine {
 
     static int driver_of(int kind) { return kind == 0 ? DRV_CHAIN1 : kind == 3 ? DRV_HYBRID : DRV_CHAIN; }
 
+    // The slots' arenas back to the device, with the graphs that point at them.
+    int drop_slots() {
+        GSB_CK(cudaStreamSynchronize(stream));
+        for (auto kv = graphs.begin(); kv != graphs.end();)
+            if ((kv->first & 0xffff) > 1) { cudaGraphExecDestroy(kv->second); kv = graphs.erase(kv); }
+            else ++kv;
+        cudaFree(slot_mem);
+        slot_mem = nullptr;
+        slot_bytes = 0;
+        return 0;
+    }
+
     // The graph of one launch of `nslots` items of mode `kind`.
     int graph(int kind, int nslots, cudaGraphExec_t *out) {
         const int key = kind << 16 | nslots;
         auto it = graphs.find(key);
         if (it != graphs.end()) { *out = it->second; return 0; }
         if (slot_need(nslots) > slot_bytes) {   // the slots' arenas, allocated on first use
-            GSB_CK(cudaStreamSynchronize(stream));
-            for (auto kv = graphs.begin(); kv != graphs.end();)            // those that point at the old ones
-                if ((kv->first & 0xffff) > 1) { cudaGraphExecDestroy(kv->second); kv = graphs.erase(kv); }
-                else ++kv;
-            cudaFree(slot_mem);
-            slot_mem = nullptr;
-            slot_bytes = 0;
+            if (int rc = drop_slots()) return rc;
             const size_t bytes = slot_need(nslots);
             if (cudaMalloc(&slot_mem, bytes) != cudaSuccess) {
                 cudaGetLastError();
@@ -1635,16 +1641,26 @@ static StepArgs dump_args(const Engine *E, int K) {
     return a;
 }
 
-static int ensure_dump(Engine *E, size_t bytes) {
-    if (E->dump_bytes >= bytes) return 0;
-    cudaFree(E->d_dump);
-    E->d_dump = nullptr;
-    E->dump_bytes = 0;
-    cudaError_t e = cudaMalloc(&E->d_dump, bytes);
-    if (e != cudaSuccess) { cudaGetLastError(); return fail(GSB_E_ALLOC, "allocation of the dump buffer failed"); }
-    E->dump_bytes = bytes;
+// A buffer of the engine for the tables of a call, of at least `bytes`; the slots' arenas make room for it.
+static int ensure_buffer(Engine *E, void *&p, size_t &have, size_t bytes, const char *what) {
+    if (have >= bytes) return 0;
+    cudaFree(p);
+    p = nullptr;
+    have = 0;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess && E->slot_bytes) {
+        cudaGetLastError();
+        if (int rc = E->drop_slots()) return rc;
+        e = cudaMalloc(&p, bytes);
+    }
+    if (e != cudaSuccess) {
+        p = nullptr;
+        return fail(GSB_E_ALLOC, std::string("allocation of ") + what + " failed");
+    }
+    have = bytes;
     return 0;
 }
+static int ensure_dump(Engine *E, size_t bytes) { return ensure_buffer(E, E->d_dump, E->dump_bytes, bytes, "the dump buffer"); }
 
 int gsb_prefix(gsb_engine *e, const int8_t *forced, int K, void *dump, double *logscale, double *log2p_prefix) {
     if (!e) return fail(GSB_E_STATE, "null engine");
@@ -1745,17 +1761,7 @@ int gsb_resume(gsb_engine *e, const int8_t *forced, int K, uint64_t seed, int64_
     memcpy(small.data() + ns8, f.data(), ns8);
     memcpy(small.data() + 2 * ns8, cs.data(), ns8);
     memcpy(small.data() + 3 * ns8, tperm.data(), 2 * ns8);
-    if (E->small_bytes < small.size()) {
-        cudaFree(E->d_small);
-        E->d_small = nullptr;
-        E->small_bytes = 0;
-        if (cudaMalloc(&E->d_small, small.size()) != cudaSuccess) {
-            cudaGetLastError();
-            E->d_small = nullptr;
-            return fail(GSB_E_ALLOC, "allocation of the slice descriptors failed");
-        }
-        E->small_bytes = small.size();
-    }
+    if ((rc = ensure_buffer(E, E->d_small, E->small_bytes, small.size(), "the slice descriptors"))) return rc;
     GSB_CK(cudaMemcpyAsync(E->d_small, small.data(), small.size(), cudaMemcpyHostToDevice, E->stream));
     const char *sp = (const char *)E->d_small;
     ResumeArgs ra;

@@ -263,3 +263,29 @@ def test_fused_kernels_by_items(fake, count, prec):
             call()
             one, several = dev.fake_count(FUSED_ONE), dev.fake_count(FUSED_SEVERAL)
             assert (one > 0, several > 0) == (count == 1, count > 1) and dev.fake_count(FUSED_WRONG) == 0
+
+
+@pytest.mark.parametrize("prec", [128, 64])
+def test_tables_take_the_place_of_slots(fake, prec):
+    """A dump or a resume that finds no memory beside the slots' arenas takes theirs; a later call of several strings goes
+    on with as many as fit."""
+    gsb, dev = fake
+    text = plan(36)
+    entry = 16 if prec == 128 else 8
+    with gsb.Engine.from_text(text, precision=prec) as eng:
+        lines = np.zeros((64, eng.ns), np.int8)
+        K = max(range(eng.ns), key=lambda k: np.ldexp(eng.dump_shape(k)[1], eng.dump_shape(k)[0]))
+        nk, ntq = eng.dump_shape(K)
+        table = (entry * ntq) << nk
+        slices = 20
+        eng.chain(lines)
+        arenas = (64 * entry) << int(text.split()[2])
+        assert arenas > (slices + 1) * table
+        dev.fake_set_capacity(dev.fake_used() + table // 2)
+        dump, ls, _ = eng.prefix(lines[0], K)
+        eng.chain(lines)
+        eng.resume(lines[0], K, 1, 0, [dump] * slices, [ls] * slices)
+        eng.chain(lines)
+        dev.fake_reset()
+        eng.chain(lines)
+        assert dev.fake_count(FAILED) == 0 and dev.fake_count(REPLAYS) < 64
