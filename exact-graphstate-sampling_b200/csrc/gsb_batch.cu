@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <exception>
@@ -69,12 +70,20 @@ struct alignas(16) BPass {
     BStep st[FUSE_MAX_STEPS];
 };
 static_assert(sizeof(BPass) % 16 == 0, "descriptors are copied in 16-byte words");
+constexpr int BATCH_WORDS = (int)(sizeof(BPass) / 16), BATCH_NEAR_WORDS = 32;   // of a descriptor; of one with a single step
+static_assert(offsetof(BPass, st) + sizeof(BStep) <= 16 * BATCH_NEAR_WORDS, "one word per lane of a warp");
 // Slots of a thread: the values between two steps of a chunk's classes.  More classes per chunk spread a step's
 // descriptor loads over more work, fewer leave room for more CTAs: 512 instances of widths 7-20 in complex64 took 22.7,
 // 21.8 and 41 ms at 128, 256 and 512 B.
 constexpr int BATCH_SLOT_BYTES = 256;
 constexpr int BATCH_CLUSTER = 8;      // CTAs of a cluster team
 constexpr int BATCH_MAX_BLOCK = 512;
+// Instances up to this width take one step per pass, and a warp keeps both tables of their items in its lanes' slots (2^8
+// entries of complex128 twice: 8 KB).  A warp's item is a chain of dependent passes with a table read in each, so what bounds
+// it is the latency of those reads and of the code between them: through L2, and through the code of the wide passes, 320
+// items of widths 1-3 took 67 us in complex64 and 75 us in complex128 (single steps with generic code 43 and 41 us, now 22 and
+// 22), 4,000 items of widths 5-9 321 and 376 us (225 and 227; now 170 and 193).
+constexpr int BATCH_NEAR_R = 8;
 
 struct BInst {
     int ns, R, K, n;
@@ -101,6 +110,7 @@ struct BatchArgs {
 // Teams.  sum() gives every thread the same total (fixed order) and is also the barrier between two passes: partial sums
 // alternate between two buffers, so a block needs one __syncthreads and a cluster one cluster barrier per pass.
 struct BlockTeam {
+    static constexpr bool WARP = false;
     int buf = 0;
     __device__ int rank() const { return threadIdx.x; }
     __device__ int size() const { return blockDim.x; }
@@ -122,6 +132,7 @@ struct BlockTeam {
 };
 
 struct WarpTeam {
+    static constexpr bool WARP = true;
     __device__ int rank() const { return threadIdx.x & 31; }
     __device__ int size() const { return 32; }
     __device__ int log2size() const { return 5; }
@@ -136,6 +147,7 @@ struct WarpTeam {
 
 // The CTAs of a cluster.
 struct ClusterTeam {
+    static constexpr bool WARP = false;
     int buf = 0;
     __device__ int rank() const { return (int)(cg::this_cluster().block_rank() * blockDim.x + threadIdx.x); }
     __device__ int size() const { return (int)(cg::this_cluster().num_blocks() * blockDim.x); }
@@ -418,6 +430,65 @@ __device__ __noinline__ double team_pass(const BPass &p, uint32_t r, int ls, con
     return nb;
 }
 
+// A pass of one step by a warp, of at most 2^BATCH_NEAR_R classes: short code for any shape with NTQ offsets.  The classes are
+// the step's cosets; columns past the last one are 0.
+template <typename E, int NTQ>
+__device__ __forceinline__ double near_step(const BPass &p, const E *in, E *out, int bit, double scale) {
+    typedef typename ArithOf<E>::T T;
+    const BStep &s = p.st[0];
+    const uint32_t r = threadIdx.x & 31;
+    if (r >> min(p.nb, 5)) return 0;
+    uint32_t base = 0, cls = r, z[NTQ];
+#pragma unroll
+    for (int j = 0; j < 5; j++)
+        if ((r >> j) & 1) base ^= p.col[j];
+#pragma unroll
+    for (int t = 0; t < NTQ; t++) z[t] = p.zin[t];
+    const uint32_t z0 = p.zout[0], z1 = p.zout[1], lam = s.lam, count = p.nb > 5 ? 1u << (p.nb - 5) : 1;
+    const int m = s.m, tau0 = s.tau0, tau1 = s.tau1, par = s.par ^ (s.mpar & 1 ? (1 << NTQ) - 1 : 0);
+    const double *M = s.M + 4 * bit;
+    const T m0r = (T)(scale * M[0]), m0i = (T)(scale * M[1]), m1r = (T)(scale * M[2]), m1i = (T)(scale * M[3]);
+    double nb = 0;
+    for (uint32_t n = 0;;) {
+        E v[NTQ];
+#pragma unroll
+        for (int t = 0; t < NTQ; t++) v[t] = in[base ^ z[t]];
+        T a0r = 0, a0i = 0, a1r = 0, a1i = 0, b0r = 0, b0i = 0, b1r = 0, b1i = 0;
+#pragma unroll
+        for (int t = 0; t < NTQ; t++) {
+            if ((tau0 >> t) & 1) { a1r += v[t].x; a1i += v[t].y; } else { a0r += v[t].x; a0i += v[t].y; }
+            const int neg = (par >> t) & 1;
+            const T yr = signed_by(v[t].x, neg), yi = signed_by(v[t].y, neg);
+            if ((tau1 >> t) & 1) { b1r += yr; b1i += yi; } else { b0r += yr; b0i += yi; }
+        }
+        const int neg = __popc(cls & lam) & 1;
+        const T wr = signed_by(m1r, neg), wi = signed_by(m1i, neg);
+        T re = m0r * a0r - m0i * a0i + wr * b0r - wi * b0i, im = m0r * a0i + m0i * a0r + wr * b0i + wi * b0r;
+        out[base ^ z0] = mk2(re, im);
+        T nn = re * re + im * im;
+        if (m == 2) {
+            re = m0r * a1r - m0i * a1i + wr * b1r - wi * b1i;
+            im = m0r * a1i + m0i * a1r + wr * b1i + wi * b1r;
+            out[base ^ z1] = mk2(re, im);
+            nn += re * re + im * im;
+        }
+        nb += (double)nn;
+        if (++n >= count) break;
+        const int j = 5 + __ffs((int)n) - 1;
+        base ^= p.col[j];
+        cls ^= 1u << j;
+    }
+    return nb;
+}
+template <typename E>
+__device__ __noinline__ double near_pass(const BPass &p, const E *in, E *out, int bit, double scale) {
+    switch (p.st[0].ntq) {
+        case 1: return near_step<E, 1>(p, in, out, bit, scale);
+        case 2: return near_step<E, 2>(p, in, out, bit, scale);
+        default: return near_step<E, 4>(p, in, out, bit, scale);
+    }
+}
+
 struct ChainState {
     double prev, lsc, scale;
     int ek, dead;
@@ -441,11 +512,11 @@ __device__ __forceinline__ void chain_update(ChainState &cs, double nb) {
 // the last one written to `last`, otherwise the arena.  desc: two descriptor buffers; the next pass's descriptor is
 // fetched during a pass.  Ends behind a team barrier (the last sum): tables complete, buffers free.
 template <typename E, typename TM>
-__device__ void run_passes(TM &tm, const BPass *passes, int a, int b, const int8_t *bits, const E *first, E *arena, E *last,
-                           BPass *desc, E *slots, int stride, ChainState &cs) {
-    constexpr int WORDS = (int)(sizeof(BPass) / 16), PER = (WORDS + 31) / 32;
+__device__ void run_passes(TM &tm, const BPass *passes, int a, int b, int words, const int8_t *bits, const E *first, E *arena,
+                           E *last, BPass *desc, E *slots, int stride, ChainState &cs) {
+    constexpr int PER = (BATCH_WORDS + 31) / 32;
     const int l = tm.local(), nl = tm.nlocal();
-    for (int i = l; i < WORDS; i += nl) reinterpret_cast<int4 *>(desc)[i] = reinterpret_cast<const int4 *>(passes + a)[i];
+    for (int i = l; i < words; i += nl) reinterpret_cast<int4 *>(desc)[i] = reinterpret_cast<const int4 *>(passes + a)[i];
     tm.sync();
     int k = 0;
     for (int i = a; i < b; i++) {
@@ -454,14 +525,17 @@ __device__ void run_passes(TM &tm, const BPass *passes, int a, int b, const int8
         if (i + 1 < b)
 #pragma unroll
             for (int q = 0; q < PER; q++)
-                if (l + q * nl < WORDS) next[q] = reinterpret_cast<const int4 *>(passes + i + 1)[l + q * nl];
-        const double nb = team_pass<E>(p, (uint32_t)tm.rank(), tm.log2size(), i == a ? first : arena,
-                                       i == b - 1 ? last : arena, bits + k, cs.scale, slots, stride);
+                if (l + q * nl < words) next[q] = reinterpret_cast<const int4 *>(passes + i + 1)[l + q * nl];
+        const E *from = i == a ? first : arena;
+        E *to = i == b - 1 ? last : arena;
+        double nb;
+        if (TM::WARP && p.d == 1 && p.nb <= BATCH_NEAR_R && p.st[0].nmem == 1) nb = near_pass<E>(p, from, to, bits[k], cs.scale);
+        else nb = team_pass<E>(p, (uint32_t)tm.rank(), tm.log2size(), from, to, bits + k, cs.scale, slots, stride);
         k += p.d;
         if (i + 1 < b)
 #pragma unroll
             for (int q = 0; q < PER; q++)
-                if (l + q * nl < WORDS) reinterpret_cast<int4 *>(desc + ((i + 1 - a) & 1))[l + q * nl] = next[q];
+                if (l + q * nl < words) reinterpret_cast<int4 *>(desc + ((i + 1 - a) & 1))[l + q * nl] = next[q];
         chain_update(cs, tm.sum(nb));
         if (cs.dead) break;
     }
@@ -475,7 +549,8 @@ __device__ void run_item(TM &tm, const BatchArgs &a, int item, E *arena, E *kept
     if (tm.rank() == 0) arena[0] = mk2((typename ArithOf<E>::T)1, (typename ArithOf<E>::T)0);
     ChainState cs{1.0, 0.0, 1.0, 0, 0};
     const int p0 = in.pass_off, p1 = p0 + in.npass[0], p2 = p1 + in.npass[1];
-    run_passes<E, TM>(tm, a.passes, p0, p1, pb, arena, arena, kept, desc, slots, stride, cs);
+    const int words = in.R <= BATCH_NEAR_R ? BATCH_NEAR_WORDS : BATCH_WORDS;
+    run_passes<E, TM>(tm, a.passes, p0, p1, words, pb, arena, arena, kept, desc, slots, stride, cs);
     const ChainState at_k = cs;
     const int nsuf_steps = in.ns - in.K;
     for (int sidx = 0; sidx < a.nsuf; sidx++) {
@@ -483,10 +558,64 @@ __device__ void run_item(TM &tm, const BatchArgs &a, int item, E *arena, E *kept
         double lp = -INFINITY;
         if (!cs.dead) {
             const int8_t *sb = a.suf_bits + in.suf_off + ((int64_t)pre * a.nsuf + sidx) * nsuf_steps;
-            run_passes<E, TM>(tm, a.passes, p1, p2, sb, kept, arena, arena, desc, slots, stride, cs);
+            run_passes<E, TM>(tm, a.passes, p1, p2, words, sb, kept, arena, arena, desc, slots, stride, cs);
             if (!cs.dead) lp = log2(cs.prev) + 2.0 * cs.lsc - in.n;
         }
         if (tm.rank() == 0) a.log2p[in.out_off + (int64_t)pre * a.nsuf + sidx] = lp;
+    }
+}
+
+// Passes a .. b - 1 of a near instance by a warp, as run_passes: every pass is one step, its descriptor one word per lane.
+template <typename E>
+__device__ __forceinline__ void near_passes(const BPass *passes, int a, int b, const int8_t *bits, const E *first, E *tab, E *last,
+                                            BPass *desc, ChainState &cs) {
+    const int lane = threadIdx.x & 31;
+    reinterpret_cast<int4 *>(desc)[lane] = reinterpret_cast<const int4 *>(passes + a)[lane];
+    int bit = bits[0];
+    __syncwarp();
+#pragma unroll 1
+    for (int i = a; i < b; i++) {
+        const BPass &p = desc[(i - a) & 1];
+        int4 next = make_int4(0, 0, 0, 0);
+        int next_bit = 0;
+        if (i + 1 < b) {
+            next = reinterpret_cast<const int4 *>(passes + i + 1)[lane];
+            next_bit = bits[i + 1 - a];
+        }
+        const E *from = i == a ? first : tab;
+        E *to = i == b - 1 ? last : tab;
+        const int ntq = p.st[0].ntq;
+        double nb;
+        if (ntq == 1) nb = near_step<E, 1>(p, from, to, bit, cs.scale);
+        else if (ntq == 2) nb = near_step<E, 2>(p, from, to, bit, cs.scale);
+        else nb = near_step<E, 4>(p, from, to, bit, cs.scale);
+        reinterpret_cast<int4 *>(desc + ((i + 1 - a) & 1))[lane] = next;
+        bit = next_bit;
+        __syncwarp();
+        chain_update(cs, warp_sum(nb));
+        if (cs.dead) break;
+    }
+}
+template <typename E>
+__device__ __noinline__ void near_item(const BatchArgs &a, int item, E *tab, BPass *desc) {
+    const int ii = item / a.npre, pre = item % a.npre;
+    const BInst in = a.inst[ii];
+    E *kept = tab + (1 << BATCH_NEAR_R);
+    if ((threadIdx.x & 31) == 0) tab[0] = mk2((typename ArithOf<E>::T)1, (typename ArithOf<E>::T)0);
+    ChainState cs{1.0, 0.0, 1.0, 0, 0};
+    const int p0 = in.pass_off, p1 = p0 + in.npass[0], p2 = p1 + in.npass[1];
+    near_passes<E>(a.passes, p0, p1, a.pre_bits + in.pre_off + (int64_t)pre * in.K, tab, tab, kept, desc, cs);
+    const ChainState at_k = cs;
+    const int nsuf_steps = in.ns - in.K;
+    for (int sidx = 0; sidx < a.nsuf; sidx++) {
+        cs = at_k;
+        double lp = -INFINITY;
+        if (!cs.dead) {
+            near_passes<E>(a.passes, p1, p2, a.suf_bits + in.suf_off + ((int64_t)pre * a.nsuf + sidx) * nsuf_steps, kept, tab, tab,
+                           desc, cs);
+            if (!cs.dead) lp = log2(cs.prev) + 2.0 * cs.lsc - in.n;
+        }
+        if ((threadIdx.x & 31) == 0) a.log2p[in.out_off + (int64_t)pre * a.nsuf + sidx] = lp;
     }
 }
 
@@ -499,7 +628,7 @@ static size_t batch_smem(int block) {
 constexpr size_t BATCH_MAX_SMEM = (227 << 10) - 2048;   // dynamic, beside the teams' static sums
 
 template <typename E>
-__global__ void __launch_bounds__(BATCH_MAX_BLOCK) k_batch(const BatchArgs a) {
+__global__ void __launch_bounds__(BATCH_MAX_BLOCK) k_batch(const __grid_constant__ BatchArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int warps = (int)(blockDim.x >> 5), w = (int)(threadIdx.x >> 5);
     BPass *desc = reinterpret_cast<BPass *>(smem);
@@ -535,13 +664,21 @@ __global__ void __launch_bounds__(BATCH_MAX_BLOCK) k_batch(const BatchArgs a) {
         run_item<E, BlockTeam>(bt, a, a.items_big[it], arena, arena + big, desc, slots, stride);
     }
     E *wa = reinterpret_cast<E *>(a.small_arena) + ((size_t)blockIdx.x * warps + (size_t)w) * 2 * small;
+    E *ws = reinterpret_cast<E *>(smem + (size_t)warps * 2 * sizeof(BPass)) + (size_t)w * (32 * BATCH_SLOT_BYTES / sizeof(E));
     WarpTeam wt;
-    for (;;) {
-        int it = 0;
-        if ((threadIdx.x & 31) == 0) it = (int)atomicAdd(&a.queues[1], 1u);
-        it = __shfl_sync(0xffffffffu, it, 0);
+    // Where there are narrow items only, every warp's first one is its own, dealt out over the blocks: the blocks that start
+    // first would otherwise take eight each.
+    const bool dealt = a.n_wide == 0 && a.n_big == 0;
+    const int warps_all = (int)gridDim.x * warps;
+    for (int it = dealt ? w * (int)gridDim.x + (int)blockIdx.x : -1;; it = -1) {
+        if (it < 0) {
+            if ((threadIdx.x & 31) == 0) it = (int)atomicAdd(&a.queues[1], 1u) + (dealt ? warps_all : 0);
+            it = __shfl_sync(0xffffffffu, it, 0);
+        }
         if (it >= a.n_small) break;
-        run_item<E, WarpTeam>(wt, a, a.items_small[it], wa, wa + small, desc + 2 * w, slots, stride);
+        const int item = a.items_small[it];
+        if (a.inst[item / a.npre].R <= BATCH_NEAR_R) near_item<E>(a, item, ws, desc + 2 * w);
+        else run_item<E, WarpTeam>(wt, a, item, wa, wa + small, desc + 2 * w, ws + (threadIdx.x & 31), 32);
     }
 }
 
@@ -740,7 +877,7 @@ static bool passes_of(const HPlan &p, int k0, int k1, int slots, std::vector<BPa
         BPass g;
         GroupPlan gp;
         int d = 1;   // a pass has at most the 2^nk cosets of each of its steps as classes
-        while (d < FUSE_MAX_STEPS && k + d < k1 && std::min(p.st[(size_t)k].nk, p.st[(size_t)(k + d)].nk) >= least) d++;
+        while (p.R > BATCH_NEAR_R && d < FUSE_MAX_STEPS && k + d < k1 && std::min(p.st[(size_t)k].nk, p.st[(size_t)(k + d)].nk) >= least) d++;
         while (d > 0 && !(plan_group(p, k, d, 0, 24, gp) && (d == 1 || gp.nb >= least) && make_pass(p, gp, slots, g))) d--;
         if (!d) return false;
         out.push_back(g);
