@@ -87,15 +87,17 @@ constexpr int BATCH_NEAR_R = 8;
 
 struct BInst {
     int ns, R, K, n;
-    int pass_off, npass[2];  // first pass; passes of the prefix, of a suffix
+    int list_off, npass[2];  // in the list of passes: those of the prefix, then those of a suffix
+    int first[2];            // the first pass of each
     int64_t pre_off;         // prefix bits: [npre][K]
     int64_t suf_off;         // suffix bits: [npre][nsuf][ns - K]
     int64_t out_off;         // log2 Pr: [npre][nsuf]
 };
 
 struct BatchArgs {
-    const BPass *passes;
+    const BPass *passes;     // every pass that some prefix length has needed
     const BInst *inst;
+    const int *list;         // the passes of the current prefix lengths, by instance
     const int *items_wide, *items_big, *items_small;   // item = inst * npre + prefix
     int n_wide, n_big, n_small, npre, nsuf;
     const int8_t *pre_bits, *suf_bits;
@@ -508,34 +510,36 @@ __device__ __forceinline__ void chain_update(ChainState &cs, double nb) {
     cs.scale = ldexp(1.0, -cs.ek);
 }
 
-// Passes a .. b - 1 of an instance with its bits (the first pass's step first): read from `first`, otherwise the arena,
-// the last one written to `last`, otherwise the arena.  desc: two descriptor buffers; the next pass's descriptor is
-// fetched during a pass.  Ends behind a team barrier (the last sum): tables complete, buffers free.
+// The n passes list[0 .. n - 1] of `passes` (the first is number p0) with their bits (the first pass's step first): read from
+// `first`, otherwise the arena, the last one written to `last`, otherwise the arena.  desc: two descriptor buffers; the next
+// pass's descriptor is fetched during a pass, its number in the pass before.  Ends behind a team barrier (the last sum): tables complete, buffers free.
 template <typename E, typename TM>
-__device__ void run_passes(TM &tm, const BPass *passes, int a, int b, int words, const int8_t *bits, const E *first, E *arena,
-                           E *last, BPass *desc, E *slots, int stride, ChainState &cs) {
+__device__ void run_passes(TM &tm, const BPass *passes, const int *list, int p0, int n, int words, const int8_t *bits,
+                           const E *first, E *arena, E *last, BPass *desc, E *slots, int stride, ChainState &cs) {
     constexpr int PER = (BATCH_WORDS + 31) / 32;
     const int l = tm.local(), nl = tm.nlocal();
-    for (int i = l; i < words; i += nl) reinterpret_cast<int4 *>(desc)[i] = reinterpret_cast<const int4 *>(passes + a)[i];
+    for (int i = l; i < words; i += nl) reinterpret_cast<int4 *>(desc)[i] = reinterpret_cast<const int4 *>(passes + p0)[i];
+    int coming = n > 1 ? list[1] : 0;
     tm.sync();
     int k = 0;
-    for (int i = a; i < b; i++) {
-        const BPass &p = desc[(i - a) & 1];
+    for (int i = 0; i < n; i++) {
+        const BPass &p = desc[i & 1];
         int4 next[PER];
-        if (i + 1 < b)
+        if (i + 1 < n)
 #pragma unroll
             for (int q = 0; q < PER; q++)
-                if (l + q * nl < words) next[q] = reinterpret_cast<const int4 *>(passes + i + 1)[l + q * nl];
-        const E *from = i == a ? first : arena;
-        E *to = i == b - 1 ? last : arena;
+                if (l + q * nl < words) next[q] = reinterpret_cast<const int4 *>(passes + coming)[l + q * nl];
+        coming = i + 2 < n ? list[i + 2] : 0;
+        const E *from = i == 0 ? first : arena;
+        E *to = i == n - 1 ? last : arena;
         double nb;
         if (TM::WARP && p.d == 1 && p.nb <= BATCH_NEAR_R && p.st[0].nmem == 1) nb = near_pass<E>(p, from, to, bits[k], cs.scale);
         else nb = team_pass<E>(p, (uint32_t)tm.rank(), tm.log2size(), from, to, bits + k, cs.scale, slots, stride);
         k += p.d;
-        if (i + 1 < b)
+        if (i + 1 < n)
 #pragma unroll
             for (int q = 0; q < PER; q++)
-                if (l + q * nl < words) reinterpret_cast<int4 *>(desc + ((i + 1 - a) & 1))[l + q * nl] = next[q];
+                if (l + q * nl < words) reinterpret_cast<int4 *>(desc + ((i + 1) & 1))[l + q * nl] = next[q];
         chain_update(cs, tm.sum(nb));
         if (cs.dead) break;
     }
@@ -548,9 +552,9 @@ __device__ void run_item(TM &tm, const BatchArgs &a, int item, E *arena, E *kept
     const int8_t *pb = a.pre_bits + in.pre_off + (int64_t)pre * in.K;
     if (tm.rank() == 0) arena[0] = mk2((typename ArithOf<E>::T)1, (typename ArithOf<E>::T)0);
     ChainState cs{1.0, 0.0, 1.0, 0, 0};
-    const int p0 = in.pass_off, p1 = p0 + in.npass[0], p2 = p1 + in.npass[1];
+    const int *list = a.list + in.list_off;
     const int words = in.R <= BATCH_NEAR_R ? BATCH_NEAR_WORDS : BATCH_WORDS;
-    run_passes<E, TM>(tm, a.passes, p0, p1, words, pb, arena, arena, kept, desc, slots, stride, cs);
+    run_passes<E, TM>(tm, a.passes, list, in.first[0], in.npass[0], words, pb, arena, arena, kept, desc, slots, stride, cs);
     const ChainState at_k = cs;
     const int nsuf_steps = in.ns - in.K;
     for (int sidx = 0; sidx < a.nsuf; sidx++) {
@@ -558,38 +562,40 @@ __device__ void run_item(TM &tm, const BatchArgs &a, int item, E *arena, E *kept
         double lp = -INFINITY;
         if (!cs.dead) {
             const int8_t *sb = a.suf_bits + in.suf_off + ((int64_t)pre * a.nsuf + sidx) * nsuf_steps;
-            run_passes<E, TM>(tm, a.passes, p1, p2, words, sb, kept, arena, arena, desc, slots, stride, cs);
+            run_passes<E, TM>(tm, a.passes, list + in.npass[0], in.first[1], in.npass[1], words, sb, kept, arena, arena, desc,
+                              slots, stride, cs);
             if (!cs.dead) lp = log2(cs.prev) + 2.0 * cs.lsc - in.n;
         }
         if (tm.rank() == 0) a.log2p[in.out_off + (int64_t)pre * a.nsuf + sidx] = lp;
     }
 }
 
-// Passes a .. b - 1 of a near instance by a warp, as run_passes: every pass is one step, its descriptor one word per lane.
+// The same for a near instance by a warp: every pass is one step, its descriptor one word per lane.
 template <typename E>
-__device__ __forceinline__ void near_passes(const BPass *passes, int a, int b, const int8_t *bits, const E *first, E *tab, E *last,
-                                            BPass *desc, ChainState &cs) {
+__device__ __forceinline__ void near_passes(const BPass *passes, const int *list, int p0, int n, const int8_t *bits,
+                                            const E *first, E *tab, E *last, BPass *desc, ChainState &cs) {
     const int lane = threadIdx.x & 31;
-    reinterpret_cast<int4 *>(desc)[lane] = reinterpret_cast<const int4 *>(passes + a)[lane];
-    int bit = bits[0];
+    reinterpret_cast<int4 *>(desc)[lane] = reinterpret_cast<const int4 *>(passes + p0)[lane];
+    int bit = bits[0], coming = n > 1 ? list[1] : 0;
     __syncwarp();
 #pragma unroll 1
-    for (int i = a; i < b; i++) {
-        const BPass &p = desc[(i - a) & 1];
+    for (int i = 0; i < n; i++) {
+        const BPass &p = desc[i & 1];
         int4 next = make_int4(0, 0, 0, 0);
         int next_bit = 0;
-        if (i + 1 < b) {
-            next = reinterpret_cast<const int4 *>(passes + i + 1)[lane];
-            next_bit = bits[i + 1 - a];
+        if (i + 1 < n) {
+            next = reinterpret_cast<const int4 *>(passes + coming)[lane];
+            next_bit = bits[i + 1];
         }
-        const E *from = i == a ? first : tab;
-        E *to = i == b - 1 ? last : tab;
+        coming = i + 2 < n ? list[i + 2] : 0;
+        const E *from = i == 0 ? first : tab;
+        E *to = i == n - 1 ? last : tab;
         const int ntq = p.st[0].ntq;
         double nb;
         if (ntq == 1) nb = near_step<E, 1>(p, from, to, bit, cs.scale);
         else if (ntq == 2) nb = near_step<E, 2>(p, from, to, bit, cs.scale);
         else nb = near_step<E, 4>(p, from, to, bit, cs.scale);
-        reinterpret_cast<int4 *>(desc + ((i + 1 - a) & 1))[lane] = next;
+        reinterpret_cast<int4 *>(desc + ((i + 1) & 1))[lane] = next;
         bit = next_bit;
         __syncwarp();
         chain_update(cs, warp_sum(nb));
@@ -603,16 +609,17 @@ __device__ __noinline__ void near_item(const BatchArgs &a, int item, E *tab, BPa
     E *kept = tab + (1 << BATCH_NEAR_R);
     if ((threadIdx.x & 31) == 0) tab[0] = mk2((typename ArithOf<E>::T)1, (typename ArithOf<E>::T)0);
     ChainState cs{1.0, 0.0, 1.0, 0, 0};
-    const int p0 = in.pass_off, p1 = p0 + in.npass[0], p2 = p1 + in.npass[1];
-    near_passes<E>(a.passes, p0, p1, a.pre_bits + in.pre_off + (int64_t)pre * in.K, tab, tab, kept, desc, cs);
+    const int *list = a.list + in.list_off;
+    near_passes<E>(a.passes, list, in.first[0], in.npass[0], a.pre_bits + in.pre_off + (int64_t)pre * in.K, tab, tab, kept, desc,
+                   cs);
     const ChainState at_k = cs;
     const int nsuf_steps = in.ns - in.K;
     for (int sidx = 0; sidx < a.nsuf; sidx++) {
         cs = at_k;
         double lp = -INFINITY;
         if (!cs.dead) {
-            near_passes<E>(a.passes, p1, p2, a.suf_bits + in.suf_off + ((int64_t)pre * a.nsuf + sidx) * nsuf_steps, kept, tab, tab,
-                           desc, cs);
+            near_passes<E>(a.passes, list + in.npass[0], in.first[1], in.npass[1],
+                           a.suf_bits + in.suf_off + ((int64_t)pre * a.nsuf + sidx) * nsuf_steps, kept, tab, tab, desc, cs);
             if (!cs.dead) lp = log2(cs.prev) + 2.0 * cs.lsc - in.n;
         }
         if ((threadIdx.x & 31) == 0) a.log2p[in.out_off + (int64_t)pre * a.nsuf + sidx] = lp;
@@ -693,8 +700,16 @@ struct BatchEngine {
     int prec = 64, dev = 0, sms = 0;
     size_t esize = 8;
     std::vector<HPlan> plans;
-    std::vector<int> K;             // prefix lengths that d_passes was made for
-    std::vector<int> pass_off, npass0, npass1;
+    std::vector<int> K;             // prefix lengths that the list was made for
+    struct Lists {
+        int off, npre, nsuf, pre0, suf0;   // in the list; passes and first pass of the prefix and of a suffix
+    };
+    std::vector<Lists> lists;
+    // per instance, entry 3 k + d - 1: the number of the pass of steps k .. k + d - 1 in d_passes, or one of these
+    enum { UNKNOWN = -1, NO_PASS = -2 };
+    std::vector<std::vector<int>> known;
+    size_t table_n = 0, table_cap = 0;   // passes in d_passes, and room
+    int *d_list = nullptr;
     std::vector<double> cost;       // per instance: entries moved by one prefix + its suffixes (relative)
     BPass *d_passes = nullptr;
     BInst *d_inst = nullptr;
@@ -706,7 +721,7 @@ struct BatchEngine {
     size_t arena_bytes = 0;
     size_t limit = SIZE_MAX;        // of the arenas' bytes, where clusters can be done without (shape_layout)
     int npre = 0, nsuf = 0;
-    int64_t pre_total = 0, suf_total = 0, out_total = 0;
+    int64_t pre_cap = 0, suf_cap = 0, out_cap = 0, out_total = 0;   // bytes, bytes, results: room; results set
     std::vector<BInst> h_inst;
     cudaStream_t stream = nullptr;
     BatchShape shape;
@@ -719,6 +734,7 @@ struct BatchEngine {
         cudaSetDevice(dev);
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
         cudaFree(d_passes);
+        cudaFree(d_list);
         cudaFree(d_inst);
         cudaFree(d_items);
         cudaFree(d_pre);
@@ -867,79 +883,147 @@ static bool make_pass(const HPlan &p, const GroupPlan &gp, int slots, BPass &g) 
     return true;
 }
 
-// Passes of steps k0 .. k1 - 1, each as long as its classes' slots allow.  A narrow instance is run by one warp by
-// default, and fusing leaves its lanes few classes with a long chain of work each: up to width 12 passes of several
-// steps have at least 2^8 classes (300 instances of widths up to 12: 0.63 ms with any number of classes, 0.43 at 2^5, 0.36
-// at 2^8).  Block and cluster teams are faster fused throughout (60 instances of widths 8-14: 0.27 against 0.33 ms).
-static bool passes_of(const HPlan &p, int k0, int k1, int slots, std::vector<BPass> &out) {
-    const int least = p.R <= 12 ? 8 : 0;
+// Passes of steps k0 .. k1 - 1, each as long as its classes' slots allow, appended to `list`; pass_at(k, d): the number of the pass
+// of steps k .. k + d - 1, or NO_PASS or UNKNOWN, which ends the list and is returned (as is NO_PASS where not even a single
+// step fits; otherwise 0).  A narrow instance is run by one warp by default, and fusing leaves its lanes few classes with a
+// long chain of work each: up to width 12 passes of several steps have at least 2^8 classes (300 instances of widths up to
+// 12: 0.63 ms with any number of classes, 0.43 at 2^5, 0.36 at 2^8).  Block and cluster teams are faster fused throughout
+// (60 instances of widths 8-14: 0.27 against 0.33 ms).
+static int least_classes(const HPlan &p) { return p.R <= 12 ? 8 : 0; }
+template <typename F>
+static int passes_of(const HPlan &p, int k0, int k1, F pass_at, std::vector<int> &list) {
+    const int least = least_classes(p);
     for (int k = k0; k < k1;) {
-        BPass g;
-        GroupPlan gp;
-        int d = 1;   // a pass has at most the 2^nk cosets of each of its steps as classes
-        while (p.R > BATCH_NEAR_R && d < FUSE_MAX_STEPS && k + d < k1 && std::min(p.st[(size_t)k].nk, p.st[(size_t)(k + d)].nk) >= least) d++;
-        while (d > 0 && !(plan_group(p, k, d, 0, 24, gp) && (d == 1 || gp.nb >= least) && make_pass(p, gp, slots, g))) d--;
-        if (!d) return false;
-        out.push_back(g);
+        int d = 1, pass = BatchEngine::NO_PASS;   // a pass has at most the 2^nk cosets of each of its steps as classes
+        while (p.R > BATCH_NEAR_R && d < FUSE_MAX_STEPS && k + d < k1 &&
+               std::min(p.st[(size_t)k].nk, p.st[(size_t)(k + d)].nk) >= least)
+            d++;
+        for (; d > 0 && (pass = pass_at(k, d)) == BatchEngine::NO_PASS; d--) {}
+        if (pass < 0) return pass;
+        list.push_back(pass);
         k += d;
     }
-    return true;
+    return 0;
 }
 
-// The pass lists for prefix lengths K (kept while they stay the same), made by the host's cores side by side: 17 us per
-// candidate pass, 20 passes per instance.
+// The pass lists for prefix lengths K.  A pass is derived once, when a list first needs it (10 us; the host's cores side by
+// side), and stays in the device's table: other prefix lengths need few new ones or none.  Two set_strings with other prefix
+// lengths: 300 instances of widths 4-5 5.4 ms with a table made for each call, 100 of width 11 3.8 ms; now 0.6 and 0.3.
 static int batch_passes(BatchEngine &E, const int *K) {
     const size_t n = E.plans.size();
     if (E.K.size() == n && std::equal(E.K.begin(), E.K.end(), K)) return 0;
-    std::vector<std::vector<BPass>> got(n);
-    std::vector<int> pre(n, 0), bad(n, 0);
+    constexpr int FRESH = 1 << 28;   // a derived pass's number until it has one in the device's table
     const int slots = BATCH_SLOT_BYTES / (int)E.esize;
-    const unsigned nt = std::max(1u, std::min({(unsigned)n, 16u, std::thread::hardware_concurrency()}));
-    std::atomic<size_t> next{0};
-    auto work = [&] {
-        for (size_t i; (i = next++) < n;) {
-            try {
-                const HPlan &p = E.plans[i];
-                bad[i] = !passes_of(p, 0, K[i], slots, got[i]);
-                pre[i] = (int)got[i].size();
-                bad[i] = bad[i] || !passes_of(p, K[i], p.ns, slots, got[i]);
-            } catch (const std::bad_alloc &) {
-                bad[i] = 2;
-            }
+    if (E.known.empty())
+        for (const HPlan &p : E.plans) E.known.emplace_back((size_t)(FUSE_MAX_STEPS * p.ns), BatchEngine::UNKNOWN);
+    std::vector<std::vector<int>> rows(n);       // E.known with this call's passes, of the instances that needed some
+    std::vector<std::vector<BPass>> derived(n);
+    std::vector<int> list, off(n), pre(n);
+    std::vector<size_t> todo;
+    // the lists with the passes at hand; false: no pass fits a step of instance *bad
+    auto assemble = [&](size_t *bad) {
+        list.clear();
+        todo.clear();
+        for (size_t i = 0; i < n; i++) {
+            const HPlan &p = E.plans[i];
+            const std::vector<int> &row = rows[i].empty() ? E.known[i] : rows[i];
+            auto at = [&](int k, int d) { return row[(size_t)(FUSE_MAX_STEPS * k + d - 1)]; };
+            off[i] = (int)list.size();
+            int rc = passes_of(p, 0, K[i], at, list);
+            pre[i] = (int)list.size() - off[i];
+            if (!rc) rc = passes_of(p, K[i], p.ns, at, list);
+            *bad = i;
+            if (rc == BatchEngine::NO_PASS) return false;
+            if (rc) todo.push_back(i);
         }
+        return true;
     };
-    std::vector<std::thread> th;
-    th.reserve(nt);
-    try {
-        for (unsigned t = 1; t < nt; t++) th.emplace_back(work);
-    } catch (const std::exception &) {   // no more threads: those there are, and this one, take all instances
+    auto derive = [&](size_t i) {
+        const HPlan &p = E.plans[i];
+        std::vector<int> row = E.known[i], any;
+        auto at = [&](int k, int d) {
+            int &x = row[(size_t)(FUSE_MAX_STEPS * k + d - 1)];
+            if (x != BatchEngine::UNKNOWN) return x;
+            BPass g;
+            GroupPlan gp;
+            x = BatchEngine::NO_PASS;
+            if (plan_group(p, k, d, 0, 24, gp) && (d == 1 || gp.nb >= least_classes(p)) && make_pass(p, gp, slots, g)) {
+                x = FRESH + (int)derived[i].size();
+                derived[i].push_back(g);
+            }
+            return x;
+        };
+        if (!passes_of(p, 0, K[i], at, any)) passes_of(p, K[i], p.ns, at, any);
+        rows[i].swap(row);
+    };
+    size_t bad = 0;
+    std::vector<BPass> fresh;
+    bool fits = assemble(&bad);
+    if (fits && !todo.empty()) {
+        const unsigned nt = std::min({(unsigned)todo.size(), 16u, std::max(1u, std::thread::hardware_concurrency())});
+        std::atomic<size_t> next{0};
+        std::atomic<bool> memory{true};
+        auto work = [&] {
+            for (size_t j; (j = next++) < todo.size();) {
+                try {
+                    derive(todo[j]);
+                } catch (const std::bad_alloc &) {
+                    memory = false;
+                }
+            }
+        };
+        std::vector<std::thread> th;
+        th.reserve(nt);
+        try {
+            for (unsigned t = 1; t < nt; t++) th.emplace_back(work);
+        } catch (const std::exception &) {   // no more threads: those there are, and this one, take all instances
+        }
+        work();
+        for (std::thread &t : th) t.join();
+        if (!memory) return fail(GSB_E_ALLOC, "no host memory for the batch's passes");
+        for (size_t i : todo) {
+            for (int &x : rows[i])
+                if (x >= FRESH) x += (int)(E.table_n + fresh.size()) - FRESH;
+            fresh.insert(fresh.end(), derived[i].begin(), derived[i].end());
+        }
+        fits = assemble(&bad);
     }
-    work();
-    for (std::thread &t : th) t.join();
-    std::vector<BPass> all;
-    std::vector<int> off(n, 0), suf(n, 0);
+    if (!fits) return fail(GSB_E_PLAN_LAYOUT, "instance " + std::to_string(bad) + " does not fit the batch kernel's passes");
+    // until the new passes are on the device the engine keeps the old lists, with the offsets that belong to them
+    const size_t need = E.table_n + fresh.size();
+    cudaError_t e = cudaSuccess;
+    if (!E.d_list) {   // at most one pass per step
+        size_t steps = 0;
+        for (const HPlan &p : E.plans) steps += (size_t)p.ns;
+        e = cudaMalloc(&E.d_list, steps * sizeof(int));
+    }
+    if (e == cudaSuccess && need > E.table_cap) {
+        const size_t cap = E.table_n ? need + need / 2 : need;
+        BPass *d = nullptr;
+        e = cudaMalloc(&d, cap * sizeof(BPass));
+        if (e == cudaSuccess && E.table_n) e = cudaMemcpy(d, E.d_passes, E.table_n * sizeof(BPass), cudaMemcpyDeviceToDevice);
+        if (e == cudaSuccess) {
+            for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);   // they point at the old table
+            E.graphs.clear();
+            cudaFree(E.d_passes);
+            E.d_passes = d;
+            E.table_cap = cap;
+        } else {
+            cudaFree(d);
+        }
+    }
+    if (e == cudaSuccess && !fresh.empty())
+        e = cudaMemcpy(E.d_passes + E.table_n, fresh.data(), fresh.size() * sizeof(BPass), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(E.d_list, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return fail(GSB_E_CUDA, std::string("the batch's pass table: ") + cudaGetErrorString(e));
+    E.table_n = need;
+    for (size_t i = 0; i < n; i++)
+        if (!rows[i].empty()) E.known[i].swap(rows[i]);
+    E.lists.resize(n);
     for (size_t i = 0; i < n; i++) {
-        if (bad[i]) return fail(GSB_E_PLAN_LAYOUT, "instance " + std::to_string(i) + " does not fit the batch kernel's passes");
-        off[i] = (int)all.size();
-        suf[i] = (int)got[i].size() - pre[i];
-        all.insert(all.end(), got[i].begin(), got[i].end());
+        const int end = i + 1 < n ? off[i + 1] : (int)list.size(), suf = off[i] + pre[i];
+        E.lists[i] = BatchEngine::Lists{off[i], pre[i], end - suf, list[(size_t)off[i]], list[(size_t)suf]};
     }
-    // until the new table is on the device the engine keeps the old one, with the offsets that belong to it
-    BPass *d = nullptr;
-    cudaError_t e = cudaMalloc(&d, all.size() * sizeof(BPass));
-    if (e == cudaSuccess) e = cudaMemcpy(d, all.data(), all.size() * sizeof(BPass), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(d);
-        return fail(GSB_E_CUDA, std::string("the batch's pass table: ") + cudaGetErrorString(e));
-    }
-    for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);   // they point at the old passes
-    E.graphs.clear();
-    cudaFree(E.d_passes);
-    E.d_passes = d;
-    E.pass_off.swap(off);
-    E.npass0.swap(pre);
-    E.npass1.swap(suf);
     E.K.assign(K, K + n);
     return 0;
 }
@@ -984,6 +1068,7 @@ static int batch_graph(BatchEngine &E, const BatchShape &sh, cudaGraphExec_t *ou
     BatchArgs a;
     a.passes = E.d_passes;
     a.inst = E.d_inst;
+    a.list = E.d_list;
     a.items_wide = E.d_items;
     a.items_big = a.items_wide + L.wide.size();
     a.items_small = a.items_big + L.big.size();
@@ -1139,15 +1224,23 @@ int gsb_batch_set_strings(gsb_batch *h, const int *K, int npre, int nsuf, const 
     } restore{prev};
     if (int rc = batch_passes(E, K)) return rc;
     for (int i = 0; i < ninst; i++) {
-        inst[(size_t)i].pass_off = E.pass_off[(size_t)i];
-        inst[(size_t)i].npass[0] = E.npass0[(size_t)i];
-        inst[(size_t)i].npass[1] = E.npass1[(size_t)i];
+        const BatchEngine::Lists &l = E.lists[(size_t)i];
+        inst[(size_t)i].list_off = l.off;
+        inst[(size_t)i].npass[0] = l.npre;
+        inst[(size_t)i].npass[1] = l.nsuf;
+        inst[(size_t)i].first[0] = l.pre0;
+        inst[(size_t)i].first[1] = l.suf0;
     }
-    // no d_inst (the last of the buffers): none yet, or a call that found no memory for them
-    const bool resize = !E.d_inst || po != E.pre_total || so != E.suf_total || oo != E.out_total || npre != E.npre || nsuf != E.nsuf;
-    if (resize) {
+    // Buffers grow and stay: a call whose strings fit them keeps the graphs as well, unless it has other counts.  No d_inst (the
+    // last of the buffers): none yet, or a call that found no memory for them.
+    const bool grow = !E.d_inst || po > E.pre_cap || so > E.suf_cap || oo > E.out_cap;
+    if (grow || npre != E.npre || nsuf != E.nsuf) {
         for (auto &kv : E.graphs) cudaGraphExecDestroy(kv.second);
         E.graphs.clear();
+    }
+    if (grow) {
+        const int64_t pre = std::max(po, E.pre_cap), suf = std::max(so, E.suf_cap), res = std::max(oo, E.out_cap);
+        E.pre_cap = E.suf_cap = E.out_cap = 0;
         cudaFree(E.d_pre);
         cudaFree(E.d_suf);
         cudaFree(E.d_out);
@@ -1156,16 +1249,17 @@ int gsb_batch_set_strings(gsb_batch *h, const int *K, int npre, int nsuf, const 
         E.d_suf = nullptr;
         E.d_out = nullptr;
         E.d_inst = nullptr;
-        BT_CK(cudaMalloc(&E.d_pre, (size_t)std::max<int64_t>(po, 1)));
-        BT_CK(cudaMalloc(&E.d_suf, (size_t)std::max<int64_t>(so, 1)));
-        BT_CK(cudaMalloc(&E.d_out, (size_t)std::max<int64_t>(oo, 1) * sizeof(double)));
+        BT_CK(cudaMalloc(&E.d_pre, (size_t)pre));
+        BT_CK(cudaMalloc(&E.d_suf, (size_t)suf));
+        BT_CK(cudaMalloc(&E.d_out, (size_t)res * sizeof(double)));
         BT_CK(cudaMalloc(&E.d_inst, (size_t)ninst * sizeof(BInst)));
-        E.pre_total = po;
-        E.suf_total = so;
-        E.out_total = oo;
-        E.npre = npre;
-        E.nsuf = nsuf;
+        E.pre_cap = pre;
+        E.suf_cap = suf;
+        E.out_cap = res;
     }
+    E.out_total = oo;
+    E.npre = npre;
+    E.nsuf = nsuf;
     BT_CK(cudaMemcpy(E.d_inst, inst.data(), (size_t)ninst * sizeof(BInst), cudaMemcpyHostToDevice));
     BT_CK(cudaMemcpy(E.d_pre, prefix_bits, (size_t)po, cudaMemcpyHostToDevice));
     BT_CK(cudaMemcpy(E.d_suf, suffix_bits, (size_t)so, cudaMemcpyHostToDevice));
@@ -1177,7 +1271,7 @@ int gsb_batch_set_strings(gsb_batch *h, const int *K, int npre, int nsuf, const 
 int gsb_batch_run(gsb_batch *h, double *log2p, float *ms) {
     if (!h || !log2p) return fail(GSB_E_USAGE, "null argument");
     BatchEngine &E = h->E;
-    if (!E.d_out) return fail(GSB_E_STATE, "no strings set (gsb_batch_set_strings)");
+    if (!E.d_inst) return fail(GSB_E_STATE, "no strings set (gsb_batch_set_strings)");
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(E.dev);
@@ -1232,7 +1326,7 @@ int gsb_batch_get_shape(const gsb_batch *h, int *block, int *small_R, int *per_s
 int gsb_batch_tune(gsb_batch *h, int reps, size_t max_bytes, int *block, int *small_R, int *per_sm, float *best_ms) {
     if (!h || reps < 1) return fail(GSB_E_USAGE, "bad argument");
     BatchEngine &E = h->E;
-    if (!E.d_out) return fail(GSB_E_STATE, "no strings set (gsb_batch_set_strings)");
+    if (!E.d_inst) return fail(GSB_E_STATE, "no strings set (gsb_batch_set_strings)");
     std::vector<double> out((size_t)std::max<int64_t>(E.out_total, 1));
     float best = 1e30f;
     E.limit = max_bytes;

@@ -9,12 +9,12 @@
 namespace {
 std::map<void *, size_t> blocks;
 size_t used = 0, capacity = (size_t)1 << 40, largest = 0;
-long mallocs = 0, failed = 0, launches = 0, attributes = 0, null_arguments = 0;
+long fail_at = 0, mallocs = 0, failed = 0, launches = 0, attributes = 0, null_arguments = 0;
 char handle;   // what every stream and event points at
-// A graph remembers the device buffers that its batched launch was given (the first three arguments: passes, instances,
-// items); a replay after one of them was freed is counted.
+// A graph remembers the device buffers that its batched launch was given (the first four arguments: passes, instances,
+// lists, items); a replay after one of them was freed is counted.
 struct Graph {
-    void *buf[3];
+    void *buf[4];
 };
 Graph captured;
 long stale = 0, replays = 0, fused_one = 0, fused_several = 0, fused_wrong = 0;
@@ -26,6 +26,7 @@ extern "C" {
 
 // capacity of the device; what was asked of it since the last reset
 void fake_set_capacity(size_t bytes) { capacity = bytes; }
+void fake_fail(long nth) { fail_at = nth; }   // the nth allocation from now on fails
 size_t fake_used(void) { return used; }
 long fake_count(int what) {
     return what == 0 ? mallocs : what == 1 ? failed : what == 2 ? launches : what == 3 ? attributes : what == 4 ? null_arguments : what == 5 ? stale : what == 6 ? replays : what == 7 ? fused_one
@@ -37,7 +38,7 @@ void fake_reset(void) { mallocs = failed = launches = attributes = null_argument
 cudaError_t cudaMalloc(void **p, size_t n) {
     mallocs++;
     *p = nullptr;
-    if (used + n > capacity) {
+    if (used + n > capacity || (fail_at && --fail_at == 0)) {
         failed++;
         return last = cudaErrorMemoryAllocation;
     }
@@ -146,8 +147,8 @@ cudaError_t cudaLaunchKernel(const void *f, dim3 grid, dim3, void **, size_t, cu
     return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **args) {
-    if (!*(void **)args[0]) null_arguments++;   // the batched launch: its first argument is the pass table
-    memcpy(captured.buf, args[0], sizeof captured.buf);
+    memcpy(captured.buf, args[0], sizeof captured.buf);   // the batched launch
+    for (void *b : captured.buf) null_arguments += !b;
     return cudaLaunchKernel(f, c->gridDim, c->blockDim, args, c->dynamicSmemBytes, c->stream);
 }
 

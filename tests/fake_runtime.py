@@ -53,6 +53,7 @@ def load():
         getattr(dev, f).restype = ctypes.c_size_t
     dev.fake_count.restype = ctypes.c_long
     dev.fake_set_capacity.argtypes = [ctypes.c_size_t]
+    dev.fake_fail.argtypes = [ctypes.c_long]
     return gsb, dev
 
 

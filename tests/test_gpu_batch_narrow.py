@@ -63,3 +63,27 @@ def test_impossible_strings(narrow, prec):
             dead = np.zeros((2, 2), bool)
             dead[(1, slice(None)) if k < K else (slice(None), 1)] = True
             assert (np.isneginf(lp) == dead).all(), (ns, k, lp)
+
+
+@pytest.mark.parametrize("prec", [128, 64])
+def test_prefix_lengths_in_any_order(narrow, prec):
+    """One batch, prefix lengths drawn anew for every instance: the passes that earlier lengths left behind and new ones."""
+    import gsb
+    import workloads
+    ws = narrow + [workloads.matching_instance(n, n, 11, 8, 2000) for n in (33, 37)]
+    ns = [len(w["steps"]) for w in ws]
+    rng = np.random.default_rng(6)
+    b = gsb.Batch([w["plan"] for w in ws], precision=prec)
+    strings = [rng.integers(0, 2, (4, n), dtype=np.int8) for n in ns]
+    ref = []
+    for w, x in zip(ws, strings):
+        with gsb.Engine.from_text(w["plan"], precision=128) as eng:
+            ref.append(eng.chain(x)[0])
+    for turn in range(12):
+        K = [int(rng.integers(1, n)) for n in ns] if turn else [1] * len(ns)
+        b.set_strings(K, [x[:, :k] for x, k in zip(strings, K)], [x[:, None, k:] for x, k in zip(strings, K)])
+        lp, _ = b.run()
+        for i, n in enumerate(ns):
+            tol = 1e-9 if prec == 128 else 6 * gsb.c64_sigma(ref[i], n)
+            assert (np.abs(lp[i][:, 0] - ref[i]) <= tol).all(), (turn, n, K[i])
+    b.close()

@@ -289,3 +289,43 @@ def test_tables_take_the_place_of_slots(fake, prec):
         dev.fake_reset()
         eng.chain(lines)
         assert dev.fake_count(FAILED) == 0 and dev.fake_count(REPLAYS) < 64
+
+
+def test_batch_without_one_of_its_buffers(fake):
+    """The same, whichever allocation of a set_strings or of the run after it fails."""
+    gsb, dev = fake
+    plans = [plan(n) for n in (18, 24)]
+    for nth in range(1, 12):
+        b = gsb.Batch(plans)
+        for K, npre in ((4, 1), (8, 2)):
+            dev.fake_fail(nth if K == 8 else 0)
+            try:
+                b.set_strings(*batch_strings(plans, K, npre=npre))
+                b.run()
+            except gsb.GsbError as e:
+                assert K == 8 and "out of memory" in str(e)
+        dev.fake_fail(0)
+        try:
+            b.run()
+        except gsb.GsbError as e:
+            assert "no strings set" in str(e)
+        b.set_strings(*batch_strings(plans, 8))
+        b.run()
+        b.close()
+    assert dev.fake_count(NULL_TABLES) == dev.fake_count(STALE_REPLAYS) == 0 < dev.fake_count(FAILED)
+
+
+def test_batch_with_other_prefix_lengths(fake):
+    """Prefix lengths that change from call to call take no device memory once their passes and strings have had room, and
+    keep the graph."""
+    gsb, dev = fake
+    plans = [plan(n) for n in (12, 18, 24, 36)]
+    b = gsb.Batch(plans)
+    for turn in range(3):
+        dev.fake_reset()
+        for K in range(1, 12):
+            b.set_strings(*batch_strings(plans, K))
+            b.run()
+    assert dev.fake_count(MALLOCS) == 0 and dev.fake_count(LAUNCHES) == 0 and dev.fake_count(REPLAYS) == 11
+    b.close()
+    assert dev.fake_used() == 0
