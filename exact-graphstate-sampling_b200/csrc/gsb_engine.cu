@@ -180,6 +180,7 @@ struct Engine {
     int fuse_depth = 0;                  // chain mode: steps fused into one pass at most (1 = none; 0: modelled, chain_cover)
     std::vector<Op> chain_ops;           // 'chain' passes
     bool prob_by_chain = false;          // 'prob' strings run the 'chain' passes (conserves)
+    std::map<std::pair<int, int>, Op> cover_ops;   // fused passes (k, d) that chain_cover tried, with the current matrices
     int hyb_K = 0;                       // gsb_set_hybrid_prefix: hybrid strings force their first hyb_K steps
     std::vector<Op> hyb_ops;             // fused 'chain' passes over those steps
     std::vector<Op> sample_ops;          // 'prob' / 'sample' passes (build_sample_ops)
@@ -1181,29 +1182,30 @@ static void chain_cover(Engine &E, int k0, int k1, std::vector<Op> &ops) {
     }
     const double latency = 8e-6 * 6e12 / (double)E.esize / E.max_slots;   // of a launch, in entries at 6 TB/s
     std::vector<double> cost((size_t)(k1 - k0) + 1, 0.0);
-    std::vector<Op> best((size_t)(k1 - k0));
+    std::vector<int> steps((size_t)(k1 - k0), 1);
     for (int k = k1 - 1; k >= k0; k--) {
         double &c = cost[(size_t)(k - k0)];
-        Op &pick = best[(size_t)(k - k0)];
-        pick = single(k);
         // a step in a run shares the run's launch with its neighbours
-        c = pick.entries + (E.in_run(k) ? latency / 8 : latency) + cost[(size_t)(k + 1 - k0)];
+        c = single_entries(p, k) + (E.in_run(k) ? latency / 8 : latency) + cost[(size_t)(k + 1 - k0)];
         if (rof(k) < GROUP_MIN_R) continue;
         for (int d = 2; d <= std::min(FUSE_MAX_STEPS, k1 - k); d++) {
+            const auto made = E.cover_ops.try_emplace(std::make_pair(k, d));
+            Op &op = made.first->second;
             GroupPlan gp;
-            Op op;
-            if (!plan_group(p, k, d, 6, GROUP_MAX_L, gp) || !fill_group(E, gp, op)) continue;
+            if (made.second && !(plan_group(p, k, d, 6, GROUP_MAX_L, gp) && fill_group(E, gp, op))) op.group = false;
+            if (!op.group) continue;
             const double rate = op.ws ? (d == 2 ? 1.0 : 0.82) : d == 2 ? 0.75 : E.prec == 64 ? 0.37 : 0.48;
             const double t = op.entries / rate + latency + cost[(size_t)(k + d - k0)];
             if (t < c) {
                 c = t;
-                pick = op;
+                steps[(size_t)(k - k0)] = d;
             }
         }
     }
-    for (int k = k0; k < k1;) {
-        ops.push_back(best[(size_t)(k - k0)]);
-        k += ops.back().d;
+    for (int k = k0; k < k1; k += ops.back().d) {
+        const int d = steps[(size_t)(k - k0)];
+        if (d == 1) ops.push_back(single(k));
+        else ops.push_back(E.cover_ops.at(std::make_pair(k, d)));
     }
 }
 
@@ -1214,6 +1216,7 @@ static void build_hyb_ops(Engine &E) {
 }
 
 static void build_chain_ops(Engine &E) {
+    E.cover_ops.clear();
     build_hyb_ops(E);
     build_sample_ops(E);
     E.chain_ops.clear();
