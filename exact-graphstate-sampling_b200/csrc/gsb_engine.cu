@@ -53,7 +53,7 @@ struct Launch {
     int grid = 1, block = 1, U = 1, tl = 0, cl = 0;
     int cap = 1;                // blocks the device holds at once
     unsigned int nchunks = 1;
-    void *fn = nullptr;
+    void *fn = nullptr, *fn_slots = nullptr;   // kernels of launches that carry one item, and several
 };
 
 struct DevGuard {
@@ -69,37 +69,35 @@ struct DevGuard {
     }
 };
 
-template <int NTQ, int M>
+// Single-step kernels, for launches of one item (SLOTS = false) or of several.
+template <int NTQ, int M, bool SLOTS>
 static void *pick_any64(bool write) {
-    return write ? (void *)k_step<float2, NTQ, M, 4, true> : (void *)k_step<float2, NTQ, M, 4, false>;
-}
-static void *pick_step_kernel(int ntq, int m, bool write) {
-    if (ntq == 4) return m == 2 ? pick_any64<4, 2>(write) : pick_any64<4, 1>(write);
-    if (ntq == 2) return m == 2 ? pick_any64<2, 2>(write) : pick_any64<2, 1>(write);
-    return m == 2 ? pick_any64<1, 2>(write) : pick_any64<1, 1>(write);
+    return write ? (void *)k_step<float2, NTQ, M, 4, true, SLOTS> : (void *)k_step<float2, NTQ, M, 4, false, SLOTS>;
 }
 
 // wide-step kernels: U = 4 coset groups per thread for 1-2 offsets, 2 for 4 offsets (register budget)
-template <int NTQ, int M>
+template <int NTQ, int M, bool SLOTS>
 static void *pick_pair64(bool write, bool fp32) {
     constexpr int U = NTQ == 4 ? 2 : 4;
-    if (fp32) return write ? (void *)k_pair64<float, NTQ, M, U, true> : (void *)k_pair64<float, NTQ, M, U, false>;
-    return write ? (void *)k_pair64<double, NTQ, M, U, true> : (void *)k_pair64<double, NTQ, M, U, false>;
+    if (fp32) return write ? (void *)k_pair64<float, NTQ, M, U, true, SLOTS> : (void *)k_pair64<float, NTQ, M, U, false, SLOTS>;
+    return write ? (void *)k_pair64<double, NTQ, M, U, true, SLOTS> : (void *)k_pair64<double, NTQ, M, U, false, SLOTS>;
 }
-template <int NTQ, int M>
+template <int NTQ, int M, bool SLOTS>
 static void *pick_wide128(bool write) {
     constexpr int U = NTQ == 4 ? 2 : 4;
-    return write ? (void *)k_wide128<NTQ, M, U, true> : (void *)k_wide128<NTQ, M, U, false>;
+    return write ? (void *)k_wide128<NTQ, M, U, true, SLOTS> : (void *)k_wide128<NTQ, M, U, false, SLOTS>;
 }
-static void *pick_wide(int prec, int ntq, int m, bool write, bool fp32) {
-    if (prec == 64) {
-        if (ntq == 4) return m == 2 ? pick_pair64<4, 2>(write, fp32) : pick_pair64<4, 1>(write, fp32);
-        if (ntq == 2) return m == 2 ? pick_pair64<2, 2>(write, fp32) : pick_pair64<2, 1>(write, fp32);
-        return m == 2 ? pick_pair64<1, 2>(write, fp32) : pick_pair64<1, 1>(write, fp32);
-    }
-    if (ntq == 4) return m == 2 ? pick_wide128<4, 2>(write) : pick_wide128<4, 1>(write);
-    if (ntq == 2) return m == 2 ? pick_wide128<2, 2>(write) : pick_wide128<2, 1>(write);
-    return m == 2 ? pick_wide128<1, 2>(write) : pick_wide128<1, 1>(write);
+enum StepKernel { STEP_ANY64, STEP_PAIR64, STEP_WIDE128 };
+template <int NTQ, int M, bool SLOTS>
+static void *pick_step_of(StepKernel kind, bool write, bool fp32) {
+    return kind == STEP_ANY64 ? pick_any64<NTQ, M, SLOTS>(write)
+           : kind == STEP_PAIR64 ? pick_pair64<NTQ, M, SLOTS>(write, fp32) : pick_wide128<NTQ, M, SLOTS>(write);
+}
+template <bool SLOTS>
+static void *pick_step(StepKernel kind, int ntq, int m, bool write, bool fp32) {
+    if (ntq == 4) return m == 2 ? pick_step_of<4, 2, SLOTS>(kind, write, fp32) : pick_step_of<4, 1, SLOTS>(kind, write, fp32);
+    if (ntq == 2) return m == 2 ? pick_step_of<2, 2, SLOTS>(kind, write, fp32) : pick_step_of<2, 1, SLOTS>(kind, write, fp32);
+    return m == 2 ? pick_step_of<1, 2, SLOTS>(kind, write, fp32) : pick_step_of<1, 1, SLOTS>(kind, write, fp32);
 }
 
 template <typename E, typename T, bool SLOTS>
@@ -295,7 +293,9 @@ struct Engine {
             L.tl = 8;
             L.cl = (wide64 ? 9 : 8) + (uw == 4 ? 2 : 1);
             L.nchunks = (unsigned int)(N >> L.cl);
-            L.fn = pick_wide(prec, a.ntq, a.m, write, arith == 32);
+            const StepKernel kind = wide64 ? STEP_PAIR64 : STEP_WIDE128;
+            L.fn = pick_step<false>(kind, a.ntq, a.m, write, arith == 32);
+            L.fn_slots = pick_step<true>(kind, a.ntq, a.m, write, arith == 32);
             L.cap = occupancy(L.fn, L.block) * sms;
             L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)L.cap);
             return L;
@@ -306,7 +306,8 @@ struct Engine {
         L.tl = 8;
         L.cl = 10;
         L.nchunks = (unsigned int)(N >> L.cl);
-        L.fn = pick_step_kernel(a.ntq, a.m, write);
+        L.fn = pick_step<false>(STEP_ANY64, a.ntq, a.m, write, true);
+        L.fn_slots = pick_step<true>(STEP_ANY64, a.ntq, a.m, write, true);
         L.cap = occupancy(L.fn, L.block) * sms;
         L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)L.cap);
         return L;
@@ -352,8 +353,8 @@ struct Engine {
         Ctx c = ctx(driver, k1, L, use_forced, use_unif);
         void *memp = arena_mem();
         void *kargs[] = {&a, &memp, &c};
-        return cudaLaunchKernel(L.fn, dim3(slot_grid(L.grid, L.cap), (unsigned)slots), dim3((unsigned)L.block), kargs, 0,
-                                stream);
+        return cudaLaunchKernel(slots == 1 ? L.fn : L.fn_slots, dim3(slot_grid(L.grid, L.cap), (unsigned)slots),
+                                dim3((unsigned)L.block), kargs, 0, stream);
     }
 
     // Steps k0 .. k1 - 1, all of one run part, as one k_run launch; norm: the branch norms of steps whose bit is drawn.

@@ -218,10 +218,10 @@ __device__ __forceinline__ void write_epilogue(const Ctx &cx, int k, int bv, dou
 }
 
 // A step of any layout (2^10 cosets or more): complex64 steps whose coset bit 0 is not arena bit 0 (k_pair64 needs that).
-template <typename E, int NTQ, int MOUT, int U, bool WRITE>
+template <typename E, int NTQ, int MOUT, int U, bool WRITE, bool SLOTS>
 __global__ void __launch_bounds__(256) k_step(const StepArgs s, E *__restrict__ mem, const Ctx c0) {
-    const Ctx cx = slot_ctx(c0);
-    mem += (size_t)blockIdx.y * cx.arena;
+    const Ctx cx = SLOTS ? slot_ctx(c0) : c0;
+    if (SLOTS) mem += (size_t)blockIdx.y * cx.arena;
     DevState *st = cx.st;
     if (*(volatile int *)&st->dead) return;
     const size_t row = (size_t)st->item * (size_t)cx.ns;
@@ -337,7 +337,9 @@ __global__ void __launch_bounds__(256) k_step(const StepArgs s, E *__restrict__ 
 //   * walk their block's range of chunks in Gray-code order, so consecutive chunks differ in one coset bit and the
 //     chunk's base address is updated with one XOR (chunk i covers cosets gray(i) * 2^chunk_log2 + [0, 2^chunk_log2));
 //   * fold the step's scale into the M row of the write pass (one uniform multiply per kernel, not per entry);
-//   * prepare the write/norm decision exactly as k_step does (same prologue, same epilogues).
+//   * prepare the write/norm decision exactly as k_step does (same prologue, same epilogues);
+//   * are built for launches of one item and of several (SLOTS), as the fused passes are: with computed pointers one item's
+//     unfused passes took 5 % longer in complex128 and 9 % in complex64 with FP64 arithmetic.
 
 struct Prologue {
     int bv;
@@ -388,10 +390,10 @@ __device__ __forceinline__ double fmaT(double a, double b, double c) { return fm
 //           complex64 build (gsamp2.cpp:32-38, 52);
 //   float : sums and rotation in FP32 (a few roundings per entry; faster on the FP32 pipe).
 // Chunk = 256 threads x U pairs = 2^(9 + log2 U) cosets; pair u of thread t covers cosets 2t + 512u + {0, 1}.
-template <typename T, int NTQ, int MOUT, int U, bool WRITE>
+template <typename T, int NTQ, int MOUT, int U, bool WRITE, bool SLOTS>
 __global__ void __launch_bounds__(256) k_pair64(const StepArgs s, float2 *__restrict__ mem, const Ctx c0) {
-    const Ctx cx = slot_ctx(c0);
-    mem += (size_t)blockIdx.y * cx.arena;
+    const Ctx cx = SLOTS ? slot_ctx(c0) : c0;
+    if (SLOTS) mem += (size_t)blockIdx.y * cx.arena;
     const Prologue P = step_prologue(s, cx, WRITE);
     if (P.skip) return;
     __shared__ uint64_t tks[40];
@@ -520,10 +522,10 @@ __global__ void __launch_bounds__(256) k_pair64(const StepArgs s, float2 *__rest
 
 // complex128 arena, one coset per thread and per 16-byte entry; FP64 arithmetic.
 // Chunk = 256 threads x U cosets = 2^(8 + log2 U) cosets; coset u of thread t is t + 256u.
-template <int NTQ, int MOUT, int U, bool WRITE>
+template <int NTQ, int MOUT, int U, bool WRITE, bool SLOTS>
 __global__ void __launch_bounds__(256) k_wide128(const StepArgs s, double2 *__restrict__ mem, const Ctx c0) {
-    const Ctx cx = slot_ctx(c0);
-    mem += (size_t)blockIdx.y * cx.arena;
+    const Ctx cx = SLOTS ? slot_ctx(c0) : c0;
+    if (SLOTS) mem += (size_t)blockIdx.y * cx.arena;
     const Prologue P = step_prologue(s, cx, WRITE);
     if (P.skip) return;
     __shared__ uint64_t tks[40];
