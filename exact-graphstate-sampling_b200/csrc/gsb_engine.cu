@@ -51,7 +51,6 @@ int fail(int code, const std::string &msg) {
 
 struct Launch {
     int grid = 1, block = 1, U = 1, tl = 0, cl = 0;
-    int cap = 1;                // blocks the device holds at once
     unsigned int nchunks = 1;
     void *fn = nullptr, *fn_slots = nullptr;   // kernels of launches that carry one item, and several
 };
@@ -181,7 +180,7 @@ struct Engine {
     std::map<std::pair<int, int>, Op> cover_ops;   // fused passes (k, d) that chain_cover tried, with the current matrices
     int hyb_K = 0;                       // gsb_set_hybrid_prefix: hybrid strings force their first hyb_K steps
     std::vector<Op> hyb_ops;             // fused 'chain' passes over those steps
-    std::vector<Op> sample_ops;          // 'prob' / 'sample' passes (build_sample_ops)
+    std::vector<Op> sample_ops;          // sampling passes (build_sample_ops)
     int withhold_loads = 0;              // test hook: fused passes issue no tile loads (their bounded waits run out)
     std::vector<OpShape> chain_shapes;   // pass lists chosen by gsb_autotune (empty: the byte-model defaults)
     std::vector<OpShape> sample_shapes;
@@ -296,8 +295,7 @@ struct Engine {
             const StepKernel kind = wide64 ? STEP_PAIR64 : STEP_WIDE128;
             L.fn = pick_step<false>(kind, a.ntq, a.m, write, arith == 32);
             L.fn_slots = pick_step<true>(kind, a.ntq, a.m, write, arith == 32);
-            L.cap = occupancy(L.fn, L.block) * sms;
-            L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)L.cap);
+            L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)(occupancy(L.fn, L.block) * sms));
             return L;
         }
         if (prec == 128 || N < 1024) return L;   // always in a run
@@ -308,8 +306,7 @@ struct Engine {
         L.nchunks = (unsigned int)(N >> L.cl);
         L.fn = pick_step<false>(STEP_ANY64, a.ntq, a.m, write, true);
         L.fn_slots = pick_step<true>(STEP_ANY64, a.ntq, a.m, write, true);
-        L.cap = occupancy(L.fn, L.block) * sms;
-        L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)L.cap);
+        L.grid = (int)std::min<uint64_t>(L.nchunks, (uint64_t)(occupancy(L.fn, L.block) * sms));
         return L;
     }
 
@@ -331,11 +328,10 @@ struct Engine {
         return c;
     }
 
-    // x extent of a launch that carries `slots` items: one item alone takes `grid` blocks, the device holds `cap`.
-    // With several items the blocks are shared out (SLOT_WAVES rounds of `cap` in all), a power of two per item so that
-    // the items' tiles, a power of two as well, split evenly.
+    // x extent of a launch that carries several items: one item alone takes `grid` blocks, the device holds `cap`.  The blocks
+    // are shared out (SLOT_WAVES rounds of `cap` in all), a power of two per item so that the items' tiles, a power of two as
+    // well, split evenly.
     unsigned slot_grid(int grid, int cap) const {
-        if (slots == 1) return (unsigned)grid;
         unsigned g = 1;
         while (2 * g * (unsigned)slots <= (unsigned)(SLOT_WAVES * cap)) g *= 2;
         return std::min((unsigned)grid, g);
@@ -353,8 +349,10 @@ struct Engine {
         Ctx c = ctx(driver, k1, L, use_forced, use_unif);
         void *memp = arena_mem();
         void *kargs[] = {&a, &memp, &c};
-        return cudaLaunchKernel(slots == 1 ? L.fn : L.fn_slots, dim3(slot_grid(L.grid, L.cap), (unsigned)slots),
-                                dim3((unsigned)L.block), kargs, 0, stream);
+        if (slots == 1) return cudaLaunchKernel(L.fn, dim3((unsigned)L.grid), dim3((unsigned)L.block), kargs, 0, stream);
+        const int cap = occupancy(L.fn_slots, L.block) * sms;
+        return cudaLaunchKernel(L.fn_slots, dim3(slot_grid(L.grid, cap), (unsigned)slots), dim3((unsigned)L.block), kargs, 0,
+                                stream);
     }
 
     // Steps k0 .. k1 - 1, all of one run part, as one k_run launch; norm: the branch norms of steps whose bit is drawn.
@@ -697,7 +695,6 @@ static bool conserves(const HPlan &p) {
 // general shape) and, per bit, the factored step's pivot (the larger of the row's two entries), its ratio
 // beta = M[b][1-piv] / M[b][piv] and cp = |M[b][piv]|^2 (exact), all rounded by round_diffused in step order.
 // Other engines use the plan's M as it is (FP64 arithmetic, or complex128).
-static bool conserves(const HPlan &p);
 static void apply_coeffs(Engine &E) {
     const HPlan &p = E.plan;
     E.prob_by_chain = conserves(p);
@@ -1088,7 +1085,8 @@ static bool ops_from_shapes(Engine &E, const std::vector<OpShape> &shapes, std::
     return true;
 }
 
-// Sampling pass list ('prob' / 'sample'): the cheapest cover of the steps, by table entries moved, with
+// Sampling pass list ('sample', and 'prob' where the plan does not conserve probability): the cheapest cover of the steps, by
+// table entries moved, with
 //   * single steps: norm pass + write pass (read, read, write);
 //   * fused passes of steps k .. k+d-1 (k+1 .. k+d-1 analytic, so their bits need no data), optionally with the
 //     branch norms of step k+d (trailing, tr = 1; at most 3 steps evaluated in one pass).  Step k's bit comes from
@@ -1409,8 +1407,9 @@ static int forced_batch(Engine *E, int kind, const int8_t *bits, int64_t nstr, d
 }
 
 // 'prob' strings (log2 Pr), by the 'chain' passes where the plan conserves probability.  The two-pass chain ends a string
-// as impossible where 1 - p rounds to 0; the one-pass chain leaves rounding noise there, so strings with a conditional
-// below PROB_FLOOR (no possible branch of a circuit comes near it) run the two passes as well.
+// as impossible where 1 - p rounds to 0; the one-pass chain leaves rounding noise there (1e-15 to 1e-13 of complex64
+// tables), so strings with a conditional below PROB_FLOOR run the two passes as well and take their result.  A branch may
+// well be possible and below it, after a small rotation: such a string costs both routes.
 constexpr double PROB_FLOOR = 1.0 / ((uint64_t)1 << 40);
 static int prob_batch(Engine *E, const int8_t *bits, int64_t nstr, double *log2p) {
     if (!E->prob_by_chain) return forced_batch(E, 1, bits, nstr, log2p, nullptr);
