@@ -81,8 +81,8 @@ constexpr int BATCH_MAX_BLOCK = 512;
 // Instances up to this width take one step per pass, and a warp keeps both tables of their items in its lanes' slots (2^8
 // entries of complex128 twice: 8 KB).  A warp's item is a chain of dependent passes with a table read in each, so what bounds
 // it is the latency of those reads and of the code between them: through L2, and through the code of the wide passes, 320
-// items of widths 1-3 took 67 us in complex64 and 75 us in complex128 (single steps with generic code 43 and 41 us, now 22 and
-// 22), 4,000 items of widths 5-9 321 and 376 us (225 and 227; now 170 and 193).
+// items of widths 1-3 took 67 us in complex64 and 75 us in complex128 (single steps with generic code 43 and 41 us, now 23 and
+// 23), 4,000 items of widths 5-9 321 and 376 us (226 and 227; now 162 and 205).
 constexpr int BATCH_NEAR_R = 8;
 
 struct BInst {
@@ -491,6 +491,8 @@ __device__ __noinline__ double near_pass(const BPass &p, const E *in, E *out, in
     }
 }
 
+// Norms: a class's squared outputs are summed in the arena's precision (at most 32 of them), classes and threads in FP64.  A
+// pass's norm only picks the power of two that scales the next one; the result is the norm of the last step's single entry.
 struct ChainState {
     double prev, lsc, scale;
     int ek, dead;
@@ -908,7 +910,7 @@ static int passes_of(const HPlan &p, int k0, int k1, F pass_at, std::vector<int>
 
 // The pass lists for prefix lengths K.  A pass is derived once, when a list first needs it (10 us; the host's cores side by
 // side), and stays in the device's table: other prefix lengths need few new ones or none.  Two set_strings with other prefix
-// lengths: 300 instances of widths 4-5 5.4 ms with a table made for each call, 100 of width 11 3.8 ms; now 0.6 and 0.3.
+// lengths: 300 instances of widths 4-5 5.4 ms with a table made for each call, 100 of width 11 3.8 ms; now 0.5 and 0.23.
 static int batch_passes(BatchEngine &E, const int *K) {
     const size_t n = E.plans.size();
     if (E.K.size() == n && std::equal(E.K.begin(), E.K.end(), K)) return 0;

@@ -4,8 +4,9 @@
 // their own, or as steps over the arena in global memory, they are bound by latency alone: the arena version of this
 // kernel took 2.5 us per step (two block barriers around scalar work in one thread, and dependent loads of the
 // descriptor, the state and the table), 54 us for each end of a 'chain' string at width 19 (now 40 for 64 strings side by
-// side), 115 us for a 20-step 'prob' (now 65; both cold), and a call of 1024 strings at n = 20 0.53 ms (now 0.11).  What
-// is left is the latency of FP64 sums, shuffles and instruction fetches, step after step.  Here
+// side; both cold).  Calls on 20 steps: one 'prob' 142 us (now 55, with one pass per step), 1024 strings by 'chain' 0.53 ms
+// (now 0.114), 100 samples 0.25 ms (now 0.146).  What is left is the latency of FP64 sums, shuffles and instruction fetches,
+// step after step.  Here
 //   * the live table sits in shared memory in compact coordinates: the addresses that the run's steps touch span a
 //     subspace of dimension D <= RUN_DIM, the host picks a basis of it (the widest step's columns first, so that its
 //     neighbouring cosets are neighbouring entries) and rewrites every step's columns in that basis;
@@ -155,8 +156,8 @@ __device__ __forceinline__ void run_pass(const RunStep &s, E *tab, int bv, doubl
 }
 
 // A step whose bit is drawn from its branch norms, with at most two cosets per thread: the cosets' sums stay in registers
-// between the norms and the write, which then reads nothing and forms no sums again (one prob at n = 20: 74 -> 67 us a
-// call, 100 samples 155 -> 148).
+// between the norms and the write, which then reads nothing and forms no sums again (100 samples of 20 steps: 155 -> 148 us a
+// call; a 'prob' of two passes per step 74 -> 67).
 struct CosetSums {
     double x[2][2], z[2][2];   // [tau][re, im]: x = 0 and signed x = 1 sums
     uint32_t base;

@@ -342,7 +342,7 @@ class Engine:
 
     def autotune(self, mode=2, reps=3):
         """Time every candidate pass on this device and keep the fastest covers of the steps (mode 0: 'chain',
-        1: 'prob' / 'sample', 2: both); returns (ms of one item before, after)."""
+        1: the sampling passes, 2: both); returns (ms of one item before, after)."""
         a, b = ctypes.c_float(), ctypes.c_float()
         _check(_lib.gsb_autotune(self.handle, int(mode), int(reps), ctypes.byref(a), ctypes.byref(b)))
         return a.value, b.value
@@ -369,7 +369,7 @@ class Engine:
         return [int(x) for x in g[:self.ns]], e[:self.ns]
 
     def passes(self, mode=0):
-        """The passes of 'chain' (mode 0) or 'prob' / 'sample' (mode 1) in launch order: a list of
+        """The passes of 'chain' (mode 0) or the sampling passes (mode 1) in launch order: a list of
         (first step, steps written, trailing branch-norm step 0/1, fused 0/1)."""
         n = ctypes.c_int()
         _check(_lib.gsb_pass_list(self.handle, int(mode), 0, None, None, None, None, ctypes.byref(n)))
@@ -402,7 +402,7 @@ class Engine:
         _check(_lib.gsb_synchronize(self.handle))
 
     def profile_steps(self, string, mode=0):
-        """Per-step kernel times (ms) of one forced string: (write [ns], norm [ns]); mode 0 chain, 1 prob."""
+        """Per-step kernel times (ms) of one forced string: (write [ns], norm [ns]); mode 0 chain, 1 sampling passes."""
         f = as_bits([string], self.ns)[0].copy()
         w = np.zeros(max(self.ns, 1), np.float32)
         nrm = np.zeros(max(self.ns, 1), np.float32)
@@ -411,6 +411,7 @@ class Engine:
         return w[:self.ns], nrm[:self.ns]
 
     def launches_per_item(self, mode):
+        """Kernel launches of one item: 0 the 'chain' passes, 1 the sampling passes, 2 'hybrid'."""
         n = ctypes.c_int64()
         _check(_lib.gsb_launches_per_item(self.handle, int(mode), ctypes.byref(n)))
         return n.value

@@ -16,6 +16,9 @@
  *     0, 1, or -1 for '?' where a mode allows it.  Multi-string arguments are row-major [nstr][nsteps].
  *   - An engine owns one arena (2^R entries of complex64 or complex128) and one CUDA stream on one device.  Calls on
  *     one engine must not overlap (one engine per host thread); different engines are independent.
+ *   - A call of several strings or samples on a plan that is neither narrow nor wide takes further arenas, 1 GB in all at most,
+ *     as many as the device has room for; the engine keeps them until it is closed, or until one of its own calls finds no
+ *     memory for dump tables (a guard engine keeps its own).
  *   - Host-buffer entry points are synchronous: they copy inputs in, run, and copy results out before returning.
  */
 #ifndef GSB_H
@@ -94,7 +97,8 @@ int gsb_dump_shape(const gsb_engine *e, int K, int *nk, int *ntq);
 
 /* 'prefix': run the forced steps 0..K-1 of one string and copy out the live table in logical (c, tq) order, entries
  * of the arena type (complex64 = 2 floats, complex128 = 2 doubles); *logscale and log2 Pr(prefix) as the reference
- * prints them (gsamp2.cpp:162-175).  dump may be NULL when only log2 Pr(prefix) (a marginal) is wanted. */
+ * prints them (gsamp2.cpp:162-175).  A prefix of probability 0 dumps zeros (log2 Pr(prefix) = -inf).  dump may be NULL when
+ * only log2 Pr(prefix) (a marginal) is wanted. */
 int gsb_prefix(gsb_engine *e, const int8_t *forced, int K, void *dump, double *logscale, double *log2p_prefix);
 
 /* 'resume': sum nslices dump tables (scaled by 2^(logscale_s - max)), read through the optional twist translation
@@ -121,7 +125,8 @@ int gsb_set_fusion(gsb_engine *e, int depth);
 /* Autotune the pass lists on this device: every candidate pass (one step; 2 or 3 fused steps; for sampling with or
  * without the next step's branch norms; tiles of up to 2^8, 2^9 or 2^10 classes) is timed alone with CUDA events,
  * and the covers of the steps with the least measured time replace the byte-model choice (mode 0: 'chain' passes,
- * 1: 'prob' / 'sample' passes, 2: both) -- if a whole item, replayed, gets faster; otherwise the previous list
+ * which 'prob' runs as well where every step conserves probability; 1: the sampling passes, 'sample' and 'prob' on
+ * other plans; 2: both) -- if a whole item, replayed, gets faster; otherwise the previous list
  * stays.  The choice survives gsb_set_matrices; gsb_set_fusion discards it.  ms_before / ms_after (may be NULL):
  * device time of one item of each tuned list before and after (summed for mode 2).  No counterpart in the
  * reference. */
@@ -129,10 +134,10 @@ int gsb_autotune(gsb_engine *e, int mode, int reps, float *ms_before, float *ms_
 /* Pass structure of 'chain' mode: group_len[k] = number of steps of the pass starting at step k (0 inside a pass);
  * entries[k] (may be NULL) = table entries the pass reads plus writes. */
 int gsb_fusion_groups(const gsb_engine *e, int *group_len, double *entries);
-/* The same for the sampling passes ('prob' / 'sample'): group_len[k] = steps written by the pass starting at step k;
+/* The same for the sampling passes ('sample', and 'prob' on plans that do not conserve probability): group_len[k] = steps written by the pass starting at step k;
  * entries[k] = table entries it reads plus writes, including the norm pass launched before it where it has one. */
 int gsb_sample_groups(const gsb_engine *e, int *group_len, double *entries);
-/* The passes of one mode (0 'chain', 1 'prob' / 'sample') in launch order: pass i starts at step k0[i], writes d[i]
+/* The passes of one list (0 'chain', 1 sampling, as for gsb_autotune) in launch order: pass i starts at step k0[i], writes d[i]
  * steps, also evaluates the branch norms of step k0[i] + d[i] when tr[i] = 1, and is a fused k_group pass when
  * fused[i] = 1 (otherwise a single-step pass, after its own norm pass in sampling mode).  *count receives the number
  * of passes; at most cap entries are written (the arrays may be NULL when cap = 0).  No counterpart in the reference:
@@ -174,10 +179,11 @@ int gsb_set_guard(gsb_engine *e, gsb_engine *g, double log2_xmin);
 int gsb_guard_evaluations(const gsb_engine *e, int64_t *count);
 
 /* Per-step kernel timing for one forced string: ms_write[k] and ms_norm[k] (0 when a pass does not run) from CUDA
- * events on the engine's stream, mode 0 = 'chain' (one pass per step), 1 = 'prob' (norm + write per step). */
+ * events on the engine's stream, mode 0 = the 'chain' passes, 1 = the sampling passes with their norm passes. */
 int gsb_profile_steps(gsb_engine *e, const int8_t *bits, int mode, float *ms_write, float *ms_norm);
 
-/* Number of kernel launches one string / sample makes in the given mode (0 chain, 1 prob/sample, 2 hybrid). */
+/* Number of kernel launches one string / sample makes: 0 the 'chain' passes ('chain', and 'prob' where every step conserves
+ * probability), 1 the sampling passes ('sample', and 'prob' on other plans), 2 'hybrid'. */
 int gsb_launches_per_item(const gsb_engine *e, int mode, int64_t *launches);
 
 /* ---- out-of-place amplitude engine (the reference's dp.cpp, dp.cpp:14-63) ----
@@ -238,7 +244,8 @@ int gsb_batch_run(gsb_batch *b, double *log2p, float *ms);
 int gsb_batch_set_shape(gsb_batch *b, int block, int small_R, int per_sm);
 int gsb_batch_get_shape(const gsb_batch *b, int *block, int *small_R, int *per_sm);
 /* Autotuner: times the candidate shapes on the current strings (reps timed runs each, arenas <= max_bytes) and
- * keeps the fastest; returns it and its mean time. */
+ * keeps the fastest; returns it and its mean time.  The bound also holds for the arenas of later runs where it decides
+ * whether the widest instances get cluster teams, which have arenas of their own. */
 int gsb_batch_tune(gsb_batch *b, int reps, size_t max_bytes, int *block, int *small_R, int *per_sm, float *best_ms);
 
 /* Test hook for the fused passes' failure path (no counterpart in the reference): with on = 1 the passes issue no
