@@ -9,7 +9,8 @@
 // run by a cluster of CTAs ("cluster team"), wide ones by a CTA ("block team"), narrow ones (R <= small_R) by one warp
 // ("warp team").  The kernel is persistent: every cluster first takes cluster items, then each of its CTAs block items,
 // then each warp warp items, with one atomic per item.  A team owns an arena of 2^R entries and a second table of the
-// same size in its slot, so a whole item runs without any grid-wide synchronisation.
+// same size in its slot, so a whole item runs without any grid-wide synchronisation.  Warp items of up to width BATCH_NEAR_R
+// have both in shared memory and a function of their own (near_item), one step per pass.
 //
 // An item's steps run in passes of up to three (gsb_fuse.h), which read and write the table once: a thread takes a few
 // classes at a time through the pass's steps, and their values between two steps sit in shared-memory slots of its own.
